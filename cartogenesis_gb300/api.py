@@ -300,7 +300,8 @@ class SeaLevelStage:
 def sequential_sum(values, mask=None, mode=0, ctx=None):
     """The reference's `var s = 0.0; for (c in cells) s += v[c]` over the cells where mask is set (all when
     mask is None), v = values (mode 0) or 1 - 0.5 values (mode 1), bit for bit, on the device. Returns
-    (sum, counts): blocks of 8192 values taken whole, pieces of 1024 reduced, pieces added one by one."""
+    (sum, counts): blocks of 8192 values taken whole, and of the other blocks the pieces of 1024 without
+    and with an addition taken alone."""
     ctx = ctx or default_context()
     x = np.ascontiguousarray(values, dtype=np.float32).ravel()
     m = None if mask is None else np.ascontiguousarray(mask, dtype=np.uint8).ravel()

@@ -15,9 +15,9 @@
 //    in key order, and one cooperative kernel runs the Kahn levels with a grid barrier between them,
 //    upward for the sums and downward for the cut, which reads each receiver's final height;
 //  - the books (uplift, cut, export to the sea and to the land, the slopes' shed) are the reference's
-//    running double sums: each round lays its terms out in the reference's order, the running total
-//    first, and sums them exactly in parallel (seq_sum_f64_dev); a term the reference skips is +0,
-//    which leaves a sum that started at +0 unchanged;
+//    running double sums: each round lays its terms out in the reference's order and adds them to the
+//    five totals exactly, side by side in one set of launches (seq_totals_f64_dev); a term the
+//    reference skips is +0, which leaves a sum that started at +0 unchanged;
 //  - the sweeps give from belt cells only and visit neighbours rows first, then columns
 //    (forEachNeighborWithLimit); every cell of a sweep reads the heights before it;
 //  - the rebound's blur sums its taps in order in double; the taps are computed on the host with
@@ -205,7 +205,7 @@ __global__ void k_frontier_list(const int* __restrict__ flag, const int* __restr
         if (flag[i]) out[pos[i]] = (int)i;
 }
 
-// The rise where the belt has begun to (BeltErosion.kt:240-248); xs[1 + l] the uplift book's term.
+// The rise where the belt has begun to (BeltErosion.kt:240-248); xs[l] the uplift book's term.
 __global__ void k_belt_rise(const int* __restrict__ list, int B, const int* __restrict__ first,
                             const float* __restrict__ rise, int round, BeltConsts k, float* __restrict__ h,
                             float* __restrict__ uplifted_m, double* __restrict__ xs) {
@@ -218,7 +218,7 @@ __global__ void k_belt_rise(const int* __restrict__ list, int B, const int* __re
             if (uplifted_m) uplifted_m[c] = __fadd_rn(uplifted_m[c], __fmul_rn(r, k.mpfu));
             term = __dmul_rn(__dmul_rn((double)r, (double)k.mpfu), k.area);
         }
-        xs[1 + l] = term;
+        xs[l] = term;
     }
 }
 
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(256) k_belt_levels(LevelArgs a) {
     }
 }
 
-// The books' terms in the reference's order after their running totals: the cut in reverse run order,
+// The books' terms in the reference's order: the cut in reverse run order,
 // the exports to the sea and to the land in run order (BeltErosion.kt:346-370).
 __global__ void k_order_terms(const int* __restrict__ order, int B, const int32_t* __restrict__ recv,
                               const uint8_t* __restrict__ belt, const uint8_t* __restrict__ land,
@@ -375,7 +375,7 @@ __global__ void k_order_terms(const int* __restrict__ order, int B, const int32_
                               const double* __restrict__ cutv, double* __restrict__ xcut,
                               double* __restrict__ xsea, double* __restrict__ xland) {
     for (size_t i = tid(); i < (size_t)B; i += nthreads()) {
-        xcut[1 + i] = cutv[order[B - 1 - i]];
+        xcut[i] = cutv[order[B - 1 - i]];
         const int c = order[i];
         const int d = recv[c];
         const double f = flux[c];
@@ -387,8 +387,8 @@ __global__ void k_order_terms(const int* __restrict__ order, int B, const int32_
             if (!land[d] || h[d] <= shoreline) sea = f;
             else lnd = f;
         }
-        xsea[1 + i] = sea;
-        xland[1 + i] = lnd;
+        xsea[i] = sea;
+        xland[i] = lnd;
     }
 }
 
@@ -674,13 +674,15 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
     CG_BUF(float, d_give, ctx, S_BT_GIVE, N);
     CG_BUF(float, d_next, ctx, S_BT_NEXT, N);
     CG_BUF(int32_t, d_order, ctx, S_BT_ORDER, (size_t)B);
-    const size_t xs_len = std::max(4 * ((size_t)B + 1), 1 + (size_t)sweeps * F);
-    CG_BUF(double, d_xs, ctx, S_BT_XS, xs_len);
+    CG_BUF(double, d_xs, ctx, S_BT_XS, 4 * (size_t)B + (size_t)sweeps * F + 1);   // the books' terms of a round
     double* xs_rise = d_xs;
-    double* xs_cut = d_xs + (B + 1);
-    double* xs_sea = d_xs + 2 * ((size_t)B + 1);
-    double* xs_land = d_xs + 3 * ((size_t)B + 1);
-    double* xs_shed = d_xs;   // after the others are summed
+    double* xs_cut = d_xs + B;
+    double* xs_sea = d_xs + 2 * (size_t)B;
+    double* xs_land = d_xs + 3 * (size_t)B;
+    double* xs_shed = d_xs + 4 * (size_t)B;
+    const SeqTotal totals[kSeqTotals] = {{xs_rise, (size_t)B, d_books}, {xs_cut, (size_t)B, d_books + 1},
+                                         {xs_sea, (size_t)B, d_books + 2}, {xs_land, (size_t)B, d_books + 3},
+                                         {xs_shed, (size_t)sweeps * F, d_books + 4}};
     CG_LAUNCH(ctx) k_widen<<<grid, 256, 0, sm>>>(d_h, N, d_routing);
     CG_CUDA(ctx, cudaMemsetAsync(d_inner, 0, N, sm));
     CG_CUDA(ctx, cudaMemsetAsync(d_routed, 0, N, sm));
@@ -729,10 +731,8 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
 
     for (int round = 0; round < k.rounds; ++round) {
         if (ctx->cancel.exchange(0)) return fail(ctx, CG_CANCELLED, "cancelled");
-        // The rise and its book (BeltErosion.kt:240-249).
+        // The rise and its book's terms (BeltErosion.kt:240-249).
         CG_LAUNCH(ctx) k_belt_rise<<<bgrid, 256, 0, sm>>>(d_swept, B, d_first, d_rise, round, k, d_h, d_uplm, xs_rise);
-        CG_CUDA(ctx, cudaMemcpyAsync(xs_rise, d_books + 0, 8, cudaMemcpyDeviceToDevice, sm));
-        CG_TRY_ST(seq_sum_f64_dev(ctx, xs_rise, (size_t)B + 1, d_books + 0));
         CG_LAUNCH(ctx) k_route_cells<<<grid, 256, 0, sm>>>(d_swept, B + F, d_h, d_routing);
         // The spill levels, the routing surface and the facet receivers (BeltErosion.kt:253-292).
         CG_LAUNCH(ctx) k_belt_masks<<<bgrid, 256, 0, sm>>>(d_swept, B, d_local, d_land, d_h, k, W, H, d_inner, d_routed);
@@ -760,21 +760,14 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
         CG_LAUNCH(ctx) k_order_terms<<<bgrid, 256, 0, sm>>>(d_order, B, d_recv, d_belt, d_land, d_h, k.shoreline,
                                                             d_flux, d_cutv, xs_cut, xs_sea, xs_land);
         CG_CHECK_LAUNCH(ctx);
-        CG_CUDA(ctx, cudaMemcpyAsync(xs_cut, d_books + 1, 8, cudaMemcpyDeviceToDevice, sm));
-        CG_CUDA(ctx, cudaMemcpyAsync(xs_sea, d_books + 2, 8, cudaMemcpyDeviceToDevice, sm));
-        CG_CUDA(ctx, cudaMemcpyAsync(xs_land, d_books + 3, 8, cudaMemcpyDeviceToDevice, sm));
-        CG_TRY_ST(seq_sum_f64_dev(ctx, xs_cut, (size_t)B + 1, d_books + 1));
-        CG_TRY_ST(seq_sum_f64_dev(ctx, xs_sea, (size_t)B + 1, d_books + 2));
-        CG_TRY_ST(seq_sum_f64_dev(ctx, xs_land, (size_t)B + 1, d_books + 3));
         // The slopes (BeltErosion.kt:373-408), the frontier's changes the shed book's terms.
         for (int s = 0; s < sweeps; ++s) {
             CG_LAUNCH(ctx) k_belt_give<<<bgrid, 256, 0, sm>>>(d_swept, B, d_h, W, H, k, d_give);
             CG_LAUNCH(ctx) k_belt_next<<<grid, 256, 0, sm>>>(d_swept, B + F, d_local, d_h, d_give, W, H, k, d_next);
-            CG_LAUNCH(ctx) k_belt_commit<<<grid, 256, 0, sm>>>(d_swept, B, F, d_next, k, d_h, xs_shed + 1 + (size_t)s * F);
+            CG_LAUNCH(ctx) k_belt_commit<<<grid, 256, 0, sm>>>(d_swept, B, F, d_next, k, d_h, xs_shed + (size_t)s * F);
         }
         CG_CHECK_LAUNCH(ctx);
-        CG_CUDA(ctx, cudaMemcpyAsync(xs_shed, d_books + 4, 8, cudaMemcpyDeviceToDevice, sm));
-        CG_TRY_ST(seq_sum_f64_dev(ctx, xs_shed, 1 + (size_t)sweeps * F, d_books + 4));
+        CG_TRY_ST(seq_totals_f64_dev(ctx, totals, kSeqTotals));
         // The crust's answer to the rock taken so far (BeltErosion.kt:413-423).
         if (rebound && ((round + 1) % kReboundRounds == 0 || round == k.rounds - 1)) {
             CG_LAUNCH(ctx) k_belt_loss<<<grid, 256, 0, sm>>>(N, d_uplm, d_rbm, d_h, d_ref, k.mpfu, d_loss);

@@ -153,13 +153,22 @@ struct DepositCounts {
 // The reference's sequential double sum (`s += v` in cell order, s from 0.0) of v = x (mode 0) or
 // v = 1 - 0.5 x (mode 1) over the cells of d_mask (all cells when null), into *d_out on the device,
 // divided by `divisor` unless it is 0; bit for bit, in parallel (cg_seqsum.cu). d_counts (3, may be
-// null) receives how the sum went: blocks of 8192 values taken whole, pieces of 1024 reduced on the
-// spot, pieces added one value at a time.
+// null) receives how the sum went: blocks of 8192 values taken whole, and of the other blocks the pieces of 1024
+// without and with an addition taken alone.
 cg_status seq_sum_dev(cg_ctx* ctx, const float* d_x, const uint8_t* d_mask, int mode, size_t n, double divisor,
                       double* d_out, long long* d_counts);
 // The same sequential sum (`s += v`, s from 0.0) over n double terms already laid out in the order the
 // reference adds them, bit for bit; a running total is carried by laying it first.
 cg_status seq_sum_f64_dev(cg_ctx* ctx, const double* d_x, size_t n, double* d_out);
+// Running totals on the device, each with the n double terms it gains in order (`*total += x[i]`), bit
+// for bit, in one set of launches.
+constexpr int kSeqTotals = 5;
+struct SeqTotal {
+    const double* x;
+    size_t n;
+    double* total;
+};
+cg_status seq_totals_f64_dev(cg_ctx* ctx, const SeqTotal* totals, int count);
 // The plate flexure of profile P3 (cg_flexure.cu). flexure_check refuses grids whose transform lines
 // do not fit a CTA's shared memory; flexure_stage_begin_dev records the field before the rounds and
 // clears the bend (and the uplift record when the world has uplift); flexure_uplifted_dev is that

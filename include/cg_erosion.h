@@ -439,9 +439,9 @@ cg_status cg_flexure_deflection(cg_ctx* ctx, const cg_erosion_params* params, co
  * (mask may be NULL). Host buffers. The stage computes these sums on the device the same way; this entry
  * point exposes the primitive on its own. The sum is not a chain of n double additions: blocks of values
  * are reduced in parallel to integer walks inside the running sum's binade (the one state a walk carries
- * is the parity of the sum's mantissa, which decides ties), and only where the sum crosses a binade are
- * values added one at a time. `counts` (3 entries, may be NULL) receives blocks of 8192 values taken
- * whole, pieces of 1024 reduced on the spot, and pieces added one value at a time.
+ * is the parity of the sum's mantissa, which decides ties), and only the value that crosses a binade is
+ * added alone. `counts` (3 entries, may be NULL) receives blocks of 8192 values taken whole, and of the
+ * other blocks the pieces of 1024 without and with an addition taken alone.
  */
 cg_status cg_sequential_sum(cg_ctx* ctx, const float* x, const uint8_t* mask, int32_t mode, int64_t n,
                             double* sum, int64_t* counts);
