@@ -7,10 +7,15 @@
 //
 // The enclosure rule labels the water's 8-connected bodies (the same union-find labels as the
 // basins, numbered by their lowest cell, which is the order the reference's scan finds them in);
-// the ocean is the largest body, the first found of that size. The belowSea notch runs on one thread
-// over the basins in the order spillways found them: only the drowned basins cut (a handful a pass),
-// and the lake-bed walk that belowSea adds follows the ponded cells as the cutting leaves them, so
-// its footprint is not known before the cut.
+// the ocean is the largest body, the first found of that size. The belowSea notch takes the drowned
+// basins in the order spillways found them, and the lake-bed walk that belowSea adds follows the ponded
+// cells as the cutting leaves them, so its footprint is not known before the cut. What bounds it is the
+// chain of dependent loads a walk is, so one CTA walks 32 basins at a time, a warp each, without
+// cutting: each lists the cells it reads and its cuts and stamps the cells it would cut, then looks
+// whether a basin before it stamped a cell it read. The basins before the first that finds one cut as
+// they would have one after another, and the next 32 start there: 11 to 17 basins a wave at 1024 x 512.
+// (One thread taking the basins in turn: 3.8 ms a pass there; one warp with the others loading ahead of
+// it 1.9; each walking twice instead of listing what it reads 0.85.)
 #include <cmath>
 
 #include "cg_common.cuh"
@@ -26,9 +31,35 @@ __global__ void k_water_mask(const uint8_t* __restrict__ land, size_t N, uint8_t
         mask[i] = land[i] ? 0 : 1;
 }
 
+// Cells per water body. Nearly every cell is the ocean's, one counter, so a warp takes a stretch of
+// kBodyRun x 32 cells and keeps the count of the body it is in, adding it once when the body changes
+// (an atomic a cell cost 230 us at 1024 x 512); cells of a mixed row of 32 go by groups of one body.
+constexpr int kBodyRun = 16;
+
 __global__ void k_body_sizes(const int* __restrict__ label, size_t N, int* __restrict__ size) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x)
-        if (label[i] >= 0) atomicAdd(&size[label[i]], 1);
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const size_t warps = (size_t)gridDim.x * blockDim.x / 32;
+    for (size_t run = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) / 32; run * (kBodyRun * 32) < N; run += warps) {
+        int body = -1, cells = 0;   // the same in every lane
+        for (int k = 0; k < kBodyRun; ++k) {
+            const size_t i = (run * kBodyRun + k) * 32 + lane;
+            const int l = i < N ? label[i] : -1;
+            const int l0 = __shfl_sync(FULL, l, 0);
+            if (__all_sync(FULL, l == l0)) {
+                if (l0 != body) {
+                    if (lane == 0 && body >= 0) atomicAdd(&size[body], cells);
+                    body = l0;
+                    cells = 0;
+                }
+                cells += 32;
+            } else {
+                const unsigned peers = __match_any_sync(FULL, l);
+                if (l >= 0 && lane == __ffs(peers) - 1) atomicAdd(&size[l], __popc(peers));
+            }
+        }
+        if (lane == 0 && body >= 0) atomicAdd(&size[body], cells);
+    }
 }
 
 // The ocean: the largest body, the lowest label (the first found) among equals.
@@ -64,27 +95,54 @@ __global__ void k_land_water_at(const float* __restrict__ h, size_t N, float sho
         rel[i] = __fdiv_rn(__fsub_rn(g, shoreline), on ? land_half : sea_half);
         mine += on ? 1 : 0;
     }
-    if (mine) atomicAdd(count, mine);
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xFFFFFFFFu, mine, o);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(count, mine);
 }
 
-// Basins whose floor stands at or above the shoreline are the rounds' notch's: their spill is
-// cleared. Counts the drowned basins that keep a spill.
-__global__ void k_mark_drowned(int* __restrict__ spill, const float* __restrict__ floor_, int count,
-                               int* __restrict__ drowned) {
-    int mine = 0;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < count; b += gridDim.x * blockDim.x) {
-        if (floor_[b] >= 0.0f) spill[b] = -1;
-        else if (spill[b] >= 0) ++mine;
+// The drowned basins, those whose floor stands below the shoreline and that have a spill, listed in
+// basin order by one CTA (the others are the rounds' notch's). The notch's one thread stepping over
+// every basin took 4.4 ms a pass at 1024 x 512.
+struct Drowned {
+    int spill, entry;
+    float level, floor_;
+};
+
+__global__ void __launch_bounds__(1024) k_list_drowned(const int* __restrict__ spill, const int* __restrict__ entry,
+                                                       const float* __restrict__ level, const float* __restrict__ floor_,
+                                                       int count, Drowned* __restrict__ list, int* __restrict__ drowned) {
+    __shared__ int warps[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int listed = 0;
+    for (int base = 0; base < count; base += 1024) {
+        const int b = base + (int)threadIdx.x;
+        const int sp = b < count ? spill[b] : -1;
+        const float fl = b < count ? floor_[b] : 0.0f;
+        const bool in = sp >= 0 && !(fl >= 0.0f);
+        const unsigned ballot = __ballot_sync(0xFFFFFFFFu, in);
+        if (lane == 0) warps[warp] = __popc(ballot);
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            before += w < warp ? warps[w] : 0;
+            all += warps[w];
+        }
+        if (in) list[listed + before + __popc(ballot & ((1u << lane) - 1u))] = Drowned{sp, entry[b], level[b], fl};
+        listed += all;
+        __syncthreads();
     }
-    if (mine) atomicAdd(drowned, mine);
+    if (threadIdx.x == 0) *drowned = listed;
 }
 
 struct NotchArgs {
     int W, H, count;
-    const int* spill;
-    const int* entry;
-    const float* level;
-    const float* floor_;
+    const Drowned* list;
+    int cap;             // cells a walk can hold
+    int* cut_cell;       // scratch, 3 cap a warp: the cells its basin cuts and the levels it cuts them to
+    float* cut_level;
+    int* chain;          // scratch, cap a warp: a margin's cells
+    int* read_cell;      // scratch, 11 cap a warp: the cells whose heights a basin's walks read
+    int* stamp;          // per cell: the wave and the first basin of it that cuts the cell
+    int wave0;           // waves stamped so far
     const uint8_t* land;
     const int32_t* dirs;
     const float* area;
@@ -103,7 +161,7 @@ __device__ __forceinline__ float jvm_minf(float a, float b) {
 }
 
 __device__ __forceinline__ float step_between(const NotchArgs& a, int from, int to) {
-    const bool same_row = from / a.W == to / a.W, same_col = from % a.W == to % a.W;
+    const bool same_row = pdiv(from, a.W) == pdiv(to, a.W), same_col = pmod(from, a.W) == pmod(to, a.W);
     return (!same_row && !same_col) ? a.step_diag : (!same_row ? a.step_ns : 1.0f);
 }
 
@@ -123,105 +181,199 @@ __device__ bool take_down(const NotchArgs& a, int cell, float cut_level, bool lo
     return false;
 }
 
-// HydraulicErosion.breach with belowSea on (HydraulicErosion.kt:1931-2171), the basins in order.
-__global__ void k_notch_below_sea(NotchArgs a) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    int cells = 0;
-    for (int b = 0; b < a.count; ++b) {
-        const int spill = a.spill[b];
-        if (spill < 0) continue;
-        const float level = a.level[b], floor_ = a.floor_[b];
-        if (level - floor_ <= 0.0f) continue;
-        float fall = 0.0f, length = 0.0f, last_step = 1.0f;
-        int walked = 0, cell = spill;
-        while (cell >= 0 && a.land[cell] && length < a.reach) {
-            fall = level - a.rel[cell];
-            if (fall > level - floor_) break;
-            const int next = a.dirs[cell];
-            last_step = next >= 0 ? step_between(a, cell, next) : 1.0f;
-            length += last_step;
-            walked++;
-            cell = next;
-        }
-        if (fall <= 1e-6f * (float)walked && cell >= 0 && !a.land[cell]) {   // outletFallToTheWater
-            fall = level - a.rel[cell];
-            length += last_step;
-        }
-        if (walked == 0) continue;
-        float slope = fall / length * (float)a.W;
-        if (slope < 0.0f) slope = 0.0f;
-        const float power = a.coefficient * sqrtf(a.area[spill] / a.land_cells) * slope;
-        const float drop = jvm_minf(power, level - floor_);
-        if (drop <= 0.0f) continue;
-        const float new_level = level - drop;
-        float from_lip = 0.0f;
-        cell = spill;
-        while (cell >= 0 && a.land[cell] && from_lip < a.reach) {
-            const float cut_level = new_level - from_lip * a.gradient;
-            if (a.rel[cell] <= cut_level) break;
-            if (take_down(a, cell, cut_level, true)) cells++;
-            const int next = a.dirs[cell];
-            from_lip += next >= 0 ? step_between(a, cell, next) : 1.0f;
-            cell = next;
-        }
-        const int entry = a.entry[b];
-        float back = 0.0f;
-        if (entry >= 0 && entry != spill) {
-            int margin_cells = 0, walker = entry;
-            float widths = 0.0f;
-            while (walker >= 0 && walker != spill && a.land[walker] && widths <= a.reach) {
-                const int next = a.dirs[walker];
-                widths += next >= 0 ? step_between(a, walker, next) : 1.0f;
-                margin_cells++;
-                walker = next;
-            }
-            if (walker == spill) {
-                // The margin from the lip back towards the entry: the chain entry -> ... -> spill,
-                // walked backwards by recounting from the entry (margin_cells stays within the reach).
-                int downstream = spill;
-                for (int i = margin_cells - 1; i >= 0; --i) {
-                    int m = entry;
-                    for (int j = 0; j < i; ++j) m = a.dirs[m];
-                    back += step_between(a, m, downstream);
-                    const float cut_level = new_level + back * a.gradient;
-                    if (a.rel[m] <= cut_level) break;
-                    if (take_down(a, m, cut_level, true)) cells++;
-                    downstream = m;
-                }
-            }
-        }
-        // The sill on the basin's own side: up the inflow of the largest catchment across the bed.
-        int from = entry >= 0 ? entry : spill;
-        while (back <= a.reach) {
-            int best = -1;
-            float best_area = -1.0f;
-            const int col = from % a.W, row = from / a.W;
-            for (int rs = -1; rs <= 1; ++rs) {
-                const int nr = row + rs;
-                if (nr < 0 || nr >= a.H) continue;
-                for (int cs = -1; cs <= 1; ++cs) {
-                    if (rs == 0 && cs == 0) continue;
-                    const int n = nr * a.W + ((col + cs) & (a.W - 1));
-                    if (a.land[n] && a.dirs[n] == from && a.ground[n] - a.rel[n] > a.pond_depth) {
-                        const float ar = a.area[n];
-                        const bool ties = ar == best_area && (best < 0 || n < best);
-                        if (ar > best_area || ties) {
-                            best_area = ar;
-                            best = n;
-                        }
-                    }
-                }
-            }
-            if (best < 0) break;
-            back += step_between(a, best, from);
-            if (back > a.reach) break;
-            const float cut_level = new_level + back * a.gradient;
-            if (a.rel[best] <= cut_level) break;
-            if (take_down(a, best, cut_level, false)) cells++;
-            from = best;
-        }
+// A wave of the notch: `kNotchWarps` basins, `rank` this warp's among them. A stamp orders waves, then
+// the basins of a wave, the first the greatest.
+constexpr int kNotchWarps = 32;
+struct NotchTurn {
+    int wave, rank;
+    int* cut_cell;
+    float* cut_level;
+    int* chain;
+    int* read_cell;
+    int reads;
+    __device__ int stamp() const { return wave * kNotchWarps + (kNotchWarps - 1 - rank); }
+    __device__ void read(int cell) {   // a walk's read, the same cell in every lane
+        if ((threadIdx.x & 31) == 0) read_cell[reads] = cell;
+        ++reads;
     }
-    *a.cells = cells;
+    __device__ void read_where(bool mine, int cell) {   // a cell of each lane that asks
+        const unsigned lanes = __ballot_sync(0xFFFFFFFFu, mine);
+        if (mine) read_cell[reads + __popc(lanes & ((1u << (threadIdx.x & 31)) - 1u))] = cell;
+        reads += __popc(lanes);
+    }
+};
+
+// HydraulicErosion.breach with belowSea on (HydraulicErosion.kt:1931-2171) for one basin, by a warp; the
+// walks run the same in every lane. The cuts are listed, not made: every cell of a basin's three walks
+// is a different one, and no walk reads a cell another of them cuts. Returns their number, and in
+// *lowers_ground the first so many of them that take the filled surface down too.
+__device__ int notch_basin(const NotchArgs& a, const Drowned& d, NotchTurn& t, int* lowers_ground) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const int spill = d.spill;
+    const float level = d.level, floor_ = d.floor_;
+    *lowers_ground = 0;
+    if (level - floor_ <= 0.0f) return 0;
+    float fall = 0.0f, length = 0.0f, last_step = 1.0f;
+    int walked = 0, cell = spill;
+    while (cell >= 0 && a.land[cell] && length < a.reach) {
+        t.read(cell);
+        fall = level - a.rel[cell];
+        if (fall > level - floor_) break;
+        const int next = a.dirs[cell];
+        last_step = next >= 0 ? step_between(a, cell, next) : 1.0f;
+        length += last_step;
+        walked++;
+        cell = next;
+    }
+    if (fall <= 1e-6f * (float)walked && cell >= 0 && !a.land[cell]) {   // outletFallToTheWater
+        fall = level - a.rel[cell];
+        length += last_step;
+    }
+    if (walked == 0) return 0;
+    float slope = fall / length * (float)a.W;
+    if (slope < 0.0f) slope = 0.0f;
+    const float power = a.coefficient * sqrtf(a.area[spill] / a.land_cells) * slope;
+    const float drop = jvm_minf(power, level - floor_);
+    if (drop <= 0.0f) return 0;
+    const float new_level = level - drop;
+    float from_lip = 0.0f;
+    int n = 0;
+    cell = spill;
+    while (cell >= 0 && a.land[cell] && from_lip < a.reach) {
+        const float cut_level = new_level - from_lip * a.gradient;
+        t.read(cell);
+        if (a.rel[cell] <= cut_level) break;
+        if (lane == 0) {
+            t.cut_cell[n] = cell;
+            t.cut_level[n] = cut_level;
+        }
+        ++n;
+        const int next = a.dirs[cell];
+        from_lip += next >= 0 ? step_between(a, cell, next) : 1.0f;
+        cell = next;
+    }
+    const int entry = d.entry;
+    float back = 0.0f;
+    if (entry >= 0 && entry != spill) {
+        int margin_cells = 0, walker = entry;
+        float widths = 0.0f;
+        while (walker >= 0 && walker != spill && a.land[walker] && widths <= a.reach) {
+            const int next = a.dirs[walker];
+            widths += next >= 0 ? step_between(a, walker, next) : 1.0f;
+            if (lane == 0) t.chain[margin_cells] = walker;
+            margin_cells++;
+            walker = next;
+        }
+        __syncwarp();
+        if (walker == spill) {
+            // The margin from the lip back towards the entry: the chain entry -> ... -> spill, walked
+            // backwards over its listed cells (distinct, as a forest's chain is).
+            int downstream = spill;
+            for (int i = margin_cells - 1; i >= 0; --i) {
+                const int m = t.chain[i];
+                back += step_between(a, m, downstream);
+                const float cut_level = new_level + back * a.gradient;
+                t.read(m);
+                if (a.rel[m] <= cut_level) break;
+                if (lane == 0) {
+                    t.cut_cell[n] = m;
+                    t.cut_level[n] = cut_level;
+                }
+                ++n;
+                downstream = m;
+            }
+        }
+        __syncwarp();   // the chain is read before the next walk writes it
+    }
+    // The sill on the basin's own side: up the inflow of the largest catchment across the bed. A step
+    // reads only cells upstream of `from`, which no cut of this basin touched.
+    int from = entry >= 0 ? entry : spill;
+    *lowers_ground = n;
+    while (back <= a.reach) {
+        const int k = lane < 4 ? lane : lane + 1;   // lanes 0-7: the neighbours, rows then columns
+        const int nr = pdiv(from, a.W) + k / 3 - 1;
+        int best = -1;
+        float best_area = -1.0f;
+        const int nb = nr * a.W + ((pmod(from, a.W) + k % 3 - 1) & (a.W - 1));
+        const bool donor = lane < 8 && nr >= 0 && nr < a.H && a.land[nb] && a.dirs[nb] == from;
+        t.read_where(donor, nb);
+        if (donor) {
+            const float ar = a.area[nb];
+            if (a.ground[nb] - a.rel[nb] > a.pond_depth && ar >= -1.0f) {
+                best = nb;
+                best_area = ar;
+            }
+        }
+        for (int o = 4; o > 0; o >>= 1) {   // the largest catchment, ties on the lower index
+            const int ob = __shfl_down_sync(FULL, best, o);
+            const float oa = __shfl_down_sync(FULL, best_area, o);
+            if (ob >= 0 && (best < 0 || oa > best_area || (oa == best_area && ob < best))) {
+                best = ob;
+                best_area = oa;
+            }
+        }
+        best = __shfl_sync(FULL, best, 0);
+        if (best < 0) break;
+        back += step_between(a, best, from);
+        if (back > a.reach) break;
+        const float cut_level = new_level + back * a.gradient;
+        if (a.rel[best] <= cut_level) break;
+        if (lane == 0) {
+            t.cut_cell[n] = best;
+            t.cut_level[n] = cut_level;
+        }
+        ++n;
+        from = best;
+    }
+    return n;
+}
+
+// The drowned basins in waves of up to 32, in order. The first basin of a wave never finds a clash, so
+// every wave cuts at least one.
+__global__ void __launch_bounds__(32 * kNotchWarps) k_notch_below_sea(NotchArgs a) {
+    __shared__ int first_clash;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    NotchTurn t;
+    t.wave = a.wave0;
+    t.rank = warp;
+    t.cut_cell = a.cut_cell + (size_t)warp * 3 * a.cap;
+    t.cut_level = a.cut_level + (size_t)warp * 3 * a.cap;
+    t.chain = a.chain + (size_t)warp * a.cap;
+    t.read_cell = a.read_cell + (size_t)warp * 11 * a.cap;
+    int cells = 0;
+    for (int b0 = 0; b0 < a.count;) {
+        ++t.wave;
+        t.reads = 0;
+        if (threadIdx.x == 0) first_clash = kNotchWarps;
+        const int b = b0 + warp;
+        int n = 0, lowers = 0;
+        Drowned d{};
+        if (b < a.count) {
+            d = a.list[b];
+            n = notch_basin(a, d, t, &lowers);
+            __syncwarp();
+            for (int i = lane; i < n; i += 32) atomicMax(&a.stamp[t.cut_cell[i]], t.stamp());
+        }
+        __syncthreads();
+        bool clash = false;
+        for (int i = lane; i < t.reads; i += 32) {
+            const int stamp = __ldcg(&a.stamp[t.read_cell[i]]);
+            clash |= stamp > t.stamp() && stamp < (t.wave + 1) * kNotchWarps;
+        }
+        if (__any_sync(0xFFFFFFFFu, clash) && lane == 0) atomicMin(&first_clash, warp);
+        __syncthreads();
+        const int go = min(first_clash, a.count - b0);
+        if (warp < go)
+            for (int i = lane; i < n; i += 32)
+                if (take_down(a, t.cut_cell[i], t.cut_level[i], i < lowers)) ++cells;
+        __syncthreads();   // the cuts are made, and first_clash read, before the next wave
+        b0 += go;
+    }
+    cells = __reduce_add_sync(0xFFFFFFFFu, cells);
+    if (threadIdx.x == 0) *a.cells = 0;
+    __syncthreads();
+    if (lane == 0 && cells) atomicAdd(a.cells, cells);
 }
 
 cg_status enclose_dev(cg_ctx* ctx, int W, int H, uint8_t* d_land, float* d_rel, const float* d_h, float shoreline,
@@ -298,6 +450,7 @@ extern "C" cg_status cg_sea_level_cut(cg_ctx* ctx, const cg_erosion_params* p, c
     CG_TRY_ST(enclose_dev(ctx, W, H, d_land, d_rel, d_h, s, land_half, largest_lake, &n));
     int run = 0;
     bool have_terrain = false;
+    int waves = 0;
     for (int pass = 0; post_cut_outlet && pass < 16 && n > 0; ++pass) {   // MAX_POST_CUT_OUTLET_PASSES
         CG_TRY_ST(fill_depressions_dev(ctx, W, H, d_land, d_rel, d_filled, nullptr, nullptr));
         FlatCounts fc{0, 0, 0};
@@ -310,8 +463,19 @@ extern "C" cg_status cg_sea_level_cut(cg_ctx* ctx, const cg_erosion_params* p, c
         int count = 0;
         CG_TRY_ST(basins_dev(ctx, W, H, d_land, d_rel, d_filled, d_recv, rates.pond_depth, d_bl, &bas, &count));
         if (count == 0) break;
+        CG_BUF(Drowned, d_list, ctx, S_SL_LIST, (size_t)count);
+        // A walk's cells are distinct and their summed steps stay within the reach; twice that leaves room
+        // for the rounding of the sums.
+        const float least = std::fmin(1.0f, rates.step_ns);
+        const size_t cap = (size_t)std::fmin((double)N, 2.0 * std::ceil((double)rates.outlet_reach_cells / least) + 64.0) + 4;
+        CG_BUF(int, d_chain, ctx, S_SL_CHAIN, 18 * kNotchWarps * cap);
+        CG_BUF(int, d_stamp, ctx, S_SL_STAMP, N);
+        if (pass == 0 || waves > (1 << 24)) {   // stamps stay within an int
+            CG_CUDA(ctx, cudaMemsetAsync(d_stamp, 0, N * sizeof(int), sm));
+            waves = 0;
+        }
         CG_CUDA(ctx, cudaMemsetAsync(d_words, 0, 4 * sizeof(int), sm));
-        CG_LAUNCH(ctx) k_mark_drowned<<<(count + 255) / 256, 256, 0, sm>>>(bas.spill, bas.floor_, count, d_words);
+        CG_LAUNCH(ctx) k_list_drowned<<<1, 1024, 0, sm>>>(bas.spill, bas.entry, bas.level, bas.floor_, count, d_list, d_words);
         CG_CHECK_LAUNCH(ctx);
         int drowned = 0;
         CG_CUDA(ctx, cudaMemcpyAsync(&drowned, d_words, sizeof(int), cudaMemcpyDeviceToHost, sm));
@@ -325,11 +489,16 @@ extern "C" cg_status cg_sea_level_cut(cg_ctx* ctx, const cg_erosion_params* p, c
         NotchArgs a;
         a.W = W;
         a.H = H;
-        a.count = count;
-        a.spill = bas.spill;
-        a.entry = bas.entry;
-        a.level = bas.level;
-        a.floor_ = bas.floor_;
+        a.count = drowned;
+        a.list = d_list;
+        a.chain = d_chain;
+        a.cut_cell = d_chain + kNotchWarps * cap;
+        a.cut_level = (float*)(d_chain + 4 * kNotchWarps * cap);
+        a.read_cell = d_chain + 7 * kNotchWarps * cap;
+        a.cap = (int)cap;
+        a.stamp = d_stamp;
+        a.wave0 = waves;
+        waves += drowned;   // a wave cuts a basin at least
         a.land = d_land;
         a.dirs = d_recv;
         a.area = d_area;
@@ -345,7 +514,7 @@ extern "C" cg_status cg_sea_level_cut(cg_ctx* ctx, const cg_erosion_params* p, c
         a.step_ns = rates.step_ns;
         a.step_diag = rates.step_diag;
         a.cells = d_words + 1;
-        CG_LAUNCH(ctx) k_notch_below_sea<<<1, 32, 0, sm>>>(a);
+        CG_LAUNCH(ctx) k_notch_below_sea<<<1, 32 * kNotchWarps, 0, sm>>>(a);
         CG_CHECK_LAUNCH(ctx);
         int cut = 0;
         CG_CUDA(ctx, cudaMemcpyAsync(&cut, d_words + 1, sizeof(int), cudaMemcpyDeviceToHost, sm));
