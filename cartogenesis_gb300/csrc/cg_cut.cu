@@ -21,6 +21,7 @@
 #include "cg_common.cuh"
 #include "cg_fpemu.h"
 #include "cg_internal.h"
+#include "cg_seqwalk.cuh"
 
 namespace cg {
 
@@ -67,18 +68,27 @@ __global__ void k_cut_init(CutState* s) {
     s->degenerate = 0;
 }
 
-__global__ void k_minmax(const float* __restrict__ h, size_t N, CutState* s) {
+__global__ void __launch_bounds__(256) k_minmax(const float* __restrict__ h, size_t N, CutState* s) {
     unsigned lo = 0xFFFFFFFFu, hi = 0u;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
         unsigned k = ordered_key(h[i]);
         lo = min(lo, k);
         hi = max(hi, k);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
-    }
+    // One atomic a CTA: every warp's, on the two words, took 13 us of a 512 x 256 cut.
+    __shared__ unsigned wlo[8], whi[8];
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
     if ((threadIdx.x & 31) == 0) {
+        wlo[threadIdx.x >> 5] = lo;
+        whi[threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+            lo = min(lo, wlo[w]);
+            hi = max(hi, whi[w]);
+        }
         atomicMin(&s->lo_key, lo);
         atomicMax(&s->hi_key, hi);
     }
@@ -113,43 +123,67 @@ __global__ void __launch_bounds__(512) k_row_counts(const float* __restrict__ h,
 }
 
 // One warp per bin: the reference's sequential sum `histogram[bin] += rowWeights[row]`, in cell
-// order, replayed exactly, 32 rows at a time (cg::warp_seq_sum).
-__global__ void k_bin_sums(const unsigned* __restrict__ counts, const double* __restrict__ w, int H,
-                           const CutState* s, double* __restrict__ hist) {
+// order, replayed exactly, 32 rows at a time (cg::warp_seq_sum). The rows that hold none of the bin's
+// cells (most rows of a small grid) are dropped first: the others queue up in order in shared memory.
+__global__ void __launch_bounds__(256) k_bin_sums(const unsigned* __restrict__ counts, const double* __restrict__ w,
+                                                  int H, const CutState* s, double* __restrict__ hist) {
+    __shared__ int q_row[8][64];
+    __shared__ unsigned q_cnt[8][64];
     const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (b >= BINS || s->degenerate) return;
-    double acc = 0.0;
+    double acc = 0.0, before;
+    int queued = 0;
+    unsigned next = lane < H ? counts[(size_t)lane * BINS + b] : 0u;
     for (int base = 0; base < H; base += 32) {
-        int r = base + lane;
-        unsigned c = r < H ? counts[(size_t)r * BINS + b] : 0u;
-        double wr = r < H ? w[r] : 0.0;
-        if (!__any_sync(0xFFFFFFFFu, c != 0u)) continue;
-        double before;
-        acc = warp_seq_sum(acc, wr, (int64_t)c, &before);
+        const int r = base + lane;
+        const unsigned c = next;
+        next = r + 32 < H ? counts[(size_t)(r + 32) * BINS + b] : 0u;
+        const unsigned rows = __ballot_sync(0xFFFFFFFFu, c != 0u);
+        if (!rows) continue;
+        if (c != 0u) {
+            const int at = queued + __popc(rows & ((1u << lane) - 1u));
+            q_row[warp][at] = r;
+            q_cnt[warp][at] = c;
+        }
+        queued += __popc(rows);
+        __syncwarp();
+        if (queued >= 32) {
+            acc = warp_seq_sum(acc, w[q_row[warp][lane]], (int64_t)q_cnt[warp][lane], &before);
+            __syncwarp();
+            if (lane < queued - 32) {
+                q_row[warp][lane] = q_row[warp][32 + lane];
+                q_cnt[warp][lane] = q_cnt[warp][32 + lane];
+            }
+            queued -= 32;
+            __syncwarp();
+        }
     }
+    if (queued > 0)
+        acc = warp_seq_sum(acc, lane < queued ? w[q_row[warp][lane]] : 0.0,
+                           lane < queued ? (int64_t)q_cnt[warp][lane] : 0, &before);
     if (lane == 0) hist[b] = acc;
 }
 
-// SeaLevelStage.kt:614-622: the first bin that brings the weight below up to the target. The
-// histogram is staged in shared memory by the CTA; one thread then takes the reference's sums.
-__global__ void __launch_bounds__(256) k_bracket_bin(const double* __restrict__ hist, double target, CutState* s) {
-    __shared__ double sh[BINS];
+// SeaLevelStage.kt:614-622: the first bin that brings the weight below up to the target, the bins'
+// sequential sum taken by the CTA's scan (one thread adding 4096 doubles in turn took 140 us).
+__global__ void __launch_bounds__(seqwalk::kSSThreads) k_bracket_bin(const double* __restrict__ hist, double target,
+                                                                     CutState* s) {
+    using namespace seqwalk;
+    static_assert(BINS <= kSSBlock, "the histogram is one block of values");
+    __shared__ CtaSum sh;
     if (s->degenerate) return;
-    for (int b = threadIdx.x; b < BINS; b += blockDim.x) sh[b] = hist[b];
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    double below = 0.0;
-    int bracket = BINS - 1;
-    for (int b = 0; b < BINS; ++b) {
-        if (below + sh[b] >= target) {
-            bracket = b;
-            break;
-        }
-        below += sh[b];
+    if (threadIdx.x == 0) {
+        sh.s = 0.0;
+        sh.hit = -1;
     }
-    s->bracket_bin = bracket;
-    s->below_bracket = below;
+    const SumIn<double> in{hist, nullptr, 0, BINS, nullptr, nullptr, 0.0, nullptr, 0};
+    __syncthreads();
+    cta_advance<true>(in, 0, BINS, sh, target);
+    if (threadIdx.x == 0) {
+        s->bracket_bin = sh.hit >= 0 ? sh.hit : BINS - 1;
+        s->below_bracket = sh.hit >= 0 ? sh.below : sh.s;
+    }
 }
 
 __global__ void k_bracket_collect(const float* __restrict__ h, size_t N, CutState* s, long long* __restrict__ keys) {
@@ -174,32 +208,33 @@ __global__ void k_bracket_collect(const float* __restrict__ h, size_t N, CutStat
     }
 }
 
-// Bitonic sort of up to 16384 keys in one CTA's shared memory (padding with the largest key).
+// Up to SMALL_SORT keys sorted by rank, over the whole GPU: a warp takes RANK_KEYS keys, its lanes count
+// the keys below each, and each goes to its count (the keys are distinct: they hold their cell). n^2 / 4
+// loads and n^2 compares beat the n log^2 n of a bitonic network in one CTA, whose 66 steps of one CTA
+// take 80 us at 2048 keys, up to 16384 keys; past that the network over chunks below is the faster.
 constexpr int SMALL_SORT = 16384;
-__global__ void __launch_bounds__(1024) k_sort_small(long long* keys, const CutState* s) {
-    extern __shared__ long long sk[];
-    int n = s->count;
-    if (s->degenerate || n <= 1 || n > SMALL_SORT) return;
-    int P2 = 1;
-    while (P2 < n) P2 <<= 1;
-    for (int i = threadIdx.x; i < P2; i += blockDim.x) sk[i] = i < n ? keys[i] : LLONG_MAX;
-    __syncthreads();
-    for (int k = 2; k <= P2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < P2; i += blockDim.x) {
-                int l = i ^ j;
-                if (l > i) {
-                    bool up = (i & k) == 0;
-                    long long a = sk[i], b = sk[l];
-                    if ((a > b) == up) {
-                        sk[i] = b;
-                        sk[l] = a;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) keys[i] = sk[i];
+constexpr int RANK_KEYS = 4;
+__global__ void __launch_bounds__(256) k_sort_rank(const long long* __restrict__ keys, int n, long long* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * RANK_KEYS;
+    if (k0 >= n) return;
+    long long mine[RANK_KEYS];
+    int below[RANK_KEYS];
+#pragma unroll
+    for (int k = 0; k < RANK_KEYS; ++k) {
+        mine[k] = k0 + k < n ? keys[k0 + k] : LLONG_MIN;
+        below[k] = 0;
+    }
+    for (int i = lane; i < n; i += 32) {
+        const long long other = keys[i];
+#pragma unroll
+        for (int k = 0; k < RANK_KEYS; ++k) below[k] += other < mine[k] ? 1 : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < RANK_KEYS; ++k) {
+        const int rank = __reduce_add_sync(0xFFFFFFFFu, below[k]);
+        if (lane == 0 && k0 + k < n) out[rank] = mine[k];
+    }
 }
 
 // One compare-exchange stage of a global bitonic sort over P2 slots, padded with the largest key.
@@ -487,7 +522,7 @@ cg_status percentile_cut_dev(cg_ctx* ctx, int W, int H, const float* d_h, float 
     CG_LAUNCH(ctx) k_cut_prepare<<<1, 1, 0, sm>>>(d_s, target);
     CG_LAUNCH(ctx) k_row_counts<<<H, 512, 0, sm>>>(d_h, W, d_s, d_counts);
     CG_LAUNCH(ctx) k_bin_sums<<<BINS * 32 / 256, 256, 0, sm>>>(d_counts, d_w, H, d_s, d_hist);
-    CG_LAUNCH(ctx) k_bracket_bin<<<1, 256, 0, sm>>>(d_hist, target, d_s);
+    CG_LAUNCH(ctx) k_bracket_bin<<<1, seqwalk::kSSThreads, 0, sm>>>(d_hist, target, d_s);
     CG_LAUNCH(ctx) k_bracket_collect<<<grid, 256, 0, sm>>>(d_h, N, d_s, d_keys);
     CG_CHECK_LAUNCH(ctx);
     CutState hs;
@@ -495,13 +530,10 @@ cg_status percentile_cut_dev(cg_ctx* ctx, int W, int H, const float* d_h, float 
     CG_CUDA(ctx, cudaStreamSynchronize(sm));
     if (!hs.degenerate && hs.count > 1) {
         if (hs.count <= SMALL_SORT) {
-            // Set on every call (it is cheap): a flag kept across calls would be shared by every
-            // context and device of the process.
-            CG_CUDA(ctx, cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)(SMALL_SORT * sizeof(long long))));
-            int P2 = 1;
-            while (P2 < hs.count) P2 <<= 1;
-            CG_LAUNCH(ctx) k_sort_small<<<1, 1024, P2 * sizeof(long long), sm>>>(d_keys, d_s);
+            CG_BUF(long long, d_sorted, ctx, S_BRACKET2, SMALL_SORT);
+            const int warps = (hs.count + RANK_KEYS - 1) / RANK_KEYS;
+            CG_LAUNCH(ctx) k_sort_rank<<<(warps + 7) / 8, 256, 0, sm>>>(d_keys, hs.count, d_sorted);
+            d_keys = d_sorted;
         } else {
             int P2 = 1;
             while (P2 < hs.count) P2 <<= 1;

@@ -17,59 +17,77 @@
 #define CG_HD __host__ __device__ __forceinline__
 #else
 #define CG_HD inline
-#include <cmath>
 #endif
+#include <cstring>
 
 namespace cg {
 
+CG_HD int64_t fp_bits(double x) {
+#ifdef __CUDA_ARCH__
+    return __double_as_longlong(x);
+#else
+    int64_t b;
+    std::memcpy(&b, &x, 8);
+    return b;
+#endif
+}
+CG_HD double fp_of(int64_t b) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double(b);
+#else
+    double x;
+    std::memcpy(&x, &b, 8);
+    return x;
+#endif
+}
+
+// Integer arithmetic on the doubles' bits throughout: GB300 issues FP64 instructions at about 1/64 of
+// its integer rate, and in the sea-level histogram's 4096 bins the divisions and scalings of a
+// floating-point form were most of the time.
 CG_HD double seq_repeat_add(double s, double w, int64_t c) {
     const int64_t TOP = (int64_t)1 << 53;   // m ranges over [2^52, 2^53) within a binade
+    const int64_t MANT = ((int64_t)1 << 52) - 1;
+    const int64_t wb = fp_bits(w);
+    const int ew = (int)(wb >> 52);
+    const int64_t mw = (wb & MANT) | (MANT + 1);
     while (c > 0) {
-        if (s == 0.0) {   // fl(0 + w) = w
+        const int64_t sb = fp_bits(s);
+        const int es = (int)(sb >> 52);
+        const int shift = es - ew;   // w / U = mw / 2^shift
+        int64_t m = (sb & MANT) | (MANT + 1);
+        // No binade to speak of (a zero or subnormal sum or term), or a term past the binade, or a step
+        // that leaves it: one addition in hardware.
+        if (es == 0 || ew == 0 || shift < 1 || m + (shift < 63 ? mw >> shift : 0) > TOP - 1) {
             s = s + w;
             --c;
             continue;
         }
-        int e;
-#ifdef __CUDA_ARCH__
-        e = ilogb(s);
-        double U = ldexp(1.0, e - 52);
-#else
-        e = std::ilogb(s);
-        double U = std::ldexp(1.0, e - 52);
-#endif
-        int64_t m = (int64_t)(s / U);   // exact: s is a multiple of U
-        double x = w / U;               // exact: scaling by a power of two
-        if (x >= 9.0e15) {              // the term alone reaches past the binade: one plain step
-            s = s + w;
-            --c;
-            continue;
-        }
-        int64_t q = (int64_t)x;
-        double f = x - (double)q;       // exact
-        if (m + q > TOP - 1) {          // this step leaves the binade: take it in hardware
-            s = s + w;
-            --c;
-            continue;
-        }
-        int64_t d;
-        if (f == 0.5) {
-            if ((m & 1) != 0) {         // one tie step from an odd m, which lands on an even m
-                s = (double)(m + q + ((m + q) & 1)) * U;
-                --c;
-                continue;
+        int64_t q = 0, d = 0;
+        if (shift < 63) {   // from 54 on w is below half a unit: q = d = 0
+            q = mw >> shift;
+            const int64_t rem = mw & (((int64_t)1 << shift) - 1), half = (int64_t)1 << (shift - 1);
+            if (rem == half) {
+                if ((m & 1) != 0) {     // one tie step from an odd m, which lands on an even m
+                    m += q + ((m + q) & 1);
+                    s = fp_of(m == TOP ? (int64_t)(es + 1) << 52 : ((int64_t)es << 52) | (m & MANT));
+                    --c;
+                    continue;
+                }
+                d = q + (q & 1);        // from an even m every tie step adds this and keeps m even
+            } else {
+                d = q + (rem > half ? 1 : 0);
             }
-            d = q + (q & 1);            // from an even m every tie step adds this and keeps m even
-        } else {
-            d = q + (f > 0.5 ? 1 : 0);
         }
         if (d == 0) return s;           // every remaining step rounds back to s
         // Steps j = 0..t-1 stay inside the binade while m + j*d + q <= TOP - 1.
-        int64_t tmax = (TOP - 1 - q - m) / d + 1;
-        int64_t t = c < tmax ? c : tmax;
-        m += t * d;
+        int64_t t = c;
+        if (c >= ((int64_t)1 << 22) || d >= ((int64_t)1 << 40) || m + (c - 1) * d + q > TOP - 1) {
+            const int64_t tmax = (TOP - 1 - q - m) / d + 1;
+            t = c < tmax ? c : tmax;
+        }
+        m += t * d;                     // at most 2^53
         c -= t;
-        s = (double)m * U;               // exact (m <= 2^53)
+        s = fp_of(m == TOP ? (int64_t)(es + 1) << 52 : ((int64_t)es << 52) | (m & MANT));
     }
     return s;
 }

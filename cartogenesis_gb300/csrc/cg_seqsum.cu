@@ -31,33 +31,18 @@
 
 #include "cg_common.cuh"
 #include "cg_internal.h"
+#include "cg_seqwalk.cuh"
 
 namespace cg {
 namespace {
 
-constexpr int kSSThreads = 1024;
-constexpr int kSSPer = 8;                        // values per thread in the parallel reduction
-constexpr int kSSBlock = kSSThreads * kSSPer;    // values per block
-constexpr long long kM0 = 1LL << 52, kM1 = 1LL << 53;
+using namespace seqwalk;
+
 constexpr long long kBig = 1LL << 58;            // a partial step this large leaves any binade: give up
 constexpr int kMaxSums = 5;                      // sums of one launch
 // Sums up to this many blocks are taken by one CTA from the first value. A block taken so costs about
 // 2.5 us, the parallel form's three launches about 25 us before its first block.
 constexpr int kDirectBlocks = 10;
-
-// The values summed: float fields (widened exactly), or double terms already in summation order.
-template <typename T>
-struct SumIn {
-    const T* x;
-    const uint8_t* mask;   // may be null: every value (float fields only)
-    int mode;              // 0: x, 1: 1 - 0.5 x (the cover's shielding factor; float fields only)
-    size_t n;
-    const double* init;    // the sum before the first value (may be null: +0)
-    double* out;           // may be `init`
-    double divisor;        // the sum is divided by it unless it is 0
-    long long* counts;     // may be null: how the sum went (3)
-    int first_block;       // this sum's first entry in the launch's estimates and walks
-};
 
 // The sums of one launch.
 template <typename T>
@@ -71,7 +56,7 @@ struct Walk {
     int out[2];                        // parity of m leaving
     int fail;                          // a value the integer walk cannot hold (it leaves the binade)
     int spec;                          // the binade and sign it was made for (exponent | sign << 11), -1: none
-    int zero;                          // every value is a zero: the block leaves any sum but -0 as it was
+    int zero;                          // no value adds anything
 };
 
 __device__ __forceinline__ Walk walk_identity() {
@@ -106,99 +91,6 @@ __device__ __forceinline__ Walk walk_then(const Walk& a, const Walk& b) {
     w.spec = a.spec;
     if (w.step[0] > kBig || w.step[0] < -kBig || w.step[1] > kBig || w.step[1] < -kBig) w.fail = 1;
     return w;
-}
-
-__device__ __forceinline__ bool value_at(const SumIn<float>& in, size_t i, float* v) {
-    if (i >= in.n) return false;
-    if (in.mask && !in.mask[i]) return false;
-    const float x = in.x[i];
-    *v = in.mode == 1 ? __fsub_rn(1.0f, __fmul_rn(0.5f, x)) : x;
-    return true;
-}
-
-__device__ __forceinline__ bool value_at(const SumIn<double>& in, size_t i, double* v) {
-    if (i >= in.n) return false;
-    *v = in.x[i];
-    return true;
-}
-
-// One value's step in the binade with exponent field ef (u = 2^(ef - 1075)), for a sum of sign `neg`:
-// the step r when it is not a tie, else the tie's floor f (r = f + ((parity + f) & 1)). An absent value
-// (a masked cell) adds nothing, as the reference skips it; +0 and -0 add nothing to a nonzero sum.
-struct Step {
-    long long r;
-    int tie, fail;
-};
-
-__device__ __forceinline__ Step step_of(float v, int ef, int neg) {
-    Step s{0, 0, 0};
-    const uint32_t b = __float_as_uint(v);
-    const int fe = (int)((b >> 23) & 0xFF);
-    if (fe == 0xFF) {
-        s.fail = 1;
-        return s;
-    }
-    long long M = (long long)(b & 0x7FFFFF);
-    if (fe != 0) M |= 1LL << 23;
-    if (M == 0) return s;
-    const bool negative = ((b >> 31) != 0) != (neg != 0);   // y's sign: x's, flipped for a negative sum
-    // y = M 2^k with k = (max(fe, 1) - 150) - (ef - 1075)
-    const int k = (fe == 0 ? 1 : fe) - 150 - ef + 1075;
-    if (k >= 0) {
-        if (k > 29) {
-            s.fail = 1;
-            return s;
-        }
-        s.r = negative ? -(M << k) : (M << k);
-        return s;
-    }
-    const int sh = -k;
-    if (sh >= 40) return s;   // |y| < 2^-16: rounds to 0
-    const long long a = M >> sh, frac = M & ((1LL << sh) - 1), half = 1LL << (sh - 1);
-    if (frac == half) {
-        s.tie = 1;
-        s.r = negative ? -(a + 1) : a;   // floor(y)
-    } else {
-        const long long r = a + (frac > half ? 1 : 0);
-        s.r = negative ? -r : r;
-    }
-    return s;
-}
-
-// The same for a double value: y = M 2^k with M < 2^53 and k = max(fe, 1) - ef. A value of 2^58 u or
-// more, or NaN or infinity, is left to the serial additions; below u / 4 it adds nothing.
-__device__ __forceinline__ Step step_of(double v, int ef, int neg) {
-    Step s{0, 0, 0};
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    const int fe = (int)((b >> 52) & 0x7FF);
-    if (fe == 0x7FF) {
-        s.fail = 1;
-        return s;
-    }
-    long long M = (long long)(b & ((1ULL << 52) - 1));
-    if (fe != 0) M |= 1LL << 52;
-    if (M == 0) return s;
-    const bool negative = ((b >> 63) != 0) != (neg != 0);
-    const int k = (fe == 0 ? 1 : fe) - ef;
-    if (k >= 0) {
-        if (k > 5) {
-            s.fail = 1;
-            return s;
-        }
-        s.r = negative ? -(M << k) : (M << k);
-        return s;
-    }
-    const int sh = -k;
-    if (sh >= 55) return s;   // |y| < 2^-2: rounds to 0
-    const long long a = M >> sh, frac = M & ((1LL << sh) - 1), half = 1LL << (sh - 1);
-    if (frac == half) {
-        s.tie = 1;
-        s.r = negative ? -(a + 1) : a;
-    } else {
-        const long long r = a + (frac > half ? 1 : 0);
-        s.r = negative ? -r : r;
-    }
-    return s;
 }
 
 // The walk of a run of values in order, for both entering parities.
@@ -254,270 +146,6 @@ __device__ Walk cta_walk(const Walk& mine, Walk* sh_warps) {
     return total;
 }
 
-// A run's step and leaving parity for each entering parity (bit q of `out`: the parity left from q).
-struct Run {
-    long long step[2];
-    unsigned out;
-};
-__device__ __forceinline__ long long wrap_add(long long a, long long b) {   // past a crossing the sums are not read
-    return (long long)((unsigned long long)a + (unsigned long long)b);
-}
-__device__ __forceinline__ Run run_then(const Run& a, const Run& b) {
-    Run r;
-    const unsigned p0 = a.out & 1u, p1 = (a.out >> 1) & 1u;
-    r.step[0] = wrap_add(a.step[0], p0 ? b.step[1] : b.step[0]);
-    r.step[1] = wrap_add(a.step[1], p1 ? b.step[1] : b.step[0]);
-    r.out = ((b.out >> p0) & 1u) | (((b.out >> p1) & 1u) << 1);
-    return r;
-}
-// The inclusive scan of the warp's runs. Without ties both parities step alike: one sum does.
-__device__ __forceinline__ Run warp_scan(Run r, bool ties) {
-    const int lane = threadIdx.x & 31;
-    for (int o = 1; o < 32; o <<= 1) {
-        Run a;
-        a.step[0] = __shfl_up_sync(0xFFFFFFFFu, r.step[0], o);
-        if (ties) {
-            a.step[1] = __shfl_up_sync(0xFFFFFFFFu, r.step[1], o);
-            a.out = __shfl_up_sync(0xFFFFFFFFu, r.out, o);
-            if (lane >= o) r = run_then(a, r);
-        } else if (lane >= o) {
-            r.step[0] = wrap_add(a.step[0], r.step[0]);
-        }
-    }
-    return r;
-}
-__device__ __forceinline__ Run run_from(const Run& r, int src) {
-    Run o;
-    o.step[0] = __shfl_sync(0xFFFFFFFFu, r.step[0], src);
-    o.step[1] = __shfl_sync(0xFFFFFFFFu, r.step[1], src);
-    o.out = __shfl_sync(0xFFFFFFFFu, r.out, src);
-    return o;
-}
-__device__ __forceinline__ Run run_identity() { return Run{{0, 0}, 2u}; }
-
-// A step's own run (a step that leaves any binade is marked by the caller).
-__device__ __forceinline__ Run run_of(const Step& st) {
-    Run r;
-    if (st.tie) {
-        r.step[0] = st.r + (st.r & 1);
-        r.step[1] = st.r + ((1 + st.r) & 1);
-        r.out = 0u;
-    } else {
-        r.step[0] = r.step[1] = st.r;
-        r.out = (st.r & 1) ? 1u : 2u;
-    }
-    return r;
-}
-
-// A normal sum's binade: exponent field, sign, and m.
-struct Binade {
-    int ef, neg;
-    long long m;
-    bool normal;
-};
-__device__ __forceinline__ Binade binade_of(double s) {
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(s);
-    Binade b;
-    b.ef = (int)((bits >> 52) & 0x7FF);
-    b.neg = (int)(bits >> 63);
-    b.m = (long long)(bits & ((1ULL << 52) - 1)) | kM0;
-    b.normal = b.ef != 0 && b.ef != 0x7FF;
-    return b;
-}
-__device__ __forceinline__ double sum_of(const Binade& b, long long m) {
-    return __longlong_as_double((long long)(((unsigned long long)b.neg << 63) | ((unsigned long long)b.ef << 52) |
-                                            (unsigned long long)(m - kM0)));
-}
-// The value moves no further than a binade's width: its step is a plain integer.
-__device__ __forceinline__ bool plain_step(const Step& st) { return !st.fail && st.r < kM1 && st.r > -kM1; }
-// The partial m stays strictly inside the binade: then the exact sum it rounds lies in [2^52, 2^53) u
-// and was rounded to the binade's ulp (a sum rounding to 2^52 itself may have come from below, where
-// the ulp is u / 2).
-__device__ __forceinline__ bool inside(long long m) { return m > kM0 && m < kM1; }
-
-struct CtaSum {
-    Run warps[kSSThreads / 32];
-    int exits[kSSThreads / 32];
-    double s;        // the running sum
-    int pos;         // values of the block taken
-    unsigned alone;  // the block's pieces of 1024 holding an addition taken alone
-};
-
-// Whether a value added to a sum that is no normal number may change it: a zero leaves +0 and the
-// subnormals as they are, NaN stays, and infinity goes only with NaN or the other infinity.
-template <typename T>
-__device__ __forceinline__ bool changes_off_binade(double s, T v) {
-    if (s != s) return false;
-    if (isinf(s)) return v != v || (isinf(v) && (v > (T)0) != (s > 0.0));
-    return v != (T)0 || __double_as_longlong(s) == (long long)(1ULL << 63);
-}
-
-// One warp's walk over the block's values from `pos`, 32 at a time, until a window holds no value taken
-// alone. Every lane holds the same s and pos.
-template <typename T>
-__device__ __forceinline__ void warp_windows(const SumIn<T>& in, size_t base, int len, double& s, int& pos,
-                                             unsigned& alone) {
-    const unsigned FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    bool crossed = true;
-    while (crossed && pos < len) {
-        T v = 0;
-        const bool has = pos + lane < len && value_at(in, base + pos + lane, &v);
-        const Binade b = binade_of(s);
-        bool leaves;
-        long long before = b.m, last = b.m;
-        if (b.normal) {
-            Step st{0, 0, 0};
-            if (has) st = step_of(v, b.ef, b.neg);
-            leaves = !plain_step(st);
-            const Run mine = leaves ? run_identity() : run_of(st);
-            const Run incl = warp_scan(mine, __any_sync(FULL, st.tie));
-            const bool ties = __any_sync(FULL, st.tie);
-            const int q = ties ? (int)(b.m & 1) : 0;
-            const long long after = wrap_add(b.m, q ? incl.step[1] : incl.step[0]);
-            before = __shfl_up_sync(FULL, after, 1);
-            if (lane == 0) before = b.m;
-            leaves = leaves || (has && v != (T)0 && !inside(after));
-            last = __shfl_sync(FULL, after, 31);
-        } else {
-            leaves = has && changes_off_binade(s, v);
-        }
-        const unsigned out = __ballot_sync(FULL, leaves);
-        if (!out) {
-            if (b.normal) s = sum_of(b, last);
-            pos += 32;
-            crossed = false;
-        } else {
-            const int e = __ffs(out) - 1;
-            const double from = b.normal ? sum_of(b, __shfl_sync(FULL, before, e)) : s;
-            s = __shfl_sync(FULL, __dadd_rn(from, (double)v), e);
-            alone |= 1u << ((pos + e) / kSSThreads);
-            pos += e + 1;
-        }
-    }
-    pos = min(pos, len);
-}
-
-// The block's `len` values (a thread's kSSPer consecutive ones in v, its present ones in `has`) added to
-// sh.s in order, by the whole CTA. sh.s is set and visible before the call and after it.
-template <typename T>
-__device__ void cta_advance(const SumIn<T>& in, size_t base, int len, const T (&v)[kSSPer], unsigned has, CtaSum& sh) {
-    const unsigned FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int first = (int)threadIdx.x * kSSPer;
-    int pos = 0;
-    if (threadIdx.x == 0) sh.alone = 0;
-    while (pos < len) {
-        const double s = sh.s;
-        const Binade b = binade_of(s);
-        const unsigned live = first + kSSPer <= pos ? 0u : first >= pos ? has : has & (0xFFu << (pos - first));
-        int exit_at = INT_MAX;
-        long long m = b.m, before = 0;   // before: the partial m at this thread's exit
-        T vx = 0;
-        if (b.normal) {
-            long long r[kSSPer];
-            unsigned tie = 0, off = 0;
-            Run mine = run_identity();
-#pragma unroll
-            for (int t = 0; t < kSSPer; ++t) {
-                Step st{0, 0, 0};
-                if (live & (1u << t)) st = step_of(v[t], b.ef, b.neg);
-                if (!plain_step(st)) {
-                    off |= 1u << t;
-                    st = Step{0, 0, 0};
-                }
-                r[t] = st.r;
-                tie |= (unsigned)st.tie << t;
-                mine.step[0] = wrap_add(mine.step[0], st.r);
-            }
-            const bool ties = __syncthreads_or(tie != 0);
-            if (ties) {
-                mine = run_identity();
-#pragma unroll
-                for (int t = 0; t < kSSPer; ++t) mine = run_then(mine, run_of(Step{r[t], (int)((tie >> t) & 1u), 0}));
-            }
-            const Run incl = warp_scan(mine, ties);
-            if (lane == 31) sh.warps[warp] = incl;
-            __syncthreads();
-            const Run wincl = warp_scan(sh.warps[lane], ties);   // every warp scans the warps' totals
-            Run start = run_from(wincl, warp > 0 ? warp - 1 : 0);
-            if (warp == 0) start = run_identity();
-            Run excl;
-            excl.step[0] = __shfl_up_sync(FULL, incl.step[0], 1);
-            excl.step[1] = __shfl_up_sync(FULL, incl.step[1], 1);
-            excl.out = __shfl_up_sync(FULL, incl.out, 1);
-            if (lane == 0) excl = run_identity();
-            if (ties) {
-                start = run_then(start, excl);
-                m = wrap_add(m, (b.m & 1) ? start.step[1] : start.step[0]);
-            } else {
-                m = wrap_add(wrap_add(m, start.step[0]), excl.step[0]);
-            }
-#pragma unroll
-            for (int t = 0; t < kSSPer; ++t) {
-                if (exit_at != INT_MAX) continue;
-                const long long rt = (tie & (1u << t)) ? r[t] + ((m + r[t]) & 1) : r[t];
-                const long long next = wrap_add(m, rt);
-                if ((live & (1u << t)) && v[t] != (T)0 && ((off & (1u << t)) || !inside(next))) {
-                    exit_at = first + t;
-                    before = m;
-                    vx = v[t];
-                } else {
-                    m = next;
-                }
-            }
-        } else {
-#pragma unroll
-            for (int t = 0; t < kSSPer; ++t)
-                if (exit_at == INT_MAX && (live & (1u << t)) && changes_off_binade(s, v[t])) {
-                    exit_at = first + t;
-                    vx = v[t];
-                }
-        }
-        const int wmin = __reduce_min_sync(FULL, exit_at);
-        if (lane == 0) sh.exits[warp] = wmin;
-        __syncthreads();
-        const int at = __reduce_min_sync(FULL, sh.exits[lane]);
-        if (at == INT_MAX) {
-            if (threadIdx.x == kSSThreads - 1 && b.normal) sh.s = sum_of(b, m);
-            pos = len;
-        } else {
-            if (exit_at == at) {
-                sh.s = __dadd_rn(b.normal ? sum_of(b, before) : s, (double)vx);
-                sh.alone |= 1u << (at / kSSThreads);
-            }
-            __syncthreads();
-            if (warp == 0) {
-                double t = sh.s;
-                int p = at + 1;
-                unsigned alone = 0;
-                warp_windows(in, base, len, t, p, alone);
-                if (lane == 0) {
-                    sh.s = t;
-                    sh.pos = p;
-                    sh.alone |= alone;
-                }
-            }
-            __syncthreads();
-            pos = sh.pos;
-        }
-        __syncthreads();   // sh.s and sh.pos are read before the next scan writes them
-    }
-}
-
-// A thread's kSSPer consecutive values of the block at `base`: the bits of the present ones.
-template <typename T>
-__device__ __forceinline__ unsigned load_values(const SumIn<T>& in, size_t base, T (&v)[kSSPer]) {
-    unsigned has = 0;
-    const size_t i0 = base + (size_t)threadIdx.x * kSSPer;
-#pragma unroll
-    for (int t = 0; t < kSSPer; ++t) {
-        v[t] = 0;
-        if (value_at(in, i0 + t, &v[t])) has |= 1u << t;
-    }
-    return has;
-}
-
 template <typename T>
 __device__ __forceinline__ void finish_sum(const SumIn<T>& in, double s, long long whole, long long reduced,
                                            long long alone) {
@@ -529,8 +157,7 @@ __device__ __forceinline__ void finish_sum(const SumIn<T>& in, double s, long lo
     }
 }
 
-// Sums of few blocks, a CTA each, from the first value to the last; the next block's values are loaded
-// while this one's are added.
+// Sums of few blocks, a CTA each, from the first value to the last.
 template <typename T>
 __global__ void __launch_bounds__(kSSThreads) k_ss_direct(SumJobs<T> jobs) {
     __shared__ CtaSum sh;
@@ -538,12 +165,8 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_direct(SumJobs<T> jobs) {
     if (threadIdx.x == 0) sh.s = in.init ? *in.init : 0.0;
     __syncthreads();
     long long whole = 0, reduced = 0, alone = 0;
-    T v[kSSPer];
-    unsigned has = load_values(in, 0, v);
     for (size_t base = 0; base < in.n; base += kSSBlock) {
-        T nv[kSSPer];
-        const unsigned nhas = load_values(in, base + kSSBlock, nv);
-        cta_advance(in, base, (int)(in.n - base < (size_t)kSSBlock ? in.n - base : (size_t)kSSBlock), v, has, sh);
+        cta_advance(in, base, (int)(in.n - base < (size_t)kSSBlock ? in.n - base : (size_t)kSSBlock), sh);
         if (threadIdx.x == 0) {
             const int a = __popc(sh.alone);
             whole += a == 0;
@@ -551,9 +174,6 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_direct(SumJobs<T> jobs) {
             alone += a;
         }
         __syncthreads();   // sh.alone is read before the next block clears it
-#pragma unroll
-        for (int t = 0; t < kSSPer; ++t) v[t] = nv[t];
-        has = nhas;
     }
     if (threadIdx.x == 0) finish_sum(in, sh.s, whole, reduced, alone);
 }
@@ -614,7 +234,7 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_walks(SumJobs<T> jobs, const 
 #pragma unroll
     for (int t = 0; t < kSSPer; ++t)
         if (has & (1u << t)) {
-            if (v[t] != (T)0) lw.w.zero = 0;
+            lw.w.zero = 0;
             if (sp >= 0) lw.add(step_of(v[t], sp & 0x7FF, sp >> 11));
         }
     Walk total = cta_walk(lw.w, sh_warps);
@@ -645,7 +265,7 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_chain(SumJobs<T> jobs, const 
                 Walk w = walk_identity();
                 if (k < blocks) w = walks[in.first_block + k];
                 const Binade b = binade_of(s);
-                const bool zero = k < blocks && w.zero && __double_as_longlong(s) != (long long)(1ULL << 63);
+                const bool zero = k < blocks && w.zero;
                 bool ok = zero || (k < blocks && b.normal && !w.fail && w.spec == (b.ef | (b.neg << 11)));
                 Run mine = run_identity();
                 if (ok && !zero) {
@@ -683,9 +303,7 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_chain(SumJobs<T> jobs, const 
         j = sh_block;
         if (j >= blocks) break;
         const size_t base = (size_t)j * kSSBlock;
-        T v[kSSPer];
-        const unsigned has = load_values(in, base, v);
-        cta_advance(in, base, (int)(in.n - base < (size_t)kSSBlock ? in.n - base : (size_t)kSSBlock), v, has, sh);
+        cta_advance(in, base, (int)(in.n - base < (size_t)kSSBlock ? in.n - base : (size_t)kSSBlock), sh);
         if (threadIdx.x == 0) {
             const int a = __popc(sh.alone);
             whole += a == 0;
