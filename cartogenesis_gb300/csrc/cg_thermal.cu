@@ -2,15 +2,26 @@
 //
 // One sweep is two passes in the reference: every cell's give rate from its 8 neighbours, then
 // every cell's new height from its neighbours' give rates. Here one CTA owns a 64 x 32 tile and
-// loads it with a halo of 2K cells into shared memory; it runs K sweeps there (K = 2, or 1 for an
-// odd remainder), each sweep's region shrinking by two cells a side (one for the give pass, one for
-// the move pass), and writes the tile back once. The passes are compute-bound, and the halo's
-// redundant work grows with K while the memory traffic it saves is small next to the compute, so
-// K stays at 2: global traffic is one read and one write per two sweeps.
+// loads it with a halo of 4 cells into shared memory; it runs two sweeps there (or one, for an odd
+// remainder), each sweep's region shrinking by two cells a side (one for the give pass, one for
+// the move pass), and writes the tile back once.
+//
+// The passes are bound by instruction issue, so they issue little for a cell at rest (most cells are, in
+// most sweeps) and share work between the passes: a cell gives only if it stands above its lowest
+// neighbour by more than the least limit, and that lowest is kept row by row as a 3 x 3 window slides
+// down a thread's column; the give pass also takes what the cell itself gives off its height, with the
+// falls it has at hand, so the move pass only adds what comes in and leaves a cell alone when no
+// neighbour gives. A thread takes a column of 8 to 10 rows, so that four runs of rows times the
+// region's columns are one step of the CTA's 288 threads (92% busy over the four passes) and the
+// window's two extra rows cost a fifth of the loads. The 384 launches of an 8192 x 4096 stage take 89.5
+// ms (113 with each pass running its whole rule on 4-row columns), 192 sweeps at 4096 x 2048 5.5 ms
+// (6.5). Queueing the active cells and running the rules on 32 of them at a time was slower (10.4 ms):
+// the queue's own instructions are as many as the rules'.
 //
 // The arithmetic per cell is the reference's, in the same neighbour order, in float, with no
-// fused multiply-add, so the result is bit-identical to ErosionStage.thermalSweep. Tiles away from
-// the poles take a path without the per-neighbour row checks; both paths compute the same values.
+// fused multiply-add, so the result is bit-identical to ErosionStage.thermalSweep. Rows off the grid
+// hold NaN, which no comparison of the rules lets through. Limits below zero (no preset has them) take
+// a plain per-cell form of the same rules.
 #include <cuda.h>
 
 #include <cmath>
@@ -24,20 +35,23 @@ namespace {
 
 constexpr int TX = 64;
 constexpr int TY = 32;
-constexpr int THREADS = 256;   // 32 x 8
 constexpr int KMAX = 2;
+constexpr int HALO = 2 * KMAX;
+constexpr int RW = TX + 2 * HALO;   // region width
+constexpr int RH = TY + 2 * HALO;   // region height
+constexpr int THREADS = 288;        // four runs of rows times up to 70 columns, a thread each
 
 struct ThermalArgs {
     float limit[8];
-    float lim0[8];   // max(limit, 0)
     float settled;
     float rate;
-    float min_lim0;  // the least of lim0
-    int plain;       // every limit >= 0 and settled >= 0: the shortcuts below are exact
+    float ew, ns, diag;   // the limits by neighbour kind
+    float least;          // the least of them
+    int plain;            // every limit >= 0 and settled >= 0: the forms below are exact
 };
 
 // Settled-tile skip (the reference's own skip, ErosionStage.kt:269-342, restated for fused launches).
-// A launch of K sweeps carries any change at most 2K cells, less than a tile's side, so a tile can
+// A launch carries any change at most 4 cells, less than a tile's side, so a tile can
 // change only if a cell of it or of one of its 8 neighbouring tiles changed in the previous launch.
 // `prev` holds those per-tile "changed" bits (null: compute every tile); each launch writes its own
 // into `cur`. A skipped tile is not even copied: the launches ping-pong between two buffers, and a
@@ -48,10 +62,9 @@ struct TileFlags {
 };
 
 // The region load by the tensor memory accelerator: one cp.async.bulk.tensor.2d per CTA of the
-// whole (TX + 2 HALO) x (TY + 2 HALO) region, rows off the grid filled with zeros by the copy
-// itself. Used for K = 2 (the region's first column, x0 = 64 bx - 4, is 16-byte aligned as TMA
-// requires) on tiles whose region does not wrap east-west; the two wrapping tile columns and the
-// odd single-sweep launch load by threads. `err` (device) is set when a copy's wait runs out, after
+// whole RW x RH region, rows off the grid filled with NaN by the copy itself. Used on tiles whose
+// region does not wrap east-west (its first column, 64 bx - 4, is 16-byte aligned as TMA requires); the
+// two wrapping tile columns load by threads. `err` (device) is set when a copy's wait runs out, after
 // which the CTA waits once more for its copy and leaves without computing; the host reports it.
 struct RegionLoad {
     CUtensorMap map;   // the source field, box = the region
@@ -77,209 +90,192 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, int tries) {
     return false;
 }
 
-// Per-cell rules, written without branches: the conditions become predicated adds in the
-// reference's neighbour order, so the sums round exactly as the reference's loop does.
-// Neighbours by name: E/W the same row, S/N the rows below/above, and the diagonals SE (+1,+1),
-// NE (+1,-1), SW (-1,+1), NW (-1,-1) as (column step, row step).
-struct Window {
-    float nw, n, ne, w, c, e, sw, s, se;   // the 3 x 3 block around a cell
+// Neighbours in the reference's order: E, W, S, N, then SE, NE, SW, NW.
+struct Around {
+    float v[8];
 };
+__device__ __forceinline__ float limit_of(const ThermalArgs& a, int n) { return n >= 4 ? a.diag : n >= 2 ? a.ns : a.ew; }
 
-// The give rate of a cell away from the poles with plain limits (every limit and the settled share
-// >= 0), the same bits as give_rate with fewer instructions:
-//  - a cell no drop of which exceeds the least max(limit, 0) gives nothing. Float subtraction is
-//    monotone, so c - min(neighbours) bounds every drop from above, and then the excess stays +0,
-//    which is not above the settled share (>= 0): the rate is +0, as the full rule returns;
-//  - the steepest drop as a running max: the reference keeps the larger of the two, and the heights
-//    are finite; the max may return -0 where the rule keeps +0, which changes neither the rate's
-//    products nor any sum (every sum starts at +0 and adds terms >= 0).
-__device__ __forceinline__ float give_rate_plain(const Window& v, const ThermalArgs& a) {
-    const float lowest = fminf(fminf(fminf(v.e, v.w), fminf(v.s, v.n)), fminf(fminf(v.se, v.ne), fminf(v.sw, v.nw)));
-    if (__fsub_rn(v.c, lowest) <= a.min_lim0) return 0.0f;
-    const float nb[8] = {v.e, v.w, v.s, v.n, v.se, v.ne, v.sw, v.nw};
-    float excess = 0.0f, steepest = 0.0f;
+// The give pass's rule on a cell of height c that stands above its lowest neighbour by more than the least
+// limit (ErosionStage.kt:283-311 and the giving half of 313-340), limits >= 0: returns its give rate and
+// takes what it gives off c. A fall counts when it is above its limit; a fall at or below it enters the
+// sums as +0, which changes no bit of a sum that starts at +0 and gains only terms >= 0. The steepest
+// fall is that to the lowest neighbour (float subtraction is monotone).
+__device__ __forceinline__ float give(float& c, const Around& nb, float lowest, const ThermalArgs& a) {
+    float over[8];
+    float excess = 0.0f;
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
-        const float drop = __fsub_rn(v.c, nb[n]);
-        steepest = fmaxf(steepest, drop);
-        const float over = __fsub_rn(drop, a.limit[n]);
-        if (drop > a.lim0[n]) excess = __fadd_rn(excess, over);
+        over[n] = fmaxf(__fsub_rn(__fsub_rn(c, nb.v[n]), limit_of(a, n)), 0.0f);
+        excess = __fadd_rn(excess, over[n]);
     }
-    float g = 0.0f;
-    if (excess > a.settled) {
-        const float p = __fmul_rn(a.rate, excess), q = __fmul_rn(steepest, 0.5f);
-        g = __fdiv_rn(p <= q ? p : q, excess);
-    }
-    return g;
+    if (!(excess > a.settled)) return 0.0f;
+    const float p = __fmul_rn(a.rate, excess), q = __fmul_rn(__fsub_rn(c, lowest), 0.5f);
+    const float rate = __fdiv_rn(p <= q ? p : q, excess);
+    float given = 0.0f;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) given = __fadd_rn(given, __fmul_rn(rate, over[n]));
+    c = __fsub_rn(c, given);
+    return rate;
 }
 
-// The new height of a cell away from the poles with plain limits, the same bits as `moved`: with a
-// limit >= 0 a drop that moves material either way has magnitude |incoming|, so one absolute value
-// replaces the select of the sign; a term is added as +0 where the rule skips it (sums start at +0
-// and gain only terms >= 0, so adding +0 changes no bit).
-__device__ __forceinline__ float moved_plain(const Window& v, const Window& g, const ThermalArgs& a) {
-    const float nb[8] = {v.e, v.w, v.s, v.n, v.se, v.ne, v.sw, v.nw};
-    const float gn[8] = {g.e, g.w, g.s, g.n, g.se, g.ne, g.sw, g.nw};
-    float received = 0.0f, given = 0.0f;
+// The move pass's rule on a cell of height c: what the neighbours that stand above it by more than their
+// limits give it (ErosionStage.kt:313-340).
+__device__ __forceinline__ float received(float c, const Around& nb, const Around& g, const ThermalArgs& a) {
+    float sum = 0.0f;
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
-        const float limit = a.limit[n];
-        const float incoming = __fsub_rn(nb[n], v.c);
-        const bool in = incoming > limit;
-        const bool out = incoming < -limit;
-        const float p = __fmul_rn(in ? gn[n] : g.c, __fsub_rn(fabsf(incoming), limit));
-        received = __fadd_rn(received, in ? p : 0.0f);
-        given = __fadd_rn(given, out ? p : 0.0f);
+        const float over = __fsub_rn(__fsub_rn(nb.v[n], c), limit_of(a, n));
+        const float p = __fmul_rn(g.v[n], over);
+        if (over > 0.0f) sum = __fadd_rn(sum, p);
     }
-    return __fadd_rn(__fsub_rn(v.c, given), received);
+    return sum;
 }
 
-// The give rate of a cell (ErosionStage.kt:283-311). `lim0[n]` is max(limit, 0): a drop counts
-// towards the excess when it is positive and above the limit. `has_s` / `has_n`: the rows below /
-// above exist (false only at the poles).
-__device__ __forceinline__ float give_rate(const Window& v, bool has_s, bool has_n, const ThermalArgs& a) {
-    const float nb[8] = {v.e, v.w, v.s, v.n, v.se, v.ne, v.sw, v.nw};
+// This thread's column and run of rows [row0, row1) of the region's rows and columns [M, R - M).
+struct Run {
+    int col, row0, row1;
+};
+template <int M>
+__device__ __forceinline__ bool run_of(Run& r) {
+    constexpr int COLS = RW - 2 * M, PER = (RH - 2 * M + 3) / 4;
+    static_assert(4 * COLS <= THREADS, "a thread takes one run");
+    const int part = (int)threadIdx.x / COLS;
+    r.col = M + (int)threadIdx.x - part * COLS;
+    r.row0 = M + part * PER;
+    r.row1 = min(r.row0 + PER, RH - M);
+    return part < 4;
+}
+// A change at this row counts for the tile's flag where the column and row are the tile's own.
+__device__ __forceinline__ bool own_col(int col) { return col >= HALO && col < HALO + TX; }
+__device__ __forceinline__ bool own_row(int row) { return row >= HALO && row < HALO + TY; }
+
+// The give pass from h: rates into g, what is left of the heights into left. The left height is
+// (c - given) + 0, since the reference adds what a cell receives, if only +0. Returns whether any of the
+// thread's cells gives.
+template <int M>
+__device__ __forceinline__ bool give_pass(const float* __restrict__ h, float* __restrict__ left, float* __restrict__ g,
+                                          const ThermalArgs& a, bool& changed) {
+    Run r;
+    if (!run_of<M>(r)) return false;
+    bool any = false;
+    unsigned moved = 0;
+    const bool own = own_col(r.col);
+    const float* p = h + (r.row0 - 1) * RW + r.col;
+    float nw = p[-1], n = p[0], ne = p[1], w = p[RW - 1], c = p[RW], e = p[RW + 1];
+    float top = fminf(fminf(nw, n), ne), mid = fminf(fminf(w, c), e);
+#pragma unroll 3
+    for (int row = r.row0; row < r.row1; ++row) {
+        const int i = row * RW + r.col;
+        const float sw = h[i + RW - 1], s = h[i + RW], se = h[i + RW + 1];
+        const float bot = fminf(fminf(sw, s), se);
+        const float lowest = fminf(fminf(top, mid), bot);
+        float rate = 0.0f, v = c;
+        if (__fsub_rn(c, lowest) > a.least) rate = give(v, Around{{e, w, s, n, se, ne, sw, nw}}, lowest, a);
+        v = __fadd_rn(v, 0.0f);
+        g[i] = rate;
+        left[i] = v;
+        any |= rate != 0.0f;
+        if (own_row(row)) moved |= __float_as_uint(v) ^ __float_as_uint(c);
+        nw = w, n = c, ne = e;
+        w = sw, c = s, e = se;
+        top = mid, mid = bot;
+    }
+    if (own && moved) changed = true;
+    return any;
+}
+
+// The move pass: what each cell receives, read from h and g, onto left.
+template <int M>
+__device__ __forceinline__ void move_pass(const float* __restrict__ h, float* __restrict__ left, const float* __restrict__ g,
+                                          const ThermalArgs& a, bool& changed) {
+    Run r;
+    if (!run_of<M>(r)) return;
+    unsigned moved = 0;
+    const bool own = own_col(r.col);
+    const float* p = h + (r.row0 - 1) * RW + r.col;
+    const float* q = g + (r.row0 - 1) * RW + r.col;
+    float nw = p[-1], n = p[0], ne = p[1], w = p[RW - 1], c = p[RW], e = p[RW + 1];
+    float gnw = q[-1], gn = q[0], gne = q[1], gw = q[RW - 1], gc = q[RW], ge = q[RW + 1];
+    unsigned top = __float_as_uint(gnw) | __float_as_uint(gn) | __float_as_uint(gne);
+#pragma unroll 3
+    for (int row = r.row0; row < r.row1; ++row) {
+        const int i = row * RW + r.col;
+        const float sw = h[i + RW - 1], s = h[i + RW], se = h[i + RW + 1];
+        const float gsw = g[i + RW - 1], gs = g[i + RW], gse = g[i + RW + 1];
+        const unsigned sides = __float_as_uint(gw) | __float_as_uint(ge);
+        const unsigned bot = __float_as_uint(gsw) | __float_as_uint(gs) | __float_as_uint(gse);
+        if (top | sides | bot) {   // a neighbour gives
+            const float v = __fadd_rn(left[i], received(c, Around{{e, w, s, n, se, ne, sw, nw}},
+                                                        Around{{ge, gw, gs, gn, gse, gne, gsw, gnw}}, a));
+            left[i] = v;
+            if (own_row(row)) moved |= __float_as_uint(v) ^ __float_as_uint(c);
+        }
+        top = sides | __float_as_uint(gc);
+        nw = w, n = c, ne = e;
+        w = sw, c = s, e = se;
+        gnw = gw, gn = gc, gne = ge;
+        gw = gsw, gc = gs, ge = gse;
+    }
+    if (own && moved) changed = true;
+}
+
+// The reference's rules on one cell of the region for any limits: rows off the grid are told apart by
+// `has_s` / `has_n` (the rows below and above exist).
+__device__ float give_rate(const float* h, int i, bool has_s, bool has_n, const ThermalArgs& a) {
+    const int off[8] = {1, -1, RW, -RW, RW + 1, -RW + 1, RW - 1, -RW - 1};
     const bool ok[8] = {true, true, has_s, has_n, has_s, has_n, has_s, has_n};
     float excess = 0.0f, steepest = 0.0f;
-#pragma unroll
     for (int n = 0; n < 8; ++n) {
-        const float drop = __fsub_rn(v.c, nb[n]);
-        if (ok[n] && drop > steepest) steepest = drop;
-        const float over = __fsub_rn(drop, a.limit[n]);
-        if (ok[n] && drop > a.lim0[n]) excess = __fadd_rn(excess, over);
+        if (!ok[n]) continue;
+        const float drop = __fsub_rn(h[i], h[i + off[n]]);
+        if (drop > steepest) steepest = drop;
+        if (drop > 0.0f && drop > a.limit[n]) excess = __fadd_rn(excess, __fsub_rn(drop, a.limit[n]));
     }
-    float g = 0.0f;
-    if (excess > a.settled) {
-        const float p = __fmul_rn(a.rate, excess), q = __fmul_rn(steepest, 0.5f);
-        g = __fdiv_rn(p <= q ? p : q, excess);
-    }
-    return g;
+    if (!(excess > a.settled)) return 0.0f;
+    const float p = __fmul_rn(a.rate, excess), q = __fmul_rn(steepest, 0.5f);
+    return __fdiv_rn(p <= q ? p : q, excess);
 }
 
-// The new height of a cell from its neighbours' give rates (ErosionStage.kt:313-340).
-__device__ __forceinline__ float moved(const Window& v, const Window& g, bool has_s, bool has_n,
-                                       const ThermalArgs& a) {
-    const float nb[8] = {v.e, v.w, v.s, v.n, v.se, v.ne, v.sw, v.nw};
-    const float gn[8] = {g.e, g.w, g.s, g.n, g.se, g.ne, g.sw, g.nw};
+__device__ float moved(const float* h, const float* g, int i, bool has_s, bool has_n, const ThermalArgs& a) {
+    const int off[8] = {1, -1, RW, -RW, RW + 1, -RW + 1, RW - 1, -RW - 1};
     const bool ok[8] = {true, true, has_s, has_n, has_s, has_n, has_s, has_n};
     float received = 0.0f, given = 0.0f;
-#pragma unroll
     for (int n = 0; n < 8; ++n) {
-        const float limit = a.limit[n];
-        const float incoming = __fsub_rn(nb[n], v.c);
-        const bool in = incoming > limit;
-        const bool out = !in && -incoming > limit;
-        // One product serves both branches: (incoming - limit) * g_n coming in, (-incoming - limit) * g_c
-        // going out; the sums take it only under their own condition, in the reference's order.
-        const float p = __fmul_rn(in ? gn[n] : g.c, __fsub_rn(in ? incoming : -incoming, limit));
-        if (ok[n] && in) received = __fadd_rn(received, p);
-        if (ok[n] && out) given = __fadd_rn(given, p);
+        if (!ok[n]) continue;
+        const float incoming = __fsub_rn(h[i + off[n]], h[i]);
+        if (incoming > a.limit[n])
+            received = __fadd_rn(received, __fmul_rn(g[i + off[n]], __fsub_rn(incoming, a.limit[n])));
+        else if (-incoming > a.limit[n])
+            given = __fadd_rn(given, __fmul_rn(g[i], __fsub_rn(-incoming, a.limit[n])));
     }
-    return __fadd_rn(__fsub_rn(v.c, given), received);
+    return __fadd_rn(__fsub_rn(h[i], given), received);
 }
 
-// One pass over the region's rows [M, RH - M) and columns [M, RW - M). A thread takes a column
-// segment of up to SEG rows and slides a 3 x 3 window down it, so each cell costs three
-// shared-memory loads per field instead of nine. Work items are (segment, column), columns
-// fastest, so a warp's loads are consecutive words. MOVE: the move pass (reads gv, writes dst),
-// else the give pass (writes gv).
-template <int RW, int RH, int M, bool MOVE, bool EDGE>
-__device__ __forceinline__ void pass(const float* __restrict__ hs, float* __restrict__ gv, float* __restrict__ dst,
-                                     int y0, int H, const ThermalArgs& a, int halo, bool& changed) {
-    constexpr int SEG = 4;
-    constexpr int COLS = RW - 2 * M, ROWS = RH - 2 * M;
-    constexpr int SEGS = (ROWS + SEG - 1) / SEG;
-    constexpr int ITEMS = COLS * SEGS;
-    for (int item = threadIdx.x; item < ITEMS; item += THREADS) {
-        const int col = M + item % COLS;
-        const int r0 = M + (item / COLS) * SEG;
-        const int r1 = r0 + SEG < RH - M ? r0 + SEG : RH - M;
-        const float* p = hs + (r0 - 1) * RW + col;
-        Window v;
-        v.nw = p[-1], v.n = p[0], v.ne = p[1];
-        v.w = p[RW - 1], v.c = p[RW], v.e = p[RW + 1];
-        Window g{};
-        unsigned or_top = 0, or_mid = 0;   // bitwise OR of the give rates' bits, per window row
-        if (MOVE) {
-            const float* q = gv + (r0 - 1) * RW + col;
-            g.nw = q[-1], g.n = q[0], g.ne = q[1];
-            g.w = q[RW - 1], g.c = q[RW], g.e = q[RW + 1];
-            or_top = __float_as_uint(g.nw) | __float_as_uint(g.n) | __float_as_uint(g.ne);
-            or_mid = __float_as_uint(g.w) | __float_as_uint(g.c) | __float_as_uint(g.e);
-        }
-#pragma unroll
-        for (int k = 0; k < SEG; ++k) {
-            const int ry = r0 + k;
-            if (ry >= r1) break;
-            const float* below = hs + (ry + 1) * RW + col;
-            v.sw = below[-1], v.s = below[0], v.se = below[1];
-            unsigned or_bot = 0;
-            if (MOVE) {
-                const float* gb = gv + (ry + 1) * RW + col;
-                g.sw = gb[-1], g.s = gb[0], g.se = gb[1];
-                or_bot = __float_as_uint(g.sw) | __float_as_uint(g.s) | __float_as_uint(g.se);
-            }
-            const int gy = y0 + ry;
-            const bool on = !EDGE || (gy >= 0 && gy < H);
-            const bool has_s = !EDGE || gy + 1 < H;
-            const bool has_n = !EDGE || gy - 1 >= 0;
-            if (on) {
-                if (MOVE) {
-                    // Every give rate around the cell +0: each product the rule could add is +0, so the
-                    // sums stay +0 and the cell moves to (h - 0) + 0. Rows off the grid (EDGE) are
-                    // left to the full rule.
-                    const bool still = !EDGE && (or_top | or_mid | or_bot) == 0u;
-                    const float nv = still ? __fadd_rn(__fsub_rn(v.c, 0.0f), 0.0f)
-                                           : (!EDGE && a.plain) ? moved_plain(v, g, a) : moved(v, g, has_s, has_n, a);
-                    dst[ry * RW + col] = nv;
-                    // A cell of the tile itself that moved (in any sweep) marks the tile as changed.
-                    if (__float_as_uint(nv) != __float_as_uint(v.c) && ry >= halo && ry < RH - halo &&
-                        col >= halo && col < RW - halo)
-                        changed = true;
-                } else {
-                    gv[ry * RW + col] = (!EDGE && a.plain) ? give_rate_plain(v, a) : give_rate(v, has_s, has_n, a);
-                }
-            }
-            v.nw = v.w, v.n = v.c, v.ne = v.e;
-            v.w = v.sw, v.c = v.s, v.e = v.se;
-            if (MOVE) {
-                g.nw = g.w, g.n = g.c, g.ne = g.e;
-                g.w = g.sw, g.c = g.s, g.e = g.se;
-                or_top = or_mid;
-                or_mid = or_bot;
-            }
-        }
+// One sweep by those rules over rows and columns [M + 1, R - M - 1) from h into to.
+template <int M>
+__device__ void any_sweep(const float* h, float* to, float* g, int y0, int H, const ThermalArgs& a, bool& changed) {
+    for (int i = threadIdx.x; i < RW * RH; i += THREADS) {
+        const int row = i / RW, col = i % RW, y = y0 + row;
+        if (row < M || row >= RH - M || col < M || col >= RW - M || y < 0 || y >= H) continue;
+        g[i] = give_rate(h, i, y + 1 < H, y > 0, a);
     }
-}
-
-// K sweeps on the region in shared memory: hs holds the heights and ends with the result
-// (swapping with hn each sweep); the region's valid part shrinks by two cells a side per sweep.
-template <int RW, int RH, int K, bool EDGE>
-__device__ __forceinline__ float* sweeps(float* hs, float* hn, float* gv, int y0, int H, const ThermalArgs& a,
-                                         bool& changed) {
-    constexpr int HALO = 2 * K;
-    pass<RW, RH, 1, false, EDGE>(hs, gv, nullptr, y0, H, a, HALO, changed);
     __syncthreads();
-    pass<RW, RH, 2, true, EDGE>(hs, gv, hn, y0, H, a, HALO, changed);
-    __syncthreads();
-    if constexpr (K == 2) {
-        pass<RW, RH, 3, false, EDGE>(hn, gv, nullptr, y0, H, a, HALO, changed);
-        __syncthreads();
-        pass<RW, RH, 4, true, EDGE>(hn, gv, hs, y0, H, a, HALO, changed);
-        __syncthreads();
-        return hs;
-    } else {
-        return hn;
+    for (int i = threadIdx.x; i < RW * RH; i += THREADS) {
+        const int row = i / RW, col = i % RW, y = y0 + row;
+        if (row <= M || row >= RH - M - 1 || col <= M || col >= RW - M - 1 || y < 0 || y >= H) continue;
+        to[i] = moved(h, g, i, y + 1 < H, y > 0, a);
+        if (__float_as_uint(to[i]) != __float_as_uint(h[i]) && row >= HALO && row < HALO + TY && col >= HALO &&
+            col < HALO + TX)
+            changed = true;
     }
+    __syncthreads();
 }
 
-template <int K>
-__global__ void __launch_bounds__(THREADS, 6) thermal_sweeps_kernel(const float* __restrict__ in, float* __restrict__ out,
-                                                                 int W, int H, ThermalArgs a, TileFlags fl,
-                                                                 const __grid_constant__ RegionLoad rl) {
-    constexpr int HALO = 2 * K;
-    constexpr int RW = TX + 2 * HALO;   // region width
-    constexpr int RH = TY + 2 * HALO;   // region height
+// `k` sweeps (1 or 2) of the field `in` into `out`, a CTA a tile.
+__global__ void __launch_bounds__(THREADS, 5) thermal_sweeps_kernel(const float* __restrict__ in, float* __restrict__ out,
+                                                                    int W, int H, int k, ThermalArgs a, TileFlags fl,
+                                                                    const __grid_constant__ RegionLoad rl) {
     __shared__ __align__(128) float sm_a[RW * RH];
     __shared__ __align__(16) float sm_b[RW * RH], sm_g[RW * RH];
     __shared__ __align__(8) unsigned long long bar;
@@ -303,18 +299,19 @@ __global__ void __launch_bounds__(THREADS, 6) thermal_sweeps_kernel(const float*
 
     const int x0 = blockIdx.x * TX - HALO;
     const int y0 = blockIdx.y * TY - HALO;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    if (K == 2 && rl.on && x0 >= 0 && x0 + RW <= W) {
-        const uint32_t b = smem_addr(&bar);
-        if (threadIdx.x == 0) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(RW * RH * 4) : "memory");
-            asm volatile(
-                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                ::"r"(smem_addr(sm_a)), "l"(&rl.map), "r"(x0), "r"(y0), "r"(b)
-                : "memory");
-        }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool tma = rl.on && x0 >= 0 && x0 + RW <= W;
+    const uint32_t b = smem_addr(&bar);
+    if (tma && threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(RW * RH * 4) : "memory");
+        asm volatile(
+            "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+            ::"r"(smem_addr(sm_a)), "l"(&rl.map), "r"(x0), "r"(y0), "r"(b)
+            : "memory");
+    }
+    if (tma) {
         __syncthreads();
         if (!mbar_wait(b, 1 << 22)) {
             // The copy did not land: record it, give it one more bounded wait, and leave.
@@ -326,42 +323,59 @@ __global__ void __launch_bounds__(THREADS, 6) thermal_sweeps_kernel(const float*
             return;
         }
     } else {
-        for (int ry = ty; ry < RH; ry += 8) {
+        for (int ry = warp; ry < RH; ry += THREADS / 32) {
             const int gy = y0 + ry;
             const bool valid = gy >= 0 && gy < H;
             const float* rowp = in + (size_t)(valid ? gy : 0) * W;
-            for (int rx = tx; rx < RW; rx += 32) sm_a[ry * RW + rx] = valid ? rowp[wrap_col(x0 + rx, W)] : 0.0f;
+            for (int rx = lane; rx < RW; rx += 32)
+                sm_a[ry * RW + rx] = valid ? rowp[wrap_col(x0 + rx, W)] : __int_as_float(0x7FFFFFFF);
         }
     }
     __syncthreads();
 
-    // Tiles whose region lies inside the grid's rows take the path without pole checks.
-    const bool edge = y0 < 0 || y0 + RH > H;
     bool moved_any = false;
-    const float* res = edge ? sweeps<RW, RH, K, true>(sm_a, sm_b, sm_g, y0, H, a, moved_any)
-                            : sweeps<RW, RH, K, false>(sm_a, sm_b, sm_g, y0, H, a, moved_any);
-
-    for (int yy = ty; yy < TY; yy += 8) {
-        const int gy = blockIdx.y * TY + yy;
-        if (gy >= H) continue;
-        for (int xx = tx; xx < TX; xx += 32) {
-            const int gx = blockIdx.x * TX + xx;
-            if (gx >= W) continue;
-            out[(size_t)gy * W + gx] = res[(yy + HALO) * RW + xx + HALO];
+    const float* res = sm_b;
+    if (a.plain) {
+        // A region in which no cell gives has nothing to move in the second sweep either.
+        if (__syncthreads_or(give_pass<1>(sm_a, sm_b, sm_g, a, moved_any))) {
+            move_pass<2>(sm_a, sm_b, sm_g, a, moved_any);
+            __syncthreads();
+            if (k == 2) {
+                if (__syncthreads_or(give_pass<3>(sm_b, sm_a, sm_g, a, moved_any)))
+                    move_pass<4>(sm_b, sm_a, sm_g, a, moved_any);
+                res = sm_a;
+            }
+        }
+    } else {
+        any_sweep<1>(sm_a, sm_b, sm_g, y0, H, a, moved_any);
+        if (k == 2) {
+            any_sweep<3>(sm_b, sm_a, sm_g, y0, H, a, moved_any);
+            res = sm_a;
         }
     }
-    if (fl.cur) {
-        const int changed = __syncthreads_or(moved_any);
-        if (threadIdx.x == 0) fl.cur[tile] = changed ? 1 : 0;
+    const int changed = __syncthreads_or(moved_any);   // the tile's result is in place, too
+    if (fl.cur && threadIdx.x == 0) fl.cur[tile] = changed ? 1 : 0;
+
+    if (W >= TX && (((uintptr_t)out) & 15) == 0) {
+        for (int i = threadIdx.x; i < TY * TX / 4; i += THREADS) {
+            const int yy = i / (TX / 4), xx = 4 * (i % (TX / 4)), gy = blockIdx.y * TY + yy;
+            if (gy < H)
+                *reinterpret_cast<float4*>(out + (size_t)gy * W + blockIdx.x * TX + xx) =
+                    *reinterpret_cast<const float4*>(res + (yy + HALO) * RW + xx + HALO);
+        }
+    } else {
+        for (int i = threadIdx.x; i < TY * TX; i += THREADS) {
+            const int yy = i / TX, xx = i % TX, gy = blockIdx.y * TY + yy, gx = blockIdx.x * TX + xx;
+            if (gy < H && gx < W) out[(size_t)gy * W + gx] = res[(yy + HALO) * RW + xx + HALO];
+        }
     }
 }
 
-template <int K>
-cudaError_t launch(const float* in, float* out, int W, int H, const ThermalArgs& a, cudaStream_t st,
+cudaError_t launch(const float* in, float* out, int W, int H, int k, const ThermalArgs& a, cudaStream_t st,
                    TileFlags fl = TileFlags{nullptr, nullptr}, const RegionLoad* rl = nullptr) {
     dim3 grid((W + TX - 1) / TX, (H + TY - 1) / TY);
     static const RegionLoad none{};
-    thermal_sweeps_kernel<K><<<grid, THREADS, 0, st>>>(in, out, W, H, a, fl, rl ? *rl : none);
+    thermal_sweeps_kernel<<<grid, THREADS, 0, st>>>(in, out, W, H, k, a, fl, rl ? *rl : none);
     return cudaGetLastError();
 }
 
@@ -384,12 +398,11 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// The region-load map of a field for K = 2 launches: the whole W x H field, a box of the region.
+// The region-load map of a field: the whole W x H field, a box of the region.
 // Off (threads load every tile) where the driver has no encoder or the grid is too narrow.
 RegionLoad region_load_of(const float* field, int W, int H, int* err) {
     RegionLoad rl{};
     rl.err = err;
-    constexpr int RW = TX + 8, RH = TY + 8;
     EncodeTiledFn enc = encode_tiled();
     if (!enc || !err || W < 2 * RW || (((uintptr_t)field) & 15) != 0) return rl;
     const cuuint64_t dims[2] = {(cuuint64_t)W, (cuuint64_t)H};
@@ -398,7 +411,7 @@ RegionLoad region_load_of(const float* field, int W, int H, int* err) {
     const cuuint32_t estride[2] = {1, 1};
     if (enc(&rl.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)field, dims, strides, box, estride,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NAN_REQUEST_ZERO_FMA) == CUDA_SUCCESS)
         rl.on = 1;
     return rl;
 }
@@ -406,13 +419,14 @@ RegionLoad region_load_of(const float* field, int W, int H, int* err) {
 ThermalArgs args_of(const ThermalLaunch& t) {
     ThermalArgs a;
     a.plain = t.settled >= 0.0f;
-    a.min_lim0 = 3.402823466e+38f;
     for (int n = 0; n < 8; ++n) {
         a.limit[n] = t.limit[n];
-        a.lim0[n] = t.limit[n] > 0.0f ? t.limit[n] : 0.0f;
-        a.min_lim0 = std::fmin(a.min_lim0, a.lim0[n]);
         if (!(t.limit[n] >= 0.0f)) a.plain = 0;
     }
+    a.ew = t.limit[0];
+    a.ns = t.limit[2];
+    a.diag = t.limit[4];
+    a.least = std::fmin(std::fmin(a.ew, a.ns), a.diag);
     a.settled = t.settled;
     a.rate = t.rate;
     return a;
@@ -440,8 +454,7 @@ int thermal_launches(int passes) {
 // One fused launch of k sweeps (k = thermal_step(...)) from src into dst on `stream`.
 cudaError_t thermal_launch(const float* src, float* dst, int W, int H, const ThermalLaunch& t, int k,
                            cudaStream_t stream) {
-    ThermalArgs a = args_of(t);
-    return k == 2 ? launch<2>(src, dst, W, H, a, stream) : launch<1>(src, dst, W, H, a, stream);
+    return launch(src, dst, W, H, k, args_of(t), stream);
 }
 
 // `passes` sweeps from d_a; the result lands in *result (d_a or d_b). Deterministic ping-pong.
@@ -464,8 +477,7 @@ cg_status thermal_sweeps_dev(cg_ctx* ctx, int W, int H, float* d_a, float* d_b, 
         const int k = thermal_step(passes);
         TileFlags fl{first ? nullptr : prev, cur};
         const RegionLoad* rl = &maps[src == d_a ? 0 : 1];
-        cudaError_t e = k == 2 ? launch<2>(src, dst, W, H, a, ctx->stream, fl, rl)
-                               : launch<1>(src, dst, W, H, a, ctx->stream, fl);
+        cudaError_t e = launch(src, dst, W, H, k, a, ctx->stream, fl, rl);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "thermal_sweeps_kernel", __FILE__, __LINE__);
         passes -= k;
         ctx->launches++;
