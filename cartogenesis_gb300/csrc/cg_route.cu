@@ -792,58 +792,107 @@ __global__ void __launch_bounds__(FT) k_flat_solve(FlatArgs a) {
 // pivots, ns / pivot and the run table sit in shared memory; the per-member constants (degree, the
 // member neighbours) and the potential x, which a thread reads only for its own members, stay in
 // global memory. The arithmetic per member and per run is that of k_flat_solve. A dot product is
-// each thread's partial sum in member order, then block_reduce2's fixed order, so its bits are fixed
+// each thread's partial sum in member order, then fold_partials' fixed order, so its bits are fixed
 // for a given CTA size.
 constexpr int MID_FLAT = 512;    // members at most for the 128-thread CTA
 constexpr int SM_BYTES_PER_MEMBER = 7 * 8 + 4;   // seven doubles and one run-table entry
 
-struct Sum2 {
-    __device__ double2 operator()(double2 a, double2 b) const { return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)); }
-};
-struct MinMax2 {
-    __device__ double2 operator()(double2 a, double2 b) const {
-        return make_double2(a.x < b.x ? a.x : b.x, a.y > b.y ? a.y : b.y);
-    }
+// On GB300 an FP64 warp instruction holds its partition's one FP64 unit for 64 cycles, whatever its lanes
+// or its dependences (measured: chains of additions, products and fused operations, one lane or 32, one
+// chain or four; a division 564 cycles, a reciprocal 353). So a CG iteration is as long as the FP64
+// instructions of its busiest warp, and the solvers below count those: weights of exactly 1 are not
+// multiplied by; a dot product's last stages run in one warp a value, side by side; the divisions are
+// taken by the warp that has the sum; the potential's update and the reciprocal that makes the next
+// division three operations run in the warps that wait for the column runs. Over an 8192 x 4096 stage's
+// rounds the CTA solver's launches went from 35.7 to 27.4 ms and the cluster solver's from 52.8 to 44.1
+// with these; what is left is mostly the longest run's chain, four FP64 instructions a member down and
+// two back up.
+
+struct DMin {
+    __device__ double operator()(double a, double b) const { return a < b ? a : b; }
 };
 
-// The CTA's combination of v (two values), returned to every thread. Every thread's partial goes to
-// shared memory; the first warp folds the FT / 32 partials of each lane in thread order, then a
-// butterfly over its lanes, and hands the result out. The FP64 pipe is the scarce resource: this
-// takes FT / 32 - 1 + 5 FP64 operations of one warp per value, where a butterfly in every warp
-// takes 5 in each. `buf` holds FT double2 and `out` one; the two barriers keep consecutive calls
-// apart.
+// x + 0.0 without the addition: x, but +0 for -0.
+__device__ __forceinline__ double plus_zero(double x) {
+    return __double_as_longlong(x) == (long long)(1ULL << 63) ? 0.0 : x;
+}
+
+// A thread's term added to its partial sum, the first one taken as 0 + x.
+__device__ __forceinline__ double partial_add(double sum, double x, bool first) {
+    return first ? plus_zero(x) : __dadd_rn(sum, x);
+}
+
+// One warp's combination of a CTA's FT partials in `buf`: each lane folds FT / 32 of them in thread order,
+// then a butterfly over the lanes. Every lane gets the result. FT / 32 - 1 + 5 FP64 instructions.
 template <int FT, class Op>
-__device__ __forceinline__ double2 block_reduce2(double2 v, Op op, double2* buf, double2* out) {
-    buf[threadIdx.x] = v;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double2 s = buf[threadIdx.x];
+__device__ __forceinline__ double fold_partials(const double* buf, Op op) {
+    const int lane = threadIdx.x & 31;
+    double s = buf[lane];
 #pragma unroll
-        for (int k = 1; k < FT / 32; ++k) s = op(s, buf[threadIdx.x + 32 * k]);
-        for (int o = 16; o > 0; o >>= 1) {
-            double2 t;
-            t.x = __shfl_xor_sync(0xFFFFFFFFu, s.x, o);
-            t.y = __shfl_xor_sync(0xFFFFFFFFu, s.y, o);
-            s = op(s, t);
-        }
-        if (threadIdx.x == 0) *out = s;
+    for (int k = 1; k < FT / 32; ++k) s = op(s, buf[lane + 32 * k]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = op(s, __shfl_xor_sync(0xFFFFFFFFu, s, o));
+    return s;
+}
+
+// One column run's solve (FlatRouting.ColumnRuns.solve, FlatRouting.kt:399-413): down the run with the
+// chain in registers, then back up; the next member's values are loaded ahead of the chain.
+template <bool UNITW>
+__device__ __forceinline__ void solve_run(const double* r, double* z, const double* piv, const double* rcp,
+                                          const double* coef, double ns, int first, int last) {
+    double v = div_by(plus_zero(r[first]), piv[first], rcp[first]);
+    z[first] = v;
+    double rn = 0.0, pn = 1.0, cn = 1.0;
+    if (first < last) rn = r[first + 1], pn = piv[first + 1], cn = rcp[first + 1];
+    for (int j = first + 1; j <= last; ++j) {
+        const double rj = rn, pj = pn, cj = cn;
+        if (j < last) rn = r[j + 1], pn = piv[j + 1], cn = rcp[j + 1];
+        v = div_by(__dadd_rn(rj, UNITW ? v : __dmul_rn(ns, v)), pj, cj);
+        z[j] = v;
     }
-    __syncthreads();
-    return *out;
+    double below = v, zn = 0.0, kn = 0.0;
+    if (first < last) zn = z[last - 1], kn = coef[last - 1];
+    for (int j = last - 1; j >= first; --j) {
+        const double zj = zn, kj = kn;
+        if (j > first) zn = z[j - 1], kn = coef[j - 1];
+        below = __dadd_rn(zj, __dmul_rn(kj, below));
+        z[j] = below;
+    }
+}
+
+// The runs' solves by the CTA's first threads, a run each, beside two pieces of work for the warps without
+// one: the potential's update x += step d (any warp may take any member), and 1 / rap for the division
+// by it after the dot products.
+template <int FT, bool UNITW>
+__device__ __forceinline__ void solve_runs_beside(const unsigned* s_run, int runs, const double* s_r, double* s_z,
+                                                  const double* s_piv, const double* s_rcp, const double* s_coef, double ns,
+                                                  double* x, const double* s_d, int members, double step, double rap,
+                                                  double* rcp_rap) {
+    const int busy = (min(runs, FT) + 31) / 32;                 // warps with runs
+    const int idle0 = busy < FT / 32 ? 32 * busy : 0;           // the first thread to update x
+    if ((int)threadIdx.x >= FT - 32) {
+        const double q = __drcp_rn(rap);
+        if ((threadIdx.x & 31) == 0) *rcp_rap = q;
+    }
+    for (int i = threadIdx.x; i < runs; i += FT)
+        solve_run<UNITW>(s_r, s_z, s_piv, s_rcp, s_coef, ns, (int)(s_run[i] & 0xFFFFu), (int)(s_run[i] >> 16));
+    if ((int)threadIdx.x >= idle0)
+        for (int k = (int)threadIdx.x - idle0; k < members; k += FT - idle0)
+            x[k] = __dadd_rn(x[k], __dmul_rn(step, s_d[k]));
 }
 
 __device__ __forceinline__ int nbr_lo(int v) { return (int)(short)(v & 0xFFFF); }
 __device__ __forceinline__ int nbr_hi(int v) { return v >> 16; }
 __device__ __forceinline__ int nbr_pack(int lo, int hi) { return (int)(((unsigned)lo & 0xFFFFu) | ((unsigned)hi << 16)); }
 
-template <int FT>
+template <int FT, bool UNITW>
 __global__ void __launch_bounds__(FT) k_flat_solve_sm(FlatArgs a, const int* __restrict__ list) {
     extern __shared__ double dyn[];
     __shared__ double shd[32];
     __shared__ float shf[32];
     __shared__ int shi[32];
-    __shared__ double2 red[FT];
-    __shared__ double2 red_out;
+    __shared__ double red[2][FT];
+    __shared__ double s_sum[2], s_quot[2], s_rcp_rap;
     __shared__ int s_nruns;
     const int f = list[blockIdx.x];
     const int base = a.off[f];
@@ -937,42 +986,38 @@ __global__ void __launch_bounds__(FT) k_flat_solve_sm(FlatArgs a, const int* __r
             s_coef[j] = __ddiv_rn(a.ns, p);
             s_rcp[j] = __ddiv_rn(1.0, p);
             if (j == last) break;
-            p = __dsub_rn(degree[j + 1], __ddiv_rn(__dmul_rn(a.ns, a.ns), p));
+            p = __dsub_rn(degree[j + 1], __ddiv_rn(UNITW ? 1.0 : __dmul_rn(a.ns, a.ns), p));
         }
     }
     __syncthreads();
 
-    // z = M^-1 r through the runs (FlatRouting.ColumnRuns.solve, FlatRouting.kt:399-413).
-    auto precondition = [&]() {
-        for (int i = threadIdx.x; i < runs; i += FT) {
-            const int first = (int)(s_run[i] & 0xFFFFu), last = (int)(s_run[i] >> 16);
-            double v = div_by(__dadd_rn(s_r[first], 0.0), s_piv[first], s_rcp[first]);
-            s_z[first] = v;
-            for (int j = first + 1; j <= last; ++j) {
-                v = div_by(__dadd_rn(s_r[j], __dmul_rn(a.ns, v)), s_piv[j], s_rcp[j]);
-                s_z[j] = v;
-            }
-            double below = v;
-            for (int j = last - 1; j >= first; --j) {
-                below = __dadd_rn(s_z[j], __dmul_rn(s_coef[j], below));
-                s_z[j] = below;
-            }
-        }
-    };
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double w8[8] = {a.diag, a.ns, a.diag, a.ew, a.ew, a.diag, a.ns, a.diag};   // stencil order
+    // The dot products r . r and r . z, a warp each.
+    auto norms = [&]() {
+        double nn = 0.0, na = 0.0;
+        for (int k = threadIdx.x; k < n; k += FT) {
+            const double rv = s_r[k];
+            nn = partial_add(nn, __dmul_rn(rv, rv), k == (int)threadIdx.x);
+            na = partial_add(na, __dmul_rn(rv, s_z[k]), k == (int)threadIdx.x);
+        }
+        red[0][threadIdx.x] = nn;
+        red[1][threadIdx.x] = na;
+        __syncthreads();
+    };
 
     // Preconditioned conjugate gradients (FlatRouting.kt:296-333).
-    precondition();
+    for (int i = threadIdx.x; i < runs; i += FT)
+        solve_run<UNITW>(s_r, s_z, s_piv, s_rcp, s_coef, a.ns, (int)(s_run[i] & 0xFFFFu), (int)(s_run[i] >> 16));
     __syncthreads();
-    double rn = 0.0, ra = 0.0;
-    for (int k = threadIdx.x; k < n; k += FT) {
-        const double rv = s_r[k], zv = s_z[k];
-        s_d[k] = zv;
-        rn = __dadd_rn(rn, __dmul_rn(rv, rv));
-        ra = __dadd_rn(ra, __dmul_rn(rv, zv));
+    for (int k = threadIdx.x; k < n; k += FT) s_d[k] = s_z[k];
+    norms();
+    if (warp < 2) {
+        const double v = fold_partials<FT>(red[warp], DAdd());
+        if (lane == 0) s_sum[warp] = v;
     }
-    double2 sums = block_reduce2<FT>(make_double2(rn, ra), Sum2(), red, &red_out);
-    double rnorm = sums.x, rap = sums.y;
+    __syncthreads();
+    double rnorm = s_sum[0], rap = s_sum[1];
     const double stop_at = __dmul_rn(__dmul_rn(rnorm, 1e-7), 1e-7);
     const int most = 64 + (int)(8.0 * sqrt((double)n));
     for (int it = 0; rnorm > stop_at && it < most; ++it) {
@@ -986,32 +1031,42 @@ __global__ void __launch_bounds__(FT) k_flat_solve_sm(FlatArgs a, const int* __r
             double sum = __dmul_rn(degree[k], dk);
 #pragma unroll
             for (int t = 0; t < 8; ++t)
-                if (l8[t] >= 0) sum = __dsub_rn(sum, __dmul_rn(w8[t], s_d[l8[t]]));
+                if (l8[t] >= 0) sum = __dsub_rn(sum, UNITW ? s_d[l8[t]] : __dmul_rn(w8[t], s_d[l8[t]]));
             s_ad[k] = sum;
-            e = __dadd_rn(e, __dmul_rn(dk, sum));
+            e = partial_add(e, __dmul_rn(dk, sum), k == (int)threadIdx.x);
         }
-        const double energy = block_reduce2<FT>(make_double2(e, 0.0), Sum2(), red, &red_out).x;
-        if (energy <= 0.0 || rap <= 0.0) break;
-        const double step = __ddiv_rn(rap, energy);
-        for (int k = threadIdx.x; k < n; k += FT) {
-            x[k] = __dadd_rn(x[k], __dmul_rn(step, s_d[k]));
-            s_r[k] = __dsub_rn(s_r[k], __dmul_rn(step, s_ad[k]));
+        red[0][threadIdx.x] = e;
+        __syncthreads();
+        if (warp == 0) {
+            const double energy = fold_partials<FT>(red[0], DAdd());
+            const double quot = __ddiv_rn(rap, energy);
+            if (lane == 0) {
+                s_sum[0] = energy;
+                s_quot[0] = quot;
+            }
         }
         __syncthreads();
-        precondition();
+        if (s_sum[0] <= 0.0 || rap <= 0.0) break;
+        const double step = s_quot[0];
+        for (int k = threadIdx.x; k < n; k += FT) s_r[k] = __dsub_rn(s_r[k], __dmul_rn(step, s_ad[k]));
         __syncthreads();
-        double nn = 0.0, na = 0.0;
-        for (int k = threadIdx.x; k < n; k += FT) {
-            const double rv = s_r[k];
-            nn = __dadd_rn(nn, __dmul_rn(rv, rv));
-            na = __dadd_rn(na, __dmul_rn(rv, s_z[k]));
+        solve_runs_beside<FT, UNITW>(s_run, runs, s_r, s_z, s_piv, s_rcp, s_coef, a.ns, x, s_d, n, step, rap, &s_rcp_rap);
+        __syncthreads();
+        norms();
+        if (warp < 2) {
+            const double v = fold_partials<FT>(red[warp], DAdd());
+            const double quot = warp == 1 ? div_by(v, rap, s_rcp_rap) : 0.0;
+            if (lane == 0) {
+                s_sum[warp] = v;
+                if (warp == 1) s_quot[1] = quot;
+            }
         }
-        sums = block_reduce2<FT>(make_double2(nn, na), Sum2(), red, &red_out);
-        const double improvement = __ddiv_rn(sums.y, rap);
+        __syncthreads();
+        const double improvement = s_quot[1];
+        rnorm = s_sum[0];
+        rap = s_sum[1];
         for (int k = threadIdx.x; k < n; k += FT) s_d[k] = __dadd_rn(s_z[k], __dmul_rn(improvement, s_d[k]));
         __syncthreads();
-        rnorm = sums.x;
-        rap = sums.y;
     }
     int positive = 1;
     double top = 0.0;
@@ -1043,30 +1098,34 @@ constexpr int CL_SMEM_MEMBERS = (227 * 1024 - 8192) / SM_BYTES_PER_MEMBER;   // 
 namespace cgc = cooperative_groups;
 
 
-// The CTA's combination of (u, v) (block_reduce2), sent to slot q of every CTA's `slots[par]`; after
-// the cluster barrier each CTA's first warp combines the CL slots in rank order and hands the result
-// to the CTA through shared memory (the FP64 pipe is the scarce resource: the other warps need not
-// repeat it). `par` alternates between calls: the next call's barrier keeps this call's readers
-// ahead of the call after it.
-template <class Op>
-__device__ double2 cluster_combine(double2 v, Op op, double2* warps, double2 (*slots)[CL], double2* result, int& par,
-                                   int q) {
-    const double2 cta = block_reduce2<CL_THREADS>(v, op, warps, result + 2);
-    if (threadIdx.x < CL) {
-        double2* dst = cgc::this_cluster().map_shared_rank(&slots[par][q], (int)threadIdx.x);
-        *dst = cta;
+// The cluster's combinations of up to two values, a warp each: warp v folds the CTA's partials in part[v],
+// its lanes send the result to slot q of every CTA's slots[par][v], and after the cluster barrier it
+// combines the CL slots in rank order. `then(v, sum)` runs in that warp before the results are handed to
+// the CTA through sum[v]. `par` alternates between calls: the next call's barrier keeps this call's
+// readers ahead of the call after it. Every thread of the cluster calls it.
+struct ClusterSums {
+    double part[2][CL_THREADS];
+    double slots[2][2][CL];
+    double sum[2], quot[2], rcp_rap;
+};
+template <int VALUES, class Op0, class Op1, class Then>
+__device__ __forceinline__ void cluster_combine(ClusterSums& c, int& par, int q, Op0 op0, Op1 op1, Then then) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();
+    if (warp < VALUES) {
+        const double v = warp == 0 ? fold_partials<CL_THREADS>(c.part[0], op0) : fold_partials<CL_THREADS>(c.part[1], op1);
+        if (lane < CL) *cgc::this_cluster().map_shared_rank(&c.slots[par][warp][q], lane) = v;
     }
     cgc::this_cluster().sync();
-    if (threadIdx.x < 32) {
-        double2 s = slots[par][0];
+    if (warp < VALUES) {
+        double s = c.slots[par][warp][0];
 #pragma unroll
-        for (int r = 1; r < CL; ++r) s = op(s, slots[par][r]);
-        if (threadIdx.x == 0) result[par] = s;
+        for (int r = 1; r < CL; ++r) s = warp == 0 ? op0(s, c.slots[par][warp][r]) : op1(s, c.slots[par][warp][r]);
+        then(warp, s);
+        if (lane == 0) c.sum[warp] = s;
     }
     __syncthreads();
-    const double2 s = result[par];
     par ^= 1;
-    return s;
 }
 
 // A member neighbour as owner rank (3 bits) and offset in the owner's range (13 bits); 0xFFFF is
@@ -1088,9 +1147,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CL_THREADS)
                     int* __restrict__ spill_count) {
     constexpr int FT = CL_THREADS;
     extern __shared__ double dyn[];
-    __shared__ double2 warps[FT];   // block_reduce2's partials
-    __shared__ double2 slots[2][CL];
-    __shared__ double2 result[3];   // two for the cluster's results, one for the CTA's
+    __shared__ ClusterSums cs;
     __shared__ int bound[CL + 1];
     __shared__ int s_nruns;
     __shared__ double* s_dptr[CL];
@@ -1152,8 +1209,10 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CL_THREADS)
     // the rain (:239-295), as k_flat_solve_sm does for its members.
     float lo_f = FLT_MAX;
     for (int j = threadIdx.x; j < m; j += FT) lo_f = fminf(lo_f, a.filled[mem[lo + j]]);
-    const double entry_level =
-        cluster_combine(make_double2((double)lo_f, 0.0), MinMax2(), warps, slots, result, par, q).x;
+    auto nothing = [](int, double) {};
+    cs.part[0][threadIdx.x] = (double)lo_f;
+    cluster_combine<1>(cs, par, q, DMin(), DMin(), nothing);
+    const double entry_level = cs.sum[0];
     double hi = -INFINITY;
     for (int j = threadIdx.x; j < m; j += FT) {
         const int k = lo + j;
@@ -1197,7 +1256,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CL_THREADS)
             s_run[atomicAdd(&s_nruns, 1)] = (unsigned)j | ((unsigned)(e - lo) << 16);
         }
     }
-    const double entry_height = cluster_combine(make_double2(0.0, hi), MinMax2(), warps, slots, result, par, q).y;
+    cs.part[0][threadIdx.x] = hi;
+    cluster_combine<1>(cs, par, q, DMax(), DMax(), nothing);
+    const double entry_height = cs.sum[0];
     const int runs = s_nruns;
 
     // Thomas pivots down each run (FlatRouting.kt:388-395) and ns / pivot for the way back up.
@@ -1214,36 +1275,27 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CL_THREADS)
     }
     __syncthreads();
 
-    auto precondition = [&]() {
-        for (int i = threadIdx.x; i < runs; i += FT) {
-            const int first = (int)(s_run[i] & 0xFFFFu), last = (int)(s_run[i] >> 16);
-            double v = div_by(__dadd_rn(s_r[first], 0.0), s_piv[first], s_rcp[first]);
-            s_z[first] = v;
-            for (int j = first + 1; j <= last; ++j) {
-                v = div_by(__dadd_rn(s_r[j], UNITW ? v : __dmul_rn(a.ns, v)), s_piv[j], s_rcp[j]);
-                s_z[j] = v;
-            }
-            double below = v;
-            for (int j = last - 1; j >= first; --j) {
-                below = __dadd_rn(s_z[j], __dmul_rn(s_coef[j], below));
-                s_z[j] = below;
-            }
-        }
-    };
     const double w8[8] = {a.diag, a.ns, a.diag, a.ew, a.ew, a.diag, a.ns, a.diag};   // stencil order
+    const int lane = threadIdx.x & 31;
+    auto norms = [&]() {
+        double nn = 0.0, na = 0.0;
+        for (int j = threadIdx.x; j < m; j += FT) {
+            const double rv = s_r[j];
+            nn = partial_add(nn, __dmul_rn(rv, rv), j == (int)threadIdx.x);
+            na = partial_add(na, __dmul_rn(rv, s_z[j]), j == (int)threadIdx.x);
+        }
+        cs.part[0][threadIdx.x] = nn;
+        cs.part[1][threadIdx.x] = na;
+    };
 
     // Preconditioned conjugate gradients (FlatRouting.kt:296-333).
-    precondition();
+    for (int i = threadIdx.x; i < runs; i += FT)
+        solve_run<UNITW>(s_r, s_z, s_piv, s_rcp, s_coef, a.ns, (int)(s_run[i] & 0xFFFFu), (int)(s_run[i] >> 16));
     __syncthreads();
-    double rn = 0.0, ra = 0.0;
-    for (int j = threadIdx.x; j < m; j += FT) {
-        const double rv = s_r[j], zv = s_z[j];
-        s_d[j] = zv;
-        rn = __dadd_rn(rn, __dmul_rn(rv, rv));
-        ra = __dadd_rn(ra, __dmul_rn(rv, zv));
-    }
-    double2 sums = cluster_combine(make_double2(rn, ra), Sum2(), warps, slots, result, par, q);   // also publishes d
-    double rnorm = sums.x, rap = sums.y;
+    for (int j = threadIdx.x; j < m; j += FT) s_d[j] = s_z[j];
+    norms();
+    cluster_combine<2>(cs, par, q, DAdd(), DAdd(), nothing);   // also publishes d
+    double rnorm = cs.sum[0], rap = cs.sum[1];
     const double stop_at = __dmul_rn(__dmul_rn(rnorm, 1e-7), 1e-7);
     const int most = 64 + (int)(8.0 * sqrt((double)n));
     for (int it = 0; rnorm > stop_at && it < most; ++it) {
@@ -1262,31 +1314,32 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CL_THREADS)
                 sum = __dsub_rn(sum, UNITW ? dn : __dmul_rn(w8[t], dn));
             }
             s_ad[j] = sum;
-            e = __dadd_rn(e, __dmul_rn(dk, sum));
+            e = partial_add(e, __dmul_rn(dk, sum), j == (int)threadIdx.x);
         }
-        const double energy = cluster_combine(make_double2(e, 0.0), Sum2(), warps, slots, result, par, q).x;
-        if (energy <= 0.0 || rap <= 0.0) break;
-        const double step = __ddiv_rn(rap, energy);
-        for (int j = threadIdx.x; j < m; j += FT) {
-            x[j] = __dadd_rn(x[j], __dmul_rn(step, s_d[j]));
-            s_r[j] = __dsub_rn(s_r[j], __dmul_rn(step, s_ad[j]));
-        }
+        cs.part[0][threadIdx.x] = e;
+        cluster_combine<1>(cs, par, q, DAdd(), DAdd(), [&](int, double energy) {
+            const double quot = __ddiv_rn(rap, energy);
+            if (lane == 0) cs.quot[0] = quot;
+        });
+        if (cs.sum[0] <= 0.0 || rap <= 0.0) break;
+        const double step = cs.quot[0];
+        for (int j = threadIdx.x; j < m; j += FT) s_r[j] = __dsub_rn(s_r[j], __dmul_rn(step, s_ad[j]));
         __syncthreads();
-        precondition();
+        solve_runs_beside<FT, UNITW>(s_run, runs, s_r, s_z, s_piv, s_rcp, s_coef, a.ns, x, s_d, m, step, rap, &cs.rcp_rap);
         __syncthreads();
-        double nn = 0.0, na = 0.0;
-        for (int j = threadIdx.x; j < m; j += FT) {
-            const double rv = s_r[j];
-            nn = __dadd_rn(nn, __dmul_rn(rv, rv));
-            na = __dadd_rn(na, __dmul_rn(rv, s_z[j]));
-        }
-        sums = cluster_combine(make_double2(nn, na), Sum2(), warps, slots, result, par, q);
-        const double improvement = __ddiv_rn(sums.y, rap);
+        norms();
+        cluster_combine<2>(cs, par, q, DAdd(), DAdd(), [&](int v, double sum) {
+            if (v == 0) return;
+            const double quot = div_by(sum, rap, cs.rcp_rap);
+            if (lane == 0) cs.quot[1] = quot;
+        });
+        const double improvement = cs.quot[1];
+        rnorm = cs.sum[0];
+        rap = cs.sum[1];
         for (int j = threadIdx.x; j < m; j += FT) s_d[j] = __dadd_rn(s_z[j], __dmul_rn(improvement, s_d[j]));
         cluster.sync();   // every CTA's new d before the next Laplacian reads it
-        rnorm = sums.x;
-        rap = sums.y;
     }
+    __syncthreads();   // every member's x
     int positive = 1;
     double top = 0.0;
     for (int j = threadIdx.x; j < m; j += FT) {
@@ -1294,11 +1347,14 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CL_THREADS)
         if (!(v > 0.0)) positive = 0;
         if (v > top) top = v;
     }
-    const double2 pt = cluster_combine(make_double2(positive ? 1.0 : 0.0, top), MinMax2(), warps, slots, result, par, q);
-    const double highest = pt.y;
+    cs.part[0][threadIdx.x] = positive ? 1.0 : 0.0;
+    cs.part[1][threadIdx.x] = top;
+    cluster_combine<2>(cs, par, q, DMin(), DMax(), nothing);
+    const bool all_positive = cs.sum[0] > 0.0;
+    const double highest = cs.sum[1];
 
     // FlatRouting.layInBand (FlatRouting.kt:455-489) over the cluster.
-    bool laid = pt.x > 0.0 && !(highest <= 0.0 || entry_height >= entry_level);
+    bool laid = all_positive && !(highest <= 0.0 || entry_height >= entry_level);
     if (laid) {
         const double band = __dmul_rn(__dsub_rn(entry_level, entry_height), 0.9);
         for (int j = threadIdx.x; j < m; j += FT)
@@ -1323,8 +1379,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CL_THREADS)
             }
             if (!lower) ok = 0.0;
         }
-        ok = cluster_combine(make_double2(ok, 0.0), MinMax2(), warps, slots, result, par, q).x;
-        if (ok <= 0.0) {
+        cs.part[0][threadIdx.x] = ok;
+        cluster_combine<1>(cs, par, q, DMin(), DMin(), nothing);
+        if (cs.sum[0] <= 0.0) {
             for (int j = threadIdx.x; j < m; j += FT) a.surface[mem[lo + j]] = (double)a.filled[mem[lo + j]];
             laid = false;
         }
@@ -1349,7 +1406,22 @@ __device__ __forceinline__ double seg_sum(double v) {
     return v;
 }
 
+// Two such sums for the FP64 instructions of one: a butterfly's first stage leaves the same sums in the
+// segment's two halves, so the lower half goes on with u's and the upper with v's (an addition of the same
+// two values either way round), and each half hands its result to the other.
 template <int S>
+__device__ __forceinline__ void seg_sum2(double& u, double& v) {
+    const bool upper = (threadIdx.x & (S / 2)) != 0;
+    const double keep = upper ? v : u, give = upper ? u : v;
+    double s = __dadd_rn(keep, __shfl_xor_sync(0xFFFFFFFFu, give, S / 2));
+#pragma unroll
+    for (int o = S / 4; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, o));
+    const double other = __shfl_xor_sync(0xFFFFFFFFu, s, S / 2);
+    u = upper ? other : s;
+    v = upper ? s : other;
+}
+
+template <int S, bool UNITW>
 __global__ void __launch_bounds__(32 * WF) k_flat_solve_seg(FlatArgs a, const int* __restrict__ list, int count) {
     constexpr int G = 32 / S;   // flats per warp
     const unsigned FULL = 0xFFFFFFFFu;
@@ -1442,31 +1514,19 @@ __global__ void __launch_bounds__(32 * WF) k_flat_solve_seg(FlatArgs a, const in
             s_rcp[w][j] = __ddiv_rn(1.0, p);
             if (!s_cont[w][j]) break;
             ++j;
-            p = __dsub_rn(s_right[w][j], __ddiv_rn(__dmul_rn(a.ns, a.ns), p));
+            p = __dsub_rn(s_right[w][j], __ddiv_rn(UNITW ? 1.0 : __dmul_rn(a.ns, a.ns), p));
         }
     }
     __syncwarp();
 
     // z = M^-1 r through the runs (FlatRouting.ColumnRuns.solve).
+    int last = lane;
+    if (head)
+        while (s_cont[w][last]) ++last;
     auto precondition = [&](double right) -> double {
         s_right[w][lane] = right;
         __syncwarp();
-        if (head) {
-            int j = lane;
-            double v = div_by(__dadd_rn(s_right[w][j], 0.0), s_piv[w][j], s_rcp[w][j]);
-            s_into[w][j] = v;
-            while (s_cont[w][j]) {
-                ++j;
-                v = div_by(__dadd_rn(s_right[w][j], __dmul_rn(a.ns, v)), s_piv[w][j], s_rcp[w][j]);
-                s_into[w][j] = v;
-            }
-            double below = v;
-            for (int i = j - 1; i >= lane; --i) {
-                const double u = __dadd_rn(s_into[w][i], __dmul_rn(s_coef[w][i], below));
-                s_into[w][i] = u;
-                below = u;
-            }
-        }
+        if (head) solve_run<UNITW>(s_right[w], s_into[w], s_piv[w], s_rcp[w], s_coef[w], a.ns, lane, last);
         __syncwarp();
         const double z = act ? s_into[w][lane] : 0.0;
         __syncwarp();
@@ -1478,7 +1538,8 @@ __global__ void __launch_bounds__(32 * WF) k_flat_solve_seg(FlatArgs a, const in
         double sum = __dmul_rn(deg, dv);
 #pragma unroll
         for (int t = 0; t < 8; ++t)
-            if (nb_lane[t] >= 0) sum = __dsub_rn(sum, __dmul_rn(nb_w[t], s_d[w][nb_lane[t]]));
+            if (nb_lane[t] >= 0)
+                sum = __dsub_rn(sum, UNITW ? s_d[w][nb_lane[t]] : __dmul_rn(nb_w[t], s_d[w][nb_lane[t]]));
         __syncwarp();
         return act ? sum : 0.0;
     };
@@ -1487,8 +1548,8 @@ __global__ void __launch_bounds__(32 * WF) k_flat_solve_seg(FlatArgs a, const in
     double x = 0.0, r = act ? rv : 0.0;
     double z = precondition(r);
     double d = z;
-    double rnorm = seg_sum<S>(act ? __dmul_rn(r, r) : 0.0);
-    double rap = seg_sum<S>(act ? __dmul_rn(r, z) : 0.0);
+    double rnorm = act ? __dmul_rn(r, r) : 0.0, rap = act ? __dmul_rn(r, z) : 0.0;
+    seg_sum2<S>(rnorm, rap);
     const double stop_at = __dmul_rn(__dmul_rn(rnorm, 1e-7), 1e-7);
     const int most = 64 + (int)(8.0 * sqrt((double)(n > 0 ? n : 1)));
     bool stopped = f < 0;
@@ -1504,9 +1565,9 @@ __global__ void __launch_bounds__(32 * WF) k_flat_solve_seg(FlatArgs a, const in
             x = __dadd_rn(x, __dmul_rn(step, d));
             r = __dsub_rn(r, __dmul_rn(step, ad));
         }
-        const double next_norm = seg_sum<S>(act ? __dmul_rn(r, r) : 0.0);
         const double zn = precondition(r);
-        const double next_ap = seg_sum<S>(act ? __dmul_rn(r, zn) : 0.0);
+        double next_norm = act ? __dmul_rn(r, r) : 0.0, next_ap = act ? __dmul_rn(r, zn) : 0.0;
+        seg_sum2<S>(next_norm, next_ap);
         if (go) {
             const double improvement = __ddiv_rn(next_ap, rap);
             if (act) d = __dadd_rn(zn, __dmul_rn(improvement, d));
@@ -1657,6 +1718,7 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
                 a.ns = 1.0;
                 a.diag = dg;
             }
+            const bool unit = a.ew == 1.0 && a.ns == 1.0 && a.diag == 1.0;   // square cells: no weight to multiply by
             a.off = d_off;
             a.count = d_cnt;
             a.members = d_members;
@@ -1694,21 +1756,21 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
             CG_CUDA(ctx, cudaEventRecord(ctx->join2, ctx->aux2));
             {
                 const int* small = d_lists + 3 * (size_t)flats;
-                if (ctr[5] > 0)
-                    CG_LAUNCH(ctx) k_flat_solve_seg<4><<<(ctr[5] + 8 * WF - 1) / (8 * WF), 32 * WF, 0, ctx->aux>>>(a, small, ctr[5]);
-                if (ctr[6] > 0)
-                    CG_LAUNCH(ctx) k_flat_solve_seg<8><<<(ctr[6] + 4 * WF - 1) / (4 * WF), 32 * WF, 0, ctx->aux>>>(
-                        a, small + flats, ctr[6]);
-                if (ctr[7] > 0)
-                    CG_LAUNCH(ctx) k_flat_solve_seg<16><<<(ctr[7] + 2 * WF - 1) / (2 * WF), 32 * WF, 0, ctx->aux>>>(
-                        a, small + 2 * (size_t)flats, ctr[7]);
-                if (ctr[8] > 0)
-                    CG_LAUNCH(ctx) k_flat_solve_seg<32><<<(ctr[8] + WF - 1) / WF, 32 * WF, 0, ctx->aux>>>(
-                        a, small + 3 * (size_t)flats, ctr[8]);
+                auto seg = [&](auto kernel, int width, int k) {   // list 3 + k: flats of up to `width` members
+                    const int per = (32 / width) * WF;
+                    if (ctr[5 + k] > 0)
+                        CG_LAUNCH(ctx) kernel<<<(ctr[5 + k] + per - 1) / per, 32 * WF, 0, ctx->aux>>>(
+                            a, small + k * (size_t)flats, ctr[5 + k]);
+                };
+                seg(unit ? k_flat_solve_seg<4, true> : k_flat_solve_seg<4, false>, 4, 0);
+                seg(unit ? k_flat_solve_seg<8, true> : k_flat_solve_seg<8, false>, 8, 1);
+                seg(unit ? k_flat_solve_seg<16, true> : k_flat_solve_seg<16, false>, 16, 2);
+                seg(unit ? k_flat_solve_seg<32, true> : k_flat_solve_seg<32, false>, 32, 3);
             }
-            if (ctr[0] > 0)
-                CG_LAUNCH(ctx) k_flat_solve_sm<128><<<ctr[0], 128, (size_t)ctr[3] * SM_BYTES_PER_MEMBER, ctx->aux>>>(
-                    a, d_lists);
+            if (ctr[0] > 0) {
+                auto kernel = unit ? k_flat_solve_sm<128, true> : k_flat_solve_sm<128, false>;
+                CG_LAUNCH(ctx) kernel<<<ctr[0], 128, (size_t)ctr[3] * SM_BYTES_PER_MEMBER, ctx->aux>>>(a, d_lists);
+            }
             CG_CHECK_LAUNCH(ctx);
             if (ctr[1] > 0) {
                 // Per CTA a share of the largest flat with room for the run-head rounding of its bounds;
@@ -1718,7 +1780,6 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
                 // More than half an SM's shared memory, so that no two CTAs of a cluster share an SM (and
                 // its FP64 pipe, which bounds the solve).
                 const size_t bytes = std::max((size_t)cap * SM_BYTES_PER_MEMBER, (size_t)116 * 1024);
-                const bool unit = a.ew == 1.0 && a.ns == 1.0 && a.diag == 1.0;
                 auto kernel = unit ? k_flat_solve_cl<true> : k_flat_solve_cl<false>;
                 // The attribute is the kernel's, shared by every context of the process: set it to the
                 // most any launch asks for, so that a context on another thread lowering it between this
