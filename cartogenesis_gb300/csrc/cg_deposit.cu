@@ -28,16 +28,20 @@
 //     group of log entries; and (b) a donor whose settled height a later (dry) cell of the level read
 //     in its headroom. Such a cell's own walk is taken again with its donors as the reference's walk
 //     shows them at its rank. Nothing else of the level reads that cell, so where its step hands
-//     everything on the fix is local; where it has a mouth, its fan changes with it: every fan from
-//     its rank on is undone (over the grid, from the log), the cell refitted, and those fans laid
-//     again, and the search, an atomic minimum over the log, repeats past it. Both are rare; the
-//     level schedule itself is shown on the host to give the reference walk's bits
+//     everything on the fix is local; where it has a mouth, its fan changes with it. Such a cell is
+//     found as the deposit that makes it one is logged, nearly always before its own fan's turn: the
+//     chunks then end before it, and it is refitted when every fan ranked before it has laid; fans of
+//     the same chunk ranked after it are undone first (over the grid, from the log) and laid again.
+//     (Laying the whole level, then undoing and laying again everything after each such cell, took
+//     2.5 million fans in the first round of an 8192 x 4096 draft where 0.5 million have work.) Both are
+//     rare; the level schedule itself is shown on the host to give the reference walk's bits
 //     (tests/native/deposit_host.cpp).
 // Settle is elementwise, and the mouths pass reads only each cell's receiver, so it runs receivers
 // first, level by level from the top, like the incision.
 #include <algorithm>
 #include <climits>
 #include <cooperative_groups.h>
+#include <cuda/atomic>
 #include <vector>
 
 #include "cg_common.cuh"
@@ -60,11 +64,11 @@ constexpr long long kSpinLimit = 1LL << 24;   // a lake fan's wait for its turn,
 
 // Control words of a walk.
 enum {
-    W_EVENTS = 0, W_ERROR = 1, W_MOUTH_ID = 2, W_GEN = 3, W_ABORT = 4, W_REPLAYED = 5, W_WAVEBASE = 6, W_WAVES = 7,
-    W_WAIT0 = 8, W_WAIT1 = 9, W_REFITTED = 10, W_ESTART = 11, W_DONE = 12, W_RELAID = 13, W_PAIRS = 14, W_DISTINCT = 15,
+    W_ERROR = 1, W_GEN = 3, W_ABORT = 4, W_REPLAYED = 5, W_WAVES = 7, W_REFITTED = 10, W_RELAID = 13, W_PAIRS = 14,
+    W_DISTINCT = 15,
     W_CHECK_SITE = 16, W_CHECK_VALUE = 17, W_CHECK_BOUND = 18, W_NDONOR = 19,
-    W_REFITGEN = 20, W_BEST = 21, W_TOUCHN = 22, W_NREPLAY = 23, W_NREFIT = 24, W_FGEN = 25, W_NLAKE = 26,
-    W_NSEA = 27, W_SEAWAIT0 = 28, W_SEAWAIT1 = 29, W_CUT = 30, W_RC = 31, W_WORDS = 32
+    W_REFITGEN = 20, W_CLASHES = 21, W_TOUCHN = 22, W_NREPLAY = 23, W_NREFIT = 24, W_FGEN = 25, W_NLAKE = 26,
+    W_NSEA = 27, W_INSERT = 28, W_WORDS = 32
 };
 
 struct WalkDev {
@@ -83,9 +87,8 @@ struct WalkDev {
     double* ev_carried;     // per rank: what a listed mouth carries
     int8_t* ev_kind;        // per rank: SEA or LAKE
     int* seg_events;        // per rank: listed ranks, compacted within each CTA's segment
-    int* seg_count;         // per CTA
-    int* seg_off;           // per CTA + 1: its listed mouths' first place in `events`
-    int* seg_part;          // per CTA + 1: a grid-wide scan's slice sums
+    int* seg_count;         // per CTA, twice (the levels alternate)
+    int* seg_part;          // per CTA: a grid-wide scan's slice sums
     int* events;            // the level's listed ranks, dense, in rank order
     // The round's lake fans, admitted before the walk (k_admit_lakes): per candidate mouth cell its
     // admitted cells sorted by distance and each one's level less its terrain, in a pool.
@@ -311,37 +314,67 @@ __global__ void k_widen_counts(const int* __restrict__ n, int count, long long* 
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) out[i] = n[i];
 }
 
-// An exclusive prefix sum by one CTA (every thread of it calls this), chunk after chunk; out[n]
-// receives the total. get(i) gives element i. sh is the CTA's shared scratch: no __restrict__ on it,
-// which would let the compiler keep a thread's own sh entry in a register across the barriers that
-// publish it to the other threads.
+// The exclusive prefix of v over the CTA's threads, and the CTA's total. sh holds kThreads / 32 ints and
+// is free again after the call. (No __restrict__ on it, which would let the compiler keep an entry in a
+// register across the barriers that publish it to the other threads.)
+__device__ __forceinline__ int cta_prefix(int v, int* total, int* sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) sh[warp] = incl;
+    __syncthreads();
+    int before = 0, all = 0;
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; ++i) {
+        const int t = sh[i];
+        before += i < warp ? t : 0;
+        all += t;
+    }
+    __syncthreads();
+    *total = all;
+    return before + incl - v;
+}
+
+// An exclusive prefix sum of [lo, hi) by one CTA (every thread of it calls this), kScanPer elements a
+// thread at a time, on top of `carry`; get(i) gives element i. Returns the sum past the last. A chunk of
+// 2048 mouths is one step of two barriers.
+constexpr int kScanPer = 8;
+template <class Get>
+__device__ int cta_scan_range(Get get, int lo, int hi, int carry, int* out, int* sh) {
+    for (int base = lo; base < hi; base += kThreads * kScanPer) {
+        const int i0 = base + (int)threadIdx.x * kScanPer;
+        int v[kScanPer], sum = 0;
+#pragma unroll
+        for (int t = 0; t < kScanPer; ++t) {
+            v[t] = i0 + t < hi ? get(i0 + t) : 0;
+            sum += v[t];
+        }
+        int total;
+        int run = carry + cta_prefix(sum, &total, sh);
+#pragma unroll
+        for (int t = 0; t < kScanPer; ++t) {
+            if (i0 + t < hi) out[i0 + t] = run;
+            run += v[t];
+        }
+        carry += total;
+    }
+    return carry;
+}
+
+// The exclusive prefix sum of n elements by one CTA; out[n] receives the total.
 template <class Get>
 __device__ void cta_exclusive_scan(Get get, int n, int* out, int* sh) {
-    int carry = 0;
-    for (int base = 0; base < n; base += kThreads) {
-        const int i = base + (int)threadIdx.x;
-        const int v = i < n ? get(i) : 0;
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < kThreads; o <<= 1) {
-            const int t = threadIdx.x >= (unsigned)o ? sh[threadIdx.x - o] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += t;
-            __syncthreads();
-        }
-        if (i < n) out[i] = carry + sh[threadIdx.x] - v;
-        const int chunk = sh[kThreads - 1];
-        __syncthreads();
-        carry += chunk;
-    }
-    if (threadIdx.x == 0) out[n] = carry;
+    const int total = cta_scan_range(get, 0, n, 0, out, sh);
+    if (threadIdx.x == 0) out[n] = total;
     __syncthreads();
 }
 
-// An exclusive prefix sum over the whole grid, called by every thread: each CTA sums a slice, one CTA
-// scans the slices' sums, then each CTA scans its slice from its offset; out[n] receives the total.
-// For long arrays, where one CTA stepping through them would hold the grid. `part` holds gridDim.x + 1
-// ints.
+// An exclusive prefix sum over the whole grid, called by every thread: each CTA sums a slice, then adds
+// the slices before its own and scans its slice from there; out[n] receives the total. For long arrays,
+// where one CTA stepping through them would hold the grid. `part` holds gridDim.x ints.
 template <class Get>
 __device__ void grid_exclusive_scan(Get get, int n, int* out, int* part, int* sh) {
     cgr::grid_group grid = cgr::this_grid();
@@ -349,38 +382,16 @@ __device__ void grid_exclusive_scan(Get get, int n, int* out, int* part, int* sh
     const int lo = min(n, (int)blockIdx.x * per), hi = min(n, lo + per);
     int sum = 0;
     for (int i = lo + (int)threadIdx.x; i < hi; i += kThreads) sum += get(i);
-    sh[threadIdx.x] = sum;
-    __syncthreads();
-    for (int o = kThreads / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-    __syncthreads();
+    int total;
+    cta_prefix(sum, &total, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = total;
     grid.sync();
-    if (blockIdx.x == 0) {
-        const int* pp = part;
-        cta_exclusive_scan([=](int i) { return __ldcg(&pp[i]); }, (int)gridDim.x, part, sh);
-    }
-    grid.sync();
-    int carry = __ldcg(&part[blockIdx.x]);
-    for (int base = lo; base < hi; base += kThreads) {
-        const int i = base + (int)threadIdx.x;
-        const int v = i < hi ? get(i) : 0;
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < kThreads; o <<= 1) {
-            const int t = threadIdx.x >= (unsigned)o ? sh[threadIdx.x - o] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += t;
-            __syncthreads();
-        }
-        if (i < hi) out[i] = carry + sh[threadIdx.x] - v;
-        const int chunk = sh[kThreads - 1];
-        __syncthreads();
-        carry += chunk;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = __ldcg(&part[gridDim.x]);
+    int before = 0;
+    for (int i = (int)threadIdx.x; i < (int)blockIdx.x; i += kThreads) before += __ldcg(&part[i]);
+    int carry;
+    cta_prefix(before, &carry, sh);
+    const int end = cta_scan_range(get, lo, hi, carry, out, sh);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = end;
 }
 
 // An index check of the laying schedule: v must lie in [0, hi). A failure records its site, value and
@@ -398,52 +409,106 @@ __device__ __forceinline__ bool index_ok(const WalkDev& w, long long v, long lon
     return false;
 }
 
+// A lake fan before its turn: what its laying needs and no earlier fan can change, loaded while it waits.
+constexpr int kLakeAhead = 2;   // admitted cells a lane loads at a time
+struct LakeFan {
+    int n;
+    const int* sorted;
+    const double* base;
+    int x[kLakeAhead];
+    double b[kLakeAhead];
+    __device__ __forceinline__ void load(int i0, int lane) {
+#pragma unroll
+        for (int u = 0; u < kLakeAhead; ++u) {
+            const int i = i0 + 32 * u + lane;
+            x[u] = i < n ? sorted[i] : -1;
+            b[u] = i < n ? base[i] : 0.0;
+        }
+    }
+};
+
+__device__ __forceinline__ bool above_zero(double x) { return __double_as_longlong(x) > 0; }
+__device__ __forceinline__ bool below(double x, double y) { return __double_as_longlong(x) < __double_as_longlong(y); }
+
 // A lake fan's laying by one warp (lay_admitted's loop over the distance-sorted admitted cells). A
-// fan's cells are distinct, so laying into one changes no other's need: the warp reads 32 needs at
-// once and lays into the ones above zero one after another, in order, while the budget lasts. The
-// deposits go to the slot's own log.
-__device__ void lay_lake_warp(const WalkDev& w, int s, double budget, int lane) {
+// fan's cells are distinct, so laying into one changes no other's need: the warp reads 64 cells at
+// once and takes the ones with a need above zero in order while the budget lasts. All of those but the
+// last take their whole need, which does not depend on what the ones before them took, so every lane
+// works out its cell's deposit at once, and only the subtractions from the budget run in order: even
+// lanes carry what remains and odd lanes what is laid, one FP64 instruction a cell. The first cell
+// whose need is not below what remains takes what remains. Everything another fan may have laid is
+// read through L2. The deposits go to the slot's own log; odd lanes return what was laid.
+__device__ double lay_lake_warp(const WalkDev& w, int s, LakeFan& fan, double budget, int lane) {
     const unsigned FULL = 0xFFFFFFFFu;
-    const int n = w.slot_n[s];
-    const int* sorted = w.pool_cells + w.slot_off[s];
-    const double* base = w.pool_base + w.slot_off[s];
     Touch* log = w.slot_touch + (size_t)s * w.cap;
-    double remaining = budget, laid = 0.0;
+    const bool odd = lane & 1;
+    double acc = odd ? 0.0 : budget;
     int logged = 0;
-    for (int i0 = 0; i0 < n && remaining > 0.0; i0 += 32) {
-        const int i = i0 + lane;
-        int x = -1;
-        double need = 0.0;
-        if (i < n) {
-            x = sorted[i];
-            if (index_ok(w, x, (long long)w.p.W * w.p.H, 9)) need = __dsub_rn(base[i], (double)__ldcg(&w.f.sediment[x]));
+    for (int i0 = 0; i0 < fan.n; i0 += 32 * kLakeAhead) {
+        if (i0 > 0) fan.load(i0, lane);
+        float prior[kLakeAhead], settled[kLakeAhead];
+        bool valid[kLakeAhead];
+#pragma unroll
+        for (int u = 0; u < kLakeAhead; ++u) {
+            valid[u] = i0 + 32 * u + lane < fan.n && index_ok(w, fan.x[u], (long long)w.p.W * w.p.H, 9);
+            prior[u] = valid[u] ? __ldcg(&w.f.sediment[fan.x[u]]) : 0.0f;
+            settled[u] = valid[u] ? __ldcg(&w.f.settled[fan.x[u]]) : 0.0f;
         }
-        unsigned live = __ballot_sync(FULL, i < n && need > 0.0);
-        while (live && remaining > 0.0) {
-            const int j = __ffs(live) - 1;
-            live &= live - 1;
-            double moved = 0.0;
-            if (lane == j) {
-                // HydraulicErosion.raise and the settled height's rise, through L2: an earlier fan on
-                // this cell may have laid on another SM in this same wave.
-                const float prior = __ldcg(&w.f.sediment[x]), settled = __ldcg(&w.f.settled[x]);
-                const float now = (float)((double)prior + (need < remaining ? need : remaining));
-                __stcg(&w.f.sediment[x], now);
-                moved = (double)now - (double)prior;
-                const float increment = (float)(moved * (double)w.p.to_relative);
-                __stcg(&w.f.settled[x], settled + increment);
-                log[logged] = Touch{x, settled, prior, increment};
+#pragma unroll
+        for (int u = 0; u < kLakeAhead; ++u) {
+            const double need = __dsub_rn(fan.b[u], (double)prior[u]);
+            unsigned live = __ballot_sync(FULL, valid[u] && above_zero(need));
+            while (live) {
+                if (!above_zero(__shfl_sync(FULL, acc, 0))) {
+                    live = 0;
+                    i0 = fan.n;   // nothing remains
+                    break;
+                }
+                float now = (float)((double)prior[u] + need);
+                double moved = (double)now - (double)prior[u];
+                double rem = 0.0, laid = 0.0;   // before this lane's cell
+                for (unsigned m = live; m; m &= m - 1) {
+                    const int j = __ffs(m) - 1;
+                    const double mv = __shfl_sync(FULL, moved, j);
+                    const double r = __shfl_sync(FULL, acc, 0), l = __shfl_sync(FULL, acc, 1);
+                    if (lane == j) {
+                        rem = r;
+                        laid = l;
+                    }
+                    acc = __dadd_rn(acc, odd ? mv : -mv);
+                }
+                const unsigned whole = __ballot_sync(FULL, above_zero(rem) && below(need, rem));
+                const unsigned part = live & ~whole;
+                const int p = part ? __ffs(part) - 1 : 32;   // the first that does not take its whole need
+                if (part) {
+                    const double r = __shfl_sync(FULL, rem, p), l = __shfl_sync(FULL, laid, p);
+                    acc = odd ? l : r;
+                    if (above_zero(r)) {
+                        if (lane == p) {
+                            now = (float)((double)prior[u] + r);
+                            moved = (double)now - (double)prior[u];
+                        }
+                        const double mv = __shfl_sync(FULL, moved, p);
+                        acc = __dadd_rn(acc, odd ? mv : -mv);
+                    }
+                }
+                const bool last = part && above_zero(__shfl_sync(FULL, rem, p & 31));
+                const unsigned lays = live & ((p < 32 ? (1u << p) : 0u) - 1u) | (last ? 1u << p : 0u);
+                if ((lays >> lane) & 1u) {
+                    // HydraulicErosion.raise and the settled height's rise.
+                    const float increment = (float)(moved * (double)w.p.to_relative);
+                    __stcg(&w.f.sediment[fan.x[u]], now);
+                    __stcg(&w.f.settled[fan.x[u]], settled[u] + increment);
+                    log[logged + __popc(lays & ((1u << lane) - 1u))] = Touch{fan.x[u], settled[u], prior[u], increment};
+                }
+                logged += __popc(lays);
+                live = part ? live & ~((2u << p) - 1u) : 0u;
             }
-            moved = __shfl_sync(FULL, moved, j);
-            ++logged;
-            remaining -= moved;
-            laid += moved;
         }
     }
-    if (lane == 0) {
-        w.slot_laid[s] = laid;
-        w.slot_touch_n[s] = logged;
-    }
+    if (lane == 1) w.slot_laid[s] = acc;
+    if (lane == 0) w.slot_touch_n[s] = logged;
+    return acc;
 }
 
 // The kind of a cell's step (own_walk's answer), read from the fixed fields alone.
@@ -511,13 +576,13 @@ __device__ bool refit_cell(const WalkDev& w, int c) {
     return true;
 }
 
-// The walk made the reference's again from rank rc (the earliest mouth conflict), once every fan
-// ranked at or after rc is undone (undo_from_grid) and the level's log cut back to before them: the
-// conflicted cell's own walk taken again on the state the reference's walk shows it (its own state
-// before the walk, and its donors as every fan ranked before it left them, which is now the current
-// state); its mouth listed or unlisted as its new load decides. ec is the index of the first event
-// ranked at or after rc, the first to lay again; *n is updated.
-__device__ void refit_mouth_cell(const WalkDev& w, int rc, int ec, int refit_gen, int* n) {
+// The conflicted cell of rank rc refitted, once every fan ranked before it has laid and none after it:
+// its own walk taken again on the state the reference's walk shows it (its own state before the walk,
+// and its donors as every fan ranked before it left them, which is now the current state); its mouth
+// listed or not as its new load decides. ec is the index of the first event ranked at or after rc. A
+// mouth that has nothing to lay any more keeps its place with no kind; returns whether one that had
+// none has to be listed at ec.
+__device__ bool refit_mouth_cell(const WalkDev& w, int rc, int ec, int n) {
     const int c = w.order[rc];
     w.f.settled[c] = w.s0[rc];
     w.f.sediment[c] = w.d0[rc];
@@ -527,21 +592,11 @@ __device__ void refit_mouth_cell(const WalkDev& w, int rc, int ec, int refit_gen
     const int kind = own_walk(w.p, w.f, c, carried, &used, &incised, &deposited);
     w.used[c] = used ? 1 : 0;
     if (kind == LAKE) w.handoff[c] = carried;
-    w.mark[c] = refit_gen;
-    const bool listed = ec < *n && w.events[ec] == rc;
+    const bool listed = ec < n && w.events[ec] == rc;
     const bool live = (kind == SEA || kind == LAKE) && mouth_live(w, c, carried, kind);
-    if (live) {
-        w.ev_carried[rc] = carried;
-        w.ev_kind[rc] = (int8_t)kind;
-        if (!listed) {
-            for (int e = *n; e > ec; --e) w.events[e] = w.events[e - 1];
-            w.events[ec] = rc;
-            ++*n;
-        }
-    } else if (listed) {
-        for (int e = ec; e + 1 < *n; ++e) w.events[e] = w.events[e + 1];
-        --*n;
-    }
+    if (live) w.ev_carried[rc] = carried;
+    if (live || listed) w.ev_kind[rc] = live ? (int8_t)kind : (int8_t)ON;
+    return live && !listed;
 }
 
 // The level log's entries [cut, T) undone over the grid, called by every thread: a cell takes back
@@ -564,25 +619,17 @@ __device__ void undo_from_grid(const WalkDev& w, int cut, int T) {
 // The level-log entry t's event (recorded as the log is assembled).
 __device__ __forceinline__ int event_of(const WalkDev& w, int t, int) { return w.touch_ev[t]; }
 
-// The earliest cell of level L, ranked after a fan of the level that raised one of its donors, whose
-// headroom read that donor and which has a mouth of its own (its step ends at the sea or in a lake):
-// its own walk, and so its fan, are not the reference's. Cells refitted already (mark = the level's
-// refit generation) are final and skipped. Over the grid: each thread takes log entries and the
-// lowest rank found wins (atomicMin into W_BEST, INT_MAX when there is none).
-__device__ void mouth_conflicts_grid(const WalkDev& w, int L, int n) {
-    const int T = *(volatile int*)&w.words[W_TOUCHN];
-    const int refit_gen = *(volatile int*)&w.words[W_REFITGEN];
-    int best = INT_MAX;
-    for (int t = (int)(blockIdx.x * blockDim.x + threadIdx.x); t < T; t += (int)(gridDim.x * blockDim.x)) {
-        const int x = w.touches[t].cell;
-        if (!w.f.land[x]) continue;
-        const int rr = w.f.dirs[x];
-        if (rr < 0 || !w.f.land[rr] || level_of_cell(w, rr) != L) continue;
-        const int r = w.rank_of[rr];
-        if (r >= best || !w.used[rr] || w.mark[rr] == refit_gen || kind_of(w, rr) == ON) continue;
-        if (r > w.events[event_of(w, t, n)]) best = r;
-    }
-    if (best != INT_MAX) atomicMin(&w.words[W_BEST], best);
+// Whether the deposit into cell x by the fan of rank `rank` of level L makes a mouth conflict: x's
+// receiver lies on the level, is ranked after the fan, read its donors' settled heights and has a mouth of
+// its own (its step ends at the sea or in a lake), so its own walk, and with it its fan, are not the
+// reference's. Such a cell is listed once a level (its mark), by rank.
+__device__ __forceinline__ void find_conflict(const WalkDev& w, int L, int x, int rank, int gen) {
+    if (!w.f.land[x]) return;
+    const int rr = w.f.dirs[x];
+    if (rr < 0 || !w.f.land[rr] || level_of_cell(w, rr) != L) return;
+    const int r = w.rank_of[rr];
+    if (r <= rank || !w.used[rr] || kind_of(w, rr) == ON) return;
+    if (atomicExch(&w.mark[rr], gen) != gen) w.refit[atomicAdd(&w.words[W_CLASHES], 1)] = r;
 }
 
 // The last repairs of level L, with its final log of n events, called by every thread of the grid:
@@ -713,9 +760,12 @@ __device__ void final_repairs_grid(const WalkDev& w, int L, int n, int touch_n, 
 __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
     cgr::grid_group grid = cgr::this_grid();
     __shared__ int warp_counts[kThreads / 32];
-    __shared__ int sh_scan[kThreads];
+    __shared__ int sh_scan[kThreads / 32];
+    __shared__ int sh_clash;
     __shared__ int block_base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), stride = (int)(gridDim.x * blockDim.x);
+    const int gwarp = tid >> 5, nwarps = stride >> 5;
     const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
     unsigned long long tm[T_COUNT] = {0, 0, 0, 0, 0};
     unsigned long long t0 = 0;
@@ -761,37 +811,72 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
             }
             __syncthreads();
         }
-        if (threadIdx.x == 0) w.seg_count[blockIdx.x] = block_base;
-        grid.sync();
         // The listed mouths, dense and in rank order: each CTA's segment at the offset of the ones before.
-        if (blockIdx.x == 0) {
-            const int* sc = w.seg_count;
-            cta_exclusive_scan([=](int i) { return sc[i]; }, (int)gridDim.x, w.seg_off, sh_scan);
-            if (threadIdx.x == 0) w.words[W_EVENTS] = w.seg_off[gridDim.x];
+        // The counts alternate between two arrays, so a CTA that goes on to the next level leaves this one's.
+        int* counts = w.seg_count + (L & 1) * gridDim.x;
+        if (threadIdx.x == 0) __stcg(&counts[blockIdx.x], block_base);
+        grid.sync();
+        int before = 0, all = 0;
+        for (int i = (int)threadIdx.x; i < (int)gridDim.x; i += kThreads) {
+            const int c = __ldcg(&counts[i]);
+            before += i < (int)blockIdx.x ? c : 0;
+            all += c;
+        }
+        int at, n;
+        cta_prefix(before, &at, sh_scan);
+        cta_prefix(all, &n, sh_scan);
+        if (n == 0) {   // no mouth of the level has anything to lay
+            if (timer) tm[T_WALKS] += now_ns() - t0;
+            continue;
+        }
+        for (int i = threadIdx.x; i < block_base; i += blockDim.x) w.events[at + i] = w.seg_events[s_lo + i];
+        if (tid == 0) {
+            w.words[W_REFITGEN] = ++w.words[W_GEN];
+            w.words[W_CLASHES] = 0;
         }
         grid.sync();
-        for (int i = threadIdx.x; i < block_base; i += blockDim.x) w.events[w.seg_off[blockIdx.x] + i] = w.seg_events[s_lo + i];
-        grid.sync();
         if (timer) tm[T_WALKS] += now_ns() - t0;
-        const int n = *(volatile int*)&w.words[W_EVENTS];
-        const int lane = threadIdx.x & 31;
-        const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-        const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-        int touch_n = 0;   // the level's log length (kept by the one thread that writes the log)
-        int n_now = n, e_start = 0;
-        int refit_gen = 0;   // thread 0's mark for the level's refitted mouth cells (a fresh generation)
-        // B, and C's mouth conflicts: lay the events from e_start in rank order (chunks of `slots`); then
-        // if a cell with a mouth read a donor an earlier fan raised, make the walk the reference's again
-        // from that cell (refit_mouth_cell) and lay what follows it again. Each pass moves past at least
-        // one such cell, so there are at most as many passes as the level has cells, and one more.
-        const int passes = hi - lo + 1;
-        for (int pass = 0; pass <= passes; ++pass) {
-            for (int e0 = e_start; e0 < n_now; e0 += w.slots) {
+        const int clash_gen = *(volatile int*)&w.words[W_REFITGEN];
+        // B, and C's mouth conflicts: the events laid in rank order, in chunks of up to `slots` that end
+        // before the lowest conflicted cell known; when every event before that cell is laid, it is
+        // refitted and the laying goes on from it. Everything here but the work itself is the same in
+        // every thread: e0 the next event to lay, n_now the events, touch_n the level log's length.
+        int touch_n = 0, n_now = n, e0 = 0;
+        long long turns = 0;
+        for (;; ++turns) {
+            // A turn lays an event or refits a cell, each once, and a refit undoes at most a chunk.
+            if (turns > 4LL * (hi - lo + 1) + 16) {
+                if (timer) w.words[W_ERROR] |= 8;
+                break;
+            }
+            int rc = INT_MAX, limit = n_now;
+            const int clashes = *(volatile int*)&w.words[W_CLASHES];
+            if (clashes > 0) {
+                if (threadIdx.x == 0) sh_clash = INT_MAX;
+                __syncthreads();
+                int lowest = INT_MAX;
+                for (int i = (int)threadIdx.x; i < clashes; i += kThreads) lowest = min(lowest, __ldcg(&w.refit[i]));
+                lowest = __reduce_min_sync(0xFFFFFFFFu, lowest);
+                if (lane == 0 && lowest != INT_MAX) atomicMin(&sh_clash, lowest);
+                __syncthreads();
+                rc = sh_clash;
+                if (rc != INT_MAX) {   // the first event ranked at or after it
+                    int a = 0, b = n_now;
+                    while (a < b) {
+                        const int m = (a + b) >> 1;
+                        if (w.events[m] < rc) a = m + 1;
+                        else b = m;
+                    }
+                    limit = a;
+                }
+                __syncthreads();   // sh_clash is read before the next turn writes it
+            }
+            if (e0 >= limit && rc == INT_MAX) break;   // every event is laid, no conflict is left
+            if (e0 < limit) {
                 if (timer) t0 = now_ns();
-                const int e1 = min(n_now, e0 + w.slots);
+                const int e1 = min(limit, e0 + w.slots);
                 // The chunk's lake fans, their admissions taken from the round's pool.
-                for (int e = e0 + (int)(blockIdx.x * blockDim.x + threadIdx.x); e < e1;
-                     e += (int)(gridDim.x * blockDim.x)) {
+                for (int e = e0 + tid; e < e1; e += stride) {
                     const int k = w.events[e];
                     const bool lake = w.ev_kind[k] == LAKE;
                     bool ok = lake;
@@ -854,7 +939,7 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                 }
                 grid.sync();
                 const int P = min(*(volatile int*)&w.words[W_PAIRS], w.pair_cap);
-                for (int q = (int)(blockIdx.x * blockDim.x + threadIdx.x); q < P; q += (int)(gridDim.x * blockDim.x)) {
+                for (int q = tid; q < P; q += stride) {
                     int a = 0, b = S;   // the slot whose pairs hold q: poff[a] <= q < poff[a + 1]
                     while (b - a > 1) {
                         const int m = (a + b) >> 1;
@@ -899,14 +984,14 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                 grid.sync();
                 // Every pair is counted on exactly one distinct cell.
                 if (blockIdx.x == 0 && threadIdx.x == 0 && __ldcg(&w.doff[D]) != P) check_failed(w, w.doff[D], P, 13);
-                for (int q = (int)(blockIdx.x * blockDim.x + threadIdx.x); q < P; q += (int)(gridDim.x * blockDim.x)) {
+                for (int q = tid; q < P; q += stride) {
                     const int d = w.cell_d[w.pair_cell[q]];
                     if (!index_ok(w, d, D, 5)) continue;
                     const int at = w.doff[d] + w.pair_pos[q];
                     if (index_ok(w, at, P, 6)) w.group[at] = q;
                 }
                 grid.sync();
-                for (int q = (int)(blockIdx.x * blockDim.x + threadIdx.x); q < P; q += (int)(gridDim.x * blockDim.x)) {
+                for (int q = tid; q < P; q += stride) {
                     const int x = w.pair_cell[q];
                     const int d = w.cell_d[x];
                     if (!index_ok(w, d, D, 5)) continue;
@@ -930,7 +1015,7 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                     if (pred) atomicAdd(&w.blockers[w.pair_fan[q]], 1);
                 }
                 grid.sync();
-                for (int q = (int)(blockIdx.x * blockDim.x + threadIdx.x); q < P; q += (int)(gridDim.x * blockDim.x))
+                for (int q = tid; q < P; q += stride)
                     w.cell_cnt[w.pair_cell[q]] = 0;   // every cell's count back to 0 for the next chunk
                 int waves = 0;
                 if (timer) {
@@ -951,26 +1036,40 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                     for (int sl = gwarp; sl < S; sl += nwarps) {
                         const int kind_slot = w.slot_state[sl];
                         if (kind_slot != 1 && kind_slot != 2) continue;
+                        // What no earlier mouth changes is loaded before the wait.
+                        const int rank = w.events[e0 + sl];
+                        const int c = w.order[rank];
+                        const double carried = w.ev_carried[rank];
+                        const int q0 = w.poff[sl], q1 = min(w.poff[sl + 1], P);   // P: past an overflow
+                        const int succ0 = q0 + lane < q1 ? w.pair_succ[q0 + lane] : -1;
+                        LakeFan fan{};
+                        double budget = 0.0;
+                        if (kind_slot == 1) {
+                            fan.n = w.slot_n[sl];
+                            fan.sorted = w.pool_cells + w.slot_off[sl];
+                            fan.base = w.pool_base + w.slot_off[sl];
+                            fan.load(0, lane);
+                            budget = mouth_budget(w.p, w.f, c, carried, LAKE);
+                        }
                         int go = 1;
                         if (lane == 0) {
                             long long spins = 0;
-                            while (*(volatile int*)&w.blockers[sl] != 0) {
+                            cuda::atomic_ref<int, cuda::thread_scope_device> waits(w.blockers[sl]);
+                            while (waits.load(cuda::memory_order_acquire) != 0) {
                                 if (*(volatile int*)&w.words[W_ABORT] || ++spins > kSpinLimit) {
                                     atomicOr(&w.words[W_ERROR], 4);
                                     atomicExch(&w.words[W_ABORT], 1);
                                     go = 0;
                                     break;
                                 }
-                                __nanosleep(64);
+                                __nanosleep(32);
                             }
                         }
                         if (!__shfl_sync(0xFFFFFFFFu, go, 0)) continue;
-                        __threadfence();
-                        const int rank = w.events[e0 + sl];
-                        const int c = w.order[rank];
-                        const double carried = w.ev_carried[rank];
+                        __syncwarp();
+                        double laid = 0.0;
                         if (kind_slot == 1) {
-                            lay_lake_warp(w, sl, mouth_budget(w.p, w.f, c, carried, LAKE), lane);
+                            laid = lay_lake_warp(w, sl, fan, budget, lane);
                         } else {
                             uint32_t* bits = w.warp_bits + (size_t)gwarp * w.box_words;
                             for (int j = lane; j < w.box_words; j += 32) bits[j] = 0u;
@@ -990,14 +1089,13 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                                 w.slot_touch_n[sl] = log.count;
                             }
                         }
+                        // What was laid is visible before the mouths after it are let go.
                         __syncwarp();
                         __threadfence();
-                        for (int q = w.poff[sl] + lane; q < min(w.poff[sl + 1], P); q += 32)   // P: past an overflow
+                        if (succ0 >= 0 && index_ok(w, succ0, S, 11)) atomicSub(&w.blockers[succ0], 1);
+                        for (int q = q0 + 32 + lane; q < q1; q += 32)
                             if (w.pair_succ[q] >= 0 && index_ok(w, w.pair_succ[q], S, 11)) atomicSub(&w.blockers[w.pair_succ[q]], 1);
-                        if (lane == 0) {
-                            if (kind_slot == 1) w.handoff[c] = __dsub_rn(carried, w.slot_laid[sl]);
-                            w.slot_state[sl] = 0;
-                        }
+                        if (kind_slot == 1 && lane == 1) w.handoff[c] = __dsub_rn(carried, laid);
                     }
                     grid.sync();
                     ++waves;
@@ -1008,93 +1106,69 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                     t0 = t;
                 }
                 // The chunk's deposits into the level's log in rank order: each event's entries at the
-                // offset of the events before it.
+                // offset of the events before it. A deposit that makes a mouth conflict lists it.
                 if (blockIdx.x == 0) {
                     const int* tn = w.slot_touch_n;
-                    cta_exclusive_scan([=](int i) { return tn[i]; }, S, w.poff, sh_scan);
-                    if (threadIdx.x == 0) {
-                        w.words[W_WAVES] += waves;
-                        w.words[W_TOUCHN] = touch_n;
-                    }
+                    cta_exclusive_scan([=](int i) { return __ldcg(&tn[i]); }, S, w.poff, sh_scan);
+                    if (threadIdx.x == 0) w.words[W_WAVES] += waves;
                 }
                 grid.sync();
                 {
-                    const int base = *(volatile int*)&w.words[W_TOUCHN];
-                    const int total = w.poff[S];
-                    const int room = w.touch_cap - base;
+                    const int total = __ldcg(&w.poff[S]);
+                    const int room = w.touch_cap - touch_n;
                     const int copied = total < room ? total : room;
-                    if (total > room && blockIdx.x == 0 && threadIdx.x == 0) w.words[W_ERROR] |= 1;
-                    const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), stride = (int)(gridDim.x * blockDim.x);
-                    for (int e = tid; e < S; e += stride) w.ev_touch[e0 + e] = base + min(w.poff[e], copied);
+                    if (total > room && timer) w.words[W_ERROR] |= 1;
+                    for (int e = tid; e < S; e += stride) w.ev_touch[e0 + e] = touch_n + min(__ldcg(&w.poff[e]), copied);
                     for (int q = tid; q < copied; q += stride) {
                         int a = 0, b = S;
                         while (b - a > 1) {
                             const int m = (a + b) >> 1;
-                            if (w.poff[m] <= q) a = m;
+                            if (__ldcg(&w.poff[m]) <= q) a = m;
                             else b = m;
                         }
-                        w.touches[base + q] = w.slot_touch[(size_t)a * w.cap + (q - w.poff[a])];
-                        w.touch_ev[base + q] = e0 + a;
+                        const Touch t = w.slot_touch[(size_t)a * w.cap + (q - __ldcg(&w.poff[a]))];
+                        w.touches[touch_n + q] = t;
+                        w.touch_ev[touch_n + q] = e0 + a;
+                        find_conflict(w, L, t.cell, w.events[e0 + a], clash_gen);
                     }
-                    if (blockIdx.x == 0 && threadIdx.x == 0) touch_n = base + copied;
+                    touch_n += copied;
                 }
+                e0 = e1;
                 if (timer) tm[T_SEAS] += now_ns() - t0;
                 grid.sync();
+                continue;
             }
+            // Every event before the conflicted cell is laid; those after it in its chunk are undone.
             if (timer) t0 = now_ns();
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                w.ev_touch[n_now] = touch_n;
-                if (pass == 0) refit_gen = ++w.words[W_GEN];
-                w.words[W_REFITGEN] = refit_gen;
-                w.words[W_BEST] = INT_MAX;
-                w.words[W_TOUCHN] = touch_n;
-            }
-            grid.sync();
-            mouth_conflicts_grid(w, L, n_now);
-            grid.sync();
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                const int best = *(volatile int*)&w.words[W_BEST];
-                const int rc = best == INT_MAX ? -1 : best;
-                if (rc < 0) {
-                    w.words[W_DONE] = 1;
-                } else {
-                    if (pass == passes) w.words[W_ERROR] |= 8;
-                    int a = 0, b = n_now;   // the first event ranked at or after rc (events are in rank order)
-                    while (a < b) {
-                        const int m = (a + b) >> 1;
-                        if (w.events[m] < rc) a = m + 1;
-                        else b = m;
-                    }
-                    w.words[W_ESTART] = a;
-                    w.words[W_CUT] = a < n_now ? w.ev_touch[a] : touch_n;
-                    w.words[W_RC] = rc;
-                    w.words[W_DONE] = 0;
-                }
-            }
-            grid.sync();
-            if (!*(volatile int*)&w.words[W_DONE]) {
-                // Every fan ranked at or after rc undone, the log cut back to before them, the cell refitted.
-                const int cut = *(volatile int*)&w.words[W_CUT];
-                undo_from_grid(w, cut, *(volatile int*)&w.words[W_TOUCHN]);
+            grid.sync();   // every thread has read the conflicts and the events
+            if (limit < e0) {
+                const int cut = __ldcg(&w.ev_touch[limit]);
+                undo_from_grid(w, cut, touch_n);
+                touch_n = cut;
                 grid.sync();
-                if (blockIdx.x == 0 && threadIdx.x == 0) {
-                    touch_n = cut;
-                    int nn = n_now;
-                    refit_mouth_cell(w, w.words[W_RC], w.words[W_ESTART], refit_gen, &nn);
-                    w.words[W_EVENTS] = nn;
-                    w.words[W_RELAID]++;
-                }
+            }
+            if (tid == 0) {
+                w.words[W_INSERT] = refit_mouth_cell(w, rc, limit, n_now) ? 1 : 0;
+                w.words[W_RELAID]++;
+                for (int i = 0; i < clashes; ++i)
+                    if (w.refit[i] == rc) w.refit[i] = INT_MAX;
             }
             grid.sync();
+            if (*(volatile int*)&w.words[W_INSERT]) {   // the events from `limit` on move up by one
+                int* kept = w.seg_events + lo;
+                for (int i = limit + tid; i < n_now; i += stride) kept[i - limit] = w.events[i];
+                grid.sync();
+                for (int i = limit + tid; i < n_now; i += stride) w.events[i + 1] = __ldcg(&kept[i - limit]);
+                if (tid == 0) w.events[limit] = rc;
+                ++n_now;
+                grid.sync();
+            }
+            e0 = limit;
             if (timer) tm[T_REPAIRS] += now_ns() - t0;
-            if (*(volatile int*)&w.words[W_DONE]) break;
-            e_start = *(volatile int*)&w.words[W_ESTART];
-            n_now = *(volatile int*)&w.words[W_EVENTS];
-            grid.sync();
         }
         // C: the last repairs, with every deposit of the level in its log.
         if (timer) t0 = now_ns();
-        if (n_now > 0) final_repairs_grid(w, L, n_now, touch_n, sh_scan);
+        final_repairs_grid(w, L, n_now, touch_n, sh_scan);
         grid.sync();
         if (timer) tm[T_REPAIRS] += now_ns() - t0;
     }
@@ -1420,10 +1494,9 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_deposit_levels, kThreads, 0));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "deposition kernel cannot be resident");
     const int cgrid = ctx->num_sms * (per_sm < 2 ? per_sm : 2);
-    CG_BUF(int, d_segc, ctx, S_DEPSEGC, 3 * (size_t)cgrid + 2);
+    CG_BUF(int, d_segc, ctx, S_DEPSEGC, 3 * (size_t)cgrid);
     w.seg_count = d_segc;
-    w.seg_off = d_segc + cgrid;
-    w.seg_part = d_segc + 2 * (size_t)cgrid + 1;
+    w.seg_part = d_segc + 2 * (size_t)cgrid;
     // A heap per warp, for the sea lobes.
     w.heap_warps = cgrid * (kThreads / 32);
     const size_t HC = (size_t)w.heap_warps * cap;
