@@ -19,9 +19,9 @@
 //     (fan, cell) pairs and the sea lobes' (lobe, box tile) pairs grouped by cell or tile, each mouth
 //     counting the earlier mouths on its cells or tiles and learning the next ones. A mouth's warp
 //     waits for its count to reach 0 (a bounded poll inside the cooperative launch), lays (a lake fan
-//     as a scan of its sorted cells, 32 needs at a time; a sea lobe whole on lane 0, its admission
-//     reading the sediment earlier lobes laid), and releases the next ones. Every deposit is logged,
-//     and the level's log is assembled in rank order from the mouths' own logs.
+//     as a scan of its sorted cells; a sea lobe whole, its admission reading the sediment earlier lobes
+//     laid), and releases the next ones. Every deposit is logged, and the level's log is assembled in
+//     rank order from the mouths' own logs.
 //  C. a fan changes only sea cells and ponded land, which no own walk reads, except (a) a ponded cell
 //     of the fan's own level ranked after it, whose settled height took its own subtraction before
 //     the fan's addition instead of after: its settled height is replayed in rank order from its
@@ -130,6 +130,8 @@ struct WalkDev {
     float* heap_keys;
     float* heap_pens;
     int* heap_admitted;
+    unsigned long long* heap_sorted;   // per warp: a sea lobe's admitted cells by distance (`cap`)
+    int lobe_words;         // words of a lobe's box in shared memory, even; 0: lobes take the heap
     int* stamp;             // per cell: the stage's fan stamps
     // The level's fan deposits, for the repairs.
     Touch* touches;
@@ -427,8 +429,17 @@ struct LakeFan {
     }
 };
 
-__device__ __forceinline__ bool above_zero(double x) { return __double_as_longlong(x) > 0; }
-__device__ __forceinline__ bool below(double x, double y) { return __double_as_longlong(x) < __double_as_longlong(y); }
+// FP64 comparisons on the integer pipes (an FP64 instruction holds its unit 64 cycles), with a NaN's
+// answers: x > 0; !(x <= 0); x < y for an x that is above 0 or NaN and a y above 0.
+__device__ __forceinline__ bool above_zero(double x) {
+    return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7FF0000000000000ull;
+}
+__device__ __forceinline__ bool not_below_zero(double x) {
+    return __double_as_longlong(x) > 0 || (unsigned long long)__double_as_longlong(x) > 0xFFF0000000000000ull;
+}
+__device__ __forceinline__ bool below(double x, double y) {
+    return (unsigned long long)__double_as_longlong(x) < (unsigned long long)__double_as_longlong(y);
+}
 
 // A lake fan's laying by one warp (lay_admitted's loop over the distance-sorted admitted cells). A
 // fan's cells are distinct, so laying into one changes no other's need: the warp reads 64 cells at
@@ -457,7 +468,7 @@ __device__ double lay_lake_warp(const WalkDev& w, int s, LakeFan& fan, double bu
 #pragma unroll
         for (int u = 0; u < kLakeAhead; ++u) {
             const double need = __dsub_rn(fan.b[u], (double)prior[u]);
-            unsigned live = __ballot_sync(FULL, valid[u] && above_zero(need));
+            unsigned live = __ballot_sync(FULL, valid[u] && not_below_zero(need));
             while (live) {
                 if (!above_zero(__shfl_sync(FULL, acc, 0))) {
                     live = 0;
@@ -509,6 +520,226 @@ __device__ double lay_lake_warp(const WalkDev& w, int s, LakeFan& fan, double bu
     if (lane == 1) w.slot_laid[s] = acc;
     if (lane == 0) w.slot_touch_n[s] = logged;
     return acc;
+}
+
+// A warp's scratch in shared memory for a sea lobe's admission: the frontier, unordered (its key and cell
+// as one integer that orders as the heap does, and its penalty), and the visited bits of the lobe's box.
+constexpr int kFrontier = 384;       // frontier cells at most; a lobe that needs more takes the heap
+constexpr int kLobeBoxWords = 1024;  // box words at most; larger boxes take the heap
+struct Lobe {
+    unsigned long long* key;
+    float* pen;
+    uint32_t* bits;
+};
+__host__ __device__ inline size_t lobe_bytes(int words) { return (size_t)kFrontier * 12 + (size_t)words * 4; }
+
+// admit (DeltaFan.growFan's best-first growth) of a sea lobe by one warp: the frontier's least (key, cell)
+// by a scan of the lanes and two reductions, its eight neighbours a lane each. The order cells enter an
+// unordered frontier does not matter, and the eight are different cells (the grid is at least 4 wide).
+// Returns the admitted count, or -1 where the frontier or the list would overflow or a height is NaN. One cell costs about a
+// load's latency and 200 instructions, where one lane with a heap in global memory took 2.5 us.
+__device__ int admit_sea_warp(const WalkDev& w, const Rim& m, const Lobe& lobe, int* admitted, int* outside) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const Params& p = w.p;
+    for (int j = lane; j < w.box_words; j += 32) lobe.bits[j] = 0u;
+    __syncwarp();
+    BoxVisited visited{lobe.bits, p.W, m.apex_column, m.apex_row, w.box_x, w.box_y, outside};
+    if (lane == 0) {
+        visited.mark(m.apex);
+        lobe.key[0] = (unsigned)m.apex;   // key 0
+        lobe.pen[0] = 0.0f;
+    }
+    int size = 1, count = 0;
+    const float apex_top = w.f.surface[m.apex] + ld_l2(&w.f.sediment[m.apex]);
+    bool nan = apex_top != apex_top;
+    while (size > 0) {
+        __syncwarp();
+        unsigned long long best = ~0ull;
+        int at = 0;
+        for (int i = lane; i < size; i += 32) {
+            const unsigned long long k = lobe.key[i];
+            if (k < best) {
+                best = k;
+                at = i;
+            }
+        }
+        const unsigned hi = __reduce_min_sync(FULL, (unsigned)(best >> 32));
+        const unsigned lo = __reduce_min_sync(FULL, (unsigned)(best >> 32) == hi ? (unsigned)best : 0xFFFFFFFFu);
+        const unsigned owner = __ballot_sync(FULL, best == (((unsigned long long)hi << 32) | lo));
+        at = __shfl_sync(FULL, at, __ffs(owner) - 1);
+        const int cur = (int)lo;
+        const float penalty = lobe.pen[at];
+        if (count >= w.cap) return -1;
+        __syncwarp();
+        --size;
+        if (lane == 0) {
+            admitted[count] = cur;
+            lobe.key[at] = lobe.key[size];
+            lobe.pen[at] = lobe.pen[size];
+        }
+        ++count;
+        __syncwarp();
+        bool push = false;
+        int n = 0;
+        float key = 0.0f, np = 0.0f;
+        if (lane < 8) {
+            const int k = lane < 4 ? lane : lane + 1;   // rows, then columns, the cell itself left out
+            const int sy = k / 3 - 1, sx = k % 3 - 1;
+            const int nr = pdiv(cur, p.W) + sy;
+            if (nr >= 0 && nr < p.H) {
+                n = nr * p.W + wrap_col(pmod(cur, p.W) + sx, p.W);
+                const float top = w.f.surface[n] + ld_l2(&w.f.sediment[n]);   // read beside the land, not after it
+                nan |= top != top;
+                if (!visited.seen(n) && mouth_accepts(p, w.f, true, n)) {
+                    const float co = rim_column_offset(m, n), ro = rim_row_offset(m, n);
+                    const float distance = sqrt_rn(co * co + ro * ro);
+                    const float depth = p.shoreline - top;
+                    const float advance = 1.0f + kDepthCost * (depth > 0.0f ? depth : 0.0f) / p.shelf_depth;
+                    np = penalty + step_of(p, sx, sy) * (advance - 1.0f);
+                    key = distance + np;
+                    push = !(key > rim_radius(m, co, ro, distance));
+                }
+            }
+        }
+        const unsigned pushes = __ballot_sync(FULL, push);
+        if (size + __popc(pushes) > kFrontier) return -1;
+        if (push) {
+            const int slot = size + __popc(pushes & ((1u << lane) - 1u));
+            lobe.key[slot] = ((unsigned long long)__float_as_uint(key) << 32) | (unsigned)n;
+            lobe.pen[slot] = np;
+            const int i = visited.index(n);
+            atomicOr(&lobe.bits[i >> 5], 1u << (i & 31));
+        }
+        size += __popc(pushes);
+    }
+    return __any_sync(FULL, nan) ? -1 : count;
+}
+
+// n keys ascending by one warp, in place: the all-ascending bitonic network (each merge first compares i
+// with its mirror, so a partner past the end never moves).
+__device__ void sort_warp(unsigned long long* key, int n) {
+    const int lane = threadIdx.x & 31;
+    for (int k = 2; k < 2 * n; k <<= 1) {
+        for (int j = k - 1; j > 0; j = (j == k - 1) ? (k >> 2) : (j >> 1)) {
+            for (int i = lane; i < n; i += 32) {
+                const int l = i ^ j;
+                if (l > i && l < n) {
+                    const unsigned long long a = key[i], b = key[l];
+                    if (a > b) {
+                        key[i] = b;
+                        key[l] = a;
+                    }
+                }
+            }
+            __syncwarp();
+            if (k == 2) break;
+        }
+    }
+}
+
+// A sea lobe whole by one warp: its rim, its admission, and its laying, the admitted cells sorted by
+// distance and cell (the laying heap's pop order) and taken 32 at a time. A lobe lays whole cells, so every
+// deposit is the cell's whole need, worked out by its lane; what remains of the budget runs in order, as
+// in lay_lake_warp, and the first cell whose need is above it ends the lobe. Returns false where the
+// admission needs the heap. With lane 0 running the whole lobe a four-round 8192 x 4096 stage spent
+// 466 ms depositing, with the warp 407 ms; the twelve rounds at 1024 x 512 went from 36 to 35 ms.
+__device__ bool sea_lobe_warp(const WalkDev& w, int c, double carried, const Lobe& lobe, int* admitted,
+                              unsigned long long* sorted, TouchLog& log, int* outside) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const Params& p = w.p;
+    double remaining = mouth_budget(p, w.f, c, carried, SEA);
+    Rim m;
+    const int receiver = w.f.dirs[c];
+    rim_init(m, receiver, p.W, p.r, p.step_ns, p.step_diag, (float)p.reach_cells,
+             (float)shortest_x(pmod(receiver, p.W) - pmod(c, p.W), p.W), (float)(pdiv(receiver, p.W) - pdiv(c, p.W)),
+             fan_hash(p.seed, mouth_key(receiver, p.reach_cells, p.W)), true);
+    // rim_prune, a groove's steps a lane each: a ray that meets land or leaves the map is dropped.
+    int kept = 0;
+    const float stride = 1.0f < m.row_scale ? 1.0f : m.row_scale;
+    for (int g = 0; g < m.distributaries; ++g) {
+        const float rx = m.groove_x[g], ry = m.groove_y[g];
+        const float far = (float)(int)rim_radius(m, rx, ry, 1.0f);
+        bool blocked = false;
+        float base = 0.0f;
+        while (!blocked && base <= far) {
+            float along = base, next = base;
+            for (int t = 0; t < 32; ++t) {   // the reference's running sum of strides
+                next += stride;
+                if (t <= lane) along = next;
+            }
+            bool mine = false;
+            if (along <= far) {
+                const int row = m.apex_row + (int)(ry * along / m.row_scale);
+                int column = (m.apex_column + (int)(rx * along)) % p.W;
+                if (column < 0) column += p.W;
+                mine = row < 0 || row >= p.H || w.f.land[row * p.W + column];
+            }
+            blocked = __any_sync(FULL, mine);
+            base = next;
+        }
+        if (blocked) continue;
+        m.groove_x[kept] = rx;
+        m.groove_y[kept] = ry;
+        ++kept;
+    }
+    m.live = kept;
+    if (remaining <= 0.0 || !mouth_accepts(p, w.f, true, m.apex)) return true;
+    const int count = admit_sea_warp(w, m, lobe, admitted, outside);
+    if (count < 0) return false;
+    for (int i = lane; i < count; i += 32) {
+        const int x = admitted[i];
+        const float co = rim_column_offset(m, x), ro = rim_row_offset(m, x);
+        sorted[i] = ((unsigned long long)__float_as_uint(sqrt_rn(co * co + ro * ro)) << 32) | (unsigned)x;
+    }
+    __syncwarp();
+    sort_warp(sorted, count);
+    for (int i0 = 0; i0 < count && remaining > 0.0; i0 += 32) {
+        const int i = i0 + lane;
+        int x = 0;
+        float prior = 0.0f, settled = 0.0f;
+        double need = 0.0;
+        if (i < count) {
+            x = (int)(sorted[i] & 0xFFFFFFFFull);
+            prior = ld_l2(&w.f.sediment[x]);
+            settled = ld_l2(&w.f.settled[x]);
+            const float co = rim_column_offset(m, x), ro = rim_row_offset(m, x);
+            float fraction = sqrt_rn(co * co + ro * ro) / m.reach_cells;
+            if (fraction > 1.0f) fraction = 1.0f;
+            float level = p.delta_top + (p.rim_top - p.delta_top) * fraction;
+            if (rim_grooved(m, co, ro)) level = p.shoreline + (level - p.shoreline) * kGrooveKeep;
+            need = (double)level - (double)w.f.surface[x] - (double)prior;
+        }
+        const float now = (float)((double)prior + need);
+        const double moved = (double)now - (double)prior;
+        unsigned live = __ballot_sync(FULL, i < count && above_zero(need));
+        double before = 0.0;
+        for (unsigned u = live; u; u &= u - 1) {
+            const int j = __ffs(u) - 1;
+            if (lane == j) before = remaining;
+            remaining -= __shfl_sync(FULL, moved, j);
+        }
+        const unsigned whole = __ballot_sync(FULL, above_zero(before) && !below(before, need));
+        const unsigned stop = live & ~whole;
+        if (stop) {   // nothing remains, or not the whole of the next cell
+            live &= (1u << (__ffs(stop) - 1)) - 1u;
+            remaining = 0.0;
+        }
+        if ((live >> lane) & 1u) {
+            const int at = log.count + __popc(live & ((1u << lane) - 1u));
+            const float increment = (float)(moved * (double)p.to_relative);
+            if (at < log.capacity) log.touches[at] = Touch{x, settled, prior, increment};
+            st_l2(&w.f.sediment[x], now);
+            st_l2(&w.f.settled[x], settled + increment);
+        }
+        log.count += __popc(live);
+        if (log.count > log.capacity) {
+            log.count = log.capacity;
+            log.overflow = 1;
+        }
+    }
+    return true;
 }
 
 // The kind of a cell's step (own_walk's answer), read from the fixed fields alone.
@@ -767,6 +998,14 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
     const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), stride = (int)(gridDim.x * blockDim.x);
     const int gwarp = tid >> 5, nwarps = stride >> 5;
     const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
+    extern __shared__ unsigned long long lobe_smem[];   // a Lobe per warp, where the grid's lobes fit one
+    Lobe lobe{nullptr, nullptr, nullptr};
+    if (w.lobe_words > 0) {
+        char* mine = (char*)lobe_smem + (size_t)warp * lobe_bytes(w.lobe_words);
+        lobe.key = (unsigned long long*)mine;
+        lobe.pen = (float*)(mine + (size_t)kFrontier * 8);
+        lobe.bits = (uint32_t*)(mine + (size_t)kFrontier * 12);
+    }
     unsigned long long tm[T_COUNT] = {0, 0, 0, 0, 0};
     unsigned long long t0 = 0;
     for (int L = 0; L < w.levels; ++L) {
@@ -1071,23 +1310,26 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                         if (kind_slot == 1) {
                             laid = lay_lake_warp(w, sl, fan, budget, lane);
                         } else {
-                            uint32_t* bits = w.warp_bits + (size_t)gwarp * w.box_words;
-                            for (int j = lane; j < w.box_words; j += 32) bits[j] = 0u;
-                            __syncwarp();
-                            if (lane == 0) {
-                                Heap h = warp_heap(w, gwarp);
-                                TouchLog log{w.slot_touch + (size_t)sl * w.cap, w.cap, 0, 0};
-                                int outside = 0;
-                                const int bx = w.box_x, by = w.box_y, W = w.p.W;
-                                mouth_with(w.p, w.f, c, carried, SEA,
-                                           [=, &outside](const Rim& m) {
-                                               return BoxVisited{bits, W, m.apex_column, m.apex_row, bx, by, &outside};
-                                           },
-                                           h, &log);
-                                if (log.overflow) atomicOr(&w.words[W_ERROR], 1);
-                                if (outside) atomicOr(&w.words[W_ERROR], 2);   // past the box its tiles cover
-                                w.slot_touch_n[sl] = log.count;
+                            TouchLog log{w.slot_touch + (size_t)sl * w.cap, w.cap, 0, 0};
+                            int outside = 0;
+                            if (!lobe.key || !sea_lobe_warp(w, c, carried, lobe, w.heap_admitted + (size_t)gwarp * w.cap,
+                                                            w.heap_sorted + (size_t)gwarp * w.cap, log, &outside)) {
+                                uint32_t* bits = w.warp_bits + (size_t)gwarp * w.box_words;
+                                for (int j = lane; j < w.box_words; j += 32) bits[j] = 0u;
+                                __syncwarp();
+                                if (lane == 0) {
+                                    Heap h = warp_heap(w, gwarp);
+                                    const int bx = w.box_x, by = w.box_y, W = w.p.W;
+                                    mouth_with(w.p, w.f, c, carried, SEA,
+                                               [=, &outside](const Rim& m) {
+                                                   return BoxVisited{bits, W, m.apex_column, m.apex_row, bx, by, &outside};
+                                               },
+                                               h, &log);
+                                }
                             }
+                            if (log.overflow) atomicOr(&w.words[W_ERROR], 1);
+                            if (outside) atomicOr(&w.words[W_ERROR], 2);   // past the box its tiles cover
+                            if (lane == 0) w.slot_touch_n[sl] = log.count;
                         }
                         // What was laid is visible before the mouths after it are let go.
                         __syncwarp();
@@ -1490,8 +1732,14 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     // The round's own counts (the fan ids, generations and wave numbers carry on through the stage).
     for (int word : {W_REPLAYED, W_WAVES, W_REFITTED, W_RELAID, W_ABORT})
         CG_CUDA(ctx, cudaMemsetAsync(d_words + word, 0, sizeof(int), sm));
+    // A lobe's scratch in shared memory, for grids at least 4 wide whose lobes' boxes fit. The attribute is
+    // the kernel's, shared by every context of the process: always set to the most a launch asks for.
+    w.lobe_words = W >= 4 && w.box_words <= kLobeBoxWords ? (w.box_words + 1) & ~1 : 0;
+    const size_t smem = w.lobe_words > 0 ? (kThreads / 32) * lobe_bytes(w.lobe_words) : 0;
+    CG_CUDA(ctx, cudaFuncSetAttribute(k_deposit_levels, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)((kThreads / 32) * lobe_bytes(kLobeBoxWords))));
     int per_sm = 0;
-    CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_deposit_levels, kThreads, 0));
+    CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_deposit_levels, kThreads, smem));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "deposition kernel cannot be resident");
     const int cgrid = ctx->num_sms * (per_sm < 2 ? per_sm : 2);
     CG_BUF(int, d_segc, ctx, S_DEPSEGC, 3 * (size_t)cgrid);
@@ -1500,7 +1748,8 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     // A heap per warp, for the sea lobes.
     w.heap_warps = cgrid * (kThreads / 32);
     const size_t HC = (size_t)w.heap_warps * cap;
-    CG_BUF(int, d_hc, ctx, S_DEPHEAP, 4 * HC);
+    CG_BUF(int, d_hc, ctx, S_DEPHEAP, 6 * HC);
+    w.heap_sorted = (unsigned long long*)(d_hc + 4 * HC);
     w.heap_cells = d_hc;
     w.heap_keys = (float*)(d_hc + HC);
     w.heap_pens = (float*)(d_hc + 2 * HC);
@@ -1509,7 +1758,7 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     w.warp_bits = d_wbits;
     void* kargs[] = {&w};
     ctx->launches++;
-    CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_deposit_levels, cgrid, kThreads, kargs, 0, sm));
+    CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_deposit_levels, cgrid, kThreads, kargs, smem, sm));
     int words[W_WORDS];
     unsigned long long timers[T_COUNT];
     CG_CUDA(ctx, cudaMemcpyAsync(words, d_words, sizeof(words), cudaMemcpyDeviceToHost, sm));
