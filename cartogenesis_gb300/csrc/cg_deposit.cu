@@ -58,6 +58,8 @@ using namespace dep;
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kAdmitThreads = 512;   // k_admit_lakes's threads an SM
+constexpr int kPoolShare = 64;       // pool entries a lake fan is first given
 constexpr int kTile = 16;   // a sea lobe's box is scheduled in tiles of kTile x kTile cells
 constexpr int kNoTouch = 0x7F7F7F7F;   // `first`'s resting value (a byte-wise memset)
 constexpr long long kSpinLimit = 1LL << 24;   // a lake fan's wait for its turn, in polls (seconds)
@@ -212,8 +214,10 @@ struct AdmitDev {
     int cap, box_words;
     const int* cand;        // candidate mouth cells
     int ncand;
-    int* cand_n;            // pass 1 writes the admitted counts
-    const long long* cand_off;   // pass 2 reads the pool offsets
+    int* cand_n;            // per candidate: admitted cells
+    long long* cand_off;    // per candidate: first pool entry
+    long long pool_cap;     // entries the pool holds; past it a fan is only counted
+    unsigned long long* pool_used;
     int* pool_cells;
     double* pool_base;
     int* h_cells;           // per thread: a heap of `cap` entries and the visited bits of a box
@@ -221,7 +225,6 @@ struct AdmitDev {
     float* h_pens;
     int* h_admitted;
     uint32_t* h_bits;
-    int fill;               // 0: count, 1: fill the pool
     int* err;
 };
 
@@ -238,9 +241,12 @@ __global__ void k_lake_candidates(Params p, Fields f, int N, int* __restrict__ c
     }
 }
 
-// A candidate's admission; pass 1 counts its admitted cells, pass 2 writes them to the pool sorted by
-// distance from the apex with the cell as the tie break (the laying heap's pop order), each with its
-// level less its terrain (lay_admitted's need before the sediment).
+// A candidate's admission. Its admitted cells take the next entries of the pool, sorted by distance from
+// the apex with the cell as the tie break (the laying heap's pop order), each with its level less its
+// terrain (lay_admitted's need before the sediment); which entries a fan takes changes nothing. The
+// pool_used total tells the host whether the pool held them all. A heap walk is a chain of dependent
+// loads, so what counts is how many run at once: in a four-round 8192 x 4096 stage a count and a filling
+// launch of 128 threads an SM took 80 ms, one launch of 256 to 512 threads an SM 21 ms.
 __global__ void __launch_bounds__(128) k_admit_lakes(AdmitDev a) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int threads = gridDim.x * blockDim.x;
@@ -259,18 +265,18 @@ __global__ void __launch_bounds__(128) k_admit_lakes(AdmitDev a) {
         Heap h{cells, keys, pens, admitted, a.cap, 0, 0};
         const int n = admit(a.p, a.f, m, false, visited, h);
         if (outside) atomicOr(a.err, 2);   // the rim reached past its box: cannot happen
-        if (!a.fill) {
-            a.cand_n[i] = n;
-            continue;
-        }
+        const long long at = (long long)atomicAdd(a.pool_used, (unsigned long long)n);
+        a.cand_n[i] = n;
+        a.cand_off[i] = at;
+        if (at + n > a.pool_cap) continue;
         h.size = 0;
         for (int k = 0; k < n; ++k) {
             const int x = admitted[k];
             const float co = rim_column_offset(m, x), ro = rim_row_offset(m, x);
             heap_push(h, x, sqrt_rn(co * co + ro * ro), 0.0f);
         }
-        int* sorted = a.pool_cells + a.cand_off[i];
-        double* base = a.pool_base + a.cand_off[i];
+        int* sorted = a.pool_cells + at;
+        double* base = a.pool_base + at;
         int got = 0, x;
         float pen;
         while (heap_pop(h, x, pen)) {
@@ -286,34 +292,6 @@ __global__ void __launch_bounds__(128) k_admit_lakes(AdmitDev a) {
             ++got;
         }
     }
-}
-
-// Exclusive prefix sum of n 64-bit counts by one CTA, chunk after chunk; out[n] receives the total.
-__global__ void __launch_bounds__(1024) k_scan64_one_block(const long long* __restrict__ in, long long* __restrict__ out,
-                                                          int n) {
-    __shared__ long long sh[1024];
-    long long carry = 0;
-    for (int base = 0; base < n; base += 1024) {
-        const int i = base + (int)threadIdx.x;
-        const long long v = i < n ? in[i] : 0;
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            const long long t = threadIdx.x >= (unsigned)o ? sh[threadIdx.x - o] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += t;
-            __syncthreads();
-        }
-        if (i < n) out[i] = carry + sh[threadIdx.x] - v;
-        const long long chunk = sh[1023];
-        __syncthreads();
-        carry += chunk;
-    }
-    if (threadIdx.x == 0) out[n] = carry;
-}
-
-__global__ void k_widen_counts(const int* __restrict__ n, int count, long long* __restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) out[i] = n[i];
 }
 
 // The exclusive prefix of v over the CTA's threads, and the CTA's total. sh holds kThreads / 32 ints and
@@ -1629,40 +1607,40 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
         a.cand_n = d_candn;
         a.cand_off = d_candoff;
         a.err = d_words + W_ERROR;
-        const int threads = ctx->num_sms * 128;
-        const size_t T = (size_t)threads;
+        // Threads: as many as the candidates, up to kAdmitThreads an SM, and no more than 4 GB of heaps
+        // allow (128 an SM at least).
+        const size_t each = cap * 16 + (size_t)w.box_words * 4;
+        int ctas = (int)std::min<long long>(((long long)ncand + 127) / 128, (long long)ctx->num_sms * (kAdmitThreads / 128));
+        ctas = std::min<long long>(ctas, std::max<long long>(ctx->num_sms, (long long)((4ull << 30) / (128 * each))));
+        const size_t T = (size_t)ctas * 128;
         CG_BUF(int, d_hc, ctx, S_DEPSLOT0, T * cap);
         CG_BUF(float, d_hk, ctx, S_DEPSLOT1, T * cap);
         CG_BUF(float, d_hp, ctx, S_DEPSLOT2, T * cap);
         CG_BUF(int, d_ha, ctx, S_DEPSLOT3, T * cap);
         CG_BUF(uint32_t, d_hb, ctx, S_DEPSLOT6, T * (size_t)w.box_words);
+        CG_BUF(unsigned long long, d_used, ctx, S_DEPCANDW, 1);
         a.h_cells = d_hc;
         a.h_keys = d_hk;
         a.h_pens = d_hp;
         a.h_admitted = d_ha;
         a.h_bits = d_hb;
-        a.pool_cells = nullptr;
-        a.pool_base = nullptr;
-        a.fill = 0;
-        CG_LAUNCH(ctx) k_admit_lakes<<<ctx->num_sms, 128, 0, sm>>>(a);
-        CG_CHECK_LAUNCH(ctx);
-        // Offsets: an exclusive scan of the counts in 64 bits.
-        CG_BUF(long long, d_wide, ctx, S_DEPCANDW, (size_t)ncand + 1);
-        CG_LAUNCH(ctx) k_widen_counts<<<(ncand + 255) / 256, 256, 0, sm>>>(d_candn, ncand, d_wide);
-        CG_CHECK_LAUNCH(ctx);
-        CG_LAUNCH(ctx) k_scan64_one_block<<<1, 1024, 0, sm>>>(d_wide, d_candoff, ncand);
-        CG_CHECK_LAUNCH(ctx);
-        CG_CUDA(ctx, cudaMemcpyAsync(&pool_total, d_candoff + ncand, sizeof(long long), cudaMemcpyDeviceToHost, sm));
-        CG_CUDA(ctx, cudaStreamSynchronize(sm));
-        CG_BUF(int, d_pc, ctx, S_DEPSLOT4, (size_t)pool_total + 1);
-        CG_BUF(double, d_pb, ctx, S_DEPSLOT5, (size_t)pool_total + 1);
-        d_pool_cells = d_pc;
-        d_pool_base = d_pb;
-        a.pool_cells = d_pc;
-        a.pool_base = d_pb;
-        a.fill = 1;
-        CG_LAUNCH(ctx) k_admit_lakes<<<ctx->num_sms, 128, 0, sm>>>(a);
-        CG_CHECK_LAUNCH(ctx);
+        a.pool_used = d_used;
+        // A pool of kPoolShare cells a candidate holds all but unusually wide lakes' fans; those are
+        // counted by the first launch and admitted again by a second with the pool they need.
+        pool_total = (long long)ncand * std::min<long long>(w.cap, kPoolShare);
+        for (;;) {
+            a.pool_cap = pool_total;
+            CG_BUF(int, d_pc, ctx, S_DEPSLOT4, (size_t)pool_total + 1);
+            CG_BUF(double, d_pb, ctx, S_DEPSLOT5, (size_t)pool_total + 1);
+            a.pool_cells = d_pool_cells = d_pc;
+            a.pool_base = d_pool_base = d_pb;
+            CG_CUDA(ctx, cudaMemsetAsync(d_used, 0, sizeof(unsigned long long), sm));
+            CG_LAUNCH(ctx) k_admit_lakes<<<ctas, 128, 0, sm>>>(a);
+            CG_CHECK_LAUNCH(ctx);
+            CG_CUDA(ctx, cudaMemcpyAsync(&pool_total, d_used, sizeof(long long), cudaMemcpyDeviceToHost, sm));
+            CG_CUDA(ctx, cudaStreamSynchronize(sm));
+            if (pool_total <= a.pool_cap) break;
+        }
     }
     w.cand_of = d_candof;
     w.cand_n = d_candn;
