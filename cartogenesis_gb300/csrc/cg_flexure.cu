@@ -7,18 +7,22 @@
 // every row and then every column, each butterfly `odd * twiddle` then `even +/- rotated` with the
 // twiddles tabulated on the host exactly as the reference tabulates them. The order of the butterflies
 // inside a stage does not matter (each writes its own pair), so a line is transformed by one CTA with
-// the whole line in shared memory (up to 8192 complex doubles, 128 KB). Columns are transformed as rows
-// of the transposed grid (a tiled transpose between the passes keeps every access coalesced); the filter
-// is applied in the forward column pass and the inverse's 1 / (W 2H) in the inverse column pass, each
-// after the pass's last butterfly, where the reference applies them.
+// the whole line in shared memory (up to 8192 complex doubles, 144 KB with the padding). Columns are
+// transformed as rows of the transposed grid (a tiled transpose between the passes keeps every access
+// coalesced); the filter is applied in the forward column pass and the inverse's 1 / (W 2H) in the inverse
+// column pass, each after the pass's last butterfly, where the reference applies them. The mirrored half
+// of the rows is never transformed (its rows are the map's own, bit for bit), and the inverse column pass
+// keeps the real parts of the map's rows alone.
 //
 // The load's mean is the reference's sequential double sum in cell order (seq_sum_dev, bit for bit).
 // Everything else is elementwise or per line.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "cg_common.cuh"
 #include "cg_internal.h"
+#include "cg_mul64.cuh"
 #include "cg_params.h"
 
 namespace cg {
@@ -26,7 +30,7 @@ namespace {
 
 constexpr int kLineThreads = 512;
 constexpr int kMaxLine = 8192;        // W and 2H: one line of complex doubles in a CTA's shared memory
-constexpr int kMinLineElems = 2048;   // short lines share a CTA, this many elements at least
+constexpr int kMinLineElems = 1024;   // short lines share a CTA, this many elements at least
 
 int log2_of(int n) {
     int l = 0;
@@ -81,85 +85,211 @@ __global__ void k_flex_load(const float* __restrict__ work, const float* __restr
     }
 }
 
-enum { SRC_GRID = 0, SRC_LOAD = 1 };
-enum { POST_NONE = 0, POST_FILTER = 1, POST_SCALE = 2 };
+enum { SRC_GRID = 0, SRC_LOAD = 1, SRC_MIRROR = 2 };
+enum { POST_NONE = 0, POST_FILTER = 1, POST_REAL = 2 };
 
 struct LineArgs {
-    double2* grid;          // `lines` lines of n complex values, line l at grid + l n
+    const double2* in;      // SRC_GRID: `lines` lines of n complex values, line l at in + l n
+    double2* out;           // the transformed lines, the same way (may be `in`)
     int n, log2n, lines, per_cta;
     const double2* tw;      // n / 2 (cos, sin)
     int inverse;
-    int src;                // SRC_LOAD: line r is map row r (r < H) or 2H - 1 - r, less the mean, imaginary 0
-    const float* load;
+    int src;                // SRC_LOAD: line r is map row r less the mean, imaginary 0
+    const float* load;      // SRC_MIRROR: lines of n / 2 values at `in`, mirrored to n
     const double* mean;
     int post;               // POST_FILTER: line c is column c, element r its padded row
     FlexConsts k;
     int W, H2;
-    double scale;           // POST_SCALE
+    double scale;           // POST_REAL: the first half's real parts times the scale, as floats, to `real`
+    float* real;            // (lines of n / 2)
 };
+
+__device__ __forceinline__ bool plain(double2 v) { return plain_value(v.x) && plain_value(v.y); }
+
+// Fft1D's butterfly: (e, o) becomes (e + o t, e - o t). The four products run on the integer pipes.
+__device__ __forceinline__ void butterfly_by(double2& e, double2& o, double wr, double wi) {
+    double rr, ri;
+    if (plain(o)) {
+        const Value x(o.x), y(o.y);
+        const Weight c(wr), s(wi);
+        rr = __dsub_rn(product(x, c), product(y, s));
+        ri = __dadd_rn(product(x, s), product(y, c));
+    } else {
+        rr = __dsub_rn(__dmul_rn(o.x, wr), __dmul_rn(o.y, wi));
+        ri = __dadd_rn(__dmul_rn(o.x, wi), __dmul_rn(o.y, wr));
+    }
+    o = make_double2(__dsub_rn(e.x, rr), __dsub_rn(e.y, ri));
+    e = make_double2(__dadd_rn(e.x, rr), __dadd_rn(e.y, ri));
+}
+__device__ __forceinline__ void butterfly(double2& e, double2& o, double2 t, int inverse) {
+    butterfly_by(e, o, t.x, inverse ? t.y : -t.y);
+}
+
+// The same for the table's first twiddle, (1, 0): o times (1, +-0) is o, but for the sign of a zero part
+// (x - y (+-0) and x (+-0) + y of a -0).
+__device__ __forceinline__ void butterfly_by_one(double2& e, double2& o, int inverse) {
+    double2 r = o;
+    if (plain(o)) {
+        const long long minus_zero = (long long)0x8000000000000000ull;
+        const long long bx = __double_as_longlong(o.x), by = __double_as_longlong(o.y);
+        if (bx == minus_zero && (by < 0) == (inverse != 0)) r.x = 0.0;
+        if (by == minus_zero && (bx < 0) != (inverse != 0)) r.y = 0.0;
+    } else {
+        const double wi = inverse ? 0.0 : -0.0;
+        r.x = __dsub_rn(o.x, __dmul_rn(o.y, wi));
+        r.y = __dadd_rn(__dmul_rn(o.x, wi), o.y);
+    }
+    o = make_double2(__dsub_rn(e.x, r.x), __dsub_rn(e.y, r.y));
+    e = make_double2(__dadd_rn(e.x, r.x), __dadd_rn(e.y, r.y));
+}
+
+// deflectionMetres' response (Isostasy.kt:344-365) to a wavenumber's squared parts; 0 at the mean, where
+// the filtered value is +0.
+__device__ __forceinline__ double2 filtered(const FlexConsts& k, double ka2, double kd2, double2 v, double2* mirror) {
+    const double k2 = __dadd_rn(ka2, kd2);
+    if (k2 == 0.0) {
+        if (mirror) *mirror = make_double2(0.0, 0.0);
+        return make_double2(0.0, 0.0);
+    }
+    const double response = __ddiv_rn(1.0, __dadd_rn(k.restoring, __dmul_rn(__dmul_rn(k.rigidity, k2), k2)));
+    if (mirror) *mirror = make_double2(__dmul_rn(mirror->x, response), __dmul_rn(mirror->y, response));
+    return make_double2(__dmul_rn(v.x, response), __dmul_rn(v.y, response));
+}
 
 // Fft1D.transform over `per_cta` lines, each whole in shared memory: the bit-reversed reordering on
 // the way in, then the butterflies stage by stage (Fft.kt:25-96), then the pass's post step.
+//
+// Bound by FP64 issue: a butterfly of ten FP64 instructions held the unit 770 cycles, and 8192 lines of
+// 8192 took 10.5 ms a pass. So the products run on the integer pipes beside the six additions; the first
+// three stages stay in registers (the eight elements u + q n / 8 land on eight neighbours, and seven of
+// their twelve twiddles are 1); a mirror pair of elements shares the filter's response; and the last
+// pass works out only the real parts of the map's rows. Later stages go two at a time, in place. The four
+// passes took 41.9 ms at 8192 x 4096 and 2.22 ms at 2048 x 1024, and take 21.5 and 1.18 ms.
 __global__ void __launch_bounds__(kLineThreads) k_fft_lines(LineArgs a) {
     extern __shared__ double2 sh[];
-    const int n = a.n, half_n = n >> 1;
+    const int n = a.n, L = a.log2n, half_n = n >> 1;
     const int l0 = blockIdx.x * a.per_cta;
-    const int elems = a.per_cta * n;
-    for (int i = threadIdx.x; i < elems; i += blockDim.x) {
-        const int l = i >> a.log2n, j = i & (n - 1);
+    const int top = L >= 6 ? L - 3 : 31;   // the same for eight neighbours
+    const int pitch = n + (n >> 3) + 8;
+    // A line's element in shared memory, spread so that neither the eighths' bit-reversed stores nor the
+    // later stages' strides of 8 fall on the same banks.
+    auto at = [=](int l, int i) { return l * pitch + i + (i >> 3) + (i >> top); };
+    auto source = [=](int l, int j) {
         const int line = l0 + l;
         double2 v = make_double2(0.0, 0.0);
-        if (line < a.lines) {
-            if (a.src == SRC_LOAD) {
-                const int row = line < a.H2 / 2 ? line : a.H2 - 1 - line;
-                v.x = __dsub_rn((double)a.load[(size_t)row * n + j], *a.mean);
-            } else {
-                v = a.grid[(size_t)line * n + j];
-            }
+        if (line >= a.lines) return v;
+        if (a.src == SRC_LOAD) v.x = __dsub_rn((double)a.load[(size_t)line * n + j], *a.mean);
+        else if (a.src == SRC_MIRROR) v = a.in[(size_t)line * half_n + (j < half_n ? j : n - 1 - j)];
+        else v = a.in[(size_t)line * n + j];
+        return v;
+    };
+    int lh = 0;
+    if (L >= 4) {
+        const int eighth = n >> 3;
+        const double2 t1 = a.tw[eighth], t2 = a.tw[2 * eighth], t3 = a.tw[3 * eighth];
+        for (int i = threadIdx.x; i < a.per_cta * eighth; i += blockDim.x) {
+            const int l = i >> (L - 3), u = i & (eighth - 1);
+            double2 r0 = source(l, u), r4 = source(l, u + eighth), r2 = source(l, u + 2 * eighth),
+                    r6 = source(l, u + 3 * eighth), r1 = source(l, u + 4 * eighth), r5 = source(l, u + 5 * eighth),
+                    r3 = source(l, u + 6 * eighth), r7 = source(l, u + 7 * eighth);
+            butterfly_by_one(r0, r1, a.inverse);
+            butterfly_by_one(r2, r3, a.inverse);
+            butterfly_by_one(r4, r5, a.inverse);
+            butterfly_by_one(r6, r7, a.inverse);
+            butterfly_by_one(r0, r2, a.inverse);
+            butterfly(r1, r3, t2, a.inverse);
+            butterfly_by_one(r4, r6, a.inverse);
+            butterfly(r5, r7, t2, a.inverse);
+            butterfly_by_one(r0, r4, a.inverse);
+            butterfly(r1, r5, t1, a.inverse);
+            butterfly(r2, r6, t2, a.inverse);
+            butterfly(r3, r7, t3, a.inverse);
+            double2* to = sh + at(l, (int)(__brev((unsigned)u) >> (32 - (L - 3))) << 3);
+            to[0] = r0;
+            to[1] = r1;
+            to[2] = r2;
+            to[3] = r3;
+            to[4] = r4;
+            to[5] = r5;
+            to[6] = r6;
+            to[7] = r7;
         }
-        const int rj = a.log2n > 0 ? (int)(__brev((unsigned)j) >> (32 - a.log2n)) : 0;
-        sh[(l << a.log2n) + rj] = v;
+        lh = 3;
+    } else {
+        for (int i = threadIdx.x; i < a.per_cta * n; i += blockDim.x) {
+            const int l = i >> L, j = i & (n - 1);
+            sh[at(l, (int)(__brev((unsigned)j) >> (32 - L)))] = source(l, j);
+        }
     }
     __syncthreads();
-    for (int lh = 0; (1 << lh) < n; ++lh) {
-        const int half = 1 << lh, tws = n >> (lh + 1);
-        for (int b = threadIdx.x; b < a.per_cta * half_n; b += blockDim.x) {
-            const int l = b >> (a.log2n - 1), k = b & (half_n - 1);
-            const int pair = k & (half - 1);
-            const int e = (l << a.log2n) + ((k >> lh) << (lh + 1)) + pair;
-            const int o = e + half;
-            const double2 t = a.tw[pair * tws];
-            const double wr = t.x, wi = a.inverse ? t.y : -t.y;
-            const double2 od = sh[o], ev = sh[e];
-            const double rr = __dsub_rn(__dmul_rn(od.x, wr), __dmul_rn(od.y, wi));
-            const double ri = __dadd_rn(__dmul_rn(od.x, wi), __dmul_rn(od.y, wr));
-            sh[e] = make_double2(__dadd_rn(ev.x, rr), __dadd_rn(ev.y, ri));
-            sh[o] = make_double2(__dsub_rn(ev.x, rr), __dsub_rn(ev.y, ri));
+    const int stages = a.post == POST_REAL ? L - 1 : L;
+    while (lh < stages) {
+        const int half = 1 << lh;
+        if (lh + 1 < stages) {
+            for (int i = threadIdx.x; i < a.per_cta * (n >> 2); i += blockDim.x) {
+                const int l = i >> (L - 2), k = i & ((n >> 2) - 1);
+                const int pair = k & (half - 1), base = ((k >> lh) << (lh + 2)) + pair;
+                double2 *p0 = sh + at(l, base), *p1 = sh + at(l, base + half), *p2 = sh + at(l, base + 2 * half),
+                        *p3 = sh + at(l, base + 3 * half);
+                double2 r0 = *p0, r1 = *p1, r2 = *p2, r3 = *p3;
+                const double2 t = a.tw[pair * (n >> (lh + 1))];
+                butterfly(r0, r1, t, a.inverse);
+                butterfly(r2, r3, t, a.inverse);
+                butterfly(r0, r2, a.tw[pair * (n >> (lh + 2))], a.inverse);
+                butterfly(r1, r3, a.tw[(pair + half) * (n >> (lh + 2))], a.inverse);
+                *p0 = r0;
+                *p1 = r1;
+                *p2 = r2;
+                *p3 = r3;
+            }
+            lh += 2;
+        } else {
+            for (int i = threadIdx.x; i < a.per_cta * half_n; i += blockDim.x) {
+                const int l = i >> (L - 1), k = i & (half_n - 1);
+                const int pair = k & (half - 1), base = ((k >> lh) << (lh + 1)) + pair;
+                double2 *p0 = sh + at(l, base), *p1 = sh + at(l, base + half);
+                double2 r0 = *p0, r1 = *p1;
+                butterfly(r0, r1, a.tw[pair * (n >> (lh + 1))], a.inverse);
+                *p0 = r0;
+                *p1 = r1;
+            }
+            lh += 1;
         }
         __syncthreads();
     }
-    for (int i = threadIdx.x; i < elems; i += blockDim.x) {
-        const int l = i >> a.log2n, j = i & (n - 1);
+    if (a.post == POST_NONE) {
+        for (int i = threadIdx.x; i < a.per_cta * n; i += blockDim.x) {
+            const int l = i >> L, j = i & (n - 1);
+            if (l0 + l < a.lines) a.out[(size_t)(l0 + l) * n + j] = sh[at(l, j)];
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < a.per_cta * half_n; i += blockDim.x) {
+        const int l = i >> (L - 1), j = i & (half_n - 1);
         const int line = l0 + l;
         if (line >= a.lines) continue;
-        double2 v = sh[i];
-        if (a.post == POST_FILTER) {   // deflectionMetres' response (Isostasy.kt:344-365)
-            const int cycles_down = j <= a.H2 / 2 ? j : j - a.H2;
-            const double kd = __dmul_rn((double)cycles_down, a.k.per_down);
-            const int cycles_across = line <= a.W / 2 ? line : line - a.W;
-            const double ka = __dmul_rn((double)cycles_across, a.k.per_across);
-            const double k2 = __dadd_rn(__dmul_rn(ka, ka), __dmul_rn(kd, kd));
-            if (k2 == 0.0) {
-                v = make_double2(0.0, 0.0);
-            } else {
-                const double response =
-                    __ddiv_rn(1.0, __dadd_rn(a.k.restoring, __dmul_rn(__dmul_rn(a.k.rigidity, k2), k2)));
-                v = make_double2(__dmul_rn(v.x, response), __dmul_rn(v.y, response));
-            }
-        } else if (a.post == POST_SCALE) {   // Fft2D.inverse's roundTripScale
-            v = make_double2(__dmul_rn(v.x, a.scale), __dmul_rn(v.y, a.scale));
+        if (a.post == POST_REAL) {   // the last stage's real parts, Fft2D.inverse's roundTripScale
+            double2 e = sh[at(l, j)], o = sh[at(l, j + half_n)];
+            const double2 t = a.tw[j];
+            const double wi = a.inverse ? t.y : -t.y;
+            const double rr = plain(o) ? __dsub_rn(product(Value(o.x), Weight(t.x)), product(Value(o.y), Weight(wi)))
+                                       : __dsub_rn(__dmul_rn(o.x, t.x), __dmul_rn(o.y, wi));
+            a.real[(size_t)line * half_n + j] = (float)__dmul_rn(__dadd_rn(e.x, rr), a.scale);
+            continue;
         }
-        a.grid[(size_t)line * n + j] = v;
+        const int cycles_across = line <= a.W / 2 ? line : line - a.W;
+        const double ka = __dmul_rn((double)cycles_across, a.k.per_across), ka2 = __dmul_rn(ka, ka);
+        const double kd = __dmul_rn((double)j, a.k.per_down);   // element n - j is -j cycles: the same square
+        double2* out = a.out + (size_t)line * n;
+        if (j > 0) {
+            double2 m = sh[at(l, n - j)];
+            out[j] = filtered(a.k, ka2, __dmul_rn(kd, kd), sh[at(l, j)], &m);
+            out[n - j] = m;
+        } else {
+            out[0] = filtered(a.k, ka2, __dmul_rn(kd, kd), sh[at(l, 0)], nullptr);
+            const double kh = __dmul_rn((double)half_n, a.k.per_down);
+            out[half_n] = filtered(a.k, ka2, __dmul_rn(kh, kh), sh[at(l, half_n)], nullptr);
+        }
     }
 }
 
@@ -178,16 +308,16 @@ __global__ void k_transpose(const double2* __restrict__ in, double2* __restrict_
     }
 }
 
-// The bend read back from the transformed grid (held column-major: W lines of 2H) and applied
+// The bend read back from the transformed grid (held column-major: W lines of H) and applied
 // (HydraulicErosion.kt:873-884): surface += (deflection - bend) / metresPerFieldUnit, deflection = bend.
-// The deflection is the real part as float, map rows only; through 32 x 32 tiles.
-__global__ void k_flex_apply(const double2* __restrict__ t, int W, int H, int H2, float mpf, float* __restrict__ work,
+// Through 32 x 32 tiles.
+__global__ void k_flex_apply(const float* __restrict__ t, int W, int H, float mpf, float* __restrict__ work,
                              float* __restrict__ defl, float* __restrict__ bend_out) {
     __shared__ float tile[32][33];
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;   // tile: rows r0.., columns c0..
     for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
         const int c = c0 + dy, r = r0 + threadIdx.x;
-        if (r < H && c < W) tile[dy][threadIdx.x] = (float)t[(size_t)c * H2 + r].x;
+        if (r < H && c < W) tile[dy][threadIdx.x] = t[(size_t)c * H + r];
     }
     __syncthreads();
     for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
@@ -204,12 +334,16 @@ __global__ void k_flex_apply(const double2* __restrict__ t, int W, int H, int H2
     }
 }
 
+size_t line_bytes(int n) { return (size_t)(n + n / 8 + 8) * sizeof(double2); }
+
+// A thread for every eight elements, 64 to kLineThreads of them: enough warps for both pipes, and small
+// CTAs where lines are short, which even out over the SMs (one line of 1024 a CTA).
 cg_status fft_pass(cg_ctx* ctx, LineArgs a, cudaStream_t sm) {
     a.log2n = log2_of(a.n);
     a.per_cta = a.n >= kMinLineElems ? 1 : kMinLineElems / a.n;
     const int ctas = (a.lines + a.per_cta - 1) / a.per_cta;
-    const size_t smem = (size_t)a.per_cta * a.n * sizeof(double2);
-    CG_LAUNCH(ctx) k_fft_lines<<<ctas, kLineThreads, smem, sm>>>(a);
+    const int threads = std::min(kLineThreads, a.per_cta * a.n / 8);
+    CG_LAUNCH(ctx) k_fft_lines<<<ctas, threads, a.per_cta * line_bytes(a.n), sm>>>(a);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }
@@ -223,7 +357,7 @@ cg_status flexure_dev(cg_ctx* ctx, const cg_erosion_params& p, const float* d_lo
     cudaStream_t sm = ctx->stream;
     if (!ctx->flex_attr) {
         CG_CUDA(ctx, cudaFuncSetAttribute(k_fft_lines, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)(kMaxLine * sizeof(double2))));
+                                          (int)line_bytes(kMaxLine)));
         ctx->flex_attr = true;
     }
     // Twiddles, tabulated once per line length.
@@ -246,10 +380,11 @@ cg_status flexure_dev(cg_ctx* ctx, const cg_erosion_params& p, const float* d_lo
     a.k = k;
     a.W = W;
     a.H2 = H2;
-    // Forward: rows (the mirrored load less its mean), then columns with the filter.
-    a.grid = d_a;
+    // Forward: rows (the load less its mean; row 2H - 1 - r is row r again, so H of them), then columns,
+    // mirrored, with the filter.
+    a.out = d_a;
     a.n = W;
-    a.lines = H2;
+    a.lines = H;
     a.tw = d_tw;
     a.inverse = 0;
     a.src = SRC_LOAD;
@@ -258,34 +393,38 @@ cg_status flexure_dev(cg_ctx* ctx, const cg_erosion_params& p, const float* d_lo
     a.post = POST_NONE;
     CG_TRY_ST(fft_pass(ctx, a, sm));
     const dim3 tb(32, 8);
-    CG_LAUNCH(ctx) k_transpose<<<dim3((W + 31) / 32, (H2 + 31) / 32), tb, 0, sm>>>(d_a, d_b, H2, W);
-    a.grid = d_b;
+    CG_LAUNCH(ctx) k_transpose<<<dim3((W + 31) / 32, (H + 31) / 32), tb, 0, sm>>>(d_a, d_b, H, W);
+    a.in = d_b;
+    a.out = d_a;
     a.n = H2;
     a.lines = W;
     a.tw = d_tw + W / 2;
-    a.src = SRC_GRID;
+    a.src = SRC_MIRROR;
     a.post = POST_FILTER;
     CG_TRY_ST(fft_pass(ctx, a, sm));
     // Inverse: rows, then columns, then the round trip's scale.
-    CG_LAUNCH(ctx) k_transpose<<<dim3((H2 + 31) / 32, (W + 31) / 32), tb, 0, sm>>>(d_b, d_a, W, H2);
-    a.grid = d_a;
+    CG_LAUNCH(ctx) k_transpose<<<dim3((H2 + 31) / 32, (W + 31) / 32), tb, 0, sm>>>(d_a, d_b, W, H2);
+    a.in = a.out = d_b;
     a.n = W;
     a.lines = H2;
     a.tw = d_tw;
     a.inverse = 1;
+    a.src = SRC_GRID;
     a.post = POST_NONE;
     CG_TRY_ST(fft_pass(ctx, a, sm));
-    CG_LAUNCH(ctx) k_transpose<<<dim3((W + 31) / 32, (H2 + 31) / 32), tb, 0, sm>>>(d_a, d_b, H2, W);
-    a.grid = d_b;
+    CG_LAUNCH(ctx) k_transpose<<<dim3((W + 31) / 32, (H2 + 31) / 32), tb, 0, sm>>>(d_b, d_a, H2, W);
+    a.in = d_a;
+    a.out = nullptr;
     a.n = H2;
     a.lines = W;
     a.tw = d_tw + W / 2;
-    a.post = POST_SCALE;
+    a.post = POST_REAL;
     a.scale = 1.0 / ((double)W * (double)H2);
+    a.real = (float*)d_b;
     CG_TRY_ST(fft_pass(ctx, a, sm));
     const float mpf = scale_of(p).relief_span();
-    CG_LAUNCH(ctx) k_flex_apply<<<dim3((H + 31) / 32, (W + 31) / 32), tb, 0, sm>>>(d_b, W, H, H2, mpf, d_work, d_defl,
-                                                                                   bend_out);
+    CG_LAUNCH(ctx) k_flex_apply<<<dim3((H + 31) / 32, (W + 31) / 32), tb, 0, sm>>>((const float*)d_b, W, H, mpf, d_work,
+                                                                                   d_defl, bend_out);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }

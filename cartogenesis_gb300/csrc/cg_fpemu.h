@@ -107,7 +107,7 @@ __device__ __forceinline__ double from_binade(int64_t m, int e) {
 // U = 2^(e-52) (d = w / U rounded to nearest, read off the bits of w), so a run of lanes is an
 // integer prefix sum of count * d. The first lane whose additions would leave the binade or meet a
 // tie is taken alone by seq_repeat_add, and the scan resumes after it.
-__device__ double warp_seq_sum(double s, double w, int64_t count, double* before) {
+__device__ inline double warp_seq_sum(double s, double w, int64_t count, double* before) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int64_t TOP = (int64_t)1 << 53;
     const int lane = threadIdx.x & 31;

@@ -12,7 +12,9 @@ B = 4 bytes per height (the REF32 field):
   relax (s sweeps, a read and a write of the field each: 2B s)   8 s
 The plate flexure (P3) is bound by the FP64 pipe instead: its two 2D transforms over the W x 2H
 mirrored grid take 5 flops per point per radix-2 stage, 20 (log2 W + log2 2H) flops per map cell
-and round, against the FP64 rate the bench measures on the GPU it runs on (cg_probe_fp64_rate).
+and round, against the FP64 rate the bench measures on the GPU it runs on (cg_probe_fp64_rate). The
+kernels take the products, 2 of the 5, on the integer pipes and skip the mirrored half of the first
+pass, so the fraction is of the transform's arithmetic and not how busy the FP64 pipe is.
 The peak is the measured HBM copy bandwidth of the GB300s (MEASURED_PEAKS.json, written by
 the pool's driver), else the recipe's fallback of 6.8 TB/s.
 """
@@ -30,7 +32,7 @@ PHASE_KERNELS = {
     "ms_deposit": "k_round_begin, k_rank_of, k_level_bounds, k_deposit_levels, k_settle, k_mouths_levels "
                   "(last round: the closing breach's cut, fill, routing and notch)",
     "ms_relax": "thermal_sweeps_kernel",
-    "ms_flexure": "k_uplift, k_flex_load, k_flex_mean, k_fft_lines, k_transpose, k_flex_apply",
+    "ms_flexure": "k_uplift, k_flex_load, k_ss_*, k_fft_lines, k_transpose, k_flex_apply",
 }
 FALLBACK_HBM_GBS = 6800.0
 
