@@ -110,11 +110,8 @@ __device__ __forceinline__ bool ratio_cannot_win(double df, double dg, double st
 //  - the share along the far edge, a / b with a = outward tc^2 and b = cdrop od^2 (rounded products,
 //    as the reference forms them), is compared with 1 as a >= b: for positive doubles fl(a/b) >= 1
 //    exactly when a >= b, since a < b puts a/b at or below the double just under 1. The division is
-//    taken once, for the winning facet, whose share the draw is compared with;
-//  - UNIT: both legs are exactly one cell width (square cells), so the products and quotients by a
-//    leg are the values themselves.
+//    taken once, for the winning facet, whose share the draw is compared with.
 // Facets are visited and compared in the reference's order, so ties resolve identically.
-template <bool UNIT>
 __device__ int facet_receiver(int W, int H, const double* __restrict__ rs, int col, int row, Steps st, long long seed) {
     const int ccs_t[4] = {1, 0, -1, 0};
     const int crs_t[4] = {0, -1, 0, 1};
@@ -143,7 +140,7 @@ __device__ int facet_receiver(int W, int H, const double* __restrict__ rs, int c
         const double cdrop = __dsub_rn(here, rs[card]);
         const double to_card = ccs != 0 ? ew : ns;     // GroundSteps.of(ccs, crs): never a diagonal here
         const double on_to_diag = ccs == 0 ? ew : ns;
-        const double cslope = UNIT ? cdrop : div_leg(cdrop, to_card);
+        const double cslope = div_leg(cdrop, to_card);
         const bool cdown = dpos(cdrop);
 #pragma unroll
         for (int turn = -1; turn <= 1; turn += 2) {
@@ -163,8 +160,8 @@ __device__ int facet_receiver(int W, int H, const double* __restrict__ rs, int c
             } else {
                 bool to_diagonal = true;   // share 1 when the cardinal is not downhill
                 if (cdown) {
-                    a = UNIT ? outward : __dmul_rn(__dmul_rn(outward, to_card), to_card);
-                    b = UNIT ? cdrop : __dmul_rn(__dmul_rn(cdrop, on_to_diag), on_to_diag);
+                    a = __dmul_rn(__dmul_rn(outward, to_card), to_card);
+                    b = __dmul_rn(__dmul_rn(cdrop, on_to_diag), on_to_diag);
                     to_diagonal = dkey(a) >= dkey(b);
                 }
                 if (to_diagonal) {
@@ -179,7 +176,7 @@ __device__ int facet_receiver(int W, int H, const double* __restrict__ rs, int c
                     }
                     m = 1;
                 } else {
-                    const double oslope = UNIT ? outward : div_leg(outward, on_to_diag);
+                    const double oslope = div_leg(outward, on_to_diag);
                     const double sq = __dadd_rn(__dmul_rn(cslope, cslope), __dmul_rn(oslope, oslope));
                     wins = false;
                     if (!sqrt_cannot_win(sq, steepest)) {
@@ -209,138 +206,172 @@ __device__ int facet_receiver(int W, int H, const double* __restrict__ rs, int c
     return dkey(draw) < dkey(share) ? fdiag : fcard;
 }
 
-// facet_receiver<true> for the 32 cells a warp holds (cell < 0: an idle lane), with the expensive
-// FP64 operations taken densely. An FP64 warp instruction holds the pipe whatever its active lanes, and
-// in the per-lane form each facet's division and square root run under a branch that only some lanes
-// take. Here every lane first settles each facet's case (cardinal, diagonal, inside) from the falls,
-// which are dense FP64 subtractions and integer comparisons; the warp then takes the diagonal
-// divisions and the inside square roots as two compacted lists, every lane one request; then each
-// lane compares its facets' slopes in the reference's order. The early outs of the per-lane form only
-// skipped slopes that could not win, so computing every slope changes no comparison's outcome.
-struct DenseFacets {
-    double sq[32 * 8];    // per lane and facet: an inside facet's squared slope, then its slope
-    double dv[32 * 4];    // per lane and diagonal: the fall, then the slope
-    int idx[32 * 8];      // the compacted requests
-};
-
-__device__ __forceinline__ int warp_exclusive_sum(int v, int lane, int* total) {
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
+// Square cells (both legs one cell width, so products and quotients by a leg are the values themselves):
+// the facets of `mask` alone, in the reference's order; facet 2 side + (turn > 0).
+__device__ __noinline__ int facet_receiver_exact(int W, int H, const double* __restrict__ rs, int col, int row,
+                                                 float diagonal, long long seed, unsigned mask) {
+    const double here = rs[row * W + col];
+    double steepest = 0.0, wa = 0.0, wb = 0.0;
+    int wmode = -1, fcard = -1, fdiag = -1;
+    for (unsigned rest = mask; rest; rest &= rest - 1) {
+        const int f = __ffs(rest) - 1, side = f >> 1, turn = (f & 1) ? 1 : -1;
+        const int ccs = side == 0 ? 1 : side == 2 ? -1 : 0, crs = side == 1 ? -1 : side == 3 ? 1 : 0;
+        const int card = neighbour_at(W, H, col + ccs, row + crs);
+        const int diag = neighbour_at(W, H, col + (ccs == 0 ? turn : ccs), row + (crs == 0 ? turn : crs));
+        if (card < 0 || diag < 0) continue;
+        const double c = __dsub_rn(here, rs[card]), df = __dsub_rn(here, rs[diag]);
+        const double o = __dsub_rn(df, c);
+        const int m = dpos(c) && !dpos(o) ? 0 : !dpos(c) || dkey(o) >= dkey(c) ? 1 : 2;
+        const double v = m == 0   ? c
+                         : m == 1 ? __ddiv_rn(df, (double)diagonal)
+                                  : __dsqrt_rn(__dadd_rn(__dmul_rn(c, c), __dmul_rn(o, o)));
+        if (dkey(v) > dkey(steepest)) {
+            steepest = v;
+            wmode = m;
+            fcard = card;
+            fdiag = diag;
+            wa = o;
+            wb = c;
+        }
     }
-    *total = __shfl_sync(0xFFFFFFFFu, x, 31);
-    return x - v;
+    if (!dpos(steepest)) return -1;
+    if (wmode < 2) return wmode == 0 ? fcard : fdiag;
+    const double share = __ddiv_rn(wa, wb);
+    if (!dpos(share)) return fcard;
+    // FlowRouting.subGridDraw (FlowRouting.kt:355-356).
+    const double draw = (double)__fmul_rn(__fadd_rn(seeded_noise(col, row, seed ^ kSubGridDrawSalt), 1.0f), 0.5f);
+    return dkey(draw) < dkey(share) ? fdiag : fcard;
 }
 
-__device__ int facet_receiver_dense(int W, int H, const double* __restrict__ rs, int cell, Steps st, long long seed,
-                                    DenseFacets& sh) {
-    const int lane = threadIdx.x & 31;
+// The facet rule on square cells, its slopes in single precision wherever that settles the answer. Only the
+// falls are taken in double, one subtraction a neighbour: a facet's case follows from comparing them (the
+// share reaches 1 when the outward fall df - c is at least c > 0, which for df < 2 c is an exact difference
+// below c, so when df >= 2 c). The squares of the slopes are then compared in float: a fall cut to a float
+// is off by under 2^-23 of itself, an inside facet's outward fall by under 2^-21 of the cardinal's, a
+// squared slope by under 8e-7 of itself, so a facet whose square is 2e-6 below the largest cannot have the
+// steepest slope, rounding and all. Facets closer than that are told apart where it needs no arithmetic
+// (the same falls in the same case; two cardinals; a cardinal against an inside facet on the same fall,
+// whose outward fall raises the slope by many units in the last place), and the rest go through the exact
+// form, as do falls too small, too large or not finite for floats, and a draw within 1e-6 of the winner's
+// share.
+//
+// The rule is bound by FP64 issue, 77 cycles a warp instruction: some 81 a cell with every slope exact,
+// here 8 and the exact form's for the few cells that need it. The two passes of a round took 3.15 ms at
+// 8192 x 4096 and 209 us at 2048 x 1024, and take 1.31 ms and 96 us.
+struct Fall {
+    double d;
+    float f;   // d cut to a float where it is above zero, else 0
+};
+
+__device__ __forceinline__ Fall fall_of(double here, double there, bool& odd) {
+    Fall v;
+    v.d = __dsub_rn(here, there);
+    const unsigned hi = (unsigned)__double2hiint(v.d), lo = (unsigned)__double2loint(v.d);
+    const unsigned a = hi & 0x7FFFFFFFu;
+    const bool down = dpos(v.d);
+    odd |= a >= (1023u + 60u) << 20 || (down && a < (1023u - 60u) << 20);
+    v.f = down ? __uint_as_float(((a - (896u << 20)) << 3) | (lo >> 29)) : 0.0f;
+    return v;
+}
+
+__device__ int facet_receiver_quick(int W, int H, const double* __restrict__ rs, int col, int row, Steps st,
+                                    long long seed) {
     const int ccs_t[4] = {1, 0, -1, 0};
     const int crs_t[4] = {0, -1, 0, 1};
-    const bool live = cell >= 0;
-    const int row = live ? pdiv(cell, W) : 0, col = live ? pmod(cell, W) : 0;
-    const double here = live ? rs[cell] : 0.0;
-    const double dg = (double)st.diag;
-    int dcell[4];
-    double dfall[4];
+    const double here = rs[row * W + col];
+    const float diagonal_sq = __frcp_rn(st.diag * st.diag);
+    bool odd = false;
+    Fall diag[4], card[4];
+    float s[8];
+    unsigned modes = 0;   // 2 bits a facet: 0 cardinal, 1 diagonal, 2 inside, 3 none
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int dcs = (k & 1) ? 1 : -1, drs = (k & 2) ? 1 : -1;
-        dcell[k] = live ? neighbour_at(W, H, col + dcs, row + drs) : -1;
-        dfall[k] = dcell[k] >= 0 ? __dsub_rn(here, rs[dcell[k]]) : 0.0;
+        const int n = neighbour_at(W, H, col + ((k & 1) ? 1 : -1), row + ((k & 2) ? 1 : -1));
+        diag[k] = fall_of(here, n >= 0 ? rs[n] : here, odd);
     }
-    int card[4];
-    double cdrop[4];
-    unsigned modes = 0;     // 2 bits per facet: 0 cardinal, 1 diagonal, 2 inside, 3 none
-    unsigned need_div = 0, need_sq = 0;
+    float most = 0.0f;
 #pragma unroll
     for (int side = 0; side < 4; ++side) {
-        card[side] = live ? neighbour_at(W, H, col + ccs_t[side], row + crs_t[side]) : -1;
-        cdrop[side] = card[side] >= 0 ? __dsub_rn(here, rs[card[side]]) : 0.0;
-        const bool cdown = dpos(cdrop[side]);
+        const int n = neighbour_at(W, H, col + ccs_t[side], row + crs_t[side]);
+        card[side] = fall_of(here, n >= 0 ? rs[n] : here, odd);
+        const Fall c = card[side];
+        const bool cdown = dpos(c.d);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int turn = t ? 1 : -1, f = side * 2 + t;
             const int dcs = ccs_t[side] == 0 ? turn : ccs_t[side];
             const int drs = crs_t[side] == 0 ? turn : crs_t[side];
-            const int k = (dcs > 0 ? 1 : 0) | (drs > 0 ? 2 : 0);
+            const Fall df = diag[(dcs > 0 ? 1 : 0) | (drs > 0 ? 2 : 0)];
             unsigned m = 3;
-            if (card[side] >= 0 && dcell[k] >= 0) {
-                const double outward = __dsub_rn(dfall[k], cdrop[side]);
-                if (cdown && !dpos(outward)) {
+            float v = 0.0f;
+            if (row + drs >= 0 && row + drs < H && n >= 0) {
+                if (cdown && dkey(df.d) <= dkey(c.d)) {
                     m = 0;
-                } else if (!cdown || dkey(outward) >= dkey(cdrop[side])) {   // a >= b, with unit legs
+                    v = c.f * c.f;
+                } else if (!cdown || dkey(df.d) >= dkey(c.d) + (1LL << 52)) {
                     m = 1;
-                    need_div |= 1u << k;
+                    v = df.f * df.f * diagonal_sq;
                 } else {
                     m = 2;
-                    need_sq |= 1u << f;
-                    sh.sq[lane * 8 + f] = __dadd_rn(__dmul_rn(cdrop[side], cdrop[side]), __dmul_rn(outward, outward));
+                    const float o = df.f - c.f;
+                    v = c.f * c.f + o * o;
                 }
             }
             modes |= m << (2 * f);
+            s[f] = v;
+            most = fmaxf(most, v);
         }
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (need_div & (1u << k)) sh.dv[lane * 4 + k] = dfall[k];
-    // The diagonal divisions, densely.
-    int total;
-    int off = warp_exclusive_sum(__popc(need_div), lane, &total);
-    for (int k = 0, j = 0; k < 4; ++k)
-        if (need_div & (1u << k)) sh.idx[off + j++] = lane * 4 + k;
-    __syncwarp();
-    for (int base = 0; base < total; base += 32)
-        if (base + lane < total) {
-            const int i = sh.idx[base + lane];
-            sh.dv[i] = __ddiv_rn(sh.dv[i], dg);
-        }
-    __syncwarp();
-    // The inside facets' square roots, densely.
-    off = warp_exclusive_sum(__popc(need_sq), lane, &total);
-    for (int f = 0, j = 0; f < 8; ++f)
-        if (need_sq & (1u << f)) sh.idx[off + j++] = lane * 8 + f;
-    __syncwarp();
-    for (int base = 0; base < total; base += 32)
-        if (base + lane < total) {
-            const int i = sh.idx[base + lane];
-            sh.sq[i] = __dsqrt_rn(sh.sq[i]);
-        }
-    __syncwarp();
-    // The facets in the reference's order; the winner's cells and falls kept as it wins.
-    double steepest = 0.0;
-    unsigned wmode = 3;
-    int fcard = -1, fdiag = -1;
-    double wout = 0.0, wdrop = 0.0;
+    // The facets that may be the steepest, in the reference's order.
+    const float least = most * 0.999998f;
+    unsigned wmode = 3, close = 0;
+    int wf = 0;
+    bool unsure = false;
+    Fall wc{0.0, 0.0f}, wd{0.0, 0.0f};
 #pragma unroll
     for (int f = 0; f < 8; ++f) {
         const unsigned m = (modes >> (2 * f)) & 3u;
         const int side = f >> 1, turn = (f & 1) ? 1 : -1;
         const int dcs = ccs_t[side] == 0 ? turn : ccs_t[side];
         const int drs = crs_t[side] == 0 ? turn : crs_t[side];
-        const int k = (dcs > 0 ? 1 : 0) | (drs > 0 ? 2 : 0);
-        if (m == 3) continue;
-        const double v = m == 0 ? cdrop[side] : m == 1 ? sh.dv[lane * 4 + k] : sh.sq[lane * 8 + f];
-        if (dkey(v) > dkey(steepest)) {
-            steepest = v;
+        const Fall c = card[side], df = diag[(dcs > 0 ? 1 : 0) | (drs > 0 ? 2 : 0)];
+        if (m == 3 || s[f] == 0.0f || s[f] < least) continue;
+        close |= 1u << f;
+        bool wins = wmode == 3;
+        if (!wins) {
+            const bool same_c = dkey(c.d) == dkey(wc.d), same_d = dkey(df.d) == dkey(wd.d);
+            if (m == 0 && wmode == 0) {
+                wins = dkey(c.d) > dkey(wc.d);
+            } else if (m == wmode && same_d && (m == 1 || same_c)) {
+                wins = false;
+            } else if (same_c && m + wmode == 2 && m != 1 && (m == 2 ? df.f - c.f : wd.f - wc.f) > 1e-6f * c.f) {
+                wins = m == 2;
+            } else {
+                unsure = true;
+            }
+        }
+        if (wins) {
             wmode = m;
-            fcard = card[side];
-            fdiag = dcell[k];
-            wout = dfall[k];
-            wdrop = cdrop[side];
+            wf = f;
+            wc = c;
+            wd = df;
         }
     }
-    __syncwarp();   // the buffers are the warp's next call's
-    if (!live || wmode == 3 || !dpos(steepest)) return -1;
-    if (wmode == 0) return fcard;
-    if (wmode == 1) return fdiag;
-    const double share = __ddiv_rn(__dsub_rn(wout, wdrop), wdrop);
-    if (!dpos(share)) return fcard;
-    // FlowRouting.subGridDraw (FlowRouting.kt:355-356).
-    const double draw = (double)__fmul_rn(__fadd_rn(seeded_noise(col, row, seed ^ kSubGridDrawSalt), 1.0f), 0.5f);
-    return dkey(draw) < dkey(share) ? fdiag : fcard;
+    // FlowRouting.subGridDraw (FlowRouting.kt:355-356) against the share along the winner's far edge.
+    bool far = wmode == 1;
+    if (wmode == 2) {
+        const float draw = __fmul_rn(__fadd_rn(seeded_noise(col, row, seed ^ kSubGridDrawSalt), 1.0f), 0.5f);
+        const float over = (wd.f - wc.f) - draw * wc.f;
+        far = over > 0.0f;
+        unsure |= fabsf(over) <= 1e-6f * wc.f;
+    }
+    if (odd) close = 0xFFu;
+    if (odd || unsure) return facet_receiver_exact(W, H, rs, col, row, st.diag, seed, close);
+    if (wmode == 3) return -1;
+    const int side = wf >> 1, turn = (wf & 1) ? 1 : -1;
+    const int ccs = side == 0 ? 1 : side == 2 ? -1 : 0, crs = side == 1 ? -1 : side == 3 ? 1 : 0;
+    const int dc = far && ccs == 0 ? turn : ccs, dr = far && crs == 0 ? turn : crs;
+    return (row + dr) * W + wrap_col(col + dc, W);
 }
 
 // FlowRouting.steepestNeighbourOf (FlowRouting.kt:320-343).
@@ -364,11 +395,11 @@ __device__ int steepest_neighbour(int W, int H, const double* __restrict__ rs, i
     return best;
 }
 
-// Receivers of land cells (sea cells get -1). The facet rule is FP64 work, and an FP64 warp
-// instruction costs the same with one lane active as with 32, so each warp compacts the land cells
-// of the chunks it scans into a small queue in shared memory and runs the rule 32 land cells at a
-// time. `near` splits the work around the flats: 0 every land cell; 1 the cells with no raised cell
-// in their 3x3 block (their surface and their neighbours' are final before the flats are solved,
+// Receivers of land cells (sea cells get -1). The facet rule's FP64 warp instructions cost the same
+// with one lane active as with 32, so each warp compacts the land cells of the chunks it scans (four cells
+// a lane, the fields' bytes a word at a time) into a small queue in shared memory and runs the rule 32 land
+// cells at a time. `near` splits the work around the flats: 0 every land cell; 1 the cells with no raised
+// cell in their 3x3 block (their surface and their neighbours' are final before the flats are solved,
 // so this pass runs beside the flat solvers) and the sea; 2 the cells with a raised cell in their
 // 3x3 block, after the flats.
 constexpr int RECV_THREADS = 256;
@@ -377,64 +408,76 @@ __device__ __forceinline__ int receiver_of(int cell, const double* __restrict__ 
                                            long long seed, int by_facet, bool unit) {
     const int row = pdiv(cell, W), col = pmod(cell, W);
     return !by_facet ? steepest_neighbour(W, H, surface, col, row, st)
-           : unit    ? facet_receiver<true>(W, H, surface, col, row, st, seed)
-                     : facet_receiver<false>(W, H, surface, col, row, st, seed);
+           : unit    ? facet_receiver_quick(W, H, surface, col, row, st, seed)
+                     : facet_receiver(W, H, surface, col, row, st, seed);
 }
 
-__device__ __forceinline__ bool near_raised(const uint8_t* __restrict__ raised, int cell, int W, int H) {
+// For the four cells from `cell`, a byte each: nonzero where a raised cell is in the cell's 3x3 block.
+__device__ __forceinline__ unsigned near_raised4(const uint8_t* __restrict__ raised, int cell, int W, int H) {
     const int row = pdiv(cell, W), col = pmod(cell, W);
-    unsigned any = 0;
+    unsigned long long any = 0;   // the columns from one before the cells to one after, a byte each
 #pragma unroll
     for (int rs = -1; rs <= 1; ++rs) {
         const int nr = row + rs;
         if (nr < 0 || nr >= H) continue;
-#pragma unroll
-        for (int cs = -1; cs <= 1; ++cs) any |= raised[nr * W + wrap_col(col + cs, W)];
+        const uint8_t* line = raised + (size_t)nr * W;
+        any |= (unsigned long long)line[wrap_col(col - 1, W)] |
+               (unsigned long long)*reinterpret_cast<const unsigned*>(line + col) << 8 |
+               (unsigned long long)line[wrap_col(col + 4, W)] << 40;
     }
-    return any != 0;
+    return (unsigned)(any | any >> 8 | any >> 16);
 }
 
-__global__ void __launch_bounds__(RECV_THREADS) k_receivers(const uint8_t* __restrict__ land,
+__global__ void __launch_bounds__(RECV_THREADS, 3) k_receivers(const uint8_t* __restrict__ land,
                                                             const double* __restrict__ surface, int W, int H,
                                                             Steps st, long long seed, int by_facet,
                                                             const uint8_t* __restrict__ raised, int near,
                                                             int32_t* __restrict__ recv) {
     const unsigned FULL = 0xFFFFFFFFu;
-    __shared__ int queue[RECV_THREADS / 32][64];
-    __shared__ DenseFacets dense[RECV_THREADS / 32];
+    __shared__ int queue[RECV_THREADS / 32][32 + 128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int* q = queue[warp];
     const bool unit = st.ew == 1.0f && st.ns == 1.0f;
-    const bool warp_dense = by_facet && unit;   // square cells: the facet rule with dense FP64 requests
     const size_t N = (size_t)W * H;
     const size_t warps = (size_t)gridDim.x * (RECV_THREADS / 32);
-    int n = 0;   // queued land cells (the same in every lane)
-    for (size_t base = ((size_t)blockIdx.x * (RECV_THREADS / 32) + warp) * 32; base < N; base += warps * 32) {
-        const size_t i = base + lane;
-        const bool is_land = i < N && land[i];
-        if (i < N && !is_land && near != 2) recv[i] = -1;
-        const bool l = is_land && (near == 0 || near_raised(raised, (int)i, W, H) == (near == 2));
-        const unsigned m = __ballot_sync(FULL, l);
-        if (l) q[n + __popc(m & ((1u << lane) - 1u))] = (int)i;
-        n += __popc(m);
+    int n = 0;   // queued land cells (the same in every lane), under 32 between chunks
+    for (size_t base = ((size_t)blockIdx.x * (RECV_THREADS / 32) + warp) * 128;; base += warps * 128) {
+        const bool last = base >= N;
+        const size_t i = base + 4 * lane;
+        unsigned is_land = 0, is_near = 0;   // a byte a cell
+        if (i < N) {
+            if (W >= 4) {
+                is_land = *reinterpret_cast<const unsigned*>(land + i);
+                if (near && is_land) is_near = near_raised4(raised, (int)i, W, H);
+            } else {   // two columns at most: a row's neighbours are the row
+                for (int k = 0; k < 4 && i + k < N; ++k) {
+                    is_land |= (unsigned)land[i + k] << (8 * k);
+                    const int row = (int)(i + k) / W;
+                    for (int c = max(0, row - 1) * W; near && c < min(H, row + 2) * W; ++c)
+                        is_near |= (unsigned)raised[c] << (8 * k);
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool on_land = (is_land >> (8 * k)) & 0xFFu;
+            if (!on_land && near != 2 && i + k < N) recv[i + k] = -1;
+            const bool l = on_land && (near == 0 || (((is_near >> (8 * k)) & 0xFFu) != 0) == (near == 2));
+            const unsigned m = __ballot_sync(FULL, l);
+            if (l) q[n + __popc(m & ((1u << lane) - 1u))] = (int)i + k;
+            n += __popc(m);
+        }
         __syncwarp();
-        if (n >= 32) {
-            const int cell = q[lane];
-            recv[cell] = warp_dense ? facet_receiver_dense(W, H, surface, cell, st, seed, dense[warp])
-                                    : receiver_of(cell, surface, W, H, st, seed, by_facet, unit);
-            __syncwarp();
-            if (lane < n - 32) q[lane] = q[32 + lane];
-            n -= 32;
+        while (n >= 32 || (last && n > 0)) {
+            const int some = min(n, 32);
+            if (lane < some) {
+                const int cell = q[n - some + lane];
+                recv[cell] = receiver_of(cell, surface, W, H, st, seed, by_facet, unit);
+            }
+            n -= some;
             __syncwarp();
         }
-    }
-    if (warp_dense) {
-        const int cell = lane < n ? q[lane] : -1;
-        const int r = facet_receiver_dense(W, H, surface, cell, st, seed, dense[warp]);
-        if (lane < n) recv[cell] = r;
-    } else if (lane < n) {
-        const int cell = q[lane];
-        recv[cell] = receiver_of(cell, surface, W, H, st, seed, by_facet, unit);
+        if (last) break;
     }
 }
 
