@@ -746,7 +746,7 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
         CG_TRY_ST(tree_walk_dev(ctx, W, H, d_belt, d_recv, nullptr, d_key, d_donors, nullptr, &levels));
         int *d_bucket = nullptr, *d_start = nullptr;
         CG_TRY_ST(level_buckets_dev(ctx, W, H, d_belt, d_key, levels, &d_bucket, &d_start));
-        CG_TRY_ST(order_from_keys_dev(ctx, W, H, d_belt, d_key, B, d_order));
+        CG_TRY_ST(order_from_keys_dev(ctx, W, H, d_belt, d_key, B, d_order, levels));
         // Discharge, the cut and the spoil's flux, level by level (BeltErosion.kt:313-370).
         la.levels = levels;
         la.bucket = d_bucket;

@@ -96,7 +96,7 @@ namespace cg {
 // Buffer slots of cg_ctx::bufs.
 enum Slot {
     S_H0, S_H1, S_GIVE, S_UPLIFT, S_ROCK, S_RAIN, S_VEG, S_RUNOFF, S_ERODE, S_LAND, S_REL, S_FILLED,
-    S_SURFACE, S_RECV, S_DONORS, S_KEY, S_ORDER, S_AREA, S_WATER, S_LABEL, S_PTR, S_PTR2, S_SCRATCH0,
+    S_SURFACE, S_RECV, S_DONORS, S_KEY, S_ORDER, S_AREA, S_WATER, S_LABEL, S_PTR, S_SCRATCH0,
     S_SCRATCH1, S_SCRATCH2, S_SCRATCH3, S_ROWW, S_HIST, S_BRACKET, S_BRACKET2, S_SMALL, S_FLATS,
     S_FLATIDX, S_FLATMEM, S_CG0, S_CG1, S_CG2, S_CG3, S_CG4, S_CG5, S_LEVELCNT, S_DEPTH, S_STATS,
     S_BASIN, S_BASIN2, S_FILLQ, S_FILLF, S_FILLFLAG, S_TILEFLAG, S_SCRATCH4, S_SCRATCH5, S_THERMFLAG,

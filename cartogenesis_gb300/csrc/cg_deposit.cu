@@ -1582,7 +1582,7 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     w.f = Fields{r.recv, r.land, r.ground, r.rel, r.area, r.surface, d_sediment, r.settled, r.incised_at};
     // The drainage order and each level's first rank.
     CG_BUF(int32_t, d_order, ctx, S_ORDER, N);
-    CG_TRY_ST(order_from_keys_dev(ctx, W, H, r.land, r.key, n, d_order));
+    CG_TRY_ST(order_from_keys_dev(ctx, W, H, r.land, r.key, n, d_order, r.levels));
     CG_BUF(int, d_rank, ctx, S_DEPRANK, N);
     CG_BUF(int, d_lstart, ctx, S_DEPLEVEL, (size_t)r.levels + 1);
     const int grid = ctx->num_sms * 8;

@@ -7,7 +7,7 @@
 // Q; when that is unique, f(n) = phi(min over neighbours of f, g(n)), a monotone fixed point. The
 // device computes that fixed point in parallel and then checks, cell by cell, whether the
 // quantised key ever left the parent open:
-//  (1) pointer jumping along strictly Q-descending neighbour chains finds every cell with such a
+//  (1) following strictly Q-descending neighbour chains to their roots finds every cell with such a
 //      chain to an outlet; those keep their own height (their first popped neighbour is lower);
 //  (2) the rest relax to the fixed point of f(n) = min_m phi(f(m), g(n)) from +inf, tile by tile
 //      in shared memory, each tile iterating to local convergence before its borders are
@@ -102,27 +102,20 @@ __global__ void k_fill_init(const uint8_t* __restrict__ land, const float* __res
     }
 }
 
-// (1) pointer jumping to the chain's root, in place: p[i] <- p[p[i]]. Whatever a concurrent update
-// lets a thread read is an ancestor of i on its chain, so the pass only jumps further, and a pass
-// that changes no pointer leaves every cell on its root. `changed` is set when some pointer moved.
-__global__ void k_jump(int* __restrict__ p, size_t N, int* __restrict__ changed) {
-    bool moved = false;
+// (1) every land cell's chain followed to its root, in place: a step replaces the cell's pointer by the one
+// it just read, p[i] <- p[p[i]], so cells above it on the chain skip what it has skipped. Whatever a
+// concurrent step lets a thread read is an ancestor of i on its chain, and the chain is finite. A cell whose
+// root is water or a polar outlet keeps its own height. One launch: jumping passes that each jumped every
+// cell once, with a host check every second pass, took 100 us at 1024 x 512 and 1.1 ms at 8192 x 4096.
+__global__ void k_drain_chains(int* p, const float* __restrict__ g, size_t N, uint8_t* cls, float* __restrict__ f) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
-        const int o = p[i];
-        const int n = p[o];
-        if (n != o) {
-            p[i] = n;
-            moved = true;
+        if (cls[i] != C_OPEN) continue;   // the roots' classes never change
+        int o = __ldcg(p + i);
+        for (int n = __ldcg(p + o); n != o; n = __ldcg(p + o)) {
+            __stcg(p + i, n);
+            o = n;
         }
-    }
-    if (__any_sync(0xFFFFFFFFu, moved) && (threadIdx.x & 31) == 0) atomicOr(changed, 1);
-}
-
-__global__ void k_mark_drained(const int* __restrict__ root, const float* __restrict__ g, size_t N,
-                               uint8_t* __restrict__ cls, float* __restrict__ f) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
-        if (cls[i] != C_OPEN) continue;
-        uint8_t rc = cls[root[i]];
+        const uint8_t rc = cls[o];
         if (rc == C_WATER || rc == C_SEED) {
             cls[i] = C_DRAINED;
             f[i] = g[i];
@@ -523,7 +516,6 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     cudaStream_t sm = ctx->stream;
     CG_BUF(uint8_t, d_cls, ctx, S_FILLFLAG, N);
     CG_BUF(int, d_ptr, ctx, S_PTR, N);
-    CG_BUF(int, d_moved, ctx, S_PTR2, 2);   // the jumping passes' change flags
     CG_BUF(int, d_pin, ctx, S_FILLQ, N);
     int tiles_x = (W + T - 1) / T, tiles_y = (H + T - 1) / T, tiles = tiles_x * tiles_y;
     // Two tile lists and their marks, two list counts, the timeout flag (zeroed before each relaxation).
@@ -551,22 +543,8 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     const int relax_grid = ctx->num_sms * std::min(per_sm, 8);
     CG_BUF(FillCounters, d_cnt, ctx, S_FILLF, 1);
     int grid = ctx->num_sms * 8;
-    CG_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, sizeof(FillCounters), sm));
     CG_LAUNCH(ctx) k_fill_init<<<grid, 256, 0, sm>>>(d_land, d_rel, W, H, d_cls, d_filled, d_ptr);
-    // Chains are at most N long: ceil(log2 N) jumps reach every root; most worlds need far fewer, so
-    // the passes stop at the first that moves no pointer (checked every second pass).
-    int jumps = 1;
-    while (((size_t)1 << jumps) < N) ++jumps;
-    for (int j = 0; j < jumps + 2; j += 2) {
-        CG_CUDA(ctx, cudaMemsetAsync(d_moved, 0, 2 * sizeof(int), sm));
-        CG_LAUNCH(ctx) k_jump<<<grid, 256, 0, sm>>>(d_ptr, N, d_moved);
-        CG_LAUNCH(ctx) k_jump<<<grid, 256, 0, sm>>>(d_ptr, N, d_moved + 1);
-        int moved[2] = {0, 0};
-        CG_CUDA(ctx, cudaMemcpyAsync(moved, d_moved, sizeof(moved), cudaMemcpyDeviceToHost, sm));
-        CG_CUDA(ctx, cudaStreamSynchronize(sm));
-        if (!moved[1]) break;
-    }
-    CG_LAUNCH(ctx) k_mark_drained<<<grid, 256, 0, sm>>>(d_ptr, d_rel, N, d_cls, d_filled);
+    CG_LAUNCH(ctx) k_drain_chains<<<grid, 256, 0, sm>>>(d_ptr, d_rel, N, d_cls, d_filled);
     CG_CHECK_LAUNCH(ctx);
 
     // Scratch of the level replays: a generation mark per cell, the level's cells and the heap, each
@@ -587,7 +565,11 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     // Each pass either settles, pins tie parents by the index rule, or replays the lowest level
     // holding a tie the index rule cannot order; the cap is a guard, not the expected exit.
     const int max_repairs = 256;
+    FillCounters zero{};
+    zero.min_level = INT_MAX;
+    zero.repair_level = INT_MAX;
     for (int repair = 0; repair <= max_repairs; ++repair) {
+        CG_CUDA(ctx, cudaMemcpyAsync(d_cnt, &zero, sizeof(zero), cudaMemcpyHostToDevice, sm));
         CG_CUDA(ctx, cudaMemsetAsync(d_lists, 0, (2 * (size_t)tiles + 4) * sizeof(int), sm));
         CG_CUDA(ctx, cudaMemsetAsync(d_marks, 0, 2 * (size_t)tiles * sizeof(int), sm));
         CG_LAUNCH(ctx) k_tiles_with_open<<<tiles, 256, 0, sm>>>(d_cls, d_filled, W, H, tiles_x, ra.mark[0], ra.list[0],
@@ -600,18 +582,14 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
             ctx->launches++;
             CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_relax_passes, relax_grid, 256, kargs, 0, sm));
         }
+        // The check runs behind the relaxation, settled or not; the host reads both together.
         int timed_out = 0;
-        CG_CUDA(ctx, cudaMemcpyAsync(&timed_out, ra.timed_out, sizeof(int), cudaMemcpyDeviceToHost, sm));
-        CG_CUDA(ctx, cudaStreamSynchronize(sm));
-        if (timed_out) return fail(ctx, CG_TIMEOUT, "fill relaxation did not settle in %d passes", ra.max_passes);
-        FillCounters zero{};
-        zero.min_level = INT_MAX;
-        zero.repair_level = INT_MAX;
-        CG_CUDA(ctx, cudaMemcpyAsync(d_cnt, &zero, sizeof(zero), cudaMemcpyHostToDevice, sm));
         CG_LAUNCH(ctx) k_check_ties<<<grid, 256, 0, sm>>>(d_filled, d_rel, d_cls, d_pin, W, H, d_cnt);
         CG_CHECK_LAUNCH(ctx);
+        CG_CUDA(ctx, cudaMemcpyAsync(&timed_out, ra.timed_out, sizeof(int), cudaMemcpyDeviceToHost, sm));
         CG_CUDA(ctx, cudaMemcpyAsync(&hc, d_cnt, sizeof(hc), cudaMemcpyDeviceToHost, sm));
         CG_CUDA(ctx, cudaStreamSynchronize(sm));
+        if (timed_out) return fail(ctx, CG_TIMEOUT, "fill relaxation did not settle in %d passes", ra.max_passes);
         if (repair == 0) tie_total = (int64_t)hc.ties;
         unresolved_total = (int64_t)hc.unresolved;
         if (hc.repaired == 0 && hc.unresolved == 0) break;

@@ -56,9 +56,10 @@ cg_status facet_receivers_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, 
 // (optional, synchronises) receives the number of Kahn levels.
 cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int32_t* d_recv,
                         const float* d_weights, long long* d_key, int32_t* d_donors, float* d_area, int* h_levels);
-// The explicit drainage order (land cells sorted by key), for callers that want it.
+// The explicit drainage order (land cells sorted by key), for callers that want it; `levels` the keys'
+// number of Kahn levels, 0 where the caller does not know it (synchronises).
 cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const long long* d_key,
-                              int land_cells, int32_t* d_order);
+                              int land_cells, int32_t* d_order, int levels = 0);
 struct InciseArgs {
     float courant_coefficient;
     float pond_depth;

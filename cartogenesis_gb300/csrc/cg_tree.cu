@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 #include <cuda/atomic>
 
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <utility>
@@ -147,15 +148,15 @@ struct WalkArgs {
 // round of loads of the other donors' keys and areas.
 __global__ void __launch_bounds__(64) k_walk(WalkArgs a) {
     const unsigned FULL = 0xFFFFFFFFu;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long local_max = 0;
-    if (idx < *a.n_sources) {
+    const int n_sources = *a.n_sources;
+    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n_sources; idx += gridDim.x * blockDim.x) {
         int c = a.sources[idx];
         long long kc = (long long)c;   // a source: level 0, its own index
         float ac = a.weights ? a.weights[c] : 0.0f;
         a.key[c] = kc;
         if (a.weights) a.area[c] = ac;
-        local_max = (unsigned long long)kc;
+        if ((unsigned long long)kc > local_max) local_max = (unsigned long long)kc;
         while (true) {
             const int d = a.down[c];
             if (d == 0xFF) break;
@@ -233,15 +234,17 @@ __global__ void k_land_flags(const uint8_t* __restrict__ land, size_t N, int* __
 
 // The drainage order as a stable LSD radix sort of the land cells' compact keys, level N + deepest
 // source (distinct, ordered as the drainage keys are), 8 bits a pass over the bits they use. A CTA
-// takes a tile of kRsTile cells: it counts its digits, the counts are scanned digit-major over the
+// takes a tile of cells: it counts its digits, the counts are scanned digit-major over the
 // tiles, and the CTA scatters its tile in order, 256 cells at a time, each cell's place among the
 // chunk's cells of its digit found with __match_any_sync within its warp and per-warp counts across
-// warps, so cells of one digit keep their order.
+// warps, so cells of one digit keep their order. A tile is 4096 cells, or fewer (whole chunks) where that
+// would leave SMs without two: the chunks of a tile follow one another, and at 60,000 cells 15 CTAs of 16
+// chunks took 14 us a pass.
 constexpr int kRsTile = 4096;
 
 __global__ void k_land_compact_ck(const uint8_t* __restrict__ land, const int* __restrict__ pos,
                                   const long long* __restrict__ key, size_t N, unsigned long long* __restrict__ ck,
-                                  int* __restrict__ vals, unsigned long long* __restrict__ kmax) {
+                                  int* __restrict__ vals, unsigned long long* __restrict__ kmax) {   // kmax or null
     unsigned long long m = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x)
         if (land[i]) {
@@ -251,6 +254,7 @@ __global__ void k_land_compact_ck(const uint8_t* __restrict__ land, const int* _
             vals[pos[i]] = (int)i;
             m = c > m ? c : m;
         }
+    if (!kmax) return;
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long t = __shfl_down_sync(0xFFFFFFFFu, m, o);
         m = t > m ? t : m;
@@ -259,19 +263,19 @@ __global__ void k_land_compact_ck(const uint8_t* __restrict__ land, const int* _
 }
 
 __global__ void __launch_bounds__(256) k_rs_hist(const unsigned long long* __restrict__ keys, int n, int shift,
-                                                 int tiles, int* __restrict__ hist) {
+                                                 int tile, int tiles, int* __restrict__ hist) {
     __shared__ int h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
-    const int lo = blockIdx.x * kRsTile, hi = min(n, lo + kRsTile);
+    const int lo = blockIdx.x * tile, hi = min(n, lo + tile);
     for (int i = lo + (int)threadIdx.x; i < hi; i += 256) atomicAdd(&h[(int)((keys[i] >> shift) & 255ull)], 1);
     __syncthreads();
     hist[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
 __global__ void __launch_bounds__(256) k_rs_scatter(const unsigned long long* __restrict__ kin,
-                                                    const int* __restrict__ vin, int n, int shift, int tiles,
-                                                    const int* __restrict__ off, unsigned long long* __restrict__ kout,
+                                                    const int* __restrict__ vin, int n, int shift, int tile,
+                                                    int tiles, const int* __restrict__ off, unsigned long long* __restrict__ kout,
                                                     int* __restrict__ vout) {
     __shared__ int base[256];
     __shared__ int wcnt[8][256];
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(256) k_rs_scatter(const unsigned long long* __
 #pragma unroll
     for (int w = 0; w < 8; ++w) wcnt[w][tid] = 0;
     __syncthreads();
-    const int lo = blockIdx.x * kRsTile, hi = min(n, lo + kRsTile);
+    const int lo = blockIdx.x * tile, hi = min(n, lo + tile);
     for (int c = lo; c < hi; c += 256) {
         const int i = c + tid;
         const bool valid = i < hi;
@@ -597,9 +601,13 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
     CG_LAUNCH(ctx) k_sources<<<grid, 256, 0, sm>>>(d_land, d_mask, N, d_donors, d_pending, d_sources, d_nsrc);
     if (d_area) CG_LAUNCH(ctx) k_area_sea<<<grid, 256, 0, sm>>>(d_land, N, d_area);
     CG_CHECK_LAUNCH(ctx);
-    int n_sources = 0;
-    CG_CUDA(ctx, cudaMemcpyAsync(&n_sources, d_nsrc, sizeof(int), cudaMemcpyDeviceToHost, sm));
-    CG_CUDA(ctx, cudaStreamSynchronize(sm));
+    // A thread a source. Up to 2^21 cells the launch is sized for as many sources as cells, up to half a
+    // million (its idle CTAs cost less than the 10 us of a host read); larger worlds read their number.
+    int n_sources = (int)std::min(N, (size_t)1 << 19);
+    if (N > (size_t)1 << 21) {
+        CG_CUDA(ctx, cudaMemcpyAsync(&n_sources, d_nsrc, sizeof(int), cudaMemcpyDeviceToHost, sm));
+        CG_CUDA(ctx, cudaStreamSynchronize(sm));
+    }
     WalkArgs a{W, H, d_down, d_mask, d_pending, d_key, d_weights, d_area, d_sources, d_nsrc, d_max};
     if (n_sources > 0) CG_LAUNCH(ctx) k_walk<<<(n_sources + 63) / 64, 64, 0, sm>>>(a);
     CG_CHECK_LAUNCH(ctx);
@@ -613,7 +621,7 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
 }
 
 cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const long long* d_key,
-                              int land_cells, int32_t* d_order) {
+                              int land_cells, int32_t* d_order, int levels) {
     size_t N = (size_t)W * H;
     cudaStream_t sm = ctx->stream;
     int grid = ctx->num_sms * 8;
@@ -621,7 +629,8 @@ cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
     CG_BUF(int, d_flag, ctx, S_SCRATCH0, N);
     CG_BUF(int, d_pos, ctx, S_SCRATCH1, N);
     const int n = land_cells;
-    const int tiles = (n + kRsTile - 1) / kRsTile;
+    const int tile = std::min(kRsTile, std::max(1, n / (2 * ctx->num_sms * 256)) * 256);
+    const int tiles = (n + tile - 1) / tile;
     CG_BUF(unsigned long long, d_keys, ctx, S_RS_KEYS, 2 * (size_t)n + 1);
     CG_BUF(int, d_vals, ctx, S_RS_VALS, 2 * (size_t)n);
     CG_BUF(int, d_hist, ctx, S_RS_HIST, 2 * (size_t)tiles * 256);
@@ -635,20 +644,23 @@ cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
     CG_CHECK_LAUNCH(ctx);
     cg_status st = exclusive_scan(ctx, d_flag, d_pos, (int)N, nullptr);
     if (st != CG_OK) return st;
-    CG_CUDA(ctx, cudaMemsetAsync(kmax, 0, sizeof(unsigned long long), sm));
-    CG_LAUNCH(ctx) k_land_compact_ck<<<grid, 256, 0, sm>>>(d_land, d_pos, d_key, N, ka, va, kmax);
+    // The largest compact key: from the levels where the caller knows them (its bits, at any rate).
+    unsigned long long hmax = levels > 0 ? (unsigned long long)levels * N - 1 : 0;
+    if (levels <= 0) CG_CUDA(ctx, cudaMemsetAsync(kmax, 0, sizeof(unsigned long long), sm));
+    CG_LAUNCH(ctx) k_land_compact_ck<<<grid, 256, 0, sm>>>(d_land, d_pos, d_key, N, ka, va, levels > 0 ? nullptr : kmax);
     CG_CHECK_LAUNCH(ctx);
-    unsigned long long hmax = 0;
-    CG_CUDA(ctx, cudaMemcpyAsync(&hmax, kmax, sizeof(hmax), cudaMemcpyDeviceToHost, sm));
-    CG_CUDA(ctx, cudaStreamSynchronize(sm));
+    if (levels <= 0) {
+        CG_CUDA(ctx, cudaMemcpyAsync(&hmax, kmax, sizeof(hmax), cudaMemcpyDeviceToHost, sm));
+        CG_CUDA(ctx, cudaStreamSynchronize(sm));
+    }
     int bits = 0;
     while (bits < 64 && (hmax >> bits) != 0) ++bits;
     for (int shift = 0; shift < bits; shift += 8) {
-        CG_LAUNCH(ctx) k_rs_hist<<<tiles, 256, 0, sm>>>(ka, n, shift, tiles, d_hist);
+        CG_LAUNCH(ctx) k_rs_hist<<<tiles, 256, 0, sm>>>(ka, n, shift, tile, tiles, d_hist);
         CG_CHECK_LAUNCH(ctx);
         st = exclusive_scan(ctx, d_hist, d_off, tiles * 256, nullptr);
         if (st != CG_OK) return st;
-        CG_LAUNCH(ctx) k_rs_scatter<<<tiles, 256, 0, sm>>>(ka, va, n, shift, tiles, d_off, kb, vb);
+        CG_LAUNCH(ctx) k_rs_scatter<<<tiles, 256, 0, sm>>>(ka, va, n, shift, tile, tiles, d_off, kb, vb);
         CG_CHECK_LAUNCH(ctx);
         std::swap(ka, kb);
         std::swap(va, vb);

@@ -8,27 +8,87 @@ namespace cg {
 
 namespace {
 
-constexpr int SCAN_BLOCK = 1024;
+constexpr int kScanThreads = 256;
+constexpr int kScanTile = 4096;         // elements a CTA scans: 16 a thread
+constexpr int kScanDirect = 1 << 13;    // tiles whose sums every CTA adds up itself
 
-__global__ void k_scan_blocks(const int* __restrict__ in, int* __restrict__ out, int* __restrict__ sums, int n) {
-    __shared__ int sh[SCAN_BLOCK];
-    int i = blockIdx.x * SCAN_BLOCK + threadIdx.x;
-    int v = i < n ? in[i] : 0;
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < SCAN_BLOCK; o <<= 1) {
-        int t = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-        __syncthreads();
-        sh[threadIdx.x] += t;
-        __syncthreads();
+// The exclusive prefix of v over the CTA's threads, and the total; sh holds kScanThreads / 32 + 1 ints.
+__device__ __forceinline__ int cta_prefix(int v, int* total, int* sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
     }
-    if (i < n) out[i] = sh[threadIdx.x] - v;   // exclusive
-    if (threadIdx.x == SCAN_BLOCK - 1) sums[blockIdx.x] = sh[threadIdx.x];
+    if (lane == 31) sh[warp] = x;
+    __syncthreads();
+    int before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+        before += w < warp ? sh[w] : 0;
+        all += sh[w];
+    }
+    __syncthreads();
+    *total = all;
+    return before + x - v;
 }
 
-__global__ void k_scan_add(int* __restrict__ out, const int* __restrict__ offs, int n) {
-    int i = blockIdx.x * SCAN_BLOCK + threadIdx.x;
-    if (i < n) out[i] += offs[blockIdx.x];
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __restrict__ in, int n, int* __restrict__ sums) {
+    __shared__ int sh[kScanThreads / 32];
+    const int base = blockIdx.x * kScanTile;
+    int v = 0;
+#pragma unroll
+    for (int k = 0; k < kScanTile / kScanThreads; ++k) {
+        const int i = base + k * kScanThreads + (int)threadIdx.x;
+        v += i < n ? in[i] : 0;
+    }
+    int total;
+    cta_prefix(v, &total, sh);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+// A tile's exclusive scan, from the sum of the tiles before it: added up here from the tiles' sums, or
+// read where they have been scanned. The last tile leaves the total.
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* __restrict__ in, int n,
+                                                             const int* __restrict__ sums, const int* __restrict__ offs,
+                                                             int* __restrict__ out, int* __restrict__ total) {
+    __shared__ int sh[kScanThreads / 32];
+    __shared__ int warp_sum[kScanThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kPer = kScanTile / kScanThreads;
+    // A warp's kPer rows of 32 elements, a row a lane-wide scan.
+    const int base = blockIdx.x * kScanTile + warp * 32 * kPer + lane;
+    int v[kPer], run = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) v[k] = base + 32 * k < n ? in[base + 32 * k] : 0;
+    int tile_offset = 0;
+    if (offs) {
+        tile_offset = offs[blockIdx.x];
+    } else if (blockIdx.x > 0) {
+        int part = 0;
+        for (int b = threadIdx.x; b < (int)blockIdx.x; b += kScanThreads) part += sums[b];
+        cta_prefix(part, &tile_offset, sh);
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        int x = v[k];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        v[k] = run + x - v[k];
+        run += __shfl_sync(0xFFFFFFFFu, x, 31);
+    }
+    if (lane == 0) warp_sum[warp] = run;
+    __syncthreads();
+    int before = tile_offset;
+    for (int w = 0; w < warp; ++w) before += warp_sum[w];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+        if (base + 32 * k < n) out[base + 32 * k] = before + v[k];
+    if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == kScanThreads - 1) *total = before + run;
 }
 
 __device__ __forceinline__ int find_root(int* parent, int a) {
@@ -112,39 +172,33 @@ __global__ void k_label_from_root(const int* __restrict__ parent, const int* __r
 
 }  // namespace
 
+// Two launches, the tiles' sums and the tiles, each CTA adding up the sums before its own: a level of
+// block scans and a pass adding their offsets took four to six. A read of up to kScanDirect sums a CTA
+// stays below the tile's own; longer inputs scan the sums first.
 cg_status exclusive_scan(cg_ctx* ctx, const int* d_in, int* d_out, int n, int* h_total) {
     if (n <= 0) {
         if (h_total) *h_total = 0;
         return CG_OK;
     }
-    // Up to three levels: 2^10 elements per block, 2^10 block sums per second-level block, and a
-    // single block over at most 2^10 second-level sums: 2^30 elements.
-    int blocks = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
-    int blocks2 = (blocks + SCAN_BLOCK - 1) / SCAN_BLOCK;
-    if (blocks2 > SCAN_BLOCK) return fail(ctx, CG_BAD_ARG, "scan of %d elements is too long", n);
-    CG_BUF(int, d_tmp, ctx, S_SCRATCH5, 2 * (size_t)blocks + 2 * (size_t)blocks2 + 4);
-    int* d_sums1 = d_tmp;                 // [blocks]
-    int* d_offs1 = d_sums1 + blocks;      // [blocks]
-    int* d_sums2 = d_offs1 + blocks;      // [blocks2]
-    int* d_offs2 = d_sums2 + blocks2;     // [blocks2]
-    int* d_total = d_offs2 + blocks2;     // [1]
-    CG_LAUNCH(ctx) k_scan_blocks<<<blocks, SCAN_BLOCK, 0, ctx->stream>>>(d_in, d_out, d_sums1, n);
-    CG_CHECK_LAUNCH(ctx);
-    if (blocks > 1) {
-        CG_LAUNCH(ctx) k_scan_blocks<<<blocks2, SCAN_BLOCK, 0, ctx->stream>>>(d_sums1, d_offs1, d_sums2, blocks);
-        if (blocks2 > 1) {
-            CG_LAUNCH(ctx) k_scan_blocks<<<1, SCAN_BLOCK, 0, ctx->stream>>>(d_sums2, d_offs2, d_total, blocks2);
-            CG_LAUNCH(ctx) k_scan_add<<<blocks2, SCAN_BLOCK, 0, ctx->stream>>>(d_offs1, d_offs2, blocks);
-        }
-        CG_LAUNCH(ctx) k_scan_add<<<blocks, SCAN_BLOCK, 0, ctx->stream>>>(d_out, d_offs1, n);
-        CG_CHECK_LAUNCH(ctx);
+    if (n > 1 << 30) return fail(ctx, CG_BAD_ARG, "scan of %d elements is too long", n);
+    const int tiles = (n + kScanTile - 1) / kScanTile;
+    const int tiles2 = tiles > kScanDirect ? (tiles + kScanTile - 1) / kScanTile : 0;
+    CG_BUF(int, d_tmp, ctx, S_SCRATCH5, 2 * (size_t)tiles + tiles2 + 1);
+    int* d_total = d_tmp;
+    int* d_sums = d_tmp + 1;
+    int* d_offs = tiles2 ? d_sums + tiles : nullptr;
+    if (tiles > 1) CG_LAUNCH(ctx) k_scan_sums<<<tiles, kScanThreads, 0, ctx->stream>>>(d_in, n, d_sums);
+    if (tiles2) {
+        int* d_sums2 = d_offs + tiles;
+        CG_LAUNCH(ctx) k_scan_sums<<<tiles2, kScanThreads, 0, ctx->stream>>>(d_sums, tiles, d_sums2);
+        CG_LAUNCH(ctx) k_scan_tiles<<<tiles2, kScanThreads, 0, ctx->stream>>>(d_sums, tiles, d_sums2, nullptr, d_offs,
+                                                                              nullptr);
     }
+    CG_LAUNCH(ctx) k_scan_tiles<<<tiles, kScanThreads, 0, ctx->stream>>>(d_in, n, d_sums, d_offs, d_out, d_total);
+    CG_CHECK_LAUNCH(ctx);
     if (h_total) {
-        int last_in, last_out;
-        CG_CUDA(ctx, cudaMemcpyAsync(&last_in, d_in + n - 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        CG_CUDA(ctx, cudaMemcpyAsync(&last_out, d_out + n - 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        CG_CUDA(ctx, cudaMemcpyAsync(h_total, d_total, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        *h_total = last_in + last_out;
     }
     return CG_OK;
 }

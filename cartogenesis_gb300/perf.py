@@ -25,7 +25,7 @@ BYTES_PER_CELL = {"ms_cut": 41.0, "ms_fill": 9.0, "ms_route": 28.0, "ms_tree": 2
                   "ms_deposit": 81.0}
 PHASE_KERNELS = {
     "ms_cut": "k_minmax, k_row_counts, k_bin_sums, k_bracket_*, k_land_and_water, k_uplift, k_unit_weights",
-    "ms_fill": "k_fill_init, k_jump, k_mark_drained, k_relax_tiles, k_check_ties",
+    "ms_fill": "k_fill_init, k_drain_chains, k_tiles_with_open, k_relax_passes, k_check_ties",
     "ms_route": "k_surface, k_cc_*, k_flat_solve_warp/_sm/_cl, k_flat_solve, k_receivers",
     "ms_tree": "k_links, k_sources, k_walk",
     "ms_incise": "k_depth_*, k_incise_levels (P1, P2: the notch's k_footprint_*, k_breach_waves)",
