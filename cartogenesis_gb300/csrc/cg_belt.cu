@@ -11,9 +11,10 @@
 //    local indices run in cell order) and gives them the same levels;
 //  - the facet rule (FlowRouting.facetReceiver) routes the belt's land over the caller-shaped surface;
 //  - the run order is the Kahn FIFO of FlowRouting.drainageOrder over the belt, so the tree walk's
-//    drainage keys (level, deepest source) order it; a cell's discharge and spoil flux add its donors
-//    in key order, and one cooperative kernel runs the Kahn levels with a grid barrier between them,
-//    upward for the sums and downward for the cut, which reads each receiver's final height;
+//    drainage keys (level, deepest source) order it; a cell's discharge (in that walk) and spoil flux (in
+//    a second one) add its donors in key order, and one cooperative kernel runs the Kahn levels downward
+//    for the cut, which reads each receiver's final height. Three level kernels with a grid barrier a
+//    level took 143 us of a round at 1024 x 512, the two walks and the cut take 62;
 //  - the books (uplift, cut, export to the sea and to the land, the slopes' shed) are the reference's
 //    running double sums: each round lays its terms out in the reference's order and adds them to the
 //    five totals exactly, side by side in one set of launches (seq_totals_f64_dev); a term the
@@ -258,18 +259,19 @@ __global__ void k_route_filled(const int* __restrict__ list, int B, const uint8_
     }
 }
 
-enum { LV_DISCHARGE = 0, LV_CUT = 1, LV_FLUX = 2 };
+// The cut, from the outlets up (BeltErosion.kt:327-351): a cell reads its receiver's final height. What the
+// receiver cannot change (the Courant number's square root and divisions, the fill, the unresolved relief)
+// is gathered for every cell at once; the levels then wait for one load and one division a cell.
+constexpr int kCutThreads = 1024;   // one CTA an SM: a shorter grid barrier than many
+constexpr int kActive = 1 << 30, kFlag = (int)(1u << 31);
 
-struct LevelArgs {
-    int W, H, levels, mode;
-    const int* bucket;          // belt cells by Kahn level
+struct CutArgs {
+    int W, levels, cells;
+    const int* order;           // belt cells in the run order, level after level
     const int* start;           // each level's first slot (levels + 1)
     const uint8_t* belt;
     const int32_t* recv;
-    const long long* key;       // drainage keys
-    const float* weights;
-    const double* inflow;
-    double* disc;
+    const double* disc;
     const uint8_t* land;
     const float* filled;
     const float* unresolved;    // or null
@@ -278,92 +280,117 @@ struct LevelArgs {
     float* eroded;
     double* flux;
     double* cutv;
+    // Per slot: the cell (kActive: something may be cut; kFlag: its receiver is land), the receiver (kFlag: a
+    // belt cell), the height and the own unresolved relief; the receiver's fill and unresolved relief; 1 + the
+    // Courant number.
+    int4* cell;
+    float2* below;
+    double* den;
+    int* split;                 // the highest level left to the whole grid
     BeltConsts k;
 };
 
-// v plus the donors' values of cell c (val), added in drainage-key order: the order the reference's
-// FIFO hands them to c. Donors sit on lower levels, final before c's level runs.
-__device__ double add_donors(const LevelArgs& a, int c, double v, const double* val) {
-    const int row = pdiv(c, a.W), col = pmod(c, a.W);
-    long long kk[8];
-    int nn[8];
-    int k = 0;
-    for (int rs = -1; rs <= 1; ++rs) {
-        const int nr = row + rs;
-        if (nr < 0 || nr >= a.H) continue;
-        for (int cs = -1; cs <= 1; ++cs) {
-            if (rs == 0 && cs == 0) continue;
-            const int n = nr * a.W + wrap_col(col + cs, a.W);
-            if (!a.belt[n] || a.recv[n] != c) continue;
-            const long long kn = a.key[n];
-            int j = k++;
-            while (j > 0 && kk[j - 1] > kn) {
-                kk[j] = kk[j - 1];
-                nn[j] = nn[j - 1];
-                --j;
-            }
-            kk[j] = kn;
-            nn[j] = n;
-        }
+__device__ void gather_cut(const CutArgs& a, int slot) {
+    const BeltConsts& k = a.k;
+    const int c = a.order[slot], d = a.recv[c];
+    const float h = a.h[c];
+    if (d < 0 || __fsub_rn(a.filled[c], h) > k.pond) {
+        a.cell[slot] = make_int4(c, 0, 0, 0);
+        return;
     }
-    for (int j = 0; j < k; ++j) v = __dadd_rn(v, __ldcg(&val[nn[j]]));
-    return v;
+    const float own = a.unresolved ? a.unresolved[c] : 0.0f;
+    const double share = __ddiv_rn(a.disc[c], (double)k.land_cells);
+    const bool same_row = pdiv(c, a.W) == pdiv(d, a.W), same_col = pmod(c, a.W) == pmod(d, a.W);
+    const float step = (!same_row && !same_col) ? k.step_diag : (!same_row ? k.step_ns : 1.0f);
+    const double cn = __ddiv_rn(__dmul_rn(__dmul_rn((double)k.courant, __dsqrt_rn(share)), (double)a.factor[c]),
+                                (double)step);
+    a.cell[slot] = make_int4(c | kActive | (a.land[d] ? kFlag : 0), d | (a.belt[d] ? kFlag : 0), __float_as_int(h),
+                             __float_as_int(own));
+    a.below[slot] = make_float2(a.filled[d], a.unresolved ? a.unresolved[d] : 0.0f);
+    a.den[slot] = __dadd_rn(1.0, cn);
 }
 
-// One cell of the cut, from the outlets up (BeltErosion.kt:327-351): its receiver's height is final.
-__device__ void cut_cell(const LevelArgs& a, int c) {
+struct CutCell {
+    int4 cell;
+    float2 below;
+    double den;
+};
+
+__device__ __forceinline__ void load_cut(const CutArgs& a, int slot, CutCell& x) {
+    x.cell = __ldcg(a.cell + slot);
+    if (x.cell.x & kActive) {
+        x.below = __ldcg(a.below + slot);
+        x.den = __ldcg(a.den + slot);
+    }
+}
+
+__device__ __forceinline__ void cut_cell(const CutArgs& a, const CutCell& x) {
     const BeltConsts& k = a.k;
+    const int c = x.cell.x & (kActive - 1);
     double t = 0.0;
-    const int d = a.recv[c];
-    if (d >= 0) {
-        const float h = __ldcg(&a.h[c]);
-        if (!(__fsub_rn(a.filled[c], h) > k.pond)) {
-            const float own = a.unresolved ? a.unresolved[c] : 0.0f;
-            const float hd = __ldcg(&a.h[d]);
-            float base;
-            if (!a.land[d] || hd <= k.shoreline) base = __fadd_rn(k.shoreline, own);
-            else if (a.belt[d] && __fsub_rn(a.filled[d], hd) > k.pond) base = __fadd_rn(a.filled[d], own);
-            else base = __fsub_rn(__fadd_rn(hd, own), a.unresolved ? a.unresolved[d] : 0.0f);
-            if (!(h <= base)) {
-                const double share = __ddiv_rn(__ldcg(&a.disc[c]), (double)k.land_cells);
-                const bool same_row = pdiv(c, a.W) == pdiv(d, a.W), same_col = pmod(c, a.W) == pmod(d, a.W);
-                const float step = (!same_row && !same_col) ? k.step_diag : (!same_row ? k.step_ns : 1.0f);
-                const double cn = __ddiv_rn(__dmul_rn(__dmul_rn((double)k.courant, __dsqrt_rn(share)), (double)a.factor[c]),
-                                            (double)step);
-                const float after = __double2float_rn(
-                    __dadd_rn((double)base, __ddiv_rn((double)__fsub_rn(h, base), __dadd_rn(1.0, cn))));
-                __stcg(&a.h[c], after);
-                const float lost = __fmul_rn(__fsub_rn(h, after), k.mpfu);
-                a.eroded[c] = __fadd_rn(a.eroded[c], lost);
-                t = __dmul_rn((double)lost, k.area);
-            }
+    if (x.cell.x & kActive) {
+        const int d = x.cell.y & ~kFlag;
+        const float h = __int_as_float(x.cell.z), own = __int_as_float(x.cell.w);
+        const float hd = __ldcg(a.h + d);
+        float base;
+        if (x.cell.x >= 0 || hd <= k.shoreline) base = __fadd_rn(k.shoreline, own);
+        else if (x.cell.y < 0 && __fsub_rn(x.below.x, hd) > k.pond) base = __fadd_rn(x.below.x, own);
+        else base = __fsub_rn(__fadd_rn(hd, own), x.below.y);
+        if (!(h <= base)) {
+            const float after =
+                __double2float_rn(__dadd_rn((double)base, __ddiv_rn((double)__fsub_rn(h, base), x.den)));
+            __stcg(a.h + c, after);
+            const float lost = __fmul_rn(__fsub_rn(h, after), k.mpfu);
+            a.eroded[c] = __fadd_rn(a.eroded[c], lost);
+            t = __dmul_rn((double)lost, k.area);
         }
     }
-    __stcg(&a.flux[c], t);
+    a.flux[c] = t;
     a.cutv[c] = t;
 }
 
-// The Kahn levels, upward for the discharge and the spoil flux, downward for the cut, one grid
-// barrier between levels.
-__global__ void __launch_bounds__(256) k_belt_levels(LevelArgs a) {
-    cgr::grid_group g = cgr::this_grid();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-    for (int s = 0; s < a.levels; ++s) {
-        const int L = a.mode == LV_CUT ? a.levels - 1 - s : s;
-        const int b1 = a.start[L + 1];
-        for (int i = a.start[L] + t; i < b1; i += nt) {
-            const int c = a.bucket[i];
-            if (a.mode == LV_DISCHARGE) {
-                const double v = add_donors(a, c, __dadd_rn((double)a.weights[c], a.inflow[c]), a.disc);
-                __stcg(&a.disc[c], v);
-            } else if (a.mode == LV_CUT) {
-                cut_cell(a, c);
-            } else {
-                const double v = add_donors(a, c, __ldcg(&a.flux[c]), a.flux);
-                __stcg(&a.flux[c], v);
+// The Kahn levels from the top down. The upper levels are small, and the first CTA takes those that fit two
+// of its passes alone, with a CTA barrier between them; the lower ones have the grid, and a grid barrier.
+// A thread's first cell of the next level is loaded before the barrier.
+__global__ void __launch_bounds__(kCutThreads) k_belt_cut(CutArgs a) {
+    cgr::grid_group grid = cgr::this_grid();
+    const int t = blockIdx.x * kCutThreads + threadIdx.x, stride = gridDim.x * kCutThreads;
+    for (int slot = t; slot < a.cells; slot += stride) gather_cut(a, slot);
+    grid.sync();
+    if (blockIdx.x == 0) {
+        int level = a.levels - 1, lo = a.start[level], hi = a.start[level + 1];
+        CutCell x{};
+        if (lo + (int)threadIdx.x < hi) load_cut(a, lo + threadIdx.x, x);
+        for (; level >= 0 && hi - lo <= 2 * kCutThreads; --level) {
+            const int slot = lo + (int)threadIdx.x;
+            if (slot < hi) cut_cell(a, x);
+            if (slot + kCutThreads < hi) {
+                load_cut(a, slot + kCutThreads, x);
+                cut_cell(a, x);
             }
+            hi = lo;
+            lo = level > 0 ? a.start[level - 1] : 0;
+            if (lo + (int)threadIdx.x < hi) load_cut(a, lo + threadIdx.x, x);
+            __syncthreads();
         }
-        g.sync();
+        if (threadIdx.x == 0) *a.split = level;
+    }
+    grid.sync();
+    const int top = *(volatile int*)a.split;
+    if (top < 0) return;
+    int lo = a.start[top], hi = a.start[top + 1];
+    CutCell x{};
+    if (lo + t < hi) load_cut(a, lo + t, x);
+    for (int level = top;; --level) {
+        for (int slot = lo + t; slot < hi; slot += stride) {
+            if (slot != lo + t) load_cut(a, slot, x);
+            cut_cell(a, x);
+        }
+        if (level == 0) break;
+        hi = lo;
+        lo = a.start[level - 1];
+        if (lo + t < hi) load_cut(a, lo + t, x);
+        grid.sync();
     }
 }
 
@@ -705,29 +732,33 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
     }
     const double crust_spread_km = kCrustKernelSpreadSpacings * opt.history_cell_km;
     int per_sm = 0;
-    CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_belt_levels, 256, 0));
-    if (per_sm < 1) return fail(ctx, CG_CUDA, "the belt's level kernel cannot be resident");
-    const int cgrid = ctx->num_sms * (per_sm < 2 ? per_sm : 2);
+    CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_belt_cut, kCutThreads, 0));
+    if (per_sm < 1) return fail(ctx, CG_CUDA, "the belt's cut kernel cannot be resident");
     const int bgrid = std::min(grid, (B + 255) / 256 + 1);
+    CG_BUF(int4, d_cut, ctx, S_BT_CUT, 2 * (size_t)B + 1);   // 32 bytes a cell
+    CG_BUF(int, d_start, ctx, S_BT_LEVELS, (size_t)B + 2);   // at most a level a cell, and the split
 
-    LevelArgs la{};
-    la.W = W;
-    la.H = H;
-    la.belt = d_belt;
-    la.recv = d_recv;
-    la.key = d_key;
-    la.weights = d_weights;
-    la.inflow = d_inflow;
-    la.disc = d_disc;
-    la.land = d_land;
-    la.filled = d_filled;
-    la.unresolved = in.unresolved;
-    la.factor = d_factor;
-    la.h = d_h;
-    la.eroded = d_eroded;
-    la.flux = d_flux;
-    la.cutv = d_cutv;
-    la.k = k;
+    CutArgs ca{};
+    ca.W = W;
+    ca.cells = B;
+    ca.order = d_order;
+    ca.start = d_start;
+    ca.belt = d_belt;
+    ca.recv = d_recv;
+    ca.disc = d_disc;
+    ca.land = d_land;
+    ca.filled = d_filled;
+    ca.unresolved = in.unresolved;
+    ca.factor = d_factor;
+    ca.h = d_h;
+    ca.eroded = d_eroded;
+    ca.flux = d_flux;
+    ca.cutv = d_cutv;
+    ca.cell = d_cut;
+    ca.below = (float2*)(d_cut + B);
+    ca.den = (double*)(ca.below + B);
+    ca.split = d_start + B + 1;
+    ca.k = k;
 
     for (int round = 0; round < k.rounds; ++round) {
         if (ctx->cancel.exchange(0)) return fail(ctx, CG_CANCELLED, "cancelled");
@@ -741,22 +772,16 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
         CG_LAUNCH(ctx) k_route_filled<<<bgrid, 256, 0, sm>>>(d_swept, B, d_routed, d_filled, d_routing);
         CG_CHECK_LAUNCH(ctx);
         CG_TRY_ST(facet_receivers_dev(ctx, W, H, d_routed, d_routing, p.seed, r, d_recv));
-        // The run order (BeltErosion.kt:296-311).
-        int levels = 0;
-        CG_TRY_ST(tree_walk_dev(ctx, W, H, d_belt, d_recv, nullptr, d_key, d_donors, nullptr, &levels));
-        int *d_bucket = nullptr, *d_start = nullptr;
-        CG_TRY_ST(level_buckets_dev(ctx, W, H, d_belt, d_key, levels, &d_bucket, &d_start));
-        CG_TRY_ST(order_from_keys_dev(ctx, W, H, d_belt, d_key, B, d_order, levels));
-        // Discharge, the cut and the spoil's flux, level by level (BeltErosion.kt:313-370).
-        la.levels = levels;
-        la.bucket = d_bucket;
-        la.start = d_start;
-        for (int mode : {LV_DISCHARGE, LV_CUT, LV_FLUX}) {
-            la.mode = mode;
-            void* kargs[] = {&la};
-            ctx->launches++;
-            CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_belt_levels, cgrid, 256, kargs, 0, sm));
-        }
+        // The run order and the discharge (BeltErosion.kt:296-325).
+        CG_TRY_ST(tree_walk_dev(ctx, W, H, d_belt, d_recv, d_weights, d_key, d_donors, nullptr, &ca.levels, d_inflow,
+                                d_disc));
+        CG_TRY_ST(order_from_keys_dev(ctx, W, H, d_belt, d_key, B, d_order, ca.levels));
+        CG_TRY_ST(level_bounds_dev(ctx, d_order, d_key, B, ca.levels, d_start));
+        // The cut and the spoil's flux (BeltErosion.kt:327-370).
+        void* kargs[] = {&ca};
+        ctx->launches++;
+        CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_belt_cut, ctx->num_sms, kCutThreads, kargs, 0, sm));
+        CG_TRY_ST(flow_walk_dev(ctx, W, H, d_key, d_flux));
         CG_LAUNCH(ctx) k_order_terms<<<bgrid, 256, 0, sm>>>(d_order, B, d_recv, d_belt, d_land, d_h, k.shoreline,
                                                             d_flux, d_cutv, xs_cut, xs_sea, xs_land);
         CG_CHECK_LAUNCH(ctx);

@@ -1451,17 +1451,6 @@ __global__ void k_rank_of(const int* __restrict__ order, int n, int* __restrict_
 }
 
 // Each level's first rank in the drainage order (level-major): level_start[levels] = n.
-__global__ void k_level_bounds(const int* __restrict__ order, const long long* __restrict__ key, int n, int levels,
-                               int* __restrict__ level_start) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const int L = (int)(key[order[k]] >> 32);
-        const int prev = k > 0 ? (int)(key[order[k - 1]] >> 32) : -1;
-        for (int l = prev + 1; l <= L; ++l) level_start[l] = k;
-        if (k == n - 1)
-            for (int l = L + 1; l <= levels; ++l) level_start[l] = n;
-    }
-}
-
 // settle(): the stage's deposition laid on the rock at once; the sediment stays as the spoil the
 // mouths pass reads (HydraulicErosion.kt:1351-1364, 1451-1462).
 __global__ void k_settle(float* __restrict__ h, const float* __restrict__ sediment, size_t N) {
@@ -1587,8 +1576,8 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     CG_BUF(int, d_lstart, ctx, S_DEPLEVEL, (size_t)r.levels + 1);
     const int grid = ctx->num_sms * 8;
     CG_LAUNCH(ctx) k_rank_of<<<grid, 256, 0, sm>>>(d_order, n, d_rank);
-    CG_LAUNCH(ctx) k_level_bounds<<<grid, 256, 0, sm>>>(d_order, r.key, n, r.levels, d_lstart);
     CG_CHECK_LAUNCH(ctx);
+    CG_TRY_ST(level_bounds_dev(ctx, d_order, r.key, n, r.levels, d_lstart));
     w.order = d_order;
     w.rank_of = d_rank;
     w.key = r.key;

@@ -53,9 +53,14 @@ cg_status facet_receivers_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, 
 // ---- drainage tree (cg_tree.cu)
 // Donor counts, the Kahn queue keys (level << 32 | deepest source) of FlowRouting.drainageOrder and,
 // if d_weights is given, FlowRouting.accumulate's areas, in one last-arriver walk. *h_levels
-// (optional, synchronises) receives the number of Kahn levels.
+// (optional, synchronises) receives the number of Kahn levels. With d_flow the sums are in double, of
+// the weights and d_inflow, into d_flow.
 cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int32_t* d_recv,
-                        const float* d_weights, long long* d_key, int32_t* d_donors, float* d_area, int* h_levels);
+                        const float* d_weights, long long* d_key, int32_t* d_donors, float* d_area, int* h_levels,
+                        const double* d_inflow = nullptr, double* d_flow = nullptr);
+// Once after a tree_walk_dev, over the tree it walked (its links, its sources and its counts, which are
+// in S_LINKS, S_SOURCES and S_DEPTH until the next user): every cell's d_flow plus its donors', in key order.
+cg_status flow_walk_dev(cg_ctx* ctx, int W, int H, long long* d_key, double* d_flow);
 // The explicit drainage order (land cells sorted by key), for callers that want it; `levels` the keys'
 // number of Kahn levels, 0 where the caller does not know it (synchronises).
 cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const long long* d_key,
@@ -72,8 +77,10 @@ struct InciseArgs {
 };
 // d_incised_at (may be NULL): per cell, what the incision took off it, in double (profile P2).
 cg_status incise_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int32_t* d_recv, const long long* d_key,
-                     int levels, const float* d_ground, const float* d_rel, const float* d_area, const float* d_erod,
+                     int levels, int land_cells, const float* d_ground, const float* d_rel, const float* d_area, const float* d_erod,
                      float* d_surface, const InciseArgs& a, double* d_incised_at = nullptr);
+// Each Kahn level's first slot in the drainage order (levels + 1 entries).
+cg_status level_bounds_dev(cg_ctx* ctx, const int* d_order, const long long* d_key, int n, int levels, int* d_start);
 // Land cells bucketed by Kahn level (the high half of the drainage key): d_bucket (N) holds them
 // level after level, d_start (levels + 1) each level's first slot. Cells within a level are in no
 // particular order.

@@ -278,7 +278,7 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
         ia.step_ns = rates.step_ns;
         ia.step_diag = rates.step_diag;
         ia.only_above_base = p.receiver_clamp != 0;
-        CG_TRY(incise_dev(ctx, W, H, d_land, d_recv, d_key, levels, d_filled, d_rel, d_area, d_erod, cur, ia,
+        CG_TRY(incise_dev(ctx, W, H, d_land, d_recv, d_key, levels, land_cells, d_filled, d_rel, d_area, d_erod, cur, ia,
                           d_incised_at));
         mark(5);
         DepositCounts dc{};

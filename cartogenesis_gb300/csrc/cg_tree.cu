@@ -14,8 +14,8 @@
 // additions in the reference's order) and carries on; the others stop. No barrier, O(N) work.
 //
 // Incision needs each receiver final before its donors: cells are bucketed by their Kahn level (a
-// receiver's level is always higher than its donors') and one cooperative kernel sweeps the levels
-// from the top down with a grid barrier between them. Every order with receivers first gives the
+// receiver's level is always higher than its donors') and one cooperative kernel gathers what the sweep
+// cannot change and then sweeps the levels from the top down with a grid barrier between them. Every order with receivers first gives the
 // same bits, because a cell reads only its receiver's final state.
 #include <cooperative_groups.h>
 #include <cuda/atomic>
@@ -135,61 +135,93 @@ struct WalkArgs {
     const uint8_t* mask;
     int32_t* pending;
     long long* key;
-    const float* weights;   // null: keys only
+    const float* weights;
     float* area;
+    const double* inflow;
+    double* flow;
     const int* sources;
     const int* n_sources;
     unsigned long long* max_key;
 };
 
+// What a walk adds up beside the keys: nothing, areas (float weights), discharges (weights and the
+// inflows from off the tree, in double), or, over a tree whose keys are known, flows that start as each
+// cell's own.
+enum { WALK_KEYS, WALK_AREA, WALK_DISCHARGE, WALK_FLOW };
+
+template <int M>
+struct WalkValue {
+    using type = double;
+};
+template <>
+struct WalkValue<WALK_AREA> {
+    using type = float;
+};
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+
 // One thread per source climbs down its receivers while it is the last donor into each. At a cell
-// r it already holds the key and area of the cell it came from; r's donor mask and weight are
+// r it already holds the key and value of the cell it came from; r's donor mask and own value are
 // loaded beside the atomic that decides whether it goes on, so a step costs the atomic and one
-// round of loads of the other donors' keys and areas.
+// round of loads of the other donors' keys and values. The counts end at 0, so a second walk over
+// the same tree counts up to the donors again.
+template <int M>
 __global__ void __launch_bounds__(64) k_walk(WalkArgs a) {
-    const unsigned FULL = 0xFFFFFFFFu;
+    using V = typename WalkValue<M>::type;
+    V* const val = M == WALK_AREA ? (V*)a.area : (V*)a.flow;
+    auto own = [&](int c) -> V {
+        if (M == WALK_AREA) return (V)a.weights[c];
+        if (M == WALK_DISCHARGE) return (V)__dadd_rn((double)a.weights[c], a.inflow[c]);
+        if (M == WALK_FLOW) return (V)a.flow[c];
+        return (V)0;
+    };
     unsigned long long local_max = 0;
     const int n_sources = *a.n_sources;
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n_sources; idx += gridDim.x * blockDim.x) {
         int c = a.sources[idx];
         long long kc = (long long)c;   // a source: level 0, its own index
-        float ac = a.weights ? a.weights[c] : 0.0f;
-        a.key[c] = kc;
-        if (a.weights) a.area[c] = ac;
+        V vc = own(c);
+        if (M != WALK_FLOW) a.key[c] = kc;
+        if (M == WALK_AREA || M == WALK_DISCHARGE) val[c] = vc;
         if ((unsigned long long)kc > local_max) local_max = (unsigned long long)kc;
         while (true) {
             const int d = a.down[c];
             if (d == 0xFF) break;
             const int r = step_to(a.W, c, d);
             const unsigned m = a.mask[r];
-            const float wr = a.weights ? a.weights[r] : 0.0f;
-            // Release: this cell's key and area are visible before its arrival is counted. Acquire:
+            const V vr = own(r);
+            const long long kr = M == WALK_FLOW ? a.key[r] : 0;
+            // Release: this cell's key and value are visible before its arrival is counted. Acquire:
             // the last donor in sees every other donor's.
             cuda::atomic_ref<int, cuda::thread_scope_device> pend(a.pending[r]);
-            if (pend.fetch_sub(1, cuda::memory_order_acq_rel) != 1) break;   // not the last donor in
-            // The donors' keys and areas (the cell just left from registers). Keys are distinct, so
-            // each donor's rank is the number of smaller keys; the areas are added in rank order.
+            if (M == WALK_FLOW) {
+                if (pend.fetch_add(1, cuda::memory_order_acq_rel) + 1 != __popc(m)) break;
+            } else {
+                if (pend.fetch_sub(1, cuda::memory_order_acq_rel) != 1) break;   // not the last donor in
+            }
+            // The donors' keys and values (the cell just left from registers). Keys are distinct, so
+            // each donor's rank is the number of smaller keys; the values are added in rank order.
             long long kt[8];
-            float at[8];
+            V vt[8];
             long long kmax = LLONG_MIN;
 #pragma unroll
             for (int t = 0; t < 8; ++t) {
                 kt[t] = LLONG_MAX;
-                at[t] = 0.0f;
+                vt[t] = (V)0;
                 if (!(m & (1u << t))) continue;
                 const int dn = step_to(a.W, r, t);
                 if (dn == c) {
                     kt[t] = kc;
-                    at[t] = ac;
+                    vt[t] = vc;
                 } else {
                     kt[t] = *((volatile long long*)&a.key[dn]);
-                    if (a.weights) at[t] = *((volatile float*)&a.area[dn]);
+                    if (M != WALK_KEYS) vt[t] = *((volatile V*)&val[dn]);
                 }
                 kmax = kt[t] > kmax ? kt[t] : kmax;
             }
-            kc = kmax + LEVEL_ONE;
-            a.key[r] = kc;
-            if (a.weights) {
+            kc = M == WALK_FLOW ? kr : kmax + LEVEL_ONE;
+            if (M != WALK_FLOW) a.key[r] = kc;
+            if (M != WALK_KEYS) {
                 int rank[8];
 #pragma unroll
                 for (int t = 0; t < 8; ++t) {
@@ -198,27 +230,29 @@ __global__ void __launch_bounds__(64) k_walk(WalkArgs a) {
                     for (int u = 0; u < 8; ++u) rank[t] += (kt[u] < kt[t]) ? 1 : 0;
                 }
                 const int n = __popc(m);
-                float sum = wr;
+                V sum = vr;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     if (j >= n) break;
-                    float pick = 0.0f;
+                    V pick = (V)0;
 #pragma unroll
-                    for (int t = 0; t < 8; ++t) pick = rank[t] == j && (m & (1u << t)) ? at[t] : pick;
-                    sum = __fadd_rn(sum, pick);
+                    for (int t = 0; t < 8; ++t) pick = rank[t] == j && (m & (1u << t)) ? vt[t] : pick;
+                    sum = add_rn(sum, pick);
                 }
-                ac = sum;
-                a.area[r] = sum;
+                vc = sum;
+                val[r] = sum;
             }
             if ((unsigned long long)kc > local_max) local_max = (unsigned long long)kc;
             c = r;
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(FULL, local_max, o);
-        if (other > local_max) local_max = other;
+    if constexpr (M != WALK_FLOW) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, local_max, o);
+            if (other > local_max) local_max = other;
+        }
+        if ((threadIdx.x & 31) == 0 && local_max) atomicMax(a.max_key, local_max);
     }
-    if ((threadIdx.x & 31) == 0 && local_max) atomicMax(a.max_key, local_max);
 }
 
 // Areas of land cells are the weights where no walk reached (sea cells hold 0).
@@ -314,6 +348,17 @@ __global__ void __launch_bounds__(256) k_rs_scatter(const unsigned long long* __
     }
 }
 
+__global__ void k_level_bounds(const int* __restrict__ order, const long long* __restrict__ key, int n, int levels,
+                               int* __restrict__ level_start) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int L = (int)(key[order[k]] >> 32);
+        const int prev = k > 0 ? (int)(key[order[k - 1]] >> 32) : -1;
+        for (int l = prev + 1; l <= L; ++l) level_start[l] = k;
+        if (k == n - 1)
+            for (int l = L + 1; l <= levels; ++l) level_start[l] = n;
+    }
+}
+
 // ---- incise
 
 // Cells bucketed by their Kahn level (the high half of their drainage key). A cell's receiver sits
@@ -325,6 +370,7 @@ __global__ void __launch_bounds__(256) k_rs_scatter(const unsigned long long* __
 // (a shared-memory atomic) after the chunk's base for that level. Level 0 holds millions of cells,
 // so atomics per warp on its cursor were the kernels' cost. Worlds with more than LVL_SMEM levels
 // take the per-warp kernels.
+constexpr int kLevelThreads = 1024;   // k_incise_levels's CTAs, one an SM: a shorter grid barrier than many
 constexpr int LVL_SMEM = 4096;
 constexpr int LVL_PER = 8;
 
@@ -417,43 +463,56 @@ struct InciseDev {
     double* incised_at; // or NULL
     const int* start;   // depth buckets, [levels + 1]
     const int* bucket;
+    int4* fixed;        // per slot of the buckets: what no other cell changes (IncisedCell)
+    float* courant;
     int levels;
     int* split;         // the highest level left to the whole grid
 };
 
-// HydraulicErosion.baseLevel (HydraulicErosion.kt:2380-2390).
-__device__ __forceinline__ float base_level(const InciseDev& d, int r) {
-    if (!d.land[r]) return d.a.shoreline;
-    float w = d.water[r];
-    if (!isnan(w)) return fmaxf(d.surface[r], w);
-    return d.surface[r];
+// A cell of HydraulicErosion.incise (HydraulicErosion.kt:2322-2359) is settled in two parts. What the
+// rest of the sweep cannot change (its receiver, its fill, its Courant number, its own height, which only
+// its own step lowers) is gathered for every cell at once before the levels run; the levels then read it in
+// slot order and wait for nothing but the receiver's height and water.
+constexpr int kUnder = 1 << 30, kLandBelow = (int)(1u << 31);
+
+__device__ void gather_incise(const InciseDev& d, int slot) {
+    const int cell = d.bucket[slot], r = d.recv[cell];
+    const float ground = d.ground[cell];
+    int flags = __fsub_rn(ground, d.rel[cell]) > d.a.pond_depth ? kUnder : 0;
+    if (r >= 0 && d.land[r]) flags |= kLandBelow;
+    // GroundSteps.between (MA/GroundSteps.kt:45-53).
+    const bool same_row = pdiv(cell, d.W) == pdiv(r, d.W), same_col = pmod(cell, d.W) == pmod(r, d.W);
+    const float step = (!same_row && !same_col) ? d.a.step_diag : (!same_row ? d.a.step_ns : 1.0f);
+    d.courant[slot] = __fdiv_rn(__fmul_rn(__fmul_rn(d.a.courant_coefficient,
+                                                    __fsqrt_rn(__fdiv_rn(d.area[cell], d.a.land_cells))),
+                                          d.erod[cell]),
+                                step);
+    const float filled_level = __fadd_rn(d.a.shoreline, __fmul_rn(ground, d.a.land_range));
+    d.fixed[slot] = make_int4(cell | flags, r, __float_as_int(filled_level), __float_as_int(d.surface[cell]));
 }
 
-// One cell of HydraulicErosion.incise (HydraulicErosion.kt:2322-2359).
-__device__ void incise_cell(const InciseDev& d, int cell) {
-    int r = d.recv[cell];
-    bool under = __fsub_rn(d.ground[cell], d.rel[cell]) > d.a.pond_depth;
+__device__ __forceinline__ void incise_cell(const InciseDev& d, int4 fixed, float courant) {
+    const int cell = fixed.x & (kUnder - 1), r = fixed.y;
+    const bool under = (fixed.x & kUnder) != 0, land_below = fixed.x < 0;
+    const float filled_level = __int_as_float(fixed.z), height = __int_as_float(fixed.w);
     if (r < 0) {
-        if (under) d.water[cell] = __fadd_rn(d.a.shoreline, __fmul_rn(d.ground[cell], d.a.land_range));
+        if (under) __stcg(d.water + cell, filled_level);
         return;
     }
-    float base_after = base_level(d, r);
-    if (under) {
-        float filled_level = __fadd_rn(d.a.shoreline, __fmul_rn(d.ground[cell], d.a.land_range));
-        float wr = d.land[r] ? d.water[r] : NAN;
-        float downstream = (d.land[r] && !isnan(wr)) ? wr : base_after;
-        d.water[cell] = fminf(filled_level, downstream);
+    // HydraulicErosion.baseLevel (HydraulicErosion.kt:2380-2390).
+    float base_after = d.a.shoreline, wr = NAN;
+    if (land_below) {
+        base_after = __ldcg(d.surface + r);
+        wr = __ldcg(d.water + r);
+        if (!isnan(wr)) base_after = fmaxf(base_after, wr);
     }
-    float height = d.surface[cell];
-    // GroundSteps.between (MA/GroundSteps.kt:45-53).
-    bool same_row = cell / d.W == r / d.W, same_col = cell % d.W == r % d.W;
-    float step = (!same_row && !same_col) ? d.a.step_diag : (!same_row ? d.a.step_ns : 1.0f);
-    float courant = __fdiv_rn(__fmul_rn(__fmul_rn(d.a.courant_coefficient,
-                                                   __fsqrt_rn(__fdiv_rn(d.area[cell], d.a.land_cells))),
-                                        d.erod[cell]),
-                              step);
-    float grades_to = base_after;   // no unresolved relief in this profile
-    bool submerged = under && height <= d.water[cell];
+    float water = NAN;
+    if (under) {
+        water = fminf(filled_level, !isnan(wr) ? wr : base_after);
+        __stcg(d.water + cell, water);
+    }
+    const float grades_to = base_after;   // no unresolved relief in this profile
+    const bool submerged = under && height <= water;
     float after;
     if (submerged || (height <= grades_to && d.a.only_above_base)) {
         after = height;
@@ -462,32 +521,69 @@ __device__ void incise_cell(const InciseDev& d, int cell) {
         after = (float)__dadd_rn(g, __ddiv_rn((double)__fsub_rn(height, grades_to), __dadd_rn(1.0, (double)courant)));
     }
     if (after != height) {
-        d.surface[cell] = after;
+        __stcg(d.surface + cell, after);
         if (d.incised_at && after < height) d.incised_at[cell] = __dsub_rn((double)height, (double)after);
     }
 }
 
 // Levels from the top down. The highest levels are the main stems of the largest rivers, a few
-// cells each: while a level fits one pass of a CTA, the first CTA takes it alone, with a CTA barrier
+// cells each: while a level fits two passes of a CTA, the first CTA takes it alone, with a CTA barrier
 // between levels (its own writes are visible to it); the rest of the grid waits at one grid barrier
-// and then sweeps the lower, larger levels with a grid barrier per level.
-__global__ void __launch_bounds__(256) k_incise_levels(InciseDev d) {
+// and then sweeps the lower, larger levels with a grid barrier per level. A thread's first cell of the next
+// level is loaded before the barrier, so a level costs a barrier, the receiver's loads and one division. With
+// the whole cell read in its level a sweep took 240 us at 2048 x 1024 and 1.85 ms at 8192 x 4096; now 158 us
+// and 1.37 ms.
+__global__ void __launch_bounds__(kLevelThreads) k_incise_levels(InciseDev d) {
     cgr::grid_group grid = cgr::this_grid();
+    const int t = blockIdx.x * kLevelThreads + threadIdx.x, stride = gridDim.x * kLevelThreads;
+    for (int slot = t; slot < d.start[d.levels]; slot += stride) gather_incise(d, slot);
+    grid.sync();
+    const int4 none = make_int4(0, -1, 0, 0);
     if (blockIdx.x == 0) {
         int level = d.levels - 1;
-        for (; level >= 0; --level) {
-            const int lo = d.start[level], hi = d.start[level + 1];
-            if (hi - lo > (int)blockDim.x) break;
-            if (lo + (int)threadIdx.x < hi) incise_cell(d, d.bucket[lo + threadIdx.x]);
+        int lo = d.start[level], hi = d.start[level + 1];
+        int4 fixed = none;
+        float courant = 0.0f;
+        auto load = [&](int slot, int end) {
+            if (slot < end) {
+                fixed = __ldcg(d.fixed + slot);
+                courant = __ldcg(d.courant + slot);
+            }
+        };
+        load(lo + (int)threadIdx.x, hi);
+        for (; level >= 0 && hi - lo <= 2 * kLevelThreads; --level) {
+            int slot = lo + (int)threadIdx.x;
+            if (slot < hi) incise_cell(d, fixed, courant);
+            slot += kLevelThreads;
+            if (slot < hi) incise_cell(d, __ldcg(d.fixed + slot), __ldcg(d.courant + slot));
+            hi = lo;
+            lo = level > 0 ? d.start[level - 1] : 0;
+            load(lo + (int)threadIdx.x, hi);
             __syncthreads();
         }
         if (threadIdx.x == 0) *d.split = level;
     }
     grid.sync();
-    const int stride = gridDim.x * blockDim.x;
-    for (int level = *(volatile int*)d.split; level >= 0; --level) {
-        const int lo = d.start[level], hi = d.start[level + 1];
-        for (int i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += stride) incise_cell(d, d.bucket[i]);
+    const int top = *(volatile int*)d.split;
+    if (top < 0) return;
+    int lo = d.start[top], hi = d.start[top + 1];
+    int4 fixed = none;
+    float courant = 0.0f;
+    if (lo + t < hi) {
+        fixed = __ldcg(d.fixed + lo + t);
+        courant = __ldcg(d.courant + lo + t);
+    }
+    for (int level = top;; --level) {
+        if (lo + t < hi) incise_cell(d, fixed, courant);
+        for (int slot = lo + t + stride; slot < hi; slot += stride)
+            incise_cell(d, __ldcg(d.fixed + slot), __ldcg(d.courant + slot));
+        if (level == 0) break;
+        hi = lo;
+        lo = d.start[level - 1];
+        if (lo + t < hi) {
+            fixed = __ldcg(d.fixed + lo + t);
+            courant = __ldcg(d.courant + lo + t);
+        }
         grid.sync();
     }
 }
@@ -583,7 +679,8 @@ __global__ void k_basin_finish(BasinDev b, int count, const uint8_t* __restrict_
 }  // namespace
 
 cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int32_t* d_recv,
-                        const float* d_weights, long long* d_key, int32_t* d_donors, float* d_area, int* h_levels) {
+                        const float* d_weights, long long* d_key, int32_t* d_donors, float* d_area, int* h_levels,
+                        const double* d_inflow, double* d_flow) {
     size_t N = (size_t)W * H;
     cudaStream_t sm = ctx->stream;
     int grid = ctx->num_sms * 8;
@@ -608,8 +705,13 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
         CG_CUDA(ctx, cudaMemcpyAsync(&n_sources, d_nsrc, sizeof(int), cudaMemcpyDeviceToHost, sm));
         CG_CUDA(ctx, cudaStreamSynchronize(sm));
     }
-    WalkArgs a{W, H, d_down, d_mask, d_pending, d_key, d_weights, d_area, d_sources, d_nsrc, d_max};
-    if (n_sources > 0) CG_LAUNCH(ctx) k_walk<<<(n_sources + 63) / 64, 64, 0, sm>>>(a);
+    WalkArgs a{W, H, d_down, d_mask, d_pending, d_key, d_weights, d_area, d_inflow, d_flow, d_sources, d_nsrc, d_max};
+    const int ctas = (n_sources + 63) / 64;
+    if (ctas > 0) {
+        if (d_flow) CG_LAUNCH(ctx) k_walk<WALK_DISCHARGE><<<ctas, 64, 0, sm>>>(a);
+        else if (d_weights) CG_LAUNCH(ctx) k_walk<WALK_AREA><<<ctas, 64, 0, sm>>>(a);
+        else CG_LAUNCH(ctx) k_walk<WALK_KEYS><<<ctas, 64, 0, sm>>>(a);
+    }
     CG_CHECK_LAUNCH(ctx);
     if (h_levels) {
         unsigned long long mk;
@@ -617,6 +719,19 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
         CG_CUDA(ctx, cudaStreamSynchronize(sm));
         *h_levels = (int)(mk >> 32) + 1;
     }
+    return CG_OK;
+}
+
+cg_status flow_walk_dev(cg_ctx* ctx, int W, int H, long long* d_key, double* d_flow) {
+    const size_t N = (size_t)W * H;
+    CG_BUF(int32_t, d_pending, ctx, S_DEPTH, N);
+    CG_BUF(uint8_t, d_links, ctx, S_LINKS, 2 * N);
+    CG_BUF(int, d_sources, ctx, S_SOURCES, N + 1);
+    WalkArgs a{W, H, d_links, d_links + N, d_pending, d_key, nullptr, nullptr, nullptr, d_flow, d_sources, d_sources + N,
+               nullptr};
+    const int ctas = ((int)std::min(N, (size_t)1 << 19) + 63) / 64;
+    CG_LAUNCH(ctx) k_walk<WALK_FLOW><<<ctas, 64, 0, ctx->stream>>>(a);
+    CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }
 
@@ -669,6 +784,13 @@ cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
     return CG_OK;
 }
 
+cg_status level_bounds_dev(cg_ctx* ctx, const int* d_order, const long long* d_key, int n, int levels, int* d_start) {
+    CG_LAUNCH(ctx) k_level_bounds<<<std::min(ctx->num_sms * 8, (n + 255) / 256), 256, 0, ctx->stream>>>(d_order, d_key, n,
+                                                                                                      levels, d_start);
+    CG_CHECK_LAUNCH(ctx);
+    return CG_OK;
+}
+
 cg_status level_buckets_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const long long* d_key, int levels,
                             int** out_bucket, int** out_start) {
     size_t N = (size_t)W * H;
@@ -695,7 +817,7 @@ cg_status level_buckets_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, co
 }
 
 cg_status incise_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int32_t* d_recv, const long long* d_key,
-                     int levels, const float* d_ground, const float* d_rel, const float* d_area, const float* d_erod,
+                     int levels, int land_cells, const float* d_ground, const float* d_rel, const float* d_area, const float* d_erod,
                      float* d_surface, const InciseArgs& args, double* d_incised_at) {
     size_t N = (size_t)W * H;
     cudaStream_t sm = ctx->stream;
@@ -733,16 +855,19 @@ cg_status incise_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int
     d.incised_at = d_incised_at;
     d.start = d_start;
     d.bucket = d_bucket;
+    CG_BUF(int4, d_fixed, ctx, S_INCFIXED, land_cells);
+    CG_BUF(float, d_courant, ctx, S_INCCOURANT, land_cells);
+    d.fixed = d_fixed;
+    d.courant = d_courant;
     d.levels = levels;
     d.split = d_cursor;   // the scatter's cursors are free by now
     int per_sm = 0;
-    CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_incise_levels, 256, 0));
+    CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_incise_levels, kLevelThreads, 0));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "incise kernel cannot be resident");
-    // Two CTAs per SM: the lower levels still fill the GPU, and a grid barrier over fewer CTAs is shorter.
-    int cgrid = ctx->num_sms * (per_sm < 2 ? per_sm : 2);
+    int cgrid = ctx->num_sms;
     void* kargs[] = {&d};
     ctx->launches++;
-    CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_incise_levels, cgrid, 256, kargs, 0, sm));
+    CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_incise_levels, cgrid, kLevelThreads, kargs, 0, sm));
     return CG_OK;
 }
 
