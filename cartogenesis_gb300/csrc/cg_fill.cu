@@ -41,7 +41,6 @@ namespace {
 
 constexpr float kStep = 1e-6f;   // FlowRouting.FLAT_GRADIENT_STEP
 constexpr int T = 32;            // tile side
-constexpr int TH = 8;            // tile rows per thread pass (block is 32 x 8)
 constexpr int kReplaySpan = 1 << 12;   // key levels (consecutive float values) one replay orders
 
 // Cell classes. PINNED: parent fixed by the index rule on a key tie; EXACT: parent fixed by
@@ -123,102 +122,123 @@ __global__ void k_drain_chains(int* p, const float* __restrict__ g, size_t N, ui
     }
 }
 
-// (2) tile relaxation. A CTA takes a 32x32 tile, loads f and g with a one-cell halo, relaxes its
-// OPEN cells to local convergence, and writes back what fell. PINNED cells take their designated
-// parent instead of the minimum. Returns (in every thread) whether a border cell fell or the tile
-// is still moving: then it and its neighbours go on the next pass's list.
+// (2) tile relaxation. A CTA takes a 32x32 tile and relaxes its OPEN cells to local convergence. A warp
+// holds four rows of the tile in registers, a column a lane: it sweeps them down and up, a row's west and
+// east neighbours by shuffles, until none of its cells falls, and only then publishes them and reads the
+// rows beside it, so the CTA's barriers come once for many cell steps. phi does not fall as its parent
+// rises, so a cell takes phi of its lowest neighbour, one phi for eight. PINNED cells take their designated
+// parent instead of the minimum. A cell's own level among its neighbours' changes nothing (phi of it is no
+// lower). Writes back what fell; returns (in every thread) whether a border cell fell or the tile is still
+// moving: then it and its neighbours go on the next pass's list.
+//
+// With eight phis a cell from shared memory and a CTA barrier for every step of a cell, a pass was as long
+// as its slowest tile's steps, 25 us at 2048 x 1024 (556 tiles) and 130 us at 8192 x 4096 (6170 tiles); it
+// takes 14 and 85 us now, most of it a tile's loads and its neighbours' marks.
 struct TileSmem {
     float sf[T + 2][T + 3];
-    float sg[T][T + 1];
-    uint8_t sc[T][T];
-    int any_border;
 };
+constexpr int kRows = T / 8;   // rows a warp holds
+constexpr int kSteps = 2 * T;  // a warp's own sweeps between barriers, at most
 
 __device__ __forceinline__ bool relax_tile(TileSmem& sm, int tile, float* __restrict__ f, const float* __restrict__ g,
                            const uint8_t* __restrict__ cls, const int* __restrict__ pin_parent, int W, int H,
                            int tiles_x, int max_sweeps) {
+    const unsigned FULL = 0xFFFFFFFFu;
     const int ty0 = (tile / tiles_x) * T, tx0 = (tile % tiles_x) * T;
     auto& sf = sm.sf;
-    auto& sg = sm.sg;
-    auto& sc = sm.sc;
-    const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;   // 32 x 8
-    for (int i = threadIdx.x; i < (T + 2) * (T + 2); i += 256) {
-        int yy = i / (T + 2), xx = i % (T + 2);
-        int gy = ty0 + yy - 1;
-        float v = INFINITY;
-        // L1-bypassing loads: neighbouring tiles on other SMs wrote these in earlier passes of the
-        // same launch, and a stale L1 line could make the tile look settled.
-        if (gy >= 0 && gy < H) v = __ldcg(f + (size_t)gy * W + wrap_col(tx0 + xx - 1, W));
-        sf[yy][xx] = v;
+    const int lx = threadIdx.x & 31, r0 = kRows * (threadIdx.x >> 5);
+    const int gx = tx0 + lx;
+    // L1-bypassing loads of the levels: neighbouring tiles on other SMs wrote these in earlier passes of
+    // the same launch, and a stale L1 line could make the tile look settled.
+    auto level = [&](int gy, int col) { return gy >= 0 && gy < H ? __ldcg(f + (size_t)gy * W + wrap_col(col, W)) : INFINITY; };
+    float c[kRows], was[kRows], gn[kRows], side[kRows];   // side: the neighbour past the tile, of the edge lanes
+    int parent[kRows];                                    // of a pinned cell, in sf; -1: an open cell, -2: settled
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+        const int gy = ty0 + r0 + k;
+        c[k] = was[k] = level(gy, gx);
+        side[k] = lx == 0 ? level(gy, tx0 - 1) : lx == T - 1 ? level(gy, tx0 + T) : INFINITY;
+        const bool in = gy < H && gx < W;
+        const size_t i = (size_t)gy * W + gx;
+        gn[k] = in ? g[i] : 0.0f;
+        const uint8_t cl = in ? cls[i] : (uint8_t)C_WATER;
+        parent[k] = cl == C_OPEN ? -1 : -2;
+        if (follows_parent(cl)) {
+            const int p = pin_parent[i], dy = pdiv(p, W) - gy;
+            int dx = pmod(p, W) - gx;
+            if (dx > 1) dx -= W;
+            if (dx < -1) dx += W;
+            parent[k] = (r0 + k + 1 + dy) * (T + 3) + lx + 1 + dx;
+        }
+        sf[r0 + k + 1][lx + 1] = c[k];
+        if (lx == 0) sf[r0 + k + 1][0] = side[k];
+        if (lx == T - 1) sf[r0 + k + 1][T + 1] = side[k];
     }
-    for (int i = threadIdx.x; i < T * T; i += 256) {
-        int yy = i / T, xx = i % T;
-        int gy = ty0 + yy, gx = tx0 + xx;
-        bool in = gy < H && gx < W;
-        sg[yy][xx] = in ? g[(size_t)gy * W + gx] : 0.0f;
-        sc[yy][xx] = in ? cls[(size_t)gy * W + gx] : (uint8_t)C_WATER;
+    if (r0 == 0 || r0 == T - kRows) {   // the rows past the tile
+        const int row = r0 == 0 ? 0 : T + 1, gy = ty0 + row - 1;
+        sf[row][lx + 1] = level(gy, gx);
+        if (lx == 0) sf[row][0] = level(gy, tx0 - 1);
+        if (lx == T - 1) sf[row][T + 1] = level(gy, tx0 + T);
     }
     __syncthreads();
     bool border_changed = false;
     int unsettled = 1;
     for (int sweep = 0; sweep < max_sweeps && unsettled; ++sweep) {
-        bool changed = false;
-        for (int yy = ly; yy < T; yy += TH) {
-            uint8_t c = sc[yy][lx];
-            if (c != C_OPEN && !follows_parent(c)) continue;
-            int gy = ty0 + yy;
-            float gn = sg[yy][lx];
-            float best = sf[yy + 1][lx + 1];
-            if (c == C_OPEN) {
-                for (int rs = -1; rs <= 1; ++rs) {
-                    int ny = gy + rs;
-                    if (ny < 0 || ny >= H) continue;
-                    for (int cs = -1; cs <= 1; ++cs) {
-                        if (rs == 0 && cs == 0) continue;
-                        float fm = sf[yy + 1 + rs][lx + 1 + cs];
-                        float v = phi(fm, gn);
-                        if (v < best) best = v;
-                    }
+        float before[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            before[k] = c[k];
+            if (parent[k] >= 0) c[k] = phi((&sf[0][0])[parent[k]], gn[k]);   // up as well as down
+        }
+        const float above = fminf(fminf(sf[r0][lx], sf[r0][lx + 1]), sf[r0][lx + 2]);
+        const float below = fminf(fminf(sf[r0 + kRows + 1][lx], sf[r0 + kRows + 1][lx + 1]), sf[r0 + kRows + 1][lx + 2]);
+        for (int step = 0; step < kSteps; ++step) {
+            float beside[kRows];
+            bool fell = false;
+#pragma unroll
+            for (int k = 0; k < kRows; ++k)
+                beside[k] = fminf(fminf(__shfl_up_sync(FULL, c[k], 1), __shfl_down_sync(FULL, c[k], 1)), side[k]);
+            auto settle = [&](int k) {
+                const float up = k > 0 ? fminf(beside[k - 1], c[k - 1]) : above;
+                const float down = k < kRows - 1 ? fminf(beside[k + 1], c[k + 1]) : below;
+                const float v = phi(fminf(fminf(up, down), beside[k]), gn[k]);
+                if (parent[k] == -1 && v < c[k]) {
+                    c[k] = v;
+                    fell = true;
                 }
-            } else {
-                int p = pin_parent[(size_t)gy * W + tx0 + lx];
-                int pr = pdiv(p, W), pc = pmod(p, W);
-                int dy = pr - gy;
-                int dx = pc - (tx0 + lx);
-                if (dx > 1) dx -= W;
-                if (dx < -1) dx += W;
-                float v = phi(sf[yy + 1 + dy][lx + 1 + dx], gn);
-                if (v != best) best = v;   // a pinned cell follows its parent up as well as down
-            }
-            if (best != sf[yy + 1][lx + 1]) {
-                sf[yy + 1][lx + 1] = best;
-                changed = true;
-                // A border cell, or the last column when the grid is narrower than a tile (its
-                // east neighbour wraps to a column this tile only sees through its halo).
-                if (yy == 0 || yy == T - 1 || lx == 0 || lx == T - 1 || tx0 + lx == W - 1) border_changed = true;
-            }
+            };
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) settle(k);
+#pragma unroll
+            for (int k = kRows - 2; k >= 0; --k) settle(k);
+            if (!__any_sync(FULL, fell)) break;
+        }
+        bool changed = false;
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            if (c[k] == before[k]) continue;
+            sf[r0 + k + 1][lx + 1] = c[k];
+            changed = true;
+            // A border cell, or the last column when the grid is narrower than a tile (its
+            // east neighbour wraps to a column this tile only sees through its halo).
+            const int yy = r0 + k;
+            if (yy == 0 || yy == T - 1 || lx == 0 || lx == T - 1 || gx == W - 1) border_changed = true;
         }
         unsettled = __syncthreads_or(changed);
     }
     // Still moving after the sweep budget: run this tile again next pass.
-    const bool again = __syncthreads_or(border_changed) || unsettled;
-    for (int yy = ly; yy < T; yy += TH) {
-        int gy = ty0 + yy, gx = tx0 + lx;
-        if (gy >= H || gx >= W) continue;
-        uint8_t c = sc[yy][lx];
-        if (c != C_OPEN && !follows_parent(c)) continue;
-        float v = sf[yy + 1][lx + 1];
-        size_t idx = (size_t)gy * W + gx;
-        if (__ldcg(f + idx) != v) f[idx] = v;
-    }
-    __syncthreads();   // the shared tile is free for the next one
+    const bool again = __syncthreads_or(border_changed) || unsettled;   // and the shared tile is free
+#pragma unroll
+    for (int k = 0; k < kRows; ++k)
+        if (parent[k] != -2 && c[k] != was[k]) f[(size_t)(ty0 + r0 + k) * W + gx] = c[k];
     return again;
 }
 
 // The relaxation passes in one cooperative launch. Pass p takes the tiles of list[p & 1] (each marked
 // in mark[p & 1]); a tile that must run again puts itself and its 8 neighbours on the other list,
 // once each (the mark), and clears its own mark for the list after next. A grid barrier separates
-// the passes; the loop ends when a pass leaves the next list empty, or at max_passes (timed_out).
+// the passes, which take turns with three list counts, so that one is cleared while no CTA reads it; the
+// loop ends when a pass leaves the next list empty, or at max_passes (timed_out).
 struct RelaxArgs {
     float* f;
     const float* g;
@@ -227,19 +247,20 @@ struct RelaxArgs {
     int W, H, tiles_x, tiles_y;
     int* list[2];
     int* mark[2];
-    int* count;   // [2]
+    int* count;   // [3]
     int* timed_out;
     int max_passes;
 };
 
-__global__ void __launch_bounds__(256) k_relax_passes(RelaxArgs a) {
+__global__ void __launch_bounds__(256, 4) k_relax_passes(RelaxArgs a) {
     cgr::grid_group grid = cgr::this_grid();
     __shared__ TileSmem sm;
-    int pass = 0;
+    int pass = 0, now = 0;   // count[now]: this pass's list
     for (; pass < a.max_passes; ++pass) {
-        const int cur = pass & 1, nxt = cur ^ 1;
-        const int n = *(volatile int*)&a.count[cur];
+        const int cur = pass & 1, nxt = cur ^ 1, then = now == 2 ? 0 : now + 1;
+        const int n = *(volatile int*)&a.count[now];
         if (n == 0) break;
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.count[then == 2 ? 0 : then + 1] = 0;   // the pass after next's
         for (int t = blockIdx.x; t < n; t += gridDim.x) {
             const int tile = __ldcg(a.list[cur] + t);
             if (threadIdx.x == 0) a.mark[cur][tile] = 0;
@@ -248,15 +269,14 @@ __global__ void __launch_bounds__(256) k_relax_passes(RelaxArgs a) {
                 const int y = tile / a.tiles_x + dy;
                 if (y >= 0 && y < a.tiles_y) {
                     const int nb = y * a.tiles_x + (tile % a.tiles_x + dx + a.tiles_x) % a.tiles_x;
-                    if (atomicExch(&a.mark[nxt][nb], 1) == 0) a.list[nxt][atomicAdd(&a.count[nxt], 1)] = nb;
+                    if (atomicExch(&a.mark[nxt][nb], 1) == 0) a.list[nxt][atomicAdd(&a.count[then], 1)] = nb;
                 }
             }
         }
         grid.sync();
-        if (blockIdx.x == 0 && threadIdx.x == 0) a.count[cur] = 0;
-        grid.sync();
+        now = then;
     }
-    if (pass == a.max_passes && blockIdx.x == 0 && threadIdx.x == 0 && *(volatile int*)&a.count[pass & 1] != 0)
+    if (pass == a.max_passes && blockIdx.x == 0 && threadIdx.x == 0 && *(volatile int*)&a.count[now] != 0)
         *a.timed_out = 1;
 }
 
@@ -518,7 +538,7 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     CG_BUF(int, d_ptr, ctx, S_PTR, N);
     CG_BUF(int, d_pin, ctx, S_FILLQ, N);
     int tiles_x = (W + T - 1) / T, tiles_y = (H + T - 1) / T, tiles = tiles_x * tiles_y;
-    // Two tile lists and their marks, two list counts, the timeout flag (zeroed before each relaxation).
+    // Two tile lists and their marks, three list counts, the timeout flag (zeroed before each relaxation).
     CG_BUF(int, d_marks, ctx, S_TILEFLAG, 2 * (size_t)tiles);
     CG_BUF(int, d_lists, ctx, S_FILLLIST, 2 * (size_t)tiles + 4);
     RelaxArgs ra;
@@ -533,7 +553,7 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     ra.list[0] = d_lists;
     ra.list[1] = d_lists + tiles;
     ra.count = d_lists + 2 * (size_t)tiles;
-    ra.timed_out = ra.count + 2;
+    ra.timed_out = ra.count + 3;
     ra.mark[0] = d_marks;
     ra.mark[1] = d_marks + tiles;
     ra.max_passes = 4 * (tiles_x + tiles_y) + 64;
