@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(256) k_bin_sums(const unsigned* __restrict__ c
 }
 
 // SeaLevelStage.kt:614-622: the first bin that brings the weight below up to the target, the bins'
-// sequential sum taken by the CTA's scan (one thread adding 4096 doubles in turn took 140 us).
+// sequential sum told apart by predicted binades and chained (one thread adding 4096 doubles in turn took
+// 140 us, a CTA scan for every binade the sum grows through 70, this 17).
 __global__ void __launch_bounds__(seqwalk::kSSThreads) k_bracket_bin(const double* __restrict__ hist, double target,
                                                                      CutState* s) {
     using namespace seqwalk;
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(seqwalk::kSSThreads) k_bracket_bin(const doubl
     }
     const SumIn<double> in{hist, nullptr, 0, BINS, nullptr, nullptr, 0.0, nullptr, 0};
     __syncthreads();
-    cta_advance<true>(in, 0, BINS, sh, target);
+    cta_advance<true>(in, 0, BINS, sh, true, target);
     if (threadIdx.x == 0) {
         s->bracket_bin = sh.hit >= 0 ? sh.hit : BINS - 1;
         s->below_bracket = sh.hit >= 0 ? sh.below : sh.s;

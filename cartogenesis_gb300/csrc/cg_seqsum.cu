@@ -10,22 +10,19 @@
 // additions inside a binade is an integer walk whose only state is m's parity, and a run's walks
 // compose: a prefix scan over the values gives every partial m at once.
 //
-// A block of 8192 values is taken by one CTA, 8 values a thread (cta_advance): a scan for the binade
-// the sum is in, the first value whose partial m leaves that binade found over the CTA, and that one
-// addition taken in hardware; crossings cluster (a sum near zero changes sign many times), so one warp
-// then goes on 32 values at a time until a window holds no crossing, and the CTA scans again from
-// there. On GB300 a dependent chain of double additions fed from shared memory takes about 80 ns an
-// addition, so a piece of 1024 taken one by one cost 80 us; a crossing costs one CTA scan, about 3 us.
-// With the pieces taken one by one the 2048 x 1024 flexure took 13.5 ms a call, with the scans 5.1; the
-// belts' replay at 1024 x 512 (five sums a round, each its own launches) 161 ms, and 79 with the scans
-// and the five sums side by side.
+// A block of 8192 values is taken by one CTA, 8 values a thread (cta_advance): a scan for the binade the
+// sum is in, and the first value whose partial m leaves that binade found over the CTA. A block with such a
+// crossing is told apart (cta_classify): a scan of the values in fixed point says which binade every
+// partial sum is in, all but those next to a power of two; the values between two binades, and the few in
+// doubt, are listed, and the chain adds those in hardware, one after another, and the runs of steps between
+// them as integers. On GB300 a dependent chain of double additions fed from shared memory takes about 80 ns
+// an addition, so a piece of 1024 taken one by one cost 80 us, and a CTA scan for every crossing 3 to 5.
 //
-// Sums of up to kDirectBlocks blocks run so from the first value, one CTA per sum. Longer ones reduce
-// their blocks in parallel first, each under the binade an estimate of the running sum gives it: a
-// block's reduction is, for each entering parity, its total step, its lowest and highest partial steps
-// (which say whether the walk stays inside the binade) and its leaving parity. One warp then chains
-// the reductions 32 at a time by a scan, and a block that is not in the binade it was reduced for, or
-// does not stay in it, is taken by cta_advance.
+// Sums of up to kDirectBlocks blocks run so from the first value, one CTA per sum. Longer ones tell their
+// blocks apart in parallel first, each after an estimate of the sum before it, with a bound of how far that
+// may be off. One warp then chains the blocks, those without a listed value 32 at a time, and a block that
+// was not told apart, or whose steps do not apply, is taken by cta_advance. At 2048 x 1024 the flexure's load takes
+// 0.18 ms (2.3 with a CTA scan for every crossing), a mean of rain 49 us (166).
 #include <climits>
 #include <cstdint>
 
@@ -38,11 +35,10 @@ namespace {
 
 using namespace seqwalk;
 
-constexpr long long kBig = 1LL << 58;            // a partial step this large leaves any binade: give up
 constexpr int kMaxSums = 5;                      // sums of one launch
-// Sums up to this many blocks are taken by one CTA from the first value. A block taken so costs about
-// 2.5 us, the parallel form's three launches about 25 us before its first block.
-constexpr int kDirectBlocks = 10;
+// Sums up to this many blocks are taken by one CTA from the first value: a block costs about 6 us so, the
+// parallel form's three launches about 20 us and little for more blocks.
+constexpr int kDirectBlocks = 3;
 
 // The sums of one launch.
 template <typename T>
@@ -50,101 +46,21 @@ struct SumJobs {
     SumIn<T> in[kMaxSums];
 };
 
-// A run of additions inside one binade, for each parity of m entering it.
-struct Walk {
-    long long step[2], lo[2], hi[2];   // total step; lowest and highest partial step (lo > hi: no values)
-    int out[2];                        // parity of m leaving
-    int fail;                          // a value the integer walk cannot hold (it leaves the binade)
-    int spec;                          // the binade and sign it was made for (exponent | sign << 11), -1: none
-    int zero;                          // no value adds anything
+// A block told apart (cta_classify) after the sum the blocks before it are estimated at: how many values are
+// listed (-1: it was not), the binade of the first run of steps, the steps of all its runs, and the pieces of
+// 1024 that hold a listed value; and a listed value, the steps of the block before it and the binade of the
+// run after it.
+struct BlockSteps {
+    long long steps;
+    int spec, listed;
+    unsigned pieces;
 };
-
-__device__ __forceinline__ Walk walk_identity() {
-    Walk w;
-    for (int q = 0; q < 2; ++q) {
-        w.step[q] = 0;
-        w.lo[q] = kBig;
-        w.hi[q] = -kBig;
-        w.out[q] = q;
-    }
-    w.fail = 0;
-    w.spec = -1;
-    w.zero = 1;
-    return w;
-}
-
-// a then b.
-__device__ __forceinline__ Walk walk_then(const Walk& a, const Walk& b) {
-    Walk w;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const bool odd = a.out[q] != 0;
-        const long long step = odd ? b.step[1] : b.step[0], lo = odd ? b.lo[1] : b.lo[0], hi = odd ? b.hi[1] : b.hi[0];
-        w.step[q] = a.step[q] + step;
-        const long long blo = a.step[q] + lo, bhi = a.step[q] + hi;
-        w.lo[q] = lo > hi ? a.lo[q] : (a.lo[q] < blo ? a.lo[q] : blo);
-        w.hi[q] = lo > hi ? a.hi[q] : (a.hi[q] > bhi ? a.hi[q] : bhi);
-        w.out[q] = odd ? b.out[1] : b.out[0];
-    }
-    w.fail = a.fail | b.fail;
-    w.zero = a.zero & b.zero;
-    w.spec = a.spec;
-    if (w.step[0] > kBig || w.step[0] < -kBig || w.step[1] > kBig || w.step[1] < -kBig) w.fail = 1;
-    return w;
-}
-
-// The walk of a run of values in order, for both entering parities.
-struct LocalWalk {
-    Walk w;
-    __device__ void init() { w = walk_identity(); }
-    __device__ void add(const Step& st) {
-        if (st.fail) w.fail = 1;
-        for (int q = 0; q < 2; ++q) {
-            const int p = w.out[q];
-            const long long r = st.tie ? st.r + ((p + (int)(st.r & 1)) & 1) : st.r;
-            w.step[q] += r;
-            if (w.step[q] < w.lo[q]) w.lo[q] = w.step[q];
-            if (w.step[q] > w.hi[q]) w.hi[q] = w.step[q];
-            w.out[q] = st.tie ? 0 : (p ^ (int)(r & 1));
-            if (w.step[q] > kBig || w.step[q] < -kBig) w.fail = 1;
-        }
-    }
+constexpr int kListed = kMostAlone;   // a block's listed values, at most; a block with more is taken by hand
+struct Listed {
+    long long steps;
+    double value;
+    int spec;
 };
-
-__device__ __forceinline__ Walk shfl_walk(const Walk& w, int from) {
-    Walk o;
-    for (int q = 0; q < 2; ++q) {
-        o.step[q] = __shfl_sync(0xFFFFFFFFu, w.step[q], from);
-        o.lo[q] = __shfl_sync(0xFFFFFFFFu, w.lo[q], from);
-        o.hi[q] = __shfl_sync(0xFFFFFFFFu, w.hi[q], from);
-        o.out[q] = __shfl_sync(0xFFFFFFFFu, w.out[q], from);
-    }
-    o.fail = __shfl_sync(0xFFFFFFFFu, w.fail, from);
-    o.zero = __shfl_sync(0xFFFFFFFFu, w.zero, from);
-    o.spec = -1;
-    return o;
-}
-
-// The warp's walks composed in lane order; lane 0 gets the result.
-__device__ __forceinline__ Walk warp_walk(Walk w) {
-    const int lane = threadIdx.x & 31;
-    for (int off = 1; off < 32; off <<= 1) {   // lane i takes lanes i .. i + 2 off - 1, a tree over the lanes
-        const Walk o = shfl_walk(w, (lane + off) & 31);
-        if ((lane & (2 * off - 1)) == 0 && lane + off < 32) w = walk_then(w, o);
-    }
-    return w;
-}
-
-// The CTA's threads' walks composed in thread order; every thread calls it, thread 0 gets the result.
-__device__ Walk cta_walk(const Walk& mine, Walk* sh_warps) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const Walk w = warp_walk(mine);
-    if (lane == 0) sh_warps[warp] = w;
-    __syncthreads();
-    Walk total = walk_identity();
-    if (warp == 0) total = warp_walk(lane < (int)(blockDim.x >> 5) ? sh_warps[lane] : walk_identity());
-    return total;
-}
 
 template <typename T>
 __device__ __forceinline__ void finish_sum(const SumIn<T>& in, double s, long long whole, long long reduced,
@@ -178,121 +94,208 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_direct(SumJobs<T> jobs) {
     if (threadIdx.x == 0) finish_sum(in, sh.s, whole, reduced, alone);
 }
 
-// A cheap estimate of each block's sum (any order): it only picks the binade each block is reduced for.
+// A block's sum and the sum of its magnitudes, and how far those may be off: where its neighbours' sums
+// begin, and how surely. In fixed point, in units of 2^-60 of what they can reach, on the integer pipes
+// (double additions held the FP64 pipe for 12 us a launch).
+struct Estimate {
+    double sum, magnitude, off;
+};
 template <typename T>
-__global__ void __launch_bounds__(kSSThreads) k_ss_estimate(SumJobs<T> jobs, double* __restrict__ est) {
-    __shared__ double part[kSSThreads / 32];
+__global__ void __launch_bounds__(kSSThreads) k_ss_estimate(SumJobs<T> jobs, Estimate* __restrict__ est) {
+    __shared__ long long sums[kSSThreads / 32], spans[kSSThreads / 32];
+    __shared__ int tops[kSSThreads / 32];
+    const unsigned FULL = 0xFFFFFFFFu;
     const SumIn<T>& in = jobs.in[blockIdx.y];
     const size_t base = (size_t)blockIdx.x * kSSBlock;
-    if (base >= in.n) return;
-    double s = 0.0;
-    for (int t = 0; t < kSSPer; ++t) {
-        T v;
-        if (value_at(in, base + (size_t)t * kSSThreads + threadIdx.x, &v)) s += (double)v;
-    }
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xFFFFFFFFu, s, off);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = part[threadIdx.x];
-        for (int off = 16; off > 0; off >>= 1) t += __shfl_down_sync(0xFFFFFFFFu, t, off);
-        if (threadIdx.x == 0) est[in.first_block + blockIdx.x] = t;
-    }
-}
-
-// Each block's walk under the binade it is expected to begin in, that of the estimates before it. A
-// thread's values are consecutive.
-template <typename T>
-__global__ void __launch_bounds__(kSSThreads) k_ss_walks(SumJobs<T> jobs, const double* __restrict__ est,
-                                                        Walk* __restrict__ walks) {
-    __shared__ Walk sh_warps[kSSThreads / 32];
-    __shared__ double part[kSSThreads / 32];
-    __shared__ int s_spec;
-    const SumIn<T>& in = jobs.in[blockIdx.y];
-    const size_t base = (size_t)blockIdx.x * kSSBlock;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (base >= in.n) return;
     T v[kSSPer];
     const unsigned has = load_values(in, base, v);
-    double s = threadIdx.x == 0 && in.init ? *in.init : 0.0;
-    for (int i = (int)threadIdx.x; i < (int)blockIdx.x; i += kSSThreads) s += est[in.first_block + i];
-    if ((int)(threadIdx.x & ~31u) < (int)blockIdx.x || threadIdx.x < 32)   // the warps that hold an estimate
-        for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xFFFFFFFFu, s, off);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = part[threadIdx.x];
-        for (int off = 16; off > 0; off >>= 1) t += __shfl_down_sync(0xFFFFFFFFu, t, off);
-        if (threadIdx.x == 0) {
-            const Binade b = binade_of(t);
-            s_spec = b.normal ? (b.ef | (b.neg << 11)) : -1;
-        }
-    }
-    __syncthreads();
-    const int sp = s_spec;
-    LocalWalk lw;
-    lw.init();
+    int top = -1;
 #pragma unroll
     for (int t = 0; t < kSSPer; ++t)
-        if (has & (1u << t)) {
-            lw.w.zero = 0;
-            if (sp >= 0) lw.add(step_of(v[t], sp & 0x7FF, sp >> 11));
+        if ((has >> t) & 1u) top = max(top, field_of(v[t]));
+    top = __reduce_max_sync(FULL, top);
+    if (lane == 0) tops[warp] = top;
+    __syncthreads();
+    top = __reduce_max_sync(FULL, tops[lane]);
+    const int unit = max(top, 1) - kTopField<T> / 2 + 14 - 59;
+    long long sum = 0, span = 0;
+    if (top < kTopField<T>) {
+#pragma unroll
+        for (int t = 0; t < kSSPer; ++t) {
+            const long long q = (has >> t) & 1u ? units_of(magnitude_of(v[t]), unit) : 0;
+            sum += q;
+            span += q < 0 ? -q : q;
         }
-    Walk total = cta_walk(lw.w, sh_warps);
-    if (threadIdx.x == 0) {
-        total.spec = sp;
-        walks[in.first_block + blockIdx.x] = total;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_down_sync(FULL, sum, o);
+        span += __shfl_down_sync(FULL, span, o);
+    }
+    if (lane == 0) {
+        sums[warp] = sum;
+        spans[warp] = span;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        sum = sums[lane];
+        span = spans[lane];
+        for (int o = 16; o > 0; o >>= 1) {
+            sum += __shfl_down_sync(FULL, sum, o);
+            span += __shfl_down_sync(FULL, span, o);
+        }
+        if (lane == 0) {
+            Estimate e{0.0, 0.0, 0.0};
+            if (top == kTopField<T>) e.off = __longlong_as_double(0x7FF0000000000000LL);
+            else if (top >= 0)
+                e = Estimate{scalbn((double)sum, unit), scalbn((double)(span + kSSBlock), unit), scalbn((double)kSSBlock, unit)};
+            est[in.first_block + blockIdx.x] = e;
+        }
     }
 }
 
-// The chain over the blocks, one CTA a sum: warp 0 takes whole blocks 32 at a time while their walks
-// apply, the CTA takes the block where one does not.
+// Each block told apart after the estimates before it. The rounded sum is off from the real sum by at most
+// 2^-53 of the magnitudes before for every addition, n of them; adding up the estimates adds 64, and the
+// estimates' own offs; all doubled for the magnitudes' own roundings.
 template <typename T>
-__global__ void __launch_bounds__(kSSThreads) k_ss_chain(SumJobs<T> jobs, const Walk* __restrict__ walks) {
+__global__ void __launch_bounds__(kSSThreads) k_ss_walks(SumJobs<T> jobs, const Estimate* __restrict__ est,
+                                                        BlockSteps* __restrict__ blocks, Listed* __restrict__ lists) {
+    __shared__ CtaSum sh;
+    __shared__ Estimate part[kSSThreads / 32];
+    __shared__ double2 start;
+    const SumIn<T>& in = jobs.in[blockIdx.y];
+    const size_t base = (size_t)blockIdx.x * kSSBlock;
+    if (base >= in.n) return;
+    Estimate s{0.0, 0.0, 0.0};
+    auto over_warp = [&]() {
+        for (int o = 16; o > 0; o >>= 1) {
+            s.sum += __shfl_down_sync(0xFFFFFFFFu, s.sum, o);
+            s.magnitude += __shfl_down_sync(0xFFFFFFFFu, s.magnitude, o);
+            s.off += __shfl_down_sync(0xFFFFFFFFu, s.off, o);
+        }
+    };
+    for (int i = (int)threadIdx.x; i < (int)blockIdx.x; i += kSSThreads) {
+        const Estimate e = est[in.first_block + i];
+        s.sum += e.sum;
+        s.magnitude += e.magnitude;
+        s.off += e.off;
+    }
+    if ((int)(threadIdx.x & ~31u) < (int)blockIdx.x) over_warp();   // the warps that hold an estimate
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        s = part[threadIdx.x];
+        if (blockIdx.x > 32) over_warp();
+        if (threadIdx.x == 0) {
+            const double init = in.init ? *in.init : 0.0;
+            start = make_double2(s.sum + init, ((double)base + 64.0) * 0x1p-52 * (s.magnitude + fabs(init)) + 2.0 * s.off);
+        }
+    }
+    __syncthreads();
+    const int len = (int)(in.n - base < (size_t)kSSBlock ? in.n - base : (size_t)kSSBlock);
+    long long steps;
+    int listed = cta_classify<false>(in, base, 0, len, start.x, start.y, sh, 0.0, &steps);
+    if (listed > kListed) listed = -1;
+    const int block = in.first_block + blockIdx.x;
+    for (int k = threadIdx.x; k < listed; k += kSSThreads)
+        lists[(size_t)block * kListed + k] = Listed{sh.steps[k], sh.values[k], sh.spec[k + 1]};
+    if (threadIdx.x == 0) {
+        unsigned pieces = 0;
+        for (int k = 0; k < listed; ++k) pieces |= 1u << (sh.at[k] / kSSThreads);
+        blocks[block] = BlockSteps{steps, sh.spec[0], listed, pieces};
+    }
+}
+
+// s after a run of steps taken for the binade `spec` (-1: unchecked); false where they do not apply.
+__device__ __forceinline__ bool take_steps(double& s, long long steps, int spec) {
+    if (steps == 0) return true;
+    const Binade b = binade_of(s);
+    const long long m = b.m + steps;
+    if (!b.normal || !inside(m) || (spec != -1 && spec != (b.ef | (b.neg << 11)))) return false;
+    s = sum_of(b, m);
+    return true;
+}
+
+// The chain over the blocks, one CTA a sum: warp 0 takes whole blocks without a listed value together, up to
+// 32 by a scan, and the listed values of the others one by one (every lane the same); a block that was not
+// told apart, or whose steps do not apply, is taken by the CTA.
+template <typename T>
+__global__ void __launch_bounds__(kSSThreads) k_ss_chain(SumJobs<T> jobs, const BlockSteps* __restrict__ heads,
+                                                        const Listed* __restrict__ lists) {
     const unsigned FULL = 0xFFFFFFFFu;
     __shared__ CtaSum sh;
     __shared__ int sh_block;
+    __shared__ Listed list[kListed];
     const SumIn<T>& in = jobs.in[blockIdx.x];
     const int blocks = (int)((in.n + kSSBlock - 1) / kSSBlock);
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) sh.s = in.init ? *in.init : 0.0;
     __syncthreads();
     long long whole = 0, reduced = 0, alone = 0;
+    auto count = [&](unsigned pieces) {
+        const int a = __popc(pieces);
+        whole += a == 0;
+        reduced += a ? kSSPer - a : 0;
+        alone += a;
+    };
     for (int j = 0; j < blocks; ++j) {
         if (threadIdx.x < 32) {
             double s = sh.s;
-            while (j < blocks) {
-                const int k = j + lane;
-                Walk w = walk_identity();
-                if (k < blocks) w = walks[in.first_block + k];
-                const Binade b = binade_of(s);
-                const bool zero = k < blocks && w.zero;
-                bool ok = zero || (k < blocks && b.normal && !w.fail && w.spec == (b.ef | (b.neg << 11)));
-                Run mine = run_identity();
-                if (ok && !zero) {
-                    mine.step[0] = w.step[0];
-                    mine.step[1] = w.step[1];
-                    mine.out = (unsigned)w.out[0] | ((unsigned)w.out[1] << 1);
+            bool by_hand = false;
+            while (j < blocks && !by_hand) {
+                const int here = min(32, blocks - j);
+                BlockSteps w{0, -1, 0, 0};
+                if (lane < here) w = heads[in.first_block + j + lane];
+                int i = 0;
+                while (i < here && !by_hand) {
+                    // The blocks from i without a listed value, in the binade the sum is in.
+                    const Binade b = binade_of(s);
+                    const bool plain = w.listed == 0 && (w.spec < 0 ? w.steps == 0 : b.normal && w.spec == (b.ef | (b.neg << 11)));
+                    long long x = lane >= i ? w.steps : 0;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const long long y = __shfl_up_sync(FULL, x, o);
+                        if (lane >= o) x = wrap_add(x, y);
+                    }
+                    const bool ok = plain && (w.steps == 0 || inside(wrap_add(b.m, x)));
+                    const unsigned stop = __ballot_sync(FULL, !ok || lane >= here) & ~((1u << i) - 1u);
+                    const int end = stop ? __ffs(stop) - 1 : 32;
+                    if (end > i) {
+                        const long long steps = __shfl_sync(FULL, x, end - 1);
+                        if (steps != 0) s = sum_of(b, wrap_add(b.m, steps));
+                        whole += end - i;
+                        i = end;
+                        continue;
+                    }
+                    // Block i alone.
+                    const int listed = __shfl_sync(FULL, w.listed, i);
+                    const long long all = __shfl_sync(FULL, w.steps, i);
+                    int spec = __shfl_sync(FULL, w.spec, i);
+                    const unsigned pieces = __shfl_sync(FULL, w.pieces, i);
+                    by_hand = listed <= 0;
+                    if (by_hand) break;
+                    for (int k = lane; k < listed; k += 32) list[k] = lists[(size_t)(in.first_block + j + i) * kListed + k];
+                    __syncwarp();
+                    double t = s;
+                    long long done = 0;
+                    bool sound = true;
+                    for (int k = 0; k < listed; ++k) {
+                        const Listed e = list[k];
+                        sound &= take_steps(t, wrap_add(e.steps, -done), spec);
+                        t = __dadd_rn(t, e.value);
+                        done = e.steps;
+                        spec = e.spec;
+                    }
+                    sound &= take_steps(t, wrap_add(all, -done), spec);
+                    __syncwarp();
+                    by_hand = !sound;
+                    if (by_hand) break;
+                    s = t;
+                    count(pieces);
+                    ++i;
                 }
-                const Run incl = warp_scan(mine, true);
-                Run excl;
-                excl.step[0] = __shfl_up_sync(FULL, incl.step[0], 1);
-                excl.step[1] = __shfl_up_sync(FULL, incl.step[1], 1);
-                excl.out = __shfl_up_sync(FULL, incl.out, 1);
-                if (lane == 0) excl = run_identity();
-                const bool odd = b.m & 1;
-                const long long m = wrap_add(b.m, odd ? excl.step[1] : excl.step[0]);
-                const long long after = wrap_add(b.m, odd ? incl.step[1] : incl.step[0]);
-                if (ok && !zero) {
-                    const int p = (int)(m & 1);
-                    ok = (p ? w.lo[1] > w.hi[1] : w.lo[0] > w.hi[0]) ||
-                         (inside(wrap_add(m, p ? w.lo[1] : w.lo[0])) && inside(wrap_add(m, p ? w.hi[1] : w.hi[0])));
-                }
-                const unsigned bad = __ballot_sync(FULL, !ok);
-                const int taken = bad ? __ffs(bad) - 1 : 32;
-                if (taken > 0 && b.normal) s = sum_of(b, __shfl_sync(FULL, after, taken - 1));
-                whole += taken;
-                j += taken;
-                if (bad) break;
+                j += i;
             }
             if (lane == 0) {
                 sh.s = s;
@@ -303,13 +306,8 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_chain(SumJobs<T> jobs, const 
         j = sh_block;
         if (j >= blocks) break;
         const size_t base = (size_t)j * kSSBlock;
-        cta_advance(in, base, (int)(in.n - base < (size_t)kSSBlock ? in.n - base : (size_t)kSSBlock), sh);
-        if (threadIdx.x == 0) {
-            const int a = __popc(sh.alone);
-            whole += a == 0;
-            reduced += a ? kSSPer - a : 0;
-            alone += a;
-        }
+        cta_advance(in, base, (int)(in.n - base < (size_t)kSSBlock ? in.n - base : (size_t)kSSBlock), sh, true);
+        if (threadIdx.x == 0) count(sh.alone);
         __syncthreads();
     }
     if (threadIdx.x == 0) finish_sum(in, sh.s, whole, reduced, alone);
@@ -331,12 +329,13 @@ cg_status seq_sums_run(cg_ctx* ctx, SumJobs<T>& jobs, int count) {
         CG_CHECK_LAUNCH(ctx);
         return CG_OK;
     }
-    CG_BUF(double, d_est, ctx, S_SS_EST, (size_t)total);
-    CG_BUF(Walk, d_walks, ctx, S_SS_WALK, (size_t)total);
+    CG_BUF(Estimate, d_est, ctx, S_SS_EST, (size_t)total);
+    CG_BUF(BlockSteps, d_heads, ctx, S_SS_WALK, (size_t)total);
+    CG_BUF(Listed, d_lists, ctx, S_SS_SPEC, (size_t)total * kListed);
     const dim3 grid(most, count);
     CG_LAUNCH(ctx) k_ss_estimate<T><<<grid, kSSThreads, 0, sm>>>(jobs, d_est);
-    CG_LAUNCH(ctx) k_ss_walks<T><<<grid, kSSThreads, 0, sm>>>(jobs, d_est, d_walks);
-    CG_LAUNCH(ctx) k_ss_chain<T><<<count, kSSThreads, 0, sm>>>(jobs, d_walks);
+    CG_LAUNCH(ctx) k_ss_walks<T><<<grid, kSSThreads, 0, sm>>>(jobs, d_est, d_heads, d_lists);
+    CG_LAUNCH(ctx) k_ss_chain<T><<<count, kSSThreads, 0, sm>>>(jobs, d_heads, d_lists);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }

@@ -14,6 +14,7 @@ namespace seqwalk {
 constexpr int kSSThreads = 1024;
 constexpr int kSSPer = 8;                        // values per thread in the parallel reduction
 constexpr int kSSBlock = kSSThreads * kSSPer;    // values per block
+constexpr int kMostAlone = 512;                  // values of a block cta_segments takes alone, at most
 constexpr long long kM0 = 1LL << 52, kM1 = 1LL << 53;
 
 // The values summed: float fields (widened exactly), or double terms already in summation order.
@@ -44,6 +45,54 @@ __device__ __forceinline__ bool value_at(const SumIn<double>& in, size_t i, doub
     if (i >= in.n) return false;
     *v = in.x[i];
     return ((unsigned long long)__double_as_longlong(*v) << 1) != 0;
+}
+
+// A thread's kSSPer consecutive values of the block at `base`: the bits of those that add something. Whole
+// runs of 16-byte aligned values by 16-byte loads: a load a value left 32 bytes between the lanes'.
+__device__ __forceinline__ void load_run(const float* x, float (&v)[kSSPer]) {
+    const float4 a = reinterpret_cast<const float4*>(x)[0], b = reinterpret_cast<const float4*>(x)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+__device__ __forceinline__ void load_run(const double* x, double (&v)[kSSPer]) {
+#pragma unroll
+    for (int t = 0; t < kSSPer / 2; ++t) {
+        const double2 a = reinterpret_cast<const double2*>(x)[t];
+        v[2 * t] = a.x, v[2 * t + 1] = a.y;
+    }
+}
+__device__ __forceinline__ bool adds(const SumIn<float>& in, float& v) {
+    if (in.mode == 1) v = __fsub_rn(1.0f, __fmul_rn(0.5f, v));
+    return (__float_as_uint(v) << 1) != 0;
+}
+__device__ __forceinline__ bool adds(const SumIn<double>&, double& v) {
+    return ((unsigned long long)__double_as_longlong(v) << 1) != 0;
+}
+template <typename T>
+__device__ __forceinline__ unsigned load_values(const SumIn<T>& in, size_t base, T (&v)[kSSPer]) {
+    unsigned has = 0;
+    const size_t i0 = base + (size_t)threadIdx.x * kSSPer;
+    if (i0 + kSSPer <= in.n && ((uintptr_t)in.x & 15) == 0 && ((uintptr_t)in.mask & 7) == 0) {
+        load_run(in.x + i0, v);
+        uint2 m = make_uint2(0x01010101u, 0x01010101u);
+        if (in.mask) m = *reinterpret_cast<const uint2*>(in.mask + i0);
+#pragma unroll
+        for (int t = 0; t < kSSPer; ++t)
+            if ((((t < 4 ? m.x : m.y) >> (8 * (t & 3))) & 0xFFu) && adds(in, v[t])) has |= 1u << t;
+        return has;
+    }
+#pragma unroll
+    for (int t = 0; t < kSSPer; ++t) {
+        v[t] = 0;
+        if (value_at(in, i0 + t, &v[t])) has |= 1u << t;
+    }
+    return has;
+}
+// The bits of a thread's values with indices in [pos, end) of the block.
+__device__ __forceinline__ unsigned within(int pos, int end) {
+    const int lo = pos - (int)threadIdx.x * kSSPer, hi = end - (int)threadIdx.x * kSSPer;
+    const unsigned below_hi = hi >= kSSPer ? 0xFFu : (hi <= 0 ? 0u : (1u << hi) - 1u);
+    const unsigned below_lo = lo >= kSSPer ? 0xFFu : (lo <= 0 ? 0u : (1u << lo) - 1u);
+    return below_hi & ~below_lo;
 }
 
 // One value's step in the binade with exponent field ef (u = 2^(ef - 1075)), for a sum of sign `neg`:
@@ -178,6 +227,13 @@ struct CtaSum {
     int hit;         // STOP: that value's index (set to -1 by the caller; -1: none has)
     int pos;         // values of the block taken
     unsigned alone;  // the block's pieces of 1024 holding an addition taken alone
+    // cta_segments: the values taken alone in order, the steps of all others before each, and the binade
+    // (exponent | sign << 11, -1: no value) of the others between it and the one before.
+    long long steps[kMostAlone + 1];
+    double values[kMostAlone];
+    int at[kMostAlone], spec[kMostAlone + 1];
+    long long totals[kSSThreads / 32];
+    int counts[kSSThreads / 32];
 };
 
 // Whether a nonzero value added to a sum that is no normal number may change it: NaN stays, and infinity
@@ -261,11 +317,16 @@ __device__ __forceinline__ int cta_scan(const SumIn<T>& in, size_t base, int fir
     if (b.normal) {
         long long r[PER], sum = 0, reach = PER;   // reach: how far the thread's partial sums can go, ties' units included
         unsigned has = 0, tie = 0, off = 0;
+        // Floats as a run (`first` is the block's start); doubles one by one, a run of them takes registers
+        // the scan has not got (35 us a book's seven blocks against 46).
+        constexpr bool kRun = PER == kSSPer && sizeof(T) == 4;
+        T x[kRun ? kSSPer : 1];
+        if constexpr (kRun) has = load_values(in, base, x) & within(pos, end);
 #pragma unroll
         for (int t = 0; t < PER; ++t) {
-            T v;
             r[t] = 0;
-            if (at0 + t >= pos && at0 + t < end && value_at(in, base + at0 + t, &v)) {
+            T& v = x[kRun ? t : 0];
+            if (kRun ? (has >> t) & 1u : at0 + t >= pos && at0 + t < end && value_at(in, base + at0 + t, &v)) {
                 const Step st = step_of(v, b.ef, b.neg);
                 has |= 1u << t;
                 if (plain_step(st)) {
@@ -341,16 +402,265 @@ __device__ __forceinline__ int cta_scan(const SumIn<T>& in, size_t base, int fir
     return at;
 }
 
+// A magnitude and its exponent: |v| = M 2^e, M < 2^53 (2^24 for floats).
+struct Magnitude {
+    unsigned long long M;
+    int e;
+    bool neg, finite;
+};
+__device__ __forceinline__ Magnitude magnitude_of(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int fe = (int)((b >> 52) & 0x7FF);
+    return Magnitude{(b & (kM0 - 1)) | (fe != 0 ? (unsigned long long)kM0 : 0ull), (fe == 0 ? 1 : fe) - 1075, (b >> 63) != 0,
+                     fe != 0x7FF};
+}
+__device__ __forceinline__ Magnitude magnitude_of(float v) {
+    const uint32_t b = __float_as_uint(v);
+    const int fe = (int)((b >> 23) & 0xFF);
+    return Magnitude{(b & 0x7FFFFFu) | (fe != 0 ? 1u << 23 : 0u), (fe == 0 ? 1 : fe) - 150, (b >> 31) != 0, fe != 0xFF};
+}
+// The exponent field's width, and a value's (nonzero values; 0: subnormal).
+template <typename T>
+constexpr int kTopField = sizeof(T) == 8 ? 0x7FF : 0xFF;
+__device__ __forceinline__ int field_of(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
+__device__ __forceinline__ int field_of(float v) { return (int)((__float_as_uint(v) >> 23) & 0xFF); }
+// The binary exponent of a nonzero magnitude: 2^x <= |v| < 2^(x + 1).
+__device__ __forceinline__ int exponent_of(const Magnitude& a) { return a.e + 63 - __clzll((long long)a.M); }
+// v in units of 2^unit, toward zero: off by less than a unit. |v| < 2^(unit + 61).
+__device__ __forceinline__ long long units_of(const Magnitude& a, int unit) {
+    const int up = a.e - unit;
+    const unsigned long long q = up >= 0 ? a.M << up : (up > -64 ? a.M >> -up : 0ull);
+    return a.neg ? -(long long)q : (long long)q;
+}
+
+// An int64 scan over the CTA: *before receives the values before this thread's, the result is
+// the total. `totals` is free again after the next barrier.
+__device__ __forceinline__ long long cta_before(long long v, long long* before, long long* totals) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x = wrap_add(x, y);
+    }
+    if (lane == 31) totals[warp] = x;
+    __syncthreads();
+    long long w = totals[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+        if (lane >= o) w = wrap_add(w, y);
+    }
+    const long long start = __shfl_sync(0xFFFFFFFFu, w, warp > 0 ? warp - 1 : 0);
+    *before = wrap_add(warp > 0 ? start : 0, wrap_add(x, -v));
+    return __shfl_sync(0xFFFFFFFFu, w, 31);
+}
+
+// The block's values [pos, len) after a sum of about `start`, crossings and all, told apart: the values to be
+// taken alone are listed in sh (steps, values, at, spec), and the steps of all others summed. The partial
+// sums are first taken in fixed point, in units of 2^-60 of what they can reach, by one integer scan: they
+// are off from the rounded sums by less than 2^20 units (a unit a value, and the rounded sums' own
+// roundings, 2^6 units each) and what `start` is off (`start_off`), which tells each partial sum's binade
+// but next to a power of two. A value whose sums before and after are surely in one binade is a step of that
+// binade, whatever the parity unless it is a tie; every other value is listed. The steps between two listed
+// values are a difference of a second scan. Returns how many values are listed, or -1 where that does not
+// apply: a sum or value that is not finite, or too many values; *all_steps receives the steps of the rest.
+// Every thread calls it, and what it wrote to sh is visible after it.
+template <bool STOP, typename T>
+__device__ int cta_classify(const SumIn<T>& in, size_t base, int pos, int len, double start, double start_off, CtaSum& sh,
+                            double stop, long long* all_steps) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int at0 = (int)threadIdx.x * kSSPer;
+    const Magnitude ms = magnitude_of(start), mo = magnitude_of(start_off);
+    T v[kSSPer];
+    const unsigned has = load_values(in, base, v) & within(pos, len);
+    // The largest exponent field, and so whether every value is finite.
+    int top = -1;
+#pragma unroll
+    for (int t = 0; t < kSSPer; ++t)
+        if ((has >> t) & 1u) top = max(top, field_of(v[t]));
+    top = __reduce_max_sync(FULL, top);
+    if (lane == 0) sh.counts[warp] = top;
+    for (int k = threadIdx.x; k <= kMostAlone; k += kSSThreads) sh.spec[k] = -1;
+    __syncthreads();
+    top = __reduce_max_sync(FULL, sh.counts[lane]);
+    *all_steps = 0;
+    if (!ms.finite || !mo.finite || top == kTopField<T>) return -1;
+    if (top < 0) return 0;   // nothing to add
+    // |every partial sum| < 2^(reach + 1): the sum before and 2^13 values.
+    const int most = max(top, 1) - kTopField<T> / 2;   // the largest value's binary exponent
+    const int reach = max(max(ms.M ? exponent_of(ms) : INT_MIN, mo.M ? exponent_of(mo) : INT_MIN) + 1, most + 13) + 1;
+    const int unit = reach - 59;
+    const long long off = (1ll << 20) + units_of(mo, unit) + 1;   // < 2^59
+    long long stop_units = 0;
+    if (STOP) {
+        const Magnitude a = magnitude_of(stop);
+        stop_units = a.M && exponent_of(a) > reach ? LLONG_MAX / 2 : units_of(a, unit);
+    }
+    long long sum = 0, span = 0, before;   // span: how far this thread's values can go
+#pragma unroll
+    for (int t = 0; t < kSSPer; ++t) {
+        const long long q = (has >> t) & 1u ? units_of(magnitude_of(v[t]), unit) : 0;
+        sum += q;
+        span += q < 0 ? -q : q;
+    }
+    cta_before(sum, &before, sh.totals);
+    const long long p0 = units_of(ms, unit) + before;
+    // The surely known binade of a partial sum: exponent field | sign << 11, or -1.
+    auto binade_at = [=](long long p) {
+        const long long a = p < 0 ? -p : p;
+        const int bit = 63 - __clzll(a);
+        if (a <= 4 * off || a - (1ll << bit) <= off || (2ll << bit) - a <= off) return -1;
+        const int ef = bit + unit + 1023;
+        return ef >= 1 && ef <= 2046 ? ef | (p < 0 ? 1 << 11 : 0) : -1;
+    };
+    auto near_stop = [=](long long was, long long p) { return STOP && p >= stop_units - 2 * off && was <= stop_units + 2 * off; };
+    long long steps = 0;
+    unsigned single = 0;
+    int spec[2] = {-1, -1};   // the binades of this thread's first steps, and of those after its last listed value
+    const int first = binade_at(p0);
+    if (first >= 0 && binade_at(p0 - span) == first && binade_at(p0 + span) == first && !near_stop(p0 - span, p0 + span)) {
+        // All of the thread's sums are surely in one binade (nearly every thread's are).
+#pragma unroll
+        for (int t = 0; t < kSSPer; ++t) {
+            if (!((has >> t) & 1u)) continue;
+            const Step st = step_of(v[t], first & 0x7FF, first >> 11);
+            if (st.tie || !plain_step(st)) single |= 1u << t;
+            else steps = wrap_add(steps, st.r);
+        }
+        if (has & ~single) spec[0] = first;
+        if (single) spec[1] = spec[0];
+    } else if (has) {
+        long long p = p0;
+        int code = first;
+#pragma unroll
+        for (int t = 0; t < kSSPer; ++t) {
+            if (!((has >> t) & 1u)) continue;
+            const long long was = p;
+            p += units_of(magnitude_of(v[t]), unit);
+            const int next = binade_at(p);
+            bool alone = code < 0 || next != code || near_stop(was, p);
+            if (!alone) {
+                const Step st = step_of(v[t], code & 0x7FF, code >> 11);
+                alone = st.tie || !plain_step(st);
+                if (!alone) {
+                    steps = wrap_add(steps, st.r);
+                    spec[single ? 1 : 0] = code;
+                }
+            }
+            if (alone) {
+                single |= 1u << t;
+                spec[1] = -1;
+            }
+            code = next;
+        }
+    }
+    __syncthreads();   // sh.totals and sh.counts are read
+    long long steps_before;
+    *all_steps = cta_before(steps, &steps_before, sh.totals);
+    int mine = __popc(single), slot = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, slot, o);
+        if (lane >= o) slot += y;
+    }
+    if (lane == 31) sh.counts[warp] = slot;
+    __syncthreads();
+    const int c = sh.counts[lane], listed = __reduce_add_sync(FULL, c);
+    slot += __reduce_add_sync(FULL, lane < warp ? c : 0) - mine;
+    if (listed > kMostAlone) return -1;
+    if (spec[0] >= 0) sh.spec[slot] = spec[0];
+    if (spec[1] >= 0) sh.spec[slot + mine] = spec[1];
+    if (single) {   // the thread's values again, for the steps between its listed ones
+        long long p = p0;
+        int code = first;
+#pragma unroll
+        for (int t = 0; t < kSSPer; ++t) {
+            if (!((has >> t) & 1u)) continue;
+            p += units_of(magnitude_of(v[t]), unit);
+            if ((single >> t) & 1u) {
+                sh.steps[slot] = steps_before;
+                sh.values[slot] = (double)v[t];
+                sh.at[slot] = at0 + t;
+                ++slot;
+            } else {
+                steps_before = wrap_add(steps_before, step_of(v[t], code & 0x7FF, code >> 11).r);
+            }
+            code = binade_at(p);
+        }
+    }
+    __syncthreads();
+    return listed;
+}
+
+// The block's values [pos, len) added to sh.s at once: told apart, then chained by one thread, one addition
+// in hardware and a few instructions a listed value, about 0.15 us, where a CTA scan for each crossing took
+// 3 to 5. The chain checks that a run of steps ends inside a binade, and that it is the one they were taken
+// for (but for runs within one thread). Returns false, with sh.s as it was, where that does not apply. sh.s
+// is set and visible before the call and after it.
+template <bool STOP, typename T>
+__device__ bool cta_segments(const SumIn<T>& in, size_t base, int pos, int len, CtaSum& sh, double stop) {
+    const double s0 = sh.s;
+    long long all_steps;
+    const int listed = cta_classify<STOP>(in, base, pos, len, s0, 0.0, sh, stop, &all_steps);
+    if (listed < 0) return false;
+    if (threadIdx.x == 0) {
+        double s = s0;
+        long long done = 0;
+        unsigned alone = 0;
+        bool sound = true;
+        int hit = -1;
+        double from = 0.0;
+        for (int k = 0; k <= listed; ++k) {
+            const long long run = wrap_add(k < listed ? sh.steps[k] : all_steps, -done);
+            if (run != 0) {
+                const Binade b = binade_of(s);
+                const long long m = b.m + run;
+                const int spec_k = sh.spec[k];
+                sound &= b.normal && inside(m) && (spec_k == -1 || spec_k == (b.ef | (b.neg << 11)));
+                s = sum_of(b, m);
+                done = wrap_add(done, run);
+            }
+            if (k == listed) break;
+            from = s;
+            s = __dadd_rn(s, sh.values[k]);
+            alone |= 1u << (sh.at[k] / kSSThreads);
+            if (STOP && reached(s, stop)) {
+                hit = sh.at[k];
+                break;
+            }
+        }
+        sh.pos = sound;
+        if (sound) {
+            sh.s = s;
+            sh.alone |= alone;
+            if (STOP && hit >= 0) {
+                sh.hit = hit;
+                sh.below = from;
+            }
+        }
+    }
+    __syncthreads();
+    return sh.pos != 0;
+}
+
 // The block's `len` values added to sh.s in order, by the whole CTA: a scan of 8 values a thread; from
-// a value taken alone on, one warp's windows and then scans of a value a thread, until 1024 values hold
-// none. sh.s is set and visible before the call and after it. STOP: as in warp_windows, through sh.hit
-// and sh.below.
+// a value taken alone on, all the rest at once by their predicted binades, or, where that does not apply,
+// one warp's windows and then scans of a value a thread, until 1024 values hold none. sh.s is set and
+// visible before the call and after it. STOP: as in warp_windows, through sh.hit and sh.below.
+// `crosses`: the caller knows that a scan would not take the block.
 template <bool STOP = false, typename T>
-__device__ void cta_advance(const SumIn<T>& in, size_t base, int len, CtaSum& sh, double stop = 0.0) {
+__device__ void cta_advance(const SumIn<T>& in, size_t base, int len, CtaSum& sh, bool crosses = false, double stop = 0.0) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int pos = 0;
-    bool wide = true;
+    bool wide = true, predict = true;
     if (threadIdx.x == 0) sh.alone = 0;
+    if (crosses) {
+        predict = false;
+        if (cta_segments<STOP>(in, base, 0, len, sh, stop)) return;
+        __syncthreads();   // sh.pos is read
+    }
     while (pos < len) {
         const double s = sh.s;
         const int end = wide ? len : min(len, pos + kSSThreads);
@@ -375,6 +685,11 @@ __device__ void cta_advance(const SumIn<T>& in, size_t base, int len, CtaSum& sh
             }
             __syncthreads();
             if (STOP && sh.hit >= 0) return;
+            if (wide && predict) {
+                predict = false;   // once a block: what it cannot take, it could not later
+                if (cta_segments<STOP>(in, base, at + 1, len, sh, stop)) return;
+                __syncthreads();   // sh.pos is read
+            }
             if (warp == 0) {
                 double t = sh.s;
                 int p = at + 1;
@@ -399,19 +714,6 @@ __device__ void cta_advance(const SumIn<T>& in, size_t base, int len, CtaSum& sh
         }
         __syncthreads();   // sh.s and sh.pos are read before the next scan writes them
     }
-}
-
-// A thread's kSSPer consecutive values of the block at `base`: the bits of those that add something.
-template <typename T>
-__device__ __forceinline__ unsigned load_values(const SumIn<T>& in, size_t base, T (&v)[kSSPer]) {
-    unsigned has = 0;
-    const size_t i0 = base + (size_t)threadIdx.x * kSSPer;
-#pragma unroll
-    for (int t = 0; t < kSSPer; ++t) {
-        v[t] = 0;
-        if (value_at(in, i0 + t, &v[t])) has |= 1u << t;
-    }
-    return has;
 }
 
 }  // namespace seqwalk
