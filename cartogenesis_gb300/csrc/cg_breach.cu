@@ -531,8 +531,7 @@ cg_status breach_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, float* d_
     ctx->launches++;
     CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_breach_waves, cgrid, 256, kargs, 0, sm));
     int q[Q_WORDS];
-    CG_CUDA(ctx, cudaMemcpyAsync(q, a.q, sizeof(q), cudaMemcpyDeviceToHost, sm));
-    CG_CUDA(ctx, cudaStreamSynchronize(sm));
+    CG_TRY_ST(read_back(ctx, {{q, a.q, sizeof(q)}}));
     if (q[Q_ERROR]) return fail(ctx, CG_CUDA, "outlet notch: waves did not converge over %d basins", count);
     if (h_cells) *h_cells = q[Q_CELLS];
     return CG_OK;

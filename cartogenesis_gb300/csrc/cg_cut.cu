@@ -94,25 +94,34 @@ __global__ void __launch_bounds__(256) k_minmax(const float* __restrict__ h, siz
     }
 }
 
-__global__ void k_cut_prepare(CutState* s, double target) {
-    float lo = from_ordered_key(s->lo_key), hi = from_ordered_key(s->hi_key);
-    s->lowest = lo;
-    s->highest = hi;
-    if (__fsub_rn(hi, lo) <= 0.0f || target <= 0.0) {
-        s->degenerate = 1;
-        s->todays = lo;
-        s->per = 0.0f;
-    } else {
-        s->per = __fdiv_rn((float)(BINS - 1), __fsub_rn(hi, lo));
-    }
+// The range and the bins' scale (SeaLevelStage.kt:590-600), from the extremes; degenerate: the answer is the lowest.
+struct CutRange {
+    float lowest, highest, per;
+    int degenerate;
+};
+__device__ __forceinline__ CutRange cut_range(const CutState* s, double target) {
+    CutRange r;
+    r.lowest = from_ordered_key(s->lo_key);
+    r.highest = from_ordered_key(s->hi_key);
+    r.degenerate = __fsub_rn(r.highest, r.lowest) <= 0.0f || target <= 0.0;
+    r.per = r.degenerate ? 0.0f : __fdiv_rn((float)(BINS - 1), __fsub_rn(r.highest, r.lowest));
+    return r;
 }
 
 // One CTA per row: exact cell counts of every bin in that row.
-__global__ void __launch_bounds__(512) k_row_counts(const float* __restrict__ h, int W, const CutState* s,
+__global__ void __launch_bounds__(512) k_row_counts(const float* __restrict__ h, int W, double target, CutState* s,
                                                     unsigned* __restrict__ counts) {
     __shared__ unsigned sh[BINS];
-    if (s->degenerate) return;
-    const float lo = s->lowest, per = s->per;
+    const CutRange r = cut_range(s, target);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // kept for the kernels after this one
+        s->lowest = r.lowest;
+        s->highest = r.highest;
+        s->per = r.per;
+        s->degenerate = r.degenerate;
+        if (r.degenerate) s->todays = r.lowest;
+    }
+    if (r.degenerate) return;
+    const float lo = r.lowest, per = r.per;
     for (int b = threadIdx.x; b < BINS; b += blockDim.x) sh[b] = 0u;
     __syncthreads();
     const float* rowp = h + (size_t)blockIdx.x * W;
@@ -215,7 +224,10 @@ __global__ void k_bracket_collect(const float* __restrict__ h, size_t N, CutStat
 // take 80 us at 2048 keys, up to 16384 keys; past that the network over chunks below is the faster.
 constexpr int SMALL_SORT = 16384;
 constexpr int RANK_KEYS = 4;
-__global__ void __launch_bounds__(256) k_sort_rank(const long long* __restrict__ keys, int n, long long* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_sort_rank(const long long* __restrict__ keys, const CutState* s,
+                                                   long long* __restrict__ out) {
+    const int n = s->count;
+    if (s->degenerate || n > SMALL_SORT) return;
     const int lane = threadIdx.x & 31;
     const int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * RANK_KEYS;
     if (k0 >= n) return;
@@ -333,7 +345,7 @@ __device__ bool walk_replay(const long long* __restrict__ keys, const double* __
 __global__ void __launch_bounds__(WALK_THREADS) k_bracket_walk(const float* __restrict__ h,
                                                                const long long* __restrict__ keys,
                                                                const double* __restrict__ w, int W, double target,
-                                                               CutState* s) {
+                                                               int most, CutState* s) {
     const int64_t TOP = (int64_t)1 << 53;
     __shared__ long long s_warp[WALK_THREADS / 32];
     __shared__ int s_hit, s_unclean, s_done;
@@ -341,6 +353,7 @@ __global__ void __launch_bounds__(WALK_THREADS) k_bracket_walk(const float* __re
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (s->degenerate) return;
     const int n = s->count;
+    if (n > most) return;   // its keys are not sorted yet
     if (n == 0) {
         if (tid == 0) s->todays = s->highest;
         return;
@@ -459,9 +472,10 @@ __global__ void __launch_bounds__(WALK_THREADS) k_bracket_walk(const float* __re
 }
 
 // SeaLevelStage.landAndWaterAt (SeaLevelStage.kt:175-200).
-__global__ void k_land_and_water(const float* __restrict__ h, size_t N, CutState* s, float lowstand,
+__global__ void k_land_and_water(const float* __restrict__ h, size_t N, int most, CutState* s, float lowstand,
                                  float land_half, float sea_half, uint8_t* __restrict__ land,
                                  float* __restrict__ rel) {
+    if (!s->degenerate && s->count > most) return;   // the shoreline is not known yet
     const float shore = __fsub_rn(s->todays, lowstand);
     int count = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
@@ -520,42 +534,41 @@ cg_status percentile_cut_dev(cg_ctx* ctx, int W, int H, const float* d_h, float 
     int grid = ctx->num_sms * 8;
     CG_LAUNCH(ctx) k_cut_init<<<1, 1, 0, sm>>>(d_s);
     CG_LAUNCH(ctx) k_minmax<<<grid, 256, 0, sm>>>(d_h, N, d_s);
-    CG_LAUNCH(ctx) k_cut_prepare<<<1, 1, 0, sm>>>(d_s, target);
-    CG_LAUNCH(ctx) k_row_counts<<<H, 512, 0, sm>>>(d_h, W, d_s, d_counts);
+    CG_LAUNCH(ctx) k_row_counts<<<H, 512, 0, sm>>>(d_h, W, target, d_s, d_counts);
     CG_LAUNCH(ctx) k_bin_sums<<<BINS * 32 / 256, 256, 0, sm>>>(d_counts, d_w, H, d_s, d_hist);
     CG_LAUNCH(ctx) k_bracket_bin<<<1, seqwalk::kSSThreads, 0, sm>>>(d_hist, target, d_s);
     CG_LAUNCH(ctx) k_bracket_collect<<<grid, 256, 0, sm>>>(d_h, N, d_s, d_keys);
     CG_CHECK_LAUNCH(ctx);
-    CutState hs;
-    CG_CUDA(ctx, cudaMemcpyAsync(&hs, d_s, sizeof(hs), cudaMemcpyDeviceToHost, sm));
-    CG_CUDA(ctx, cudaStreamSynchronize(sm));
-    if (!hs.degenerate && hs.count > 1) {
-        if (hs.count <= SMALL_SORT) {
-            CG_BUF(long long, d_sorted, ctx, S_BRACKET2, SMALL_SORT);
-            const int warps = (hs.count + RANK_KEYS - 1) / RANK_KEYS;
-            CG_LAUNCH(ctx) k_sort_rank<<<(warps + 7) / 8, 256, 0, sm>>>(d_keys, hs.count, d_sorted);
-            d_keys = d_sorted;
-        } else {
-            int P2 = 1;
-            while (P2 < hs.count) P2 <<= 1;
-            int blocks = (P2 / 2 + 255) / 256;
-            if (blocks > grid) blocks = grid;
-            CG_LAUNCH(ctx) k_pad<<<blocks, 256, 0, sm>>>(d_keys, hs.count, P2);
-            // P2 > SMALL_SORT >= SORT_CH: whole chunks of SORT_CH keys.
-            CG_LAUNCH(ctx) k_sort_chunk<<<P2 / SORT_CH, 1024, 0, sm>>>(d_keys, 0);
-            for (int k = 2 * SORT_CH; k <= P2; k <<= 1) {
-                for (int j = k >> 1; j >= SORT_CH; j >>= 1)
-                    CG_LAUNCH(ctx) k_sort_stage<<<blocks, 256, 0, sm>>>(d_keys, P2, k, j);
-                CG_LAUNCH(ctx) k_sort_chunk<<<P2 / SORT_CH, 1024, 0, sm>>>(d_keys, k);
-            }
-        }
-        CG_CHECK_LAUNCH(ctx);
-    }
-    CG_LAUNCH(ctx) k_bracket_walk<<<1, WALK_THREADS, 0, sm>>>(d_h, d_keys, d_w, W, target, d_s);
-    CG_LAUNCH(ctx) k_land_and_water<<<grid, 256, 0, sm>>>(d_h, N, d_s, lowstand_share, land_half, sea_half, d_land, d_rel);
+    // A bracket of up to SMALL_SORT cells, as nearly every one is, is sorted and walked before the host has
+    // read its size; a larger one is left as it is by those launches, and sorted and walked after.
+    CG_BUF(long long, d_sorted, ctx, S_BRACKET2, SMALL_SORT);
+    CG_LAUNCH(ctx) k_sort_rank<<<SMALL_SORT / RANK_KEYS / 8, 256, 0, sm>>>(d_keys, d_s, d_sorted);
+    auto walk = [&](const long long* keys, int most) {
+        CG_LAUNCH(ctx) k_bracket_walk<<<1, WALK_THREADS, 0, sm>>>(d_h, keys, d_w, W, target, most, d_s);
+        CG_LAUNCH(ctx) k_land_and_water<<<grid, 256, 0, sm>>>(d_h, N, most, d_s, lowstand_share, land_half, sea_half,
+                                                              d_land, d_rel);
+    };
+    walk(d_sorted, SMALL_SORT);
     CG_CHECK_LAUNCH(ctx);
-    CG_CUDA(ctx, cudaMemcpyAsync(&hs, d_s, sizeof(hs), cudaMemcpyDeviceToHost, sm));
-    CG_CUDA(ctx, cudaStreamSynchronize(sm));
+    CutState hs;
+    CG_TRY_ST(read_back(ctx, {{&hs, d_s, sizeof(hs)}}));
+    if (!hs.degenerate && hs.count > SMALL_SORT) {
+        int P2 = 1;
+        while (P2 < hs.count) P2 <<= 1;
+        int blocks = (P2 / 2 + 255) / 256;
+        if (blocks > grid) blocks = grid;
+        CG_LAUNCH(ctx) k_pad<<<blocks, 256, 0, sm>>>(d_keys, hs.count, P2);
+        // P2 > SMALL_SORT >= SORT_CH: whole chunks of SORT_CH keys.
+        CG_LAUNCH(ctx) k_sort_chunk<<<P2 / SORT_CH, 1024, 0, sm>>>(d_keys, 0);
+        for (int k = 2 * SORT_CH; k <= P2; k <<= 1) {
+            for (int j = k >> 1; j >= SORT_CH; j >>= 1)
+                CG_LAUNCH(ctx) k_sort_stage<<<blocks, 256, 0, sm>>>(d_keys, P2, k, j);
+            CG_LAUNCH(ctx) k_sort_chunk<<<P2 / SORT_CH, 1024, 0, sm>>>(d_keys, k);
+        }
+        walk(d_keys, INT_MAX);
+        CG_CHECK_LAUNCH(ctx);
+        CG_TRY_ST(read_back(ctx, {{&hs, d_s, sizeof(hs)}}));
+    }
     *h_shoreline = hs.todays - lowstand_share;
     *h_land_cells = hs.land_cells;
     return CG_OK;

@@ -32,6 +32,7 @@
 
 #include "cg_common.cuh"
 #include "cg_internal.h"
+#include "cg_util.h"
 
 namespace cg {
 
@@ -59,6 +60,7 @@ struct FillCounters {
     int min_level;      // the lowest key level holding a tie only its own pops can order
     int overflow;       // that level was too large to replay
     int repair_level;   // the lowest key level at which a pin changed a cell's level
+    int timed_out;      // the relaxation did not settle
 };
 
 // (0) classes and initial levels.
@@ -283,8 +285,14 @@ __global__ void __launch_bounds__(256, 4) k_relax_passes(RelaxArgs a) {
 // A tile is on the first pass's list if it holds a cell still to settle (a level reset to +inf).
 __global__ void k_tiles_with_open(const uint8_t* __restrict__ cls, const float* __restrict__ f, int W, int H,
                                   int tiles_x, int* __restrict__ mark, int* __restrict__ list,
-                                  int* __restrict__ count) {
+                                  int* __restrict__ count, FillCounters* cnt) {
     int tile = blockIdx.x;
+    if (tile == 0 && threadIdx.x == 0) {   // the pass's counters start over
+        FillCounters zero{};
+        zero.min_level = INT_MAX;
+        zero.repair_level = INT_MAX;
+        *cnt = zero;
+    }
     const int ty0 = (tile / tiles_x) * T, tx0 = (tile % tiles_x) * T;
     int has = 0;
     for (int i = threadIdx.x; i < T * T; i += blockDim.x) {
@@ -538,9 +546,10 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     CG_BUF(int, d_ptr, ctx, S_PTR, N);
     CG_BUF(int, d_pin, ctx, S_FILLQ, N);
     int tiles_x = (W + T - 1) / T, tiles_y = (H + T - 1) / T, tiles = tiles_x * tiles_y;
-    // Two tile lists and their marks, three list counts, the timeout flag (zeroed before each relaxation).
-    CG_BUF(int, d_marks, ctx, S_TILEFLAG, 2 * (size_t)tiles);
-    CG_BUF(int, d_lists, ctx, S_FILLLIST, 2 * (size_t)tiles + 4);
+    // Three list counts and the two tile lists' marks (zeroed before each relaxation), and the lists.
+    CG_BUF(int, d_marks, ctx, S_TILEFLAG, 2 * (size_t)tiles + 4);
+    CG_BUF(int, d_lists, ctx, S_FILLLIST, 2 * (size_t)tiles);
+    CG_BUF(FillCounters, d_cnt, ctx, S_FILLF, 1);
     RelaxArgs ra;
     ra.f = d_filled;
     ra.g = d_rel;
@@ -552,16 +561,15 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     ra.tiles_y = tiles_y;
     ra.list[0] = d_lists;
     ra.list[1] = d_lists + tiles;
-    ra.count = d_lists + 2 * (size_t)tiles;
-    ra.timed_out = ra.count + 3;
-    ra.mark[0] = d_marks;
-    ra.mark[1] = d_marks + tiles;
+    ra.count = d_marks;
+    ra.timed_out = &d_cnt->timed_out;
+    ra.mark[0] = d_marks + 4;
+    ra.mark[1] = ra.mark[0] + tiles;
     ra.max_passes = 4 * (tiles_x + tiles_y) + 64;
     int per_sm = 0;
     CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_relax_passes, 256, 0));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "k_relax_passes cannot be resident");
     const int relax_grid = ctx->num_sms * std::min(per_sm, 8);
-    CG_BUF(FillCounters, d_cnt, ctx, S_FILLF, 1);
     int grid = ctx->num_sms * 8;
     CG_LAUNCH(ctx) k_fill_init<<<grid, 256, 0, sm>>>(d_land, d_rel, W, H, d_cls, d_filled, d_ptr);
     CG_LAUNCH(ctx) k_drain_chains<<<grid, 256, 0, sm>>>(d_ptr, d_rel, N, d_cls, d_filled);
@@ -576,7 +584,6 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     int* d_list = d_replay;
     long long* d_heap = (long long*)(d_replay + cap + (cap & 1));   // 8-byte aligned
     int* d_list_n = d_replay + 3 * (size_t)cap + 2;
-    CG_CUDA(ctx, cudaMemsetAsync(d_mark, 0, N * sizeof(int), sm));
     int gen = 0;
 
     FillCounters hc;
@@ -585,15 +592,10 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     // Each pass either settles, pins tie parents by the index rule, or replays the lowest level
     // holding a tie the index rule cannot order; the cap is a guard, not the expected exit.
     const int max_repairs = 256;
-    FillCounters zero{};
-    zero.min_level = INT_MAX;
-    zero.repair_level = INT_MAX;
     for (int repair = 0; repair <= max_repairs; ++repair) {
-        CG_CUDA(ctx, cudaMemcpyAsync(d_cnt, &zero, sizeof(zero), cudaMemcpyHostToDevice, sm));
-        CG_CUDA(ctx, cudaMemsetAsync(d_lists, 0, (2 * (size_t)tiles + 4) * sizeof(int), sm));
-        CG_CUDA(ctx, cudaMemsetAsync(d_marks, 0, 2 * (size_t)tiles * sizeof(int), sm));
+        CG_CUDA(ctx, cudaMemsetAsync(d_marks, 0, (2 * (size_t)tiles + 4) * sizeof(int), sm));
         CG_LAUNCH(ctx) k_tiles_with_open<<<tiles, 256, 0, sm>>>(d_cls, d_filled, W, H, tiles_x, ra.mark[0], ra.list[0],
-                                                                ra.count);
+                                                                ra.count, d_cnt);
         CG_CHECK_LAUNCH(ctx);
         // Relax until no tile changes, in one cooperative launch. Bounded: every pass lowers some level
         // or stops, and levels only take values from a finite set; the cap is a guard, not the exit.
@@ -603,13 +605,10 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
             CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_relax_passes, relax_grid, 256, kargs, 0, sm));
         }
         // The check runs behind the relaxation, settled or not; the host reads both together.
-        int timed_out = 0;
         CG_LAUNCH(ctx) k_check_ties<<<grid, 256, 0, sm>>>(d_filled, d_rel, d_cls, d_pin, W, H, d_cnt);
         CG_CHECK_LAUNCH(ctx);
-        CG_CUDA(ctx, cudaMemcpyAsync(&timed_out, ra.timed_out, sizeof(int), cudaMemcpyDeviceToHost, sm));
-        CG_CUDA(ctx, cudaMemcpyAsync(&hc, d_cnt, sizeof(hc), cudaMemcpyDeviceToHost, sm));
-        CG_CUDA(ctx, cudaStreamSynchronize(sm));
-        if (timed_out) return fail(ctx, CG_TIMEOUT, "fill relaxation did not settle in %d passes", ra.max_passes);
+        CG_TRY_ST(read_back(ctx, {{&hc, d_cnt, sizeof(hc)}}));
+        if (hc.timed_out) return fail(ctx, CG_TIMEOUT, "fill relaxation did not settle in %d passes", ra.max_passes);
         if (repair == 0) tie_total = (int64_t)hc.ties;
         unresolved_total = (int64_t)hc.unresolved;
         if (hc.repaired == 0 && hc.unresolved == 0) break;
@@ -629,6 +628,7 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
             const int Q = hc.repaired ? std::min(hc.min_level, hc.repair_level) : hc.min_level;
             const int span = replays < 8 ? 0 : std::min(1 << std::min(replays - 8, 12), kReplaySpan);
             const int Qmax = Q + span;
+            if (replays == 0) CG_CUDA(ctx, cudaMemsetAsync(d_mark, 0, N * sizeof(int), sm));
             ++replays;
             ++gen;
             CG_CUDA(ctx, cudaMemsetAsync(d_list_n, 0, sizeof(int), sm));
@@ -638,8 +638,7 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
                                                             d_heap, cap, W, H, Q, Qmax, d_eb, d_cnt);
             CG_CHECK_LAUNCH(ctx);
             int overflow = 0;
-            CG_CUDA(ctx, cudaMemcpyAsync(&overflow, &d_cnt->overflow, sizeof(int), cudaMemcpyDeviceToHost, sm));
-            CG_CUDA(ctx, cudaStreamSynchronize(sm));
+            CG_TRY_ST(read_back(ctx, {{&overflow, &d_cnt->overflow, sizeof(int)}}));
             if (overflow) {   // cannot happen with cap = N; kept as a guard
                 unresolved_total += 1;
                 break;

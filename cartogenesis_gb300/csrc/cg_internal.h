@@ -2,6 +2,7 @@
 #pragma once
 
 #include "cg_common.cuh"
+#include "cg_util.h"
 
 namespace cg {
 
@@ -41,10 +42,12 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
 // ---- routing (cg_route.cu)
 struct FlatCounts {
     int flats, kept, raised;
+    const int* d_kept;   // `kept` on the device until the next call, for a caller that reads it later
 };
 cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const float* d_rel,
                               const float* d_filled, int64_t seed, double r, int lattice, bool by_facet,
-                              bool over_potential, int32_t* d_recv, double* d_surface, FlatCounts* counts);
+                              bool over_potential, int32_t* d_recv, double* d_surface, FlatCounts* counts,
+                              bool kept_later = false);
 
 // FlowRouting.facetReceiver at every cell of d_mask over the routing surface d_surface (-1 elsewhere).
 cg_status facet_receivers_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, const double* d_surface,
@@ -54,10 +57,11 @@ cg_status facet_receivers_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, 
 // Donor counts, the Kahn queue keys (level << 32 | deepest source) of FlowRouting.drainageOrder and,
 // if d_weights is given, FlowRouting.accumulate's areas, in one last-arriver walk. *h_levels
 // (optional, synchronises) receives the number of Kahn levels. With d_flow the sums are in double, of
-// the weights and d_inflow, into d_flow.
+// the weights and d_inflow, into d_flow. `also` is read back beside the levels.
 cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int32_t* d_recv,
                         const float* d_weights, long long* d_key, int32_t* d_donors, float* d_area, int* h_levels,
-                        const double* d_inflow = nullptr, double* d_flow = nullptr);
+                        const double* d_inflow = nullptr, double* d_flow = nullptr,
+                        ReadBack also = ReadBack{nullptr, nullptr, 0});
 // Once after a tree_walk_dev, over the tree it walked (its links, its sources and its counts, which are
 // in S_LINKS, S_SOURCES and S_DEPTH until the next user): every cell's d_flow plus its donors', in key order.
 cg_status flow_walk_dev(cg_ctx* ctx, int W, int H, long long* d_key, double* d_flow);

@@ -483,13 +483,24 @@ __global__ void __launch_bounds__(RECV_THREADS, 3) k_receivers(const uint8_t* __
 
 __global__ void k_surface(const uint8_t* __restrict__ land, const float* __restrict__ rel,
                           const float* __restrict__ filled, size_t N, double* __restrict__ surface,
-                          uint8_t* __restrict__ raised, int* __restrict__ local) {
+                          uint8_t* __restrict__ raised, int* __restrict__ local, int* __restrict__ n_raised) {
+    int count = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
         bool l = land[i] != 0;
         surface[i] = (double)(l ? filled[i] : rel[i]);
-        if (raised) raised[i] = l && filled[i] > rel[i];
+        const bool up = l && filled[i] > rel[i];
+        if (raised) raised[i] = up;
         if (local) local[i] = -1;
+        count += up;
     }
+    if (!n_raised) return;
+    __shared__ int total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    count = __reduce_add_sync(0xFFFFFFFFu, count);
+    if ((threadIdx.x & 31) == 0 && count) atomicAdd(&total, count);
+    __syncthreads();
+    if (threadIdx.x == 0 && total) atomicAdd(n_raised, total);
 }
 
 __global__ void k_flat_count(const int* __restrict__ label, size_t N, int* __restrict__ count) {
@@ -1706,11 +1717,12 @@ cg_status facet_receivers_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, 
 
 cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const float* d_rel,
                               const float* d_filled, int64_t seed, double r, int lattice, bool by_facet,
-                              bool over_potential, int32_t* d_recv, double* d_surface, FlatCounts* counts) {
+                              bool over_potential, int32_t* d_recv, double* d_surface, FlatCounts* counts,
+                              bool kept_later) {
     size_t N = (size_t)W * H;
     cudaStream_t sm = ctx->stream;
     int grid = ctx->num_sms * 8;
-    FlatCounts fc{0, 0, 0};
+    FlatCounts fc{0, 0, 0, nullptr};
     Steps steps;
     steps.ew = 1.0f;
     steps.ns = (float)r;
@@ -1718,17 +1730,20 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
     const int by = by_facet ? 1 : 0;
     bool routed = false;   // receivers already written (in two passes around the flats)
     if (!over_potential) {
-        CG_LAUNCH(ctx) k_surface<<<grid, 256, 0, sm>>>(d_land, d_rel, d_filled, N, d_surface, nullptr, nullptr);
+        CG_LAUNCH(ctx) k_surface<<<grid, 256, 0, sm>>>(d_land, d_rel, d_filled, N, d_surface, nullptr, nullptr, nullptr);
         CG_CHECK_LAUNCH(ctx);
     } else {
         CG_BUF(uint8_t, d_raised, ctx, S_FLATS, N);
         CG_BUF(int, d_local, ctx, S_FLATIDX, N);
         CG_BUF(int, d_root, ctx, S_LABEL, N);
         CG_BUF(int, d_label, ctx, S_SCRATCH2, N);
-        CG_LAUNCH(ctx) k_surface<<<grid, 256, 0, sm>>>(d_land, d_rel, d_filled, N, d_surface, d_raised, d_local);
+        CG_BUF(int, d_nraised, ctx, S_FLATCOUNT, 1);
+        CG_CUDA(ctx, cudaMemsetAsync(d_nraised, 0, sizeof(int), sm));
+        CG_LAUNCH(ctx) k_surface<<<grid, 256, 0, sm>>>(d_land, d_rel, d_filled, N, d_surface, d_raised, d_local, d_nraised);
         CG_CHECK_LAUNCH(ctx);
-        int flats = 0;
-        cg_status st = component_labels(ctx, W, H, d_raised, d_root, d_label, &flats);
+        int flats = 0, raised = 0;
+        cg_status st = component_labels(ctx, W, H, d_raised, d_root, d_label, &flats,
+                                        ReadBack{&raised, d_nraised, sizeof(int)});
         if (st != CG_OK) return st;
         if (flats > 0) {
             CG_BUF(int, d_cnt, ctx, S_CG0, 3 * (size_t)flats + 1);
@@ -1738,8 +1753,7 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
             CG_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, sizeof(int) * (3 * (size_t)flats + 1), sm));
             CG_LAUNCH(ctx) k_flat_count<<<grid, 256, 0, sm>>>(d_label, N, d_cnt);
             CG_CHECK_LAUNCH(ctx);
-            int raised = 0;
-            if ((st = exclusive_scan(ctx, d_cnt, d_off, flats, &raised)) != CG_OK) return st;
+            if ((st = exclusive_scan(ctx, d_cnt, d_off, flats, nullptr)) != CG_OK) return st;
             CG_BUF(int, d_members, ctx, S_FLATMEM, raised);
             CG_BUF(double, d_dbl, ctx, S_CG1, 10 * (size_t)raised);
             CG_LAUNCH(ctx) k_flat_scatter<<<grid, 256, 0, sm>>>(d_label, N, d_off, d_cur, d_members);
@@ -1785,8 +1799,7 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
             CG_LAUNCH(ctx) k_flat_lists<<<(flats + 255) / 256, 256, 0, sm>>>(d_cnt, flats, d_lists, d_ctr);
             CG_CHECK_LAUNCH(ctx);
             int ctr[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-            CG_CUDA(ctx, cudaMemcpyAsync(ctr, d_ctr, sizeof(ctr), cudaMemcpyDeviceToHost, sm));
-            CG_CUDA(ctx, cudaStreamSynchronize(sm));
+            CG_TRY_ST(read_back(ctx, {{ctr, d_ctr, sizeof(ctr)}}));
             // The small and mid-sized flats on the auxiliary stream, beside the few large ones, whose
             // CTAs hold an SM each for the whole solve.
             CG_CUDA(ctx, cudaEventRecord(ctx->fork, sm));
@@ -1833,8 +1846,7 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
                 CG_LAUNCH(ctx) kernel<<<ctr[1] * CL, CL_THREADS, bytes, sm>>>(a, d_lists + flats, cap,
                                                                               d_lists + 2 * (size_t)flats, d_ctr + 2);
                 CG_CHECK_LAUNCH(ctx);
-                CG_CUDA(ctx, cudaMemcpyAsync(&ctr[2], d_ctr + 2, sizeof(int), cudaMemcpyDeviceToHost, sm));
-                CG_CUDA(ctx, cudaStreamSynchronize(sm));
+                CG_TRY_ST(read_back(ctx, {{&ctr[2], d_ctr + 2, sizeof(int)}}));
             }
             if (ctr[2] > 0) {
                 a.large = d_lists + 2 * (size_t)flats;
@@ -1849,8 +1861,8 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
                                                                      by, d_raised, 2, d_recv);
             CG_CHECK_LAUNCH(ctx);
             routed = true;
-            CG_CUDA(ctx, cudaMemcpyAsync(&fc.kept, d_kept, sizeof(int), cudaMemcpyDeviceToHost, sm));
-            CG_CUDA(ctx, cudaStreamSynchronize(sm));
+            if (kept_later) fc.d_kept = d_kept;
+            else CG_TRY_ST(read_back(ctx, {{&fc.kept, d_kept, sizeof(int)}}));
             fc.flats = flats;
             fc.raised = raised;
         }

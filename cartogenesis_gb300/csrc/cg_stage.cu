@@ -191,24 +191,48 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
     }
 
     // Phase boundaries of a round, for the per-phase device times of cg_round_stats (ev[8]: the end
-    // of the uplift and the plate flexure).
-    cudaEvent_t ev[9] = {};
+    // of the uplift and the plate flexure). Two rounds' events in turn: a round's times are read after the
+    // next one's first synchronisation, so that the host does not wait for the end of a round.
+    cudaEvent_t events[2][9] = {};
     if (stats)
-        for (auto& e : ev) CG_CUDA(ctx, cudaEventCreate(&e));
+        for (auto& set : events)
+            for (auto& e : set) CG_CUDA(ctx, cudaEventCreate(&e));
     struct Events {
-        cudaEvent_t* ev;
+        cudaEvent_t (*ev)[9];
         bool on;
         ~Events() {
             if (on)
-                for (int i = 0; i < 9; ++i) cudaEventDestroy(ev[i]);
+                for (int i = 0; i < 18; ++i) cudaEventDestroy(ev[i / 9][i % 9]);
         }
-    } guard{ev, stats != nullptr};
-    auto mark = [&](int i) {
-        if (stats) cudaEventRecord(ev[i], sm);
+    } guard{events, stats != nullptr};
+    auto read_times = [&](int round) {   // of a round that is over
+        if (!stats || round < first_round) return;
+        cudaEvent_t* ev = events[round & 1];
+        float ms[8] = {0};
+        for (int i = 1; i < 8; ++i) cudaEventElapsedTime(&ms[i], ev[i - 1], ev[i]);
+        float total = 0.0f, ms_flexure = 0.0f;
+        if (flexure) {
+            cudaEventElapsedTime(&ms_flexure, ev[0], ev[8]);
+            cudaEventElapsedTime(&ms[1], ev[8], ev[1]);
+        }
+        cudaEventElapsedTime(&total, ev[0], ev[7]);
+        cg_round_stats& s = stats[round - first_round];
+        s.ms_total = total;
+        s.ms_flexure = ms_flexure;
+        s.ms_cut = ms[1];
+        s.ms_fill = ms[2];
+        s.ms_route = ms[3];
+        s.ms_tree = ms[4];
+        s.ms_incise = ms[5];
+        s.ms_deposit = ms[6];
+        s.ms_relax = ms[7];
     };
 
     for (int round = first_round; round < end_round; ++round) {
         CG_TRY(cancelled(ctx));
+        auto mark = [&](int i) {
+            if (stats) cudaEventRecord(events[round & 1][i], sm);
+        };
         float* cur = run.cur;
         const long long launches0 = ctx->launches;
         mark(0);
@@ -221,6 +245,7 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
         int land_cells;
         CG_TRY(percentile_cut_dev(ctx, W, H, cur, p.sea_level, land_half, sea_half, stand_below_today(p, round),
                                   d_land, d_rel, &shoreline, &land_cells));
+        read_times(round - 1);
         if (land_cells == 0) {   // HydraulicErosion.kt:856-858: the rounds stop where the land is gone
             run.done = true;
             run.next_round = round;
@@ -251,12 +276,13 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
         int64_t ties = 0, unresolved = 0;
         CG_TRY(fill_depressions_dev(ctx, W, H, d_land, d_rel, d_filled, &ties, &unresolved));
         mark(2);
-        FlatCounts fc{0, 0, 0};
+        FlatCounts fc{0, 0, 0, nullptr};
         CG_TRY(flow_directions_dev(ctx, W, H, d_land, d_rel, d_filled, p.seed, rates.cell_height_in_cell_widths,
-                                   lattice, p.facet_routing != 0, p.flat_potential != 0, d_recv, d_surface, &fc));
+                                   lattice, p.facet_routing != 0, p.flat_potential != 0, d_recv, d_surface, &fc, true));
         mark(3);
         int levels = 0;
-        CG_TRY(tree_walk_dev(ctx, W, H, d_land, d_recv, d_runoff, d_key, d_donors, d_area, &levels));
+        CG_TRY(tree_walk_dev(ctx, W, H, d_land, d_recv, d_runoff, d_key, d_donors, d_area, &levels, nullptr, nullptr,
+                             ReadBack{&fc.kept, fc.d_kept, fc.d_kept ? sizeof(int) : 0}));
         mark(4);
         const bool notch = p.profile >= CG_PROFILE_P1, deposition = p.profile >= CG_PROFILE_P2;
         const bool closing = round == p.hydraulic_rounds - 1;
@@ -339,16 +365,6 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
         run.next_round = round + 1;
         mark(7);
         if (stats) {
-            CG_CUDA(ctx, cudaEventSynchronize(ev[7]));
-            float ms[8] = {0};
-            for (int i = 1; i < 8; ++i) cudaEventElapsedTime(&ms[i], ev[i - 1], ev[i]);
-            float ms_flexure = 0.0f;
-            if (flexure) {
-                cudaEventElapsedTime(&ms_flexure, ev[0], ev[8]);
-                cudaEventElapsedTime(&ms[1], ev[8], ev[1]);
-            }
-            float total = 0.0f;
-            cudaEventElapsedTime(&total, ev[0], ev[7]);
             cg_round_stats& s = stats[round - first_round];
             std::memset(&s, 0, sizeof(s));
             s.round = round;
@@ -361,15 +377,6 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
             s.fill_ties = ties;
             s.fill_unresolved = unresolved;
             s.kernel_launches = ctx->launches - launches0;
-            s.ms_total = total;
-            s.ms_cut = ms[1];
-            s.ms_fill = ms[2];
-            s.ms_route = ms[3];
-            s.ms_tree = ms[4];
-            s.ms_incise = ms[5];
-            s.ms_deposit = ms[6];
-            s.ms_relax = ms[7];
-            s.ms_flexure = ms_flexure;
             s.deposit_replayed = dc.replayed;
             s.deposit_redone = dc.redone;
             s.deposit_refitted = dc.refitted;
@@ -380,6 +387,10 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
             s.ms_deposit_seas = dc.ms_seas;
             s.ms_deposit_repairs = dc.ms_repairs;
         }
+    }
+    if (stats && end_round > first_round) {
+        CG_CUDA(ctx, cudaEventSynchronize(events[(end_round - 1) & 1][7]));
+        read_times(end_round - 1);
     }
     if (run.next_round >= p.hydraulic_rounds) run.done = true;
     return CG_OK;

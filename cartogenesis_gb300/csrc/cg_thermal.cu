@@ -502,8 +502,7 @@ cg_status thermal_error_reset_dev(cg_ctx* ctx) {
 cg_status thermal_error_check(cg_ctx* ctx) {
     CG_BUF(int, d_err, ctx, S_THERMERR, 1);
     int err = 0;
-    CG_CUDA(ctx, cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    CG_TRY_ST(read_back(ctx, {{&err, d_err, sizeof(int)}}));
     if (err) return fail(ctx, CG_TIMEOUT, "thermal sweeps: a region copy did not arrive in its bounded wait");
     return CG_OK;
 }

@@ -680,7 +680,7 @@ __global__ void k_basin_finish(BasinDev b, int count, const uint8_t* __restrict_
 
 cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int32_t* d_recv,
                         const float* d_weights, long long* d_key, int32_t* d_donors, float* d_area, int* h_levels,
-                        const double* d_inflow, double* d_flow) {
+                        const double* d_inflow, double* d_flow, ReadBack also) {
     size_t N = (size_t)W * H;
     cudaStream_t sm = ctx->stream;
     int grid = ctx->num_sms * 8;
@@ -702,8 +702,7 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
     // million (its idle CTAs cost less than the 10 us of a host read); larger worlds read their number.
     int n_sources = (int)std::min(N, (size_t)1 << 19);
     if (N > (size_t)1 << 21) {
-        CG_CUDA(ctx, cudaMemcpyAsync(&n_sources, d_nsrc, sizeof(int), cudaMemcpyDeviceToHost, sm));
-        CG_CUDA(ctx, cudaStreamSynchronize(sm));
+        CG_TRY_ST(read_back(ctx, {{&n_sources, d_nsrc, sizeof(int)}}));
     }
     WalkArgs a{W, H, d_down, d_mask, d_pending, d_key, d_weights, d_area, d_inflow, d_flow, d_sources, d_nsrc, d_max};
     const int ctas = (n_sources + 63) / 64;
@@ -715,8 +714,7 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
     CG_CHECK_LAUNCH(ctx);
     if (h_levels) {
         unsigned long long mk;
-        CG_CUDA(ctx, cudaMemcpyAsync(&mk, d_max, sizeof(mk), cudaMemcpyDeviceToHost, sm));
-        CG_CUDA(ctx, cudaStreamSynchronize(sm));
+        CG_TRY_ST(read_back(ctx, {{&mk, d_max, sizeof(mk)}, also}));
         *h_levels = (int)(mk >> 32) + 1;
     }
     return CG_OK;
@@ -765,8 +763,7 @@ cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
     CG_LAUNCH(ctx) k_land_compact_ck<<<grid, 256, 0, sm>>>(d_land, d_pos, d_key, N, ka, va, levels > 0 ? nullptr : kmax);
     CG_CHECK_LAUNCH(ctx);
     if (levels <= 0) {
-        CG_CUDA(ctx, cudaMemcpyAsync(&hmax, kmax, sizeof(hmax), cudaMemcpyDeviceToHost, sm));
-        CG_CUDA(ctx, cudaStreamSynchronize(sm));
+        CG_TRY_ST(read_back(ctx, {{&hmax, kmax, sizeof(hmax)}}));
     }
     int bits = 0;
     while (bits < 64 && (hmax >> bits) != 0) ++bits;

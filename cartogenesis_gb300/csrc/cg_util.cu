@@ -1,6 +1,9 @@
 // Device building blocks shared by the phases: an exclusive prefix sum, and connected-component
 // labels over an 8-neighbour mask whose root is the component's smallest cell index (the order the
 // reference's DFS walks number components in: ascending start cell).
+#include <algorithm>
+#include <cstring>
+
 #include "cg_common.cuh"
 #include "cg_util.h"
 
@@ -172,14 +175,30 @@ __global__ void k_label_from_root(const int* __restrict__ parent, const int* __r
 
 }  // namespace
 
+cg_status read_back(cg_ctx* ctx, std::initializer_list<ReadBack> parts) {
+    size_t total = 0;
+    for (const ReadBack& p : parts) total += (p.bytes + 15) & ~(size_t)15;
+    cg_status st = CG_OK;
+    char* staging = (char*)pinned(ctx, std::max<size_t>(total, 256), &st);
+    if (st != CG_OK) return st;
+    size_t at = 0;
+    for (const ReadBack& p : parts) {
+        if (p.bytes) CG_CUDA(ctx, cudaMemcpyAsync(staging + at, p.dev, p.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        at += (p.bytes + 15) & ~(size_t)15;
+    }
+    CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    at = 0;
+    for (const ReadBack& p : parts) {
+        if (p.bytes) std::memcpy(p.host, staging + at, p.bytes);
+        at += (p.bytes + 15) & ~(size_t)15;
+    }
+    return CG_OK;
+}
+
 // Two launches, the tiles' sums and the tiles, each CTA adding up the sums before its own: a level of
 // block scans and a pass adding their offsets took four to six. A read of up to kScanDirect sums a CTA
 // stays below the tile's own; longer inputs scan the sums first.
-cg_status exclusive_scan(cg_ctx* ctx, const int* d_in, int* d_out, int n, int* h_total) {
-    if (n <= 0) {
-        if (h_total) *h_total = 0;
-        return CG_OK;
-    }
+static cg_status scan_dev(cg_ctx* ctx, const int* d_in, int* d_out, int n, int** total) {
     if (n > 1 << 30) return fail(ctx, CG_BAD_ARG, "scan of %d elements is too long", n);
     const int tiles = (n + kScanTile - 1) / kScanTile;
     const int tiles2 = tiles > kScanDirect ? (tiles + kScanTile - 1) / kScanTile : 0;
@@ -196,15 +215,22 @@ cg_status exclusive_scan(cg_ctx* ctx, const int* d_in, int* d_out, int n, int* h
     }
     CG_LAUNCH(ctx) k_scan_tiles<<<tiles, kScanThreads, 0, ctx->stream>>>(d_in, n, d_sums, d_offs, d_out, d_total);
     CG_CHECK_LAUNCH(ctx);
-    if (h_total) {
-        CG_CUDA(ctx, cudaMemcpyAsync(h_total, d_total, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    }
+    *total = d_total;
     return CG_OK;
 }
 
+cg_status exclusive_scan(cg_ctx* ctx, const int* d_in, int* d_out, int n, int* h_total) {
+    if (n <= 0) {
+        if (h_total) *h_total = 0;
+        return CG_OK;
+    }
+    int* d_total = nullptr;
+    CG_TRY_ST(scan_dev(ctx, d_in, d_out, n, &d_total));
+    return h_total ? read_back(ctx, {{h_total, d_total, sizeof(int)}}) : CG_OK;
+}
+
 cg_status component_labels(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, int* d_root, int* d_label,
-                           int* h_count) {
+                           int* h_count, ReadBack also) {
     size_t N = (size_t)W * H;
     int grid = ctx->num_sms * 8;
     CG_LAUNCH(ctx) k_cc_init<<<grid, 256, 0, ctx->stream>>>(d_mask, d_root, N);
@@ -216,8 +242,9 @@ cg_status component_labels(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, int
         CG_BUF(int, d_rank, ctx, S_SCRATCH1, N);
         CG_LAUNCH(ctx) k_root_flags<<<grid, 256, 0, ctx->stream>>>(d_root, d_flag, N);
         CG_CHECK_LAUNCH(ctx);
-        cg_status st = exclusive_scan(ctx, d_flag, d_rank, (int)N, h_count);
-        if (st != CG_OK) return st;
+        int* d_total = nullptr;
+        CG_TRY_ST(scan_dev(ctx, d_flag, d_rank, (int)N, &d_total));
+        if (h_count) CG_TRY_ST(read_back(ctx, {{h_count, d_total, sizeof(int)}, also}));
         CG_LAUNCH(ctx) k_label_from_root<<<grid, 256, 0, ctx->stream>>>(d_root, d_rank, d_label, N);
         CG_CHECK_LAUNCH(ctx);
     }
