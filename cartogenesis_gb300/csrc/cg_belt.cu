@@ -206,47 +206,39 @@ __global__ void k_frontier_list(const int* __restrict__ flag, const int* __restr
         if (flag[i]) out[pos[i]] = (int)i;
 }
 
-// The rise where the belt has begun to (BeltErosion.kt:240-248); xs[l] the uplift book's term.
-__global__ void k_belt_rise(const int* __restrict__ list, int B, const int* __restrict__ first,
-                            const float* __restrict__ rise, int round, BeltConsts k, float* __restrict__ h,
-                            float* __restrict__ uplifted_m, double* __restrict__ xs) {
-    for (size_t l = tid(); l < (size_t)B; l += nthreads()) {
-        double term = 0.0;
-        if (round >= first[l]) {
-            const int c = list[l];
-            const float r = rise[l];
-            h[c] = __fadd_rn(h[c], r);
-            if (uplifted_m) uplifted_m[c] = __fadd_rn(uplifted_m[c], __fmul_rn(r, k.mpfu));
-            term = __dmul_rn(__dmul_rn((double)r, (double)k.mpfu), k.area);
+// A round's opening. The rise where the belt has begun to (BeltErosion.kt:240-248), xs[l] the uplift book's
+// term; the belt flood's inner land and the facet rule's cells (BeltErosion.kt:257-292); and the routing
+// surface of the belt and its frontier, as yet unfilled.
+__global__ void k_belt_open(const int* __restrict__ swept, int B, int F, const int* __restrict__ first,
+                            const float* __restrict__ rise, int round, BeltConsts k, const int* __restrict__ local,
+                            const uint8_t* __restrict__ land, int W, int H, float* __restrict__ h,
+                            float* __restrict__ uplifted_m, double* __restrict__ xs, uint8_t* __restrict__ inner,
+                            uint8_t* __restrict__ routed, double* __restrict__ routing) {
+    for (size_t l = tid(); l < (size_t)(B + F); l += nthreads()) {
+        const int c = swept[l];
+        float height = h[c];
+        if (l < (size_t)B) {
+            double term = 0.0;
+            if (round >= first[l]) {
+                const float r = rise[l];
+                height = __fadd_rn(height, r);
+                h[c] = height;
+                if (uplifted_m) uplifted_m[c] = __fadd_rn(uplifted_m[c], __fmul_rn(r, k.mpfu));
+                term = __dmul_rn(__dmul_rn((double)r, (double)k.mpfu), k.area);
+            }
+            xs[l] = term;
+            const int row = pdiv(c, W), col = pmod(c, W);
+            const bool sea = !land[c] || height <= k.shoreline;
+            bool edge = row == 0 || row == H - 1;
+            for (int rs = -1; rs <= 1 && !edge && !sea; ++rs) {
+                const int nr = row + rs;
+                for (int cs = -1; cs <= 1; ++cs)
+                    if (!(rs == 0 && cs == 0) && local[nr * W + wrap_col(col + cs, W)] < 0) edge = true;
+            }
+            inner[c] = (!sea && !edge) ? 1 : 0;
+            routed[c] = sea ? 0 : 1;
         }
-        xs[l] = term;
-    }
-}
-
-__global__ void k_route_cells(const int* __restrict__ cells, int n, const float* __restrict__ h,
-                              double* __restrict__ routing) {
-    for (size_t j = tid(); j < (size_t)n; j += nthreads()) {
-        const int c = cells[j];
-        routing[c] = (double)h[c];
-    }
-}
-
-// The belt flood's inner land and the facet rule's cells (BeltErosion.kt:257-292).
-__global__ void k_belt_masks(const int* __restrict__ list, int B, const int* __restrict__ local,
-                             const uint8_t* __restrict__ land, const float* __restrict__ h, BeltConsts k, int W,
-                             int H, uint8_t* __restrict__ inner, uint8_t* __restrict__ routed) {
-    for (size_t l = tid(); l < (size_t)B; l += nthreads()) {
-        const int c = list[l];
-        const int row = pdiv(c, W), col = pmod(c, W);
-        const bool sea = !land[c] || h[c] <= k.shoreline;
-        bool edge = row == 0 || row == H - 1;
-        for (int rs = -1; rs <= 1 && !edge && !sea; ++rs) {
-            const int nr = row + rs;
-            for (int cs = -1; cs <= 1; ++cs)
-                if (!(rs == 0 && cs == 0) && local[nr * W + wrap_col(col + cs, W)] < 0) edge = true;
-        }
-        inner[c] = (!sea && !edge) ? 1 : 0;
-        routed[c] = sea ? 0 : 1;
+        routing[c] = (double)height;
     }
 }
 
@@ -419,69 +411,88 @@ __global__ void k_order_terms(const int* __restrict__ order, int B, const int32_
     }
 }
 
-// One sweep's give rates of the belt cells (BeltErosion.kt:375-390).
-__global__ void k_belt_give(const int* __restrict__ list, int B, const float* __restrict__ h, int W, int H,
-                            BeltConsts k, float* __restrict__ give) {
-    for (size_t l = tid(); l < (size_t)B; l += nthreads()) {
-        const int c = list[l];
-        const int row = pdiv(c, W), col = pmod(c, W);
-        const float here = h[c];
-        float excess = 0.0f, steepest = 0.0f;
-        for (int rs = -1; rs <= 1; ++rs) {
-            const int nr = row + rs;
-            if (nr < 0 || nr >= H) continue;
-            for (int cs = -1; cs <= 1; ++cs) {
-                if (rs == 0 && cs == 0) continue;
-                const float drop = __fsub_rn(here, h[nr * W + wrap_col(col + cs, W)]);
-                if (drop > 0.0f) {
-                    if (drop > steepest) steepest = drop;
-                    const float limit = limit_of(rs, cs, k);
-                    if (drop > limit) excess = __fadd_rn(excess, __fsub_rn(drop, limit));
-                }
-            }
-        }
-        give[c] = excess <= k.settled ? 0.0f
-                                      : __fdiv_rn(jvm_min(__fmul_rn(k.rate, excess), __fmul_rn(steepest, 0.5f)), excess);
-    }
-}
+// A round's sweeps over the belt and its frontier (BeltErosion.kt:373-408) in one cooperative launch: the
+// belt cells' give rates, then every swept cell's new height into the other field, the frontier's change
+// the shed book's terms, a grid barrier after each. The fields differ at swept cells alone, and every sweep
+// writes all of those. Three launches a sweep took 14 us at 50,000 cells, a third of it between them; a sweep
+// here takes 10.
+struct SweepArgs {
+    const int* swept;   // the belt's cells, then the frontier's
+    int B, F, W, H, sweeps;
+    const int* local;
+    float* h[2];        // the heights, and the other field
+    float* give;
+    double* xs;         // the shed terms, F a sweep
+    BeltConsts k;
+};
 
-// One sweep's new heights of the belt and its frontier (BeltErosion.kt:391-403).
-__global__ void k_belt_next(const int* __restrict__ swept, int n, const int* __restrict__ local,
-                            const float* __restrict__ h, const float* __restrict__ give, int W, int H, BeltConsts k,
-                            float* __restrict__ next) {
-    for (size_t j = tid(); j < (size_t)n; j += nthreads()) {
-        const int c = swept[j];
-        const int row = pdiv(c, W), col = pmod(c, W);
-        const float here = h[c];
-        const bool own = local[c] >= 0;
-        float received = 0.0f, given = 0.0f;
-        for (int rs = -1; rs <= 1; ++rs) {
-            const int nr = row + rs;
-            if (nr < 0 || nr >= H) continue;
-            for (int cs = -1; cs <= 1; ++cs) {
-                if (rs == 0 && cs == 0) continue;
-                const int nb = nr * W + wrap_col(col + cs, W);
+__device__ float belt_give(const SweepArgs& a, const float* h, int c) {
+    const BeltConsts& k = a.k;
+    const int row = pdiv(c, a.W), col = pmod(c, a.W);
+    const float here = __ldcg(h + c);
+    float excess = 0.0f, steepest = 0.0f;
+    for (int rs = -1; rs <= 1; ++rs) {
+        const int nr = row + rs;
+        if (nr < 0 || nr >= a.H) continue;
+        for (int cs = -1; cs <= 1; ++cs) {
+            if (rs == 0 && cs == 0) continue;
+            const float drop = __fsub_rn(here, __ldcg(h + nr * a.W + wrap_col(col + cs, a.W)));
+            if (drop > 0.0f) {
+                if (drop > steepest) steepest = drop;
                 const float limit = limit_of(rs, cs, k);
-                const float incoming = __fsub_rn(h[nb], here);
-                if (incoming > limit && local[nb] >= 0)
-                    received = __fadd_rn(received, __fmul_rn(give[nb], __fsub_rn(incoming, limit)));
-                else if (-incoming > limit && own)
-                    given = __fadd_rn(given, __fmul_rn(give[c], __fsub_rn(-incoming, limit)));
+                if (drop > limit) excess = __fadd_rn(excess, __fsub_rn(drop, limit));
             }
         }
-        next[j] = __fadd_rn(__fsub_rn(here, given), received);
     }
+    return excess <= k.settled ? 0.0f : __fdiv_rn(jvm_min(__fmul_rn(k.rate, excess), __fmul_rn(steepest, 0.5f)), excess);
 }
 
-// The sweep's heights written back; the frontier's change is the shed book's terms (BeltErosion.kt:404-407).
-__global__ void k_belt_commit(const int* __restrict__ swept, int B, int F, const float* __restrict__ next,
-                              BeltConsts k, float* __restrict__ h, double* __restrict__ xs) {
-    for (size_t j = tid(); j < (size_t)(B + F); j += nthreads()) {
-        const int c = swept[j];
-        if (j >= (size_t)B)
-            xs[j - B] = __dmul_rn(__dmul_rn((double)__fsub_rn(next[j], h[c]), (double)k.mpfu), k.area);
-        h[c] = next[j];
+__device__ float belt_next(const SweepArgs& a, const float* h, int c, float here, bool own) {
+    const BeltConsts& k = a.k;
+    const int row = pdiv(c, a.W), col = pmod(c, a.W);
+    float received = 0.0f, given = 0.0f;
+    for (int rs = -1; rs <= 1; ++rs) {
+        const int nr = row + rs;
+        if (nr < 0 || nr >= a.H) continue;
+        for (int cs = -1; cs <= 1; ++cs) {
+            if (rs == 0 && cs == 0) continue;
+            const int nb = nr * a.W + wrap_col(col + cs, a.W);
+            const float limit = limit_of(rs, cs, k);
+            const float incoming = __fsub_rn(__ldcg(h + nb), here);
+            if (incoming > limit && a.local[nb] >= 0)
+                received = __fadd_rn(received, __fmul_rn(__ldcg(a.give + nb), __fsub_rn(incoming, limit)));
+            else if (-incoming > limit && own)
+                given = __fadd_rn(given, __fmul_rn(__ldcg(a.give + c), __fsub_rn(-incoming, limit)));
+        }
     }
+    return __fadd_rn(__fsub_rn(here, given), received);
+}
+
+__global__ void __launch_bounds__(512) k_belt_sweeps(SweepArgs a) {
+    cgr::grid_group grid = cgr::this_grid();
+    const int t = blockIdx.x * 512 + threadIdx.x, stride = gridDim.x * 512, n = a.B + a.F;
+    for (int s = 0; s < a.sweeps; ++s) {
+        const float* h = a.h[s & 1];
+        float* to = a.h[(s & 1) ^ 1];
+        for (int l = t; l < a.B; l += stride) {
+            const int c = a.swept[l];
+            __stcg(a.give + c, belt_give(a, h, c));
+        }
+        grid.sync();
+        for (int j = t; j < n; j += stride) {
+            const int c = a.swept[j];
+            const float here = __ldcg(h + c), next = belt_next(a, h, c, here, j < a.B);
+            __stcg(to + c, next);
+            if (j >= a.B)
+                a.xs[(size_t)s * a.F + (j - a.B)] = __dmul_rn(__dmul_rn((double)__fsub_rn(next, here), (double)a.k.mpfu), a.k.area);
+        }
+        if (s + 1 < a.sweeps || (a.sweeps & 1)) grid.sync();
+    }
+    if (a.sweeps & 1)   // the heights are in the other field
+        for (int j = t; j < n; j += stride) {
+            const int c = a.swept[j];
+            a.h[0][c] = __ldcg(a.h[1] + c);
+        }
 }
 
 // The rock lost so far less the rebound already given (BeltErosion.kt:414-416).
@@ -522,12 +533,12 @@ __global__ void k_blur_down(const float* __restrict__ in, int W, int H, const do
     }
 }
 
-// The crust's answer (BeltErosion.kt:418-422).
+// The crust's answer (BeltErosion.kt:418-422), in both of the sweeps' fields.
 __global__ void k_belt_rebound(size_t N, const float* __restrict__ loss, float share, float mpfu,
-                               float* __restrict__ h, float* __restrict__ rbm) {
+                               float* __restrict__ h, float* __restrict__ rbm, float* __restrict__ other) {
     for (size_t i = tid(); i < N; i += nthreads()) {
         const float rebound = __fmul_rn(share, loss[i]);
-        h[i] = __fadd_rn(h[i], __fdiv_rn(__fsub_rn(rebound, rbm[i]), mpfu));
+        h[i] = other[i] = __fadd_rn(h[i], __fdiv_rn(__fsub_rn(rebound, rbm[i]), mpfu));
         rbm[i] = rebound;
     }
 }
@@ -735,6 +746,22 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
     CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_belt_cut, kCutThreads, 0));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "the belt's cut kernel cannot be resident");
     const int bgrid = std::min(grid, (B + 255) / 256 + 1);
+    CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_belt_sweeps, 512, 0));
+    if (per_sm < 1) return fail(ctx, CG_CUDA, "the belt's sweep kernel cannot be resident");
+    CG_CUDA(ctx, cudaMemcpyAsync(d_next, d_h, N * 4, cudaMemcpyDeviceToDevice, sm));
+    SweepArgs sa{};
+    sa.swept = d_swept;
+    sa.B = B;
+    sa.F = F;
+    sa.W = W;
+    sa.H = H;
+    sa.sweeps = sweeps;
+    sa.local = d_local;
+    sa.h[0] = d_h;
+    sa.h[1] = d_next;
+    sa.give = d_give;
+    sa.xs = xs_shed;
+    sa.k = k;
     CG_BUF(int4, d_cut, ctx, S_BT_CUT, 2 * (size_t)B + 1);   // 32 bytes a cell
     CG_BUF(int, d_start, ctx, S_BT_LEVELS, (size_t)B + 2);   // at most a level a cell, and the split
 
@@ -762,12 +789,11 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
 
     for (int round = 0; round < k.rounds; ++round) {
         if (ctx->cancel.exchange(0)) return fail(ctx, CG_CANCELLED, "cancelled");
-        // The rise and its book's terms (BeltErosion.kt:240-249).
-        CG_LAUNCH(ctx) k_belt_rise<<<bgrid, 256, 0, sm>>>(d_swept, B, d_first, d_rise, round, k, d_h, d_uplm, xs_rise);
-        CG_LAUNCH(ctx) k_route_cells<<<grid, 256, 0, sm>>>(d_swept, B + F, d_h, d_routing);
-        // The spill levels, the routing surface and the facet receivers (BeltErosion.kt:253-292).
-        CG_LAUNCH(ctx) k_belt_masks<<<bgrid, 256, 0, sm>>>(d_swept, B, d_local, d_land, d_h, k, W, H, d_inner, d_routed);
+        // The rise and its book's terms (BeltErosion.kt:240-249), and the round's masks.
+        CG_LAUNCH(ctx) k_belt_open<<<grid, 256, 0, sm>>>(d_swept, B, F, d_first, d_rise, round, k, d_local, d_land, W, H,
+                                                         d_h, d_uplm, xs_rise, d_inner, d_routed, d_routing);
         CG_CHECK_LAUNCH(ctx);
+        // The spill levels, the routing surface and the facet receivers (BeltErosion.kt:253-292).
         CG_TRY_ST(fill_depressions_dev(ctx, W, H, d_inner, d_h, d_filled, nullptr, nullptr));
         CG_LAUNCH(ctx) k_route_filled<<<bgrid, 256, 0, sm>>>(d_swept, B, d_routed, d_filled, d_routing);
         CG_CHECK_LAUNCH(ctx);
@@ -775,7 +801,7 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
         // The run order and the discharge (BeltErosion.kt:296-325).
         CG_TRY_ST(tree_walk_dev(ctx, W, H, d_belt, d_recv, d_weights, d_key, d_donors, nullptr, &ca.levels, d_inflow,
                                 d_disc));
-        CG_TRY_ST(order_from_keys_dev(ctx, W, H, d_belt, d_key, B, d_order, ca.levels));
+        CG_TRY_ST(order_from_keys_dev(ctx, W, H, d_belt, d_key, B, d_order, ca.levels, d_swept));
         CG_TRY_ST(level_bounds_dev(ctx, d_order, d_key, B, ca.levels, d_start));
         // The cut and the spoil's flux (BeltErosion.kt:327-370).
         void* kargs[] = {&ca};
@@ -785,13 +811,10 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
         CG_LAUNCH(ctx) k_order_terms<<<bgrid, 256, 0, sm>>>(d_order, B, d_recv, d_belt, d_land, d_h, k.shoreline,
                                                             d_flux, d_cutv, xs_cut, xs_sea, xs_land);
         CG_CHECK_LAUNCH(ctx);
-        // The slopes (BeltErosion.kt:373-408), the frontier's changes the shed book's terms.
-        for (int s = 0; s < sweeps; ++s) {
-            CG_LAUNCH(ctx) k_belt_give<<<bgrid, 256, 0, sm>>>(d_swept, B, d_h, W, H, k, d_give);
-            CG_LAUNCH(ctx) k_belt_next<<<grid, 256, 0, sm>>>(d_swept, B + F, d_local, d_h, d_give, W, H, k, d_next);
-            CG_LAUNCH(ctx) k_belt_commit<<<grid, 256, 0, sm>>>(d_swept, B, F, d_next, k, d_h, xs_shed + (size_t)s * F);
-        }
-        CG_CHECK_LAUNCH(ctx);
+        // The slopes.
+        void* sargs[] = {&sa};
+        ctx->launches++;
+        CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_belt_sweeps, ctx->num_sms, 512, sargs, 0, sm));
         CG_TRY_ST(seq_totals_f64_dev(ctx, totals, kSeqTotals));
         // The crust's answer to the rock taken so far (BeltErosion.kt:413-423).
         if (rebound && ((round + 1) % kReboundRounds == 0 || round == k.rounds - 1)) {
@@ -799,7 +822,7 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
             CG_CHECK_LAUNCH(ctx);
             CG_TRY_ST(gaussian_blur_dev(ctx, W, H, d_loss, d_tmp, crust_spread_km / sc.cell_width_km(W),
                                         crust_spread_km / sc.cell_height_km(H)));
-            CG_LAUNCH(ctx) k_belt_rebound<<<grid, 256, 0, sm>>>(N, d_loss, k.rebound_share, k.mpfu, d_h, d_rbm);
+            CG_LAUNCH(ctx) k_belt_rebound<<<grid, 256, 0, sm>>>(N, d_loss, k.rebound_share, k.mpfu, d_h, d_rbm, d_next);
             CG_CHECK_LAUNCH(ctx);
         }
     }

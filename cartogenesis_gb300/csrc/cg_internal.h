@@ -66,9 +66,10 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
 // in S_LINKS, S_SOURCES and S_DEPTH until the next user): every cell's d_flow plus its donors', in key order.
 cg_status flow_walk_dev(cg_ctx* ctx, int W, int H, long long* d_key, double* d_flow);
 // The explicit drainage order (land cells sorted by key), for callers that want it; `levels` the keys'
-// number of Kahn levels, 0 where the caller does not know it (synchronises).
+// number of Kahn levels, 0 where the caller does not know it (synchronises); d_cells the land cells in any
+// order, where the caller has them.
 cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const long long* d_key,
-                              int land_cells, int32_t* d_order, int levels = 0);
+                              int land_cells, int32_t* d_order, int levels = 0, const int* d_cells = nullptr);
 struct InciseArgs {
     float courant_coefficient;
     float pond_depth;

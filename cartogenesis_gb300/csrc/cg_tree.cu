@@ -275,6 +275,7 @@ __global__ void k_land_flags(const uint8_t* __restrict__ land, size_t N, int* __
 // would leave SMs without two: the chunks of a tile follow one another, and at 60,000 cells 15 CTAs of 16
 // chunks took 14 us a pass.
 constexpr int kRsTile = 4096;
+constexpr int kRsOneLaunch = 2048;   // cells an SM up to which the passes share one launch
 
 __global__ void k_land_compact_ck(const uint8_t* __restrict__ land, const int* __restrict__ pos,
                                   const long long* __restrict__ key, size_t N, unsigned long long* __restrict__ ck,
@@ -296,6 +297,17 @@ __global__ void k_land_compact_ck(const uint8_t* __restrict__ land, const int* _
     if ((threadIdx.x & 31) == 0 && m) atomicMax(kmax, m);
 }
 
+// The same from a list of the cells (in any order: the keys are distinct).
+__global__ void k_list_ck(const int* __restrict__ cells, int n, const long long* __restrict__ key, size_t N,
+                          unsigned long long* __restrict__ ck, int* __restrict__ vals) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int c = cells[i];
+        const unsigned long long k = (unsigned long long)key[c];
+        ck[i] = (k >> 32) * (unsigned long long)N + (k & 0xFFFFFFFFull);
+        vals[i] = c;
+    }
+}
+
 __global__ void __launch_bounds__(256) k_rs_hist(const unsigned long long* __restrict__ keys, int n, int shift,
                                                  int tile, int tiles, int* __restrict__ hist) {
     __shared__ int h[256];
@@ -307,32 +319,33 @@ __global__ void __launch_bounds__(256) k_rs_hist(const unsigned long long* __res
     hist[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void __launch_bounds__(256) k_rs_scatter(const unsigned long long* __restrict__ kin,
-                                                    const int* __restrict__ vin, int n, int shift, int tile,
-                                                    int tiles, const int* __restrict__ off, unsigned long long* __restrict__ kout,
-                                                    int* __restrict__ vout) {
-    __shared__ int base[256];
-    __shared__ int wcnt[8][256];
+struct RsSmem {
+    int base[256];
+    int wcnt[8][256];
+};
+
+// A CTA's tile [lo, hi) scattered in order, its digits' first places in sh.base.
+__device__ __forceinline__ void rs_scatter_tile(const unsigned long long* __restrict__ kin, const int* __restrict__ vin,
+                                                int lo, int hi, int shift, RsSmem& sh,
+                                                unsigned long long* __restrict__ kout, int* __restrict__ vout) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    base[tid] = off[tid * tiles + blockIdx.x];
 #pragma unroll
-    for (int w = 0; w < 8; ++w) wcnt[w][tid] = 0;
+    for (int w = 0; w < 8; ++w) sh.wcnt[w][tid] = 0;
     __syncthreads();
-    const int lo = blockIdx.x * tile, hi = min(n, lo + tile);
     for (int c = lo; c < hi; c += 256) {
         const int i = c + tid;
         const bool valid = i < hi;
-        const unsigned long long k = valid ? kin[i] : 0ull;
-        const int v = valid ? vin[i] : 0;
+        const unsigned long long k = valid ? __ldcg(kin + i) : 0ull;
+        const int v = valid ? __ldcg(vin + i) : 0;
         const int d = valid ? (int)((k >> shift) & 255ull) : 256;
         const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
         const int rank = __popc(peers & ((1u << lane) - 1u));
-        if (valid && rank == 0) wcnt[warp][d] = __popc(peers);
+        if (valid && rank == 0) sh.wcnt[warp][d] = __popc(peers);
         __syncthreads();
         if (valid) {
             int before = 0;
-            for (int w = 0; w < warp; ++w) before += wcnt[w][d];
-            const int p = base[d] + before + rank;
+            for (int w = 0; w < warp; ++w) before += sh.wcnt[w][d];
+            const int p = sh.base[d] + before + rank;
             kout[p] = k;
             vout[p] = v;
         }
@@ -340,11 +353,79 @@ __global__ void __launch_bounds__(256) k_rs_scatter(const unsigned long long* __
         int sum = 0;
 #pragma unroll
         for (int w = 0; w < 8; ++w) {
-            sum += wcnt[w][tid];
-            wcnt[w][tid] = 0;
+            sum += sh.wcnt[w][tid];
+            sh.wcnt[w][tid] = 0;
         }
-        base[tid] += sum;
+        sh.base[tid] += sum;
         __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(256) k_rs_scatter(const unsigned long long* __restrict__ kin,
+                                                    const int* __restrict__ vin, int n, int shift, int tile,
+                                                    int tiles, const int* __restrict__ off, unsigned long long* __restrict__ kout,
+                                                    int* __restrict__ vout) {
+    __shared__ RsSmem sh;
+    sh.base[threadIdx.x] = off[threadIdx.x * tiles + blockIdx.x];
+    const int lo = blockIdx.x * tile;
+    rs_scatter_tile(kin, vin, lo, min(n, lo + tile), shift, sh, kout, vout);
+}
+
+// Every pass in one cooperative launch, a CTA a tile, where the tiles are no more than the SMs: the counts,
+// a warp a digit scanning them over the tiles, and the scatter, a grid barrier after each. Four launches a
+// pass took 16 us at 50,000 cells, mostly between them; a pass here takes 10.
+struct RsArgs {
+    unsigned long long* keys[2];
+    int* vals[2];
+    int n, tile, tiles, bits;
+    int* hist;     // [tiles][256]
+    int* before;   // [tiles][256]: the cells of the digit in the tiles before
+    int* total;    // [256]
+    int* out;
+};
+__global__ void __launch_bounds__(256) k_rs_sort(RsArgs a) {
+    cgr::grid_group grid = cgr::this_grid();
+    __shared__ RsSmem sh;
+    __shared__ int warp_sum[8];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int lo = blockIdx.x * a.tile, hi = min(a.n, lo + a.tile);
+    int pass = 0;
+    for (int shift = 0; shift < a.bits; shift += 8, ++pass) {
+        const unsigned long long* kin = a.keys[pass & 1];
+        sh.base[tid] = 0;
+        __syncthreads();
+        for (int i = lo + tid; i < hi; i += 256) atomicAdd(&sh.base[(int)((__ldcg(kin + i) >> shift) & 255ull)], 1);
+        __syncthreads();
+        __stcg(a.hist + blockIdx.x * 256 + tid, sh.base[tid]);
+        grid.sync();
+        for (int d = blockIdx.x * 8 + warp; d < 256; d += gridDim.x * 8) {
+            int run = 0;
+            for (int t0 = 0; t0 < a.tiles; t0 += 32) {
+                const int v = t0 + lane < a.tiles ? __ldcg(a.hist + (t0 + lane) * 256 + d) : 0;
+                int x = v;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (t0 + lane < a.tiles) __stcg(a.before + (t0 + lane) * 256 + d, run + x - v);
+                run += __shfl_sync(0xFFFFFFFFu, x, 31);
+            }
+            if (lane == 0) __stcg(a.total + d, run);
+        }
+        grid.sync();
+        const int all = __ldcg(a.total + tid);
+        int x = all;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_sum[warp] = x;
+        __syncthreads();
+        for (int w = 0; w < warp; ++w) x += warp_sum[w];
+        sh.base[tid] = x - all + __ldcg(a.before + blockIdx.x * 256 + tid);
+        const bool last = shift + 8 >= a.bits;
+        rs_scatter_tile(kin, a.vals[pass & 1], lo, hi, shift, sh, a.keys[(pass & 1) ^ 1], last ? a.out : a.vals[(pass & 1) ^ 1]);
+        if (!last) grid.sync();
     }
 }
 
@@ -685,15 +766,14 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
     cudaStream_t sm = ctx->stream;
     int grid = ctx->num_sms * 8;
     CG_BUF(int32_t, d_pending, ctx, S_DEPTH, N);
-    CG_BUF(unsigned long long, d_max, ctx, S_STATS, 1);
-    CG_BUF(uint8_t, d_links, ctx, S_LINKS, 2 * N);
-    CG_BUF(int, d_sources, ctx, S_SOURCES, N + 1);
+    // The links and, behind them, the largest key and the number of sources: zeroed together.
+    CG_BUF(uint8_t, d_links, ctx, S_LINKS, 2 * N + 32);
+    CG_BUF(int, d_sources, ctx, S_SOURCES, N);
     uint8_t* d_down = d_links;
     uint8_t* d_mask = d_links + N;
-    int* d_nsrc = d_sources + N;
-    CG_CUDA(ctx, cudaMemsetAsync(d_mask, 0, N, sm));
-    CG_CUDA(ctx, cudaMemsetAsync(d_nsrc, 0, sizeof(int), sm));
-    CG_CUDA(ctx, cudaMemsetAsync(d_max, 0, sizeof(unsigned long long), sm));
+    unsigned long long* d_max = reinterpret_cast<unsigned long long*>(d_links + ((2 * N + 15) & ~(size_t)15));
+    int* d_nsrc = reinterpret_cast<int*>(d_max + 1);
+    CG_CUDA(ctx, cudaMemsetAsync(d_mask, 0, (uint8_t*)(d_nsrc + 1) - d_mask, sm));
     CG_LAUNCH(ctx) k_links<<<grid, 256, 0, sm>>>(d_land, d_recv, W, H, d_down, d_mask);
     CG_LAUNCH(ctx) k_sources<<<grid, 256, 0, sm>>>(d_land, d_mask, N, d_donors, d_pending, d_sources, d_nsrc);
     if (d_area) CG_LAUNCH(ctx) k_area_sea<<<grid, 256, 0, sm>>>(d_land, N, d_area);
@@ -723,10 +803,10 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
 cg_status flow_walk_dev(cg_ctx* ctx, int W, int H, long long* d_key, double* d_flow) {
     const size_t N = (size_t)W * H;
     CG_BUF(int32_t, d_pending, ctx, S_DEPTH, N);
-    CG_BUF(uint8_t, d_links, ctx, S_LINKS, 2 * N);
-    CG_BUF(int, d_sources, ctx, S_SOURCES, N + 1);
-    WalkArgs a{W, H, d_links, d_links + N, d_pending, d_key, nullptr, nullptr, nullptr, d_flow, d_sources, d_sources + N,
-               nullptr};
+    CG_BUF(uint8_t, d_links, ctx, S_LINKS, 2 * N + 32);
+    CG_BUF(int, d_sources, ctx, S_SOURCES, N);
+    const int* d_nsrc = reinterpret_cast<const int*>(d_links + ((2 * N + 15) & ~(size_t)15)) + 2;
+    WalkArgs a{W, H, d_links, d_links + N, d_pending, d_key, nullptr, nullptr, nullptr, d_flow, d_sources, d_nsrc, nullptr};
     const int ctas = ((int)std::min(N, (size_t)1 << 19) + 63) / 64;
     CG_LAUNCH(ctx) k_walk<WALK_FLOW><<<ctas, 64, 0, ctx->stream>>>(a);
     CG_CHECK_LAUNCH(ctx);
@@ -734,43 +814,68 @@ cg_status flow_walk_dev(cg_ctx* ctx, int W, int H, long long* d_key, double* d_f
 }
 
 cg_status order_from_keys_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const long long* d_key,
-                              int land_cells, int32_t* d_order, int levels) {
+                              int land_cells, int32_t* d_order, int levels, const int* d_cells) {
     size_t N = (size_t)W * H;
     cudaStream_t sm = ctx->stream;
     int grid = ctx->num_sms * 8;
     if (land_cells <= 0) return CG_OK;
-    CG_BUF(int, d_flag, ctx, S_SCRATCH0, N);
-    CG_BUF(int, d_pos, ctx, S_SCRATCH1, N);
     const int n = land_cells;
     const int tile = std::min(kRsTile, std::max(1, n / (2 * ctx->num_sms * 256)) * 256);
     const int tiles = (n + tile - 1) / tile;
     CG_BUF(unsigned long long, d_keys, ctx, S_RS_KEYS, 2 * (size_t)n + 1);
     CG_BUF(int, d_vals, ctx, S_RS_VALS, 2 * (size_t)n);
-    CG_BUF(int, d_hist, ctx, S_RS_HIST, 2 * (size_t)tiles * 256);
+    CG_BUF(int, d_hist, ctx, S_RS_HIST, 2 * (size_t)tiles * 256 + 256);
     unsigned long long* kmax = d_keys + 2 * (size_t)n;
     unsigned long long* ka = d_keys;
     unsigned long long* kb = d_keys + n;
     int* va = d_vals;
     int* vb = d_vals + n;
     int* d_off = d_hist + (size_t)tiles * 256;
-    CG_LAUNCH(ctx) k_land_flags<<<grid, 256, 0, sm>>>(d_land, N, d_flag);
-    CG_CHECK_LAUNCH(ctx);
-    cg_status st = exclusive_scan(ctx, d_flag, d_pos, (int)N, nullptr);
-    if (st != CG_OK) return st;
     // The largest compact key: from the levels where the caller knows them (its bits, at any rate).
     unsigned long long hmax = levels > 0 ? (unsigned long long)levels * N - 1 : 0;
-    if (levels <= 0) CG_CUDA(ctx, cudaMemsetAsync(kmax, 0, sizeof(unsigned long long), sm));
-    CG_LAUNCH(ctx) k_land_compact_ck<<<grid, 256, 0, sm>>>(d_land, d_pos, d_key, N, ka, va, levels > 0 ? nullptr : kmax);
-    CG_CHECK_LAUNCH(ctx);
-    if (levels <= 0) {
-        CG_TRY_ST(read_back(ctx, {{&hmax, kmax, sizeof(hmax)}}));
+    if (d_cells && levels > 0) {
+        CG_LAUNCH(ctx) k_list_ck<<<std::min(grid, (n + 255) / 256), 256, 0, sm>>>(d_cells, n, d_key, N, ka, va);
+        CG_CHECK_LAUNCH(ctx);
+    } else {
+        CG_BUF(int, d_flag, ctx, S_SCRATCH0, N);
+        CG_BUF(int, d_pos, ctx, S_SCRATCH1, N);
+        CG_LAUNCH(ctx) k_land_flags<<<grid, 256, 0, sm>>>(d_land, N, d_flag);
+        CG_CHECK_LAUNCH(ctx);
+        cg_status st = exclusive_scan(ctx, d_flag, d_pos, (int)N, nullptr);
+        if (st != CG_OK) return st;
+        if (levels <= 0) CG_CUDA(ctx, cudaMemsetAsync(kmax, 0, sizeof(unsigned long long), sm));
+        CG_LAUNCH(ctx) k_land_compact_ck<<<grid, 256, 0, sm>>>(d_land, d_pos, d_key, N, ka, va, levels > 0 ? nullptr : kmax);
+        CG_CHECK_LAUNCH(ctx);
+        if (levels <= 0) CG_TRY_ST(read_back(ctx, {{&hmax, kmax, sizeof(hmax)}}));
     }
     int bits = 0;
     while (bits < 64 && (hmax >> bits) != 0) ++bits;
+    if (bits > 0 && n <= ctx->num_sms * kRsOneLaunch) {
+        RsArgs a;
+        a.keys[0] = ka;
+        a.keys[1] = kb;
+        a.vals[0] = va;
+        a.vals[1] = vb;
+        a.n = n;
+        a.tile = std::max(1, (n + ctx->num_sms * 256 - 1) / (ctx->num_sms * 256)) * 256;
+        a.tiles = (n + a.tile - 1) / a.tile;   // no more than the SMs, and than `tiles`
+        a.bits = bits;
+        a.hist = d_hist;
+        a.before = d_off;
+        a.total = d_off + (size_t)tiles * 256;
+        a.out = d_order;
+        int per_sm = 0;
+        CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rs_sort, 256, 0));
+        if (per_sm < 1) return fail(ctx, CG_CUDA, "the order's sort cannot be resident");
+        void* kargs[] = {&a};
+        ctx->launches++;
+        CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_rs_sort, a.tiles, 256, kargs, 0, sm));
+        return CG_OK;
+    }
     for (int shift = 0; shift < bits; shift += 8) {
         CG_LAUNCH(ctx) k_rs_hist<<<tiles, 256, 0, sm>>>(ka, n, shift, tile, tiles, d_hist);
         CG_CHECK_LAUNCH(ctx);
-        st = exclusive_scan(ctx, d_hist, d_off, tiles * 256, nullptr);
+        cg_status st = exclusive_scan(ctx, d_hist, d_off, tiles * 256, nullptr);
         if (st != CG_OK) return st;
         CG_LAUNCH(ctx) k_rs_scatter<<<tiles, 256, 0, sm>>>(ka, va, n, shift, tile, tiles, d_off, kb, vb);
         CG_CHECK_LAUNCH(ctx);
