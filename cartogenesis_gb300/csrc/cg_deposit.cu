@@ -58,6 +58,7 @@ using namespace dep;
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kSlots = 2048;         // mouths a chunk holds
 constexpr int kAdmitThreads = 512;   // k_admit_lakes's threads an SM
 constexpr int kPoolShare = 64;       // pool entries a lake fan is first given
 constexpr int kTile = 16;   // a sea lobe's box is scheduled in tiles of kTile x kTile cells
@@ -66,11 +67,10 @@ constexpr long long kSpinLimit = 1LL << 24;   // a lake fan's wait for its turn,
 
 // Control words of a walk.
 enum {
-    W_ERROR = 1, W_GEN = 3, W_ABORT = 4, W_REPLAYED = 5, W_WAVES = 7, W_REFITTED = 10, W_RELAID = 13, W_PAIRS = 14,
+    W_ERROR = 1, W_GEN = 3, W_ABORT = 4, W_REPLAYED = 5, W_WAVES = 7, W_REFITTED = 10, W_RELAID = 13, W_GROUPED = 14,
     W_DISTINCT = 15,
     W_CHECK_SITE = 16, W_CHECK_VALUE = 17, W_CHECK_BOUND = 18, W_NDONOR = 19,
-    W_REFITGEN = 20, W_CLASHES = 21, W_TOUCHN = 22, W_NREPLAY = 23, W_NREFIT = 24, W_FGEN = 25, W_NLAKE = 26,
-    W_NSEA = 27, W_INSERT = 28, W_WORDS = 32
+    W_REFITGEN = 20, W_CLASHES = 21, W_TOUCHN = 22, W_NREPLAY = 23, W_NREFIT = 24, W_FGEN = 25, W_INSERT = 28, W_WORDS = 32
 };
 
 struct WalkDev {
@@ -90,7 +90,6 @@ struct WalkDev {
     int8_t* ev_kind;        // per rank: SEA or LAKE
     int* seg_events;        // per rank: listed ranks, compacted within each CTA's segment
     int* seg_count;         // per CTA, twice (the levels alternate)
-    int* seg_part;          // per CTA: a grid-wide scan's slice sums
     int* events;            // the level's listed ranks, dense, in rank order
     // The round's lake fans, admitted before the walk (k_admit_lakes): per candidate mouth cell its
     // admitted cells sorted by distance and each one's level less its terrain, in a pool.
@@ -113,7 +112,6 @@ struct WalkDev {
     // A chunk's laying schedule: each (fan, admitted cell) pair, grouped by cell, knows the fan that
     // follows it on that cell in rank order; a fan lays once every fan before it on its cells has.
     int pair_cap;
-    int* poff;              // per slot + 1: its first pair
     int* pair_fan;          // per pair: its slot
     int* pair_cell;
     int* pair_pos;          // per pair: its place in its cell's group (arrival order)
@@ -350,28 +348,6 @@ __device__ void cta_exclusive_scan(Get get, int n, int* out, int* sh) {
     const int total = cta_scan_range(get, 0, n, 0, out, sh);
     if (threadIdx.x == 0) out[n] = total;
     __syncthreads();
-}
-
-// An exclusive prefix sum over the whole grid, called by every thread: each CTA sums a slice, then adds
-// the slices before its own and scans its slice from there; out[n] receives the total. For long arrays,
-// where one CTA stepping through them would hold the grid. `part` holds gridDim.x ints.
-template <class Get>
-__device__ void grid_exclusive_scan(Get get, int n, int* out, int* part, int* sh) {
-    cgr::grid_group grid = cgr::this_grid();
-    const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int lo = min(n, (int)blockIdx.x * per), hi = min(n, lo + per);
-    int sum = 0;
-    for (int i = lo + (int)threadIdx.x; i < hi; i += kThreads) sum += get(i);
-    int total;
-    cta_prefix(sum, &total, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = total;
-    grid.sync();
-    int before = 0;
-    for (int i = (int)threadIdx.x; i < (int)blockIdx.x; i += kThreads) before += __ldcg(&part[i]);
-    int carry;
-    cta_prefix(before, &carry, sh);
-    const int end = cta_scan_range(get, lo, hi, carry, out, sh);
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = end;
 }
 
 // An index check of the laying schedule: v must lie in [0, hi). A failure records its site, value and
@@ -1015,6 +991,7 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
     const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), stride = (int)(gridDim.x * blockDim.x);
     const int gwarp = tid >> 5, nwarps = stride >> 5;
     const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
+    __shared__ int sh_poff[kSlots + 1];   // a chunk's slots' first pairs, then their first entries of its log
     extern __shared__ unsigned long long lobe_smem[];   // a Lobe per warp, where the grid's lobes fit one
     Lobe lobe{nullptr, nullptr, nullptr};
     if (w.lobe_words > 0) {
@@ -1167,6 +1144,10 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                     w.slot_touch_n[e - e0] = 0;
                     w.blockers[e - e0] = 0;
                 }
+                if (tid == 0) {
+                    w.words[W_DISTINCT] = 0;
+                    w.words[W_GROUPED] = 0;
+                }
                 grid.sync();
                 // The lake fans lay in waves, a warp each, in rank order wherever they share a cell: the
                 // chunk's (fan, cell) pairs are grouped by cell, each pair learning whether an earlier
@@ -1175,35 +1156,23 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                 // layings touch different cells). Bounded: the lowest waiting rank is never blocked, so
                 // every wave lays at least one fan.
                 const int S = e1 - e0;
-                if (blockIdx.x == 0) {
-                    const int* st = w.slot_state;
-                    const int* sn = w.slot_n;
-                    cta_exclusive_scan([=](int i) { return st[i] ? sn[i] : 0; }, S, w.poff, sh_scan);
-                    int lakes = 0, seas = 0;
-                    for (int base = 0; base < S; base += kThreads) {
-                        const int i = base + (int)threadIdx.x;
-                        lakes += __syncthreads_count(i < S && st[i] == 1);
-                        seas += __syncthreads_count(i < S && st[i] == 2);
-                    }
-                    if (threadIdx.x == 0) {
-                        w.words[W_PAIRS] = w.poff[S];
-                        w.words[W_DISTINCT] = 0;
-                        w.words[W_NLAKE] = lakes;
-                        w.words[W_NSEA] = seas;
-                        if (w.poff[S] > w.pair_cap) w.words[W_ERROR] |= 16;
-                    }
+                // Every CTA works out the slots' first pairs for itself: a scan in shared memory against one CTA's
+                // and a grid barrier, and a pair's search for its slot takes no loads.
+                {
+                    const int *st = w.slot_state, *sn = w.slot_n;
+                    cta_exclusive_scan([=](int i) { return __ldcg(&st[i]) ? __ldcg(&sn[i]) : 0; }, S, sh_poff, sh_scan);
                 }
-                grid.sync();
-                const int P = min(*(volatile int*)&w.words[W_PAIRS], w.pair_cap);
+                if (timer && sh_poff[S] > w.pair_cap) w.words[W_ERROR] |= 16;
+                const int P = min(sh_poff[S], w.pair_cap);
                 for (int q = tid; q < P; q += stride) {
                     int a = 0, b = S;   // the slot whose pairs hold q: poff[a] <= q < poff[a + 1]
                     while (b - a > 1) {
                         const int m = (a + b) >> 1;
-                        if (w.poff[m] <= q) a = m;
+                        if (sh_poff[m] <= q) a = m;
                         else b = m;
                     }
                     int x = 0;
-                    const int k = q - w.poff[a];
+                    const int k = q - sh_poff[a];
                     if (index_ok(w, k, w.slot_n[a], 12)) {
                         if (w.slot_state[a] == 2) {   // a sea lobe's tile
                             const int* box = w.slot_box + 4 * a;
@@ -1227,19 +1196,24 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                     }
                 }
                 grid.sync();
+                // Each distinct cell's group takes the next pairs' places, in whatever order.
                 const int D = *(volatile int*)&w.words[W_DISTINCT];
-                {
-                    const int* cnt = w.cell_cnt;
-                    const int* dc = w.dcell;
-                    if (D > 4 * kThreads) {   // long: over the grid
-                        grid_exclusive_scan([=](int i) { return __ldcg(&cnt[dc[i]]); }, D, w.doff, w.seg_part, sh_scan);
-                    } else if (blockIdx.x == 0) {
-                        cta_exclusive_scan([=](int i) { return __ldcg(&cnt[dc[i]]); }, D, w.doff, sh_scan);
+                for (int d0 = tid - lane; d0 < D; d0 += stride) {
+                    const int d = d0 + lane;
+                    const int cnt = d < D ? __ldcg(&w.cell_cnt[w.dcell[d]]) : 0;
+                    int incl = cnt;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                        if (lane >= o) incl += y;
                     }
+                    int first = 0;
+                    if (lane == 31) first = atomicAdd(&w.words[W_GROUPED], incl);
+                    first = __shfl_sync(0xFFFFFFFFu, first, 31);
+                    if (d < D) w.doff[d] = first + incl - cnt;
                 }
                 grid.sync();
                 // Every pair is counted on exactly one distinct cell.
-                if (blockIdx.x == 0 && threadIdx.x == 0 && __ldcg(&w.doff[D]) != P) check_failed(w, w.doff[D], P, 13);
+                if (timer && __ldcg(&w.words[W_GROUPED]) != P) check_failed(w, w.words[W_GROUPED], P, 13);
                 for (int q = tid; q < P; q += stride) {
                     const int d = w.cell_d[w.pair_cell[q]];
                     if (!index_ok(w, d, D, 5)) continue;
@@ -1279,7 +1253,6 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                     tm[T_SCHEDULE] += t - t0;
                     t0 = t;
                 }
-                const int n_lakes = *(volatile int*)&w.words[W_NLAKE], n_seas = *(volatile int*)&w.words[W_NSEA];
                 // A fan's warp waits for its count to reach 0 (the fans before it on its cells laid), inside
                 // the cooperative launch: every CTA is resident, each warp takes its slots in rank order and
                 // a count only waits on lower ranks, so the lowest waiting fan always runs. The wait is
@@ -1287,7 +1260,7 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                 // heeds, and the walk reports the error.
                 // A lake fan touches only ponded land and a sea lobe only sea cells, so the two kinds wait
                 // only on their own (their schedule ids are cells and tiles, apart) and lay in one pass.
-                if (n_lakes + n_seas > 0) {
+                if (P > 0) {   // a mouth's cells or tiles hold its apex, at least
                     for (int sl = gwarp; sl < S; sl += nwarps) {
                         const int kind_slot = w.slot_state[sl];
                         if (kind_slot != 1 && kind_slot != 2) continue;
@@ -1295,7 +1268,7 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                         const int rank = w.events[e0 + sl];
                         const int c = w.order[rank];
                         const double carried = w.ev_carried[rank];
-                        const int q0 = w.poff[sl], q1 = min(w.poff[sl + 1], P);   // P: past an overflow
+                        const int q0 = sh_poff[sl], q1 = min(sh_poff[sl + 1], P);   // P: past an overflow
                         const int succ0 = q0 + lane < q1 ? w.pair_succ[q0 + lane] : -1;
                         LakeFan fan{};
                         double budget = 0.0;
@@ -1365,26 +1338,25 @@ __global__ void __launch_bounds__(kThreads) k_deposit_levels(WalkDev w) {
                 }
                 // The chunk's deposits into the level's log in rank order: each event's entries at the
                 // offset of the events before it. A deposit that makes a mouth conflict lists it.
-                if (blockIdx.x == 0) {
-                    const int* tn = w.slot_touch_n;
-                    cta_exclusive_scan([=](int i) { return __ldcg(&tn[i]); }, S, w.poff, sh_scan);
-                    if (threadIdx.x == 0) w.words[W_WAVES] += waves;
-                }
-                grid.sync();
+                if (timer) w.words[W_WAVES] += waves;
                 {
-                    const int total = __ldcg(&w.poff[S]);
+                    const int* tn = w.slot_touch_n;
+                    cta_exclusive_scan([=](int i) { return __ldcg(&tn[i]); }, S, sh_poff, sh_scan);
+                }
+                {
+                    const int total = sh_poff[S];
                     const int room = w.touch_cap - touch_n;
                     const int copied = total < room ? total : room;
                     if (total > room && timer) w.words[W_ERROR] |= 1;
-                    for (int e = tid; e < S; e += stride) w.ev_touch[e0 + e] = touch_n + min(__ldcg(&w.poff[e]), copied);
+                    for (int e = tid; e < S; e += stride) w.ev_touch[e0 + e] = touch_n + min(sh_poff[e], copied);
                     for (int q = tid; q < copied; q += stride) {
                         int a = 0, b = S;
                         while (b - a > 1) {
                             const int m = (a + b) >> 1;
-                            if (__ldcg(&w.poff[m]) <= q) a = m;
+                            if (sh_poff[m] <= q) a = m;
                             else b = m;
                         }
-                        const Touch t = w.slot_touch[(size_t)a * w.cap + (q - __ldcg(&w.poff[a]))];
+                        const Touch t = w.slot_touch[(size_t)a * w.cap + (q - sh_poff[a])];
                         w.touches[touch_n + q] = t;
                         w.touch_ev[touch_n + q] = e0 + a;
                         find_conflict(w, L, t.cell, w.events[e0 + a], clash_gen);
@@ -1606,7 +1578,7 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     // chunks' mouth slots.
     w.cap = heap_capacity(w.p);
     w.box_words = box_words(w.p);
-    w.slots = 2048;
+    w.slots = kSlots;
     const size_t S = (size_t)w.slots, cap = (size_t)w.cap;
     CG_BUF(int, d_candof, ctx, S_DEPCANDOF, N);
     CG_BUF(int, d_cand, ctx, S_DEPCAND, (size_t)n + 2);
@@ -1683,17 +1655,16 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     CG_BUF(int, d_stn, ctx, S_DEPSLOT10, S);
     w.pair_cap = (int)std::min<size_t>(S * cap, (size_t)1 << 30);
     const size_t PC = (size_t)w.pair_cap;
-    // poff (S + 1), blockers (S + 1), then seven arrays of PC: pair_fan, pair_cell, pair_pos,
-    // pair_succ, group, dcell, and doff (its D + 1 <= PC + 1 entries run into the spare 2).
-    CG_BUF(int, d_sched, ctx, S_DEPCLAIM, 7 * PC + 2 * S + 4);
+    // blockers (S + 1), then seven arrays of PC: pair_fan, pair_cell, pair_pos, pair_succ, group, dcell
+    // and doff.
+    CG_BUF(int, d_sched, ctx, S_DEPCLAIM, 7 * PC + S + 1);
     const size_t ids = schedule_ids(W, H);
     CG_BUF(int, d_cellcnt, ctx, S_DEPCELLCNT, 2 * ids);
     w.tiles_x = (W + kTile - 1) / kTile;
     w.tiles_y = (H + kTile - 1) / kTile;
     w.box_x = box_bx(w.p);
     w.box_y = box_by(w.p);
-    w.poff = d_sched;
-    w.blockers = d_sched + S + 1;
+    w.blockers = d_sched;
     w.pair_fan = w.blockers + S + 1;
     w.pair_cell = w.pair_fan + PC;
     w.pair_pos = w.pair_cell + PC;
@@ -1746,10 +1717,12 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     int per_sm = 0;
     CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_deposit_levels, kThreads, smem));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "deposition kernel cannot be resident");
-    const int cgrid = ctx->num_sms * (per_sm < 2 ? per_sm : 2);
-    CG_BUF(int, d_segc, ctx, S_DEPSEGC, 3 * (size_t)cgrid);
+    // Two CTAs an SM on large grids, whose levels have the mouths for them; on smaller ones a grid barrier over
+    // half as many CTAs, of which a level takes a dozen, is worth more: a round's walk took 2.10 and 1.95 ms at
+    // 1024 x 512, 4.6 and 4.4 at 2048 x 1024, but 47.2 and 48.0 at 8192 x 4096.
+    const int cgrid = ctx->num_sms * (per_sm < 2 || N <= (size_t)1 << 23 ? 1 : 2);
+    CG_BUF(int, d_segc, ctx, S_DEPSEGC, 2 * (size_t)cgrid);
     w.seg_count = d_segc;
-    w.seg_part = d_segc + 2 * (size_t)cgrid;
     // A heap per warp, for the sea lobes.
     w.heap_warps = cgrid * (kThreads / 32);
     const size_t HC = (size_t)w.heap_warps * cap;
