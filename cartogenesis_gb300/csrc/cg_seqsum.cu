@@ -47,12 +47,12 @@ struct SumJobs {
 };
 
 // A block told apart (cta_classify) after the sum the blocks before it are estimated at: how many values are
-// listed (-1: it was not), the binade of the first run of steps, the steps of all its runs, and the pieces of
-// 1024 that hold a listed value; and a listed value, the steps of the block before it and the binade of the
+// listed (-1: it was not), the binade of the first run of steps, the steps of all its runs, what its first run
+// takes more from an odd sum, and the pieces of 1024 that hold a listed value; and a listed value, the steps of the block before it and the binade of the
 // run after it.
 struct BlockSteps {
     long long steps;
-    int spec, listed;
+    int spec, listed, odd;
     unsigned pieces;
 };
 constexpr int kListed = kMostAlone;   // a block's listed values, at most; a block with more is taken by hand
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_walks(SumJobs<T> jobs, const 
     __syncthreads();
     const int len = (int)(in.n - base < (size_t)kSSBlock ? in.n - base : (size_t)kSSBlock);
     long long steps;
-    int listed = cta_classify<false>(in, base, 0, len, start.x, start.y, sh, 0.0, &steps);
+    int listed = cta_classify<false>(in, base, 0, len, start.x, start.y, kParityStart, sh, 0.0, &steps);
     if (listed > kListed) listed = -1;
     const int block = in.first_block + blockIdx.x;
     for (int k = threadIdx.x; k < listed; k += kSSThreads)
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_walks(SumJobs<T> jobs, const 
     if (threadIdx.x == 0) {
         unsigned pieces = 0;
         for (int k = 0; k < listed; ++k) pieces |= 1u << (sh.at[k] / kSSThreads);
-        blocks[block] = BlockSteps{steps, sh.spec[0], listed, pieces};
+        blocks[block] = BlockSteps{steps, sh.spec[0], listed, sh.odd, pieces};
     }
 }
 
@@ -245,32 +245,36 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_chain(SumJobs<T> jobs, const 
             bool by_hand = false;
             while (j < blocks && !by_hand) {
                 const int here = min(32, blocks - j);
-                BlockSteps w{0, -1, 0, 0};
+                BlockSteps w{0, -1, 0, 0, 0};
                 if (lane < here) w = heads[in.first_block + j + lane];
                 int i = 0;
                 while (i < here && !by_hand) {
                     // The blocks from i without a listed value, in the binade the sum is in.
                     const Binade b = binade_of(s);
                     const bool plain = w.listed == 0 && (w.spec < 0 ? w.steps == 0 : b.normal && w.spec == (b.ef | (b.neg << 11)));
-                    long long x = lane >= i ? w.steps : 0;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const long long y = __shfl_up_sync(FULL, x, o);
-                        if (lane >= o) x = wrap_add(x, y);
+                    Run run = run_identity();
+                    if (lane >= i && plain) {
+                        run.step[0] = w.steps;
+                        run.step[1] = w.steps + w.odd;
+                        run.out = (unsigned)(run.step[0] & 1) | ((unsigned)(1 + run.step[1]) & 1u) << 1;
                     }
-                    const bool ok = plain && (w.steps == 0 || inside(wrap_add(b.m, x)));
+                    const bool odd = __any_sync(FULL, plain && w.odd != 0);
+                    const Run incl = warp_scan(run, odd);
+                    const long long x = odd && (b.m & 1) ? incl.step[1] : incl.step[0];
+                    const bool ok = plain && (w.spec < 0 || inside(wrap_add(b.m, x)));
                     const unsigned stop = __ballot_sync(FULL, !ok || lane >= here) & ~((1u << i) - 1u);
                     const int end = stop ? __ffs(stop) - 1 : 32;
                     if (end > i) {
                         const long long steps = __shfl_sync(FULL, x, end - 1);
-                        if (steps != 0) s = sum_of(b, wrap_add(b.m, steps));
+                        if (b.normal) s = sum_of(b, wrap_add(b.m, steps));
                         whole += end - i;
                         i = end;
                         continue;
                     }
                     // Block i alone.
                     const int listed = __shfl_sync(FULL, w.listed, i);
-                    const long long all = __shfl_sync(FULL, w.steps, i);
+                    long long all = __shfl_sync(FULL, w.steps, i);
+                    const int more = b.normal && (b.m & 1) ? __shfl_sync(FULL, w.odd, i) : 0;
                     int spec = __shfl_sync(FULL, w.spec, i);
                     const unsigned pieces = __shfl_sync(FULL, w.pieces, i);
                     by_hand = listed <= 0;
@@ -282,7 +286,7 @@ __global__ void __launch_bounds__(kSSThreads) k_ss_chain(SumJobs<T> jobs, const 
                     bool sound = true;
                     for (int k = 0; k < listed; ++k) {
                         const Listed e = list[k];
-                        sound &= take_steps(t, wrap_add(e.steps, -done), spec);
+                        sound &= take_steps(t, wrap_add(e.steps, (k == 0 ? more : 0) - done), spec);
                         t = __dadd_rn(t, e.value);
                         done = e.steps;
                         spec = e.spec;

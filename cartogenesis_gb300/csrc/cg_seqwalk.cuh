@@ -232,6 +232,7 @@ struct CtaSum {
     long long steps[kMostAlone + 1];
     double values[kMostAlone];
     int at[kMostAlone], spec[kMostAlone + 1];
+    int odd;         // cta_classify: steps more from an odd start
     long long totals[kSSThreads / 32];
     int counts[kSSThreads / 32];
 };
@@ -456,19 +457,38 @@ __device__ __forceinline__ long long cta_before(long long v, long long* before, 
     return __shfl_sync(0xFFFFFFFFu, w, 31);
 }
 
+// What is known of the parity of a sum's m: even, odd, that of the sum the block starts from or the other
+// one, or nothing; and what a run of values makes of it, a parity or (kParityKeep, + 1: the other one) a
+// change of it. A tie leaves m even, whatever it was.
+using Parity = int;
+constexpr Parity kParityEven = 0, kParityStart = 2, kParityUnknown = 4, kParityKeep = 8;
+__device__ __forceinline__ Parity parity_then(Parity a, Parity b) {
+    if (b < kParityKeep) return b;
+    return a == kParityUnknown ? a : a ^ (b & 1);   // of a change: the changes add up
+}
+// A tie's step from a sum of parity `state` (of an even start), and how much more it is from an odd start.
+__device__ __forceinline__ long long tie_value(const Step& st, Parity state) { return st.r + (((state & 1) + st.r) & 1); }
+__device__ __forceinline__ bool tie_step(const Step& st, Parity state, long long* odd) {
+    *odd = (state & 2) ? tie_value(st, state ^ 1) - tie_value(st, state) : 0;
+    return state != kParityUnknown;
+}
+
 // The block's values [pos, len) after a sum of about `start`, crossings and all, told apart: the values to be
 // taken alone are listed in sh (steps, values, at, spec), and the steps of all others summed. The partial
 // sums are first taken in fixed point, in units of 2^-60 of what they can reach, by one integer scan: they
 // are off from the rounded sums by less than 2^20 units (a unit a value, and the rounded sums' own
 // roundings, 2^6 units each) and what `start` is off (`start_off`), which tells each partial sum's binade
 // but next to a power of two. A value whose sums before and after are surely in one binade is a step of that
-// binade, whatever the parity unless it is a tie; every other value is listed. The steps between two listed
-// values are a difference of a second scan. Returns how many values are listed, or -1 where that does not
+// binade, whatever the parity unless it is a tie; a tie's step follows from the parity, which is known from
+// the tie before it on (a scan of the parities, where there are ties), is `entry`'s at the block's start, and
+// is not known after a crossing. Every other value is listed. The steps are taken for a block that starts
+// even; sh.odd is what one that starts odd takes more, before the first listed value. The steps between two
+// listed values are a difference of a second scan. Returns how many values are listed, or -1 where that does not
 // apply: a sum or value that is not finite, or too many values; *all_steps receives the steps of the rest.
 // Every thread calls it, and what it wrote to sh is visible after it.
 template <bool STOP, typename T>
-__device__ int cta_classify(const SumIn<T>& in, size_t base, int pos, int len, double start, double start_off, CtaSum& sh,
-                            double stop, long long* all_steps) {
+__device__ int cta_classify(const SumIn<T>& in, size_t base, int pos, int len, double start, double start_off, Parity entry,
+                            CtaSum& sh, double stop, long long* all_steps) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int at0 = (int)threadIdx.x * kSSPer;
@@ -483,6 +503,7 @@ __device__ int cta_classify(const SumIn<T>& in, size_t base, int pos, int len, d
     top = __reduce_max_sync(FULL, top);
     if (lane == 0) sh.counts[warp] = top;
     for (int k = threadIdx.x; k <= kMostAlone; k += kSSThreads) sh.spec[k] = -1;
+    if (threadIdx.x == 0) sh.odd = 0;
     __syncthreads();
     top = __reduce_max_sync(FULL, sh.counts[lane]);
     *all_steps = 0;
@@ -516,47 +537,87 @@ __device__ int cta_classify(const SumIn<T>& in, size_t base, int pos, int len, d
         return ef >= 1 && ef <= 2046 ? ef | (p < 0 ? 1 << 11 : 0) : -1;
     };
     auto near_stop = [=](long long was, long long p) { return STOP && p >= stop_units - 2 * off && was <= stop_units + 2 * off; };
-    long long steps = 0;
-    unsigned single = 0;
-    int spec[2] = {-1, -1};   // the binades of this thread's first steps, and of those after its last listed value
     const int first = binade_at(p0);
-    if (first >= 0 && binade_at(p0 - span) == first && binade_at(p0 + span) == first && !near_stop(p0 - span, p0 + span)) {
-        // All of the thread's sums are surely in one binade (nearly every thread's are).
-#pragma unroll
-        for (int t = 0; t < kSSPer; ++t) {
-            if (!((has >> t) & 1u)) continue;
-            const Step st = step_of(v[t], first & 0x7FF, first >> 11);
-            if (st.tie || !plain_step(st)) single |= 1u << t;
-            else steps = wrap_add(steps, st.r);
-        }
-        if (has & ~single) spec[0] = first;
-        if (single) spec[1] = spec[0];
-    } else if (has) {
+    // All of the thread's sums are surely in one binade (nearly every thread's are).
+    const bool quiet = first >= 0 && binade_at(p0 - span) == first && binade_at(p0 + span) == first &&
+                       !near_stop(p0 - span, p0 + span);
+    // The thread's values in order: whether one is to be taken alone, else its step and binade.
+    auto each = [&](auto&& take) {
         long long p = p0;
         int code = first;
 #pragma unroll
         for (int t = 0; t < kSSPer; ++t) {
             if (!((has >> t) & 1u)) continue;
-            const long long was = p;
-            p += units_of(magnitude_of(v[t]), unit);
-            const int next = binade_at(p);
-            bool alone = code < 0 || next != code || near_stop(was, p);
+            int next = code;
+            bool alone = false;
+            if (!quiet) {
+                const long long was = p;
+                p += units_of(magnitude_of(v[t]), unit);
+                next = binade_at(p);
+                alone = code < 0 || next != code || near_stop(was, p);
+            }
+            Step st{0, 0, 0};
             if (!alone) {
-                const Step st = step_of(v[t], code & 0x7FF, code >> 11);
-                alone = st.tie || !plain_step(st);
-                if (!alone) {
-                    steps = wrap_add(steps, st.r);
-                    spec[single ? 1 : 0] = code;
-                }
+                st = step_of(v[t], code & 0x7FF, code >> 11);
+                alone = !plain_step(st);
             }
-            if (alone) {
-                single |= 1u << t;
-                spec[1] = -1;
-            }
+            take(t, alone, st, code);
             code = next;
         }
+    };
+    long long steps = 0;
+    unsigned single = 0;
+    int spec[2] = {-1, -1};   // the binades of this thread's first steps, and of those after its last listed value
+    auto note = [&](int t, bool alone, long long step, int code) {
+        if (alone) {
+            single |= 1u << t;
+            spec[1] = -1;
+        } else {
+            steps = wrap_add(steps, step);
+            spec[single ? 1 : 0] = code;
+        }
+    };
+    bool tie = false;
+    Parity moves = kParityKeep;
+    each([&](int t, bool alone, const Step& st, int code) {
+        note(t, alone, st.r, code);
+        tie |= !alone && st.tie;
+        moves = parity_then(moves, alone ? kParityUnknown : st.tie ? kParityEven : kParityKeep + (int)(st.r & 1));
+    });
+    Parity enters = entry;
+    const bool ties = __syncthreads_or(tie);   // and sh.totals and sh.counts are read
+    if (ties) {
+        Parity x = moves;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const Parity y = __shfl_up_sync(FULL, x, o);
+            if (lane >= o) x = parity_then(y, x);
+        }
+        if (lane == 31) sh.counts[warp] = x;
+        __syncthreads();
+        Parity w = sh.counts[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const Parity y = __shfl_up_sync(FULL, w, o);
+            if (lane >= o) w = parity_then(y, w);
+        }
+        w = __shfl_sync(FULL, w, warp > 0 ? warp - 1 : 0);
+        x = __shfl_up_sync(FULL, x, 1);
+        if (warp > 0) enters = parity_then(enters, w);
+        if (lane > 0) enters = parity_then(enters, x);
+        steps = 0;
+        single = 0;
+        spec[0] = spec[1] = -1;
+        Parity state = enters;
+        each([&](int t, bool alone, const Step& st, int code) {
+            long long odd;
+            const bool unknown = !alone && st.tie && !tie_step(st, state, &odd);
+            if (!alone && st.tie && !unknown && odd != 0) sh.odd = (int)odd;
+            note(t, alone || unknown, st.tie && !unknown ? tie_value(st, state) : st.r, code);
+            state = parity_then(state, alone ? kParityUnknown : st.tie ? kParityEven : kParityKeep + (int)(st.r & 1));
+        });
+        __syncthreads();   // sh.counts is read
     }
-    __syncthreads();   // sh.totals and sh.counts are read
     long long steps_before;
     *all_steps = cta_before(steps, &steps_before, sh.totals);
     int mine = __popc(single), slot = mine;
@@ -573,22 +634,18 @@ __device__ int cta_classify(const SumIn<T>& in, size_t base, int pos, int len, d
     if (spec[0] >= 0) sh.spec[slot] = spec[0];
     if (spec[1] >= 0) sh.spec[slot + mine] = spec[1];
     if (single) {   // the thread's values again, for the steps between its listed ones
-        long long p = p0;
-        int code = first;
-#pragma unroll
-        for (int t = 0; t < kSSPer; ++t) {
-            if (!((has >> t) & 1u)) continue;
-            p += units_of(magnitude_of(v[t]), unit);
+        Parity state = enters;
+        each([&](int t, bool alone, const Step& st, int) {
             if ((single >> t) & 1u) {
                 sh.steps[slot] = steps_before;
                 sh.values[slot] = (double)v[t];
                 sh.at[slot] = at0 + t;
                 ++slot;
             } else {
-                steps_before = wrap_add(steps_before, step_of(v[t], code & 0x7FF, code >> 11).r);
+                steps_before = wrap_add(steps_before, st.tie ? tie_value(st, state) : st.r);
             }
-            code = binade_at(p);
-        }
+            state = parity_then(state, alone ? kParityUnknown : st.tie ? kParityEven : kParityKeep + (int)(st.r & 1));
+        });
     }
     __syncthreads();
     return listed;
@@ -603,7 +660,9 @@ template <bool STOP, typename T>
 __device__ bool cta_segments(const SumIn<T>& in, size_t base, int pos, int len, CtaSum& sh, double stop) {
     const double s0 = sh.s;
     long long all_steps;
-    const int listed = cta_classify<STOP>(in, base, pos, len, s0, 0.0, sh, stop, &all_steps);
+    const Binade b0 = binade_of(s0);
+    const int listed = cta_classify<STOP>(in, base, pos, len, s0, 0.0, b0.normal ? (Parity)(b0.m & 1) : kParityUnknown, sh,
+                                          stop, &all_steps);
     if (listed < 0) return false;
     if (threadIdx.x == 0) {
         double s = s0;
