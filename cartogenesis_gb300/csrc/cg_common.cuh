@@ -116,7 +116,7 @@ enum Slot {
     S_BT_FIRST, S_BT_RISE, S_BT_WEIGHTS, S_BT_FACTOR, S_BT_FILLED, S_BT_SURF, S_BT_RECV, S_BT_KEY,
     S_BT_DONORS, S_BT_AREA, S_BT_INFLOW, S_BT_ROUTING, S_BT_DISC, S_BT_FLUX, S_BT_CUTV, S_BT_GIVE,
     S_BT_NEXT, S_BT_ORDER, S_BT_XS, S_BT_REF, S_BT_UPLM, S_BT_RBM, S_BT_LOSS, S_BT_TMP, S_BT_TAPS,
-    S_BT_SMALL, S_BT_ERODED, S_BT_LEVELS, S_BT_CUT, S_INCFIXED, S_INCCOURANT, S_FLATCOUNT,
+    S_BT_SMALL, S_BT_ERODED, S_BT_LEVELS, S_BT_CUT, S_INCFIXED, S_INCCOURANT, S_FLATCOUNT, S_BRACKETW,
     S_COUNT
 };
 static_assert(S_COUNT <= (int)(sizeof(((cg_ctx*)nullptr)->bufs) / sizeof(DevBuf)), "a slot past the context's buffers");

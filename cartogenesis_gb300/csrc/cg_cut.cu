@@ -11,8 +11,8 @@
 //    (cg::warp_seq_sum, on the integer pipes); a row whose additions cross a binade or meet a tie is
 //    taken alone by cg::seq_repeat_add, which takes `count` equal additions in closed form
 //    (csrc/cg_fpemu.h);
-//  - the bracket: its cells are sorted on the device and walked in the reference's order by one
-//    warp with the same chunking.
+//  - the bins' walk and the bracket's, whose cells are sorted on the device: sequential sums by one CTA,
+//    inside binades as integer scans (cg_seqwalk.cuh).
 // min, max, the bin of a cell and the land/relative split are elementwise or exact reductions.
 #include <climits>
 #include <cmath>
@@ -304,171 +304,40 @@ __global__ void k_pad(long long* keys, int n, int P2) {
     for (int i = n + blockIdx.x * blockDim.x + threadIdx.x; i < P2; i += gridDim.x * blockDim.x) keys[i] = LLONG_MAX;
 }
 
-// SeaLevelStage.kt:636-644: walk the sorted bracket until the area below reaches the target.
-//
-// The walk's sum is sequential, but it rarely leaves its binade: then every entry adds a whole
-// number of units in the last place, d_i = rne(w_i / U), and the sums before the entries are an
-// integer prefix scan. One CTA takes the bracket CHUNK entries at a time: per entry d_i and whether
-// it is clean (no tie at half a unit, the step stays in the binade); a block scan of the d_i; the
-// answer is the first entry whose sum before it reaches the target, provided every earlier entry of
-// the chunk is clean. From the first entry that is not, warp 0 replays the rest of the chunk exactly
-// (32 entries at a time with cg::warp_seq_sum).
-constexpr int WALK_THREADS = 1024;
-constexpr int WALK_PER = 8;
-constexpr int WALK_CHUNK = WALK_THREADS * WALK_PER;
-
-// Warp 0's exact replay of entries [from, to) starting from `below`. Returns true with *cell the
-// answer's cell when the sum before an entry reaches the target; otherwise *below is the sum after
-// entry to - 1.
-__device__ bool walk_replay(const long long* __restrict__ keys, const double* __restrict__ w, int W, double target,
-                            int from, int to, double* below_io, int* cell_out) {
-    const unsigned FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    double below = *below_io;
-    for (int base = from; base < to; base += 32) {
-        const int i = base + lane;
-        const int cell = i < to ? (int)(keys[i] & 0xFFFFFFFFLL) : -1;
-        const double wi = i < to ? w[pdiv(cell, W)] : 0.0;
-        double before;
-        const double after = warp_seq_sum(below, wi, i < to ? 1 : 0, &before);
-        const unsigned hit = __ballot_sync(FULL, i < to && before >= target);
-        if (hit) {
-            *cell_out = __shfl_sync(FULL, cell, __ffs(hit) - 1);
-            return true;
-        }
-        below = after;
-    }
-    *below_io = below;
-    return false;
-}
-
-__global__ void __launch_bounds__(WALK_THREADS) k_bracket_walk(const float* __restrict__ h,
-                                                               const long long* __restrict__ keys,
-                                                               const double* __restrict__ w, int W, double target,
-                                                               int most, CutState* s) {
-    const int64_t TOP = (int64_t)1 << 53;
-    __shared__ long long s_warp[WALK_THREADS / 32];
-    __shared__ int s_hit, s_unclean, s_done;
-    __shared__ double s_below;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// SeaLevelStage.kt:636-644: walk the sorted bracket until the area below reaches the target: the answer is the
+// first cell whose sum before it does, so the one after the cell that brings the sum there. The sum is
+// sequential; the CTA takes it 8192 cells at a time, inside binades as integer scans (cg_seqwalk.cuh). Scans
+// with one warp replaying the rest of the chunk from the first crossing took 32 us at 2048 x 1024 and 455 at
+// 8192 x 4096, this 9 and 90.
+__global__ void __launch_bounds__(seqwalk::kSSThreads) k_bracket_walk(const float* __restrict__ h,
+                                                                      const long long* __restrict__ keys,
+                                                                      const double* __restrict__ w, int W, double target,
+                                                                      int most, CutState* s, double* __restrict__ weights) {
+    using namespace seqwalk;
+    __shared__ CtaSum sh;
     if (s->degenerate) return;
     const int n = s->count;
     if (n > most) return;   // its keys are not sorted yet
     if (n == 0) {
-        if (tid == 0) s->todays = s->highest;
+        if (threadIdx.x == 0) s->todays = s->highest;
         return;
     }
-    double below = s->below_bracket;
-    for (int base = 0; base < n; base += WALK_CHUNK) {
-        const int end = min(n, base + WALK_CHUNK);
-        if (tid == 0) {
-            s_hit = INT_MAX;
-            s_unclean = below > 0.0 ? INT_MAX : base;   // a zero sum has no binade: replay from the start
-        }
-        int e = 0;
-        double U = 1.0;
-        int64_t m = 0;
-        if (below > 0.0) {
-            e = ilogb(below);
-            U = ldexp(1.0, e - 52);
-            m = (int64_t)(below / U);
-        }
-        int64_t d[WALK_PER], q[WALK_PER];
-        bool clean[WALK_PER];
-        int64_t mine = 0;
-        const int first = base + tid * WALK_PER;
-#pragma unroll
-        for (int k = 0; k < WALK_PER; ++k) {
-            const int i = first + k;
-            d[k] = 0;
-            q[k] = 0;
-            clean[k] = true;
-            if (i < end) {
-                const int cell = (int)(keys[i] & 0xFFFFFFFFLL);
-                const double x = ldexp(w[pdiv(cell, W)], 52 - e);   // w / U, exact
-                if (!(x < 9.0e15)) {
-                    clean[k] = false;
-                } else {
-                    q[k] = (int64_t)x;
-                    const double f = x - (double)q[k];
-                    clean[k] = f != 0.5;
-                    d[k] = q[k] + (f > 0.5 ? 1 : 0);
-                }
-            }
-            mine += d[k];
-        }
-        // Exclusive block scan of the per-thread totals.
-        int64_t incl = mine;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            int64_t v = s_warp[lane], vi = v;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t t = __shfl_up_sync(0xFFFFFFFFu, vi, o);
-                if (lane >= o) vi += t;
-            }
-            s_warp[lane] = vi - v;   // exclusive over warps
-        }
-        __syncthreads();
-        int64_t run = m + s_warp[warp] + (incl - mine);   // the sum before this thread's first entry, in U
-        int hit = INT_MAX, unclean = INT_MAX;
-#pragma unroll
-        for (int k = 0; k < WALK_PER; ++k) {
-            const int i = first + k;
-            if (i >= end) break;
-            if (hit == INT_MAX && (double)run * U >= target) hit = i;
-            if (unclean == INT_MAX && (!clean[k] || run + q[k] > TOP - 1)) unclean = i;
-            run += d[k];
-        }
-        if (hit != INT_MAX) atomicMin(&s_hit, hit);
-        if (unclean != INT_MAX) atomicMin(&s_unclean, unclean);
-        __syncthreads();
-        const int h_at = s_hit, u_at = s_unclean;
-        if (h_at != INT_MAX && h_at <= u_at) {   // every entry before the answer added whole units inside the binade
-            if (tid == 0) s->todays = h[(int)(keys[h_at] & 0xFFFFFFFFLL)];
-            return;
-        }
-        // The sum before entry u_at (exact), from the thread that owns it; for a chunk that was clean
-        // throughout, the sum after its last entry.
-        if (tid == 0) s_done = 0;
-        __syncthreads();
-        {
-            int64_t r2 = m + s_warp[warp] + (incl - mine);
-#pragma unroll
-            for (int k = 0; k < WALK_PER; ++k) {
-                const int i = first + k;
-                if (i == u_at) s_below = (double)r2 * U;
-                if (i >= end) break;
-                r2 += d[k];
-                if (u_at == INT_MAX && i == end - 1) s_below = (double)r2 * U;
-            }
-        }
-        __syncthreads();
-        below = s_below;
-        if (u_at != INT_MAX) {
-            if (warp == 0) {
-                double b = below;
-                int cell;
-                if (walk_replay(keys, w, W, target, u_at, end, &b, &cell)) {
-                    if (lane == 0) {
-                        s->todays = h[cell];
-                        s_done = 1;
-                    }
-                } else if (lane == 0) {
-                    s_below = b;
-                }
-            }
-            __syncthreads();
-            if (s_done) return;
-            below = s_below;
-        }
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        sh.s = s->below_bracket;
+        sh.hit = -1;
     }
-    if (tid == 0) s->todays = h[(int)(keys[n - 1] & 0xFFFFFFFFLL)];
+    for (int i = threadIdx.x; i < n; i += kSSThreads) weights[i] = w[pdiv((int)(keys[i] & 0xFFFFFFFFLL), W)];
+    __syncthreads();
+    int answer = s->below_bracket >= target ? 0 : n;
+    const SumIn<double> in{weights, nullptr, 0, (size_t)n, nullptr, nullptr, 0.0, nullptr, 0};
+    for (int base = 0; base < n && answer == n; base += kSSBlock) {
+        cta_advance<true>(in, (size_t)base, min(n - base, kSSBlock), sh, false, target);
+        __syncthreads();
+        if (sh.hit >= 0) answer = base + sh.hit + 1;
+        __syncthreads();
+        if (answer != n) break;
+    }
+    if (threadIdx.x == 0) s->todays = h[(int)(keys[min(answer, n - 1)] & 0xFFFFFFFFLL)];
 }
 
 // SeaLevelStage.landAndWaterAt (SeaLevelStage.kt:175-200).
@@ -530,6 +399,7 @@ cg_status percentile_cut_dev(cg_ctx* ctx, int W, int H, const float* d_h, float 
     CG_BUF(unsigned, d_counts, ctx, S_HIST, (size_t)H * BINS);
     CG_BUF(double, d_hist, ctx, S_SCRATCH4, BINS);
     CG_BUF(long long, d_keys, ctx, S_BRACKET, N);
+    CG_BUF(double, d_weights, ctx, S_BRACKETW, N);   // the bracket's row weights
     cudaStream_t sm = ctx->stream;
     int grid = ctx->num_sms * 8;
     CG_LAUNCH(ctx) k_cut_init<<<1, 1, 0, sm>>>(d_s);
@@ -544,7 +414,7 @@ cg_status percentile_cut_dev(cg_ctx* ctx, int W, int H, const float* d_h, float 
     CG_BUF(long long, d_sorted, ctx, S_BRACKET2, SMALL_SORT);
     CG_LAUNCH(ctx) k_sort_rank<<<SMALL_SORT / RANK_KEYS / 8, 256, 0, sm>>>(d_keys, d_s, d_sorted);
     auto walk = [&](const long long* keys, int most) {
-        CG_LAUNCH(ctx) k_bracket_walk<<<1, WALK_THREADS, 0, sm>>>(d_h, keys, d_w, W, target, most, d_s);
+        CG_LAUNCH(ctx) k_bracket_walk<<<1, seqwalk::kSSThreads, 0, sm>>>(d_h, keys, d_w, W, target, most, d_s, d_weights);
         CG_LAUNCH(ctx) k_land_and_water<<<grid, 256, 0, sm>>>(d_h, N, most, d_s, lowstand_share, land_half, sea_half,
                                                               d_land, d_rel);
     };
