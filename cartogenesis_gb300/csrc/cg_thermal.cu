@@ -1,7 +1,7 @@
 // Musgrave thermal sweeps (ErosionStage.thermalSweep, ErosionStage.kt:235-403), fused for GB300.
 //
 // One sweep is two passes in the reference: every cell's give rate from its 8 neighbours, then
-// every cell's new height from its neighbours' give rates. Here one CTA owns a 64 x 32 tile and
+// every cell's new height from its neighbours' give rates. Here one CTA owns a tile (64 x 32, 32 x 16 on small grids) and
 // loads it with a halo of 4 cells into shared memory; it runs two sweeps there (or one, for an odd
 // remainder), each sweep's region shrinking by two cells a side (one for the give pass, one for
 // the move pass), and writes the tile back once.
@@ -11,7 +11,7 @@
 // neighbour by more than the least limit, and that lowest is kept row by row as a 3 x 3 window slides
 // down a thread's column; the give pass also takes what the cell itself gives off its height, with the
 // falls it has at hand, so the move pass only adds what comes in and leaves a cell alone when no
-// neighbour gives. A thread takes a column of 8 to 10 rows, so that four runs of rows times the
+// neighbour gives. A thread takes a column of 8 to 10 rows (4 to 6), so that four runs of rows times the
 // region's columns are one step of the CTA's 288 threads (92% busy over the four passes) and the
 // window's two extra rows cost a fifth of the loads. The 384 launches of an 8192 x 4096 stage take 89.5
 // ms (113 with each pass running its whole rule on 4-row columns), 192 sweeps at 4096 x 2048 5.5 ms
@@ -33,13 +33,26 @@ namespace cg {
 
 namespace {
 
-constexpr int TX = 64;
-constexpr int TY = 32;
 constexpr int KMAX = 2;
 constexpr int HALO = 2 * KMAX;
-constexpr int RW = TX + 2 * HALO;   // region width
-constexpr int RH = TY + 2 * HALO;   // region height
-constexpr int THREADS = 288;        // four runs of rows times up to 70 columns, a thread each
+
+// A CTA's tile, its region with the halo, and its threads: four runs of rows times up to RW - 2 columns, a
+// thread each.
+template <int X, int Y, int CTAS>
+struct Shape {
+    static constexpr int TX = X, TY = Y;
+    static constexpr int RW = TX + 2 * HALO, RH = TY + 2 * HALO;
+    static constexpr int THREADS = (4 * (RW - 2) + 31) / 32 * 32;
+    static constexpr int MIN_CTAS = CTAS;
+};
+using Wide = Shape<64, 32, 5>;    // 288 threads
+using Small = Shape<32, 16, 8>;   // 160 threads
+// A grid of fewer Wide tiles than SMs is a matter of one CTA's time, and a Small tile's columns are 4 to 6
+// rows long instead of 8 to 10: 24 sweeps at 512 x 256 took 128 us with 64 Wide tiles and take 108 with 256
+// Small ones, though nearly half of their region is halo.
+bool small_tiles(int W, int H) {
+    return (long long)((W + Wide::TX - 1) / Wide::TX) * ((H + Wide::TY - 1) / Wide::TY) < kSMs;
+}
 
 struct ThermalArgs {
     float limit[8];
@@ -63,7 +76,7 @@ struct TileFlags {
 
 // The region load by the tensor memory accelerator: one cp.async.bulk.tensor.2d per CTA of the
 // whole RW x RH region, rows off the grid filled with NaN by the copy itself. Used on tiles whose
-// region does not wrap east-west (its first column, 64 bx - 4, is 16-byte aligned as TMA requires); the
+// region does not wrap east-west (its first column, TX bx - 4, is 16-byte aligned as TMA requires); the
 // two wrapping tile columns load by threads. `err` (device) is set when a copy's wait runs out, after
 // which the CTA waits once more for its copy and leaves without computing; the host reports it.
 struct RegionLoad {
@@ -136,31 +149,34 @@ __device__ __forceinline__ float received(float c, const Around& nb, const Aroun
 struct Run {
     int col, row0, row1;
 };
-template <int M>
+template <class S, int M>
 __device__ __forceinline__ bool run_of(Run& r) {
-    constexpr int COLS = RW - 2 * M, PER = (RH - 2 * M + 3) / 4;
-    static_assert(4 * COLS <= THREADS, "a thread takes one run");
+    constexpr int COLS = S::RW - 2 * M, PER = (S::RH - 2 * M + 3) / 4;
+    static_assert(4 * COLS <= S::THREADS, "a thread takes one run");
     const int part = (int)threadIdx.x / COLS;
     r.col = M + (int)threadIdx.x - part * COLS;
     r.row0 = M + part * PER;
-    r.row1 = min(r.row0 + PER, RH - M);
+    r.row1 = min(r.row0 + PER, S::RH - M);
     return part < 4;
 }
 // A change at this row counts for the tile's flag where the column and row are the tile's own.
-__device__ __forceinline__ bool own_col(int col) { return col >= HALO && col < HALO + TX; }
-__device__ __forceinline__ bool own_row(int row) { return row >= HALO && row < HALO + TY; }
+template <class S>
+__device__ __forceinline__ bool own_col(int col) { return col >= HALO && col < HALO + S::TX; }
+template <class S>
+__device__ __forceinline__ bool own_row(int row) { return row >= HALO && row < HALO + S::TY; }
 
 // The give pass from h: rates into g, what is left of the heights into left. The left height is
 // (c - given) + 0, since the reference adds what a cell receives, if only +0. Returns whether any of the
 // thread's cells gives.
-template <int M>
+template <class S, int M>
 __device__ __forceinline__ bool give_pass(const float* __restrict__ h, float* __restrict__ left, float* __restrict__ g,
                                           const ThermalArgs& a, bool& changed) {
+    constexpr int RW = S::RW;
     Run r;
-    if (!run_of<M>(r)) return false;
+    if (!run_of<S, M>(r)) return false;
     bool any = false;
     unsigned moved = 0;
-    const bool own = own_col(r.col);
+    const bool own = own_col<S>(r.col);
     const float* p = h + (r.row0 - 1) * RW + r.col;
     float nw = p[-1], n = p[0], ne = p[1], w = p[RW - 1], c = p[RW], e = p[RW + 1];
     float top = fminf(fminf(nw, n), ne), mid = fminf(fminf(w, c), e);
@@ -176,7 +192,7 @@ __device__ __forceinline__ bool give_pass(const float* __restrict__ h, float* __
         g[i] = rate;
         left[i] = v;
         any |= rate != 0.0f;
-        if (own_row(row)) moved |= __float_as_uint(v) ^ __float_as_uint(c);
+        if (own_row<S>(row)) moved |= __float_as_uint(v) ^ __float_as_uint(c);
         nw = w, n = c, ne = e;
         w = sw, c = s, e = se;
         top = mid, mid = bot;
@@ -186,13 +202,14 @@ __device__ __forceinline__ bool give_pass(const float* __restrict__ h, float* __
 }
 
 // The move pass: what each cell receives, read from h and g, onto left.
-template <int M>
+template <class S, int M>
 __device__ __forceinline__ void move_pass(const float* __restrict__ h, float* __restrict__ left, const float* __restrict__ g,
                                           const ThermalArgs& a, bool& changed) {
+    constexpr int RW = S::RW;
     Run r;
-    if (!run_of<M>(r)) return;
+    if (!run_of<S, M>(r)) return;
     unsigned moved = 0;
-    const bool own = own_col(r.col);
+    const bool own = own_col<S>(r.col);
     const float* p = h + (r.row0 - 1) * RW + r.col;
     const float* q = g + (r.row0 - 1) * RW + r.col;
     float nw = p[-1], n = p[0], ne = p[1], w = p[RW - 1], c = p[RW], e = p[RW + 1];
@@ -209,7 +226,7 @@ __device__ __forceinline__ void move_pass(const float* __restrict__ h, float* __
             const float v = __fadd_rn(left[i], received(c, Around{{e, w, s, n, se, ne, sw, nw}},
                                                         Around{{ge, gw, gs, gn, gse, gne, gsw, gnw}}, a));
             left[i] = v;
-            if (own_row(row)) moved |= __float_as_uint(v) ^ __float_as_uint(c);
+            if (own_row<S>(row)) moved |= __float_as_uint(v) ^ __float_as_uint(c);
         }
         top = sides | __float_as_uint(gc);
         nw = w, n = c, ne = e;
@@ -222,7 +239,9 @@ __device__ __forceinline__ void move_pass(const float* __restrict__ h, float* __
 
 // The reference's rules on one cell of the region for any limits: rows off the grid are told apart by
 // `has_s` / `has_n` (the rows below and above exist).
+template <class S>
 __device__ float give_rate(const float* h, int i, bool has_s, bool has_n, const ThermalArgs& a) {
+    constexpr int RW = S::RW;
     const int off[8] = {1, -1, RW, -RW, RW + 1, -RW + 1, RW - 1, -RW - 1};
     const bool ok[8] = {true, true, has_s, has_n, has_s, has_n, has_s, has_n};
     float excess = 0.0f, steepest = 0.0f;
@@ -237,7 +256,9 @@ __device__ float give_rate(const float* h, int i, bool has_s, bool has_n, const 
     return __fdiv_rn(p <= q ? p : q, excess);
 }
 
+template <class S>
 __device__ float moved(const float* h, const float* g, int i, bool has_s, bool has_n, const ThermalArgs& a) {
+    constexpr int RW = S::RW;
     const int off[8] = {1, -1, RW, -RW, RW + 1, -RW + 1, RW - 1, -RW - 1};
     const bool ok[8] = {true, true, has_s, has_n, has_s, has_n, has_s, has_n};
     float received = 0.0f, given = 0.0f;
@@ -253,18 +274,19 @@ __device__ float moved(const float* h, const float* g, int i, bool has_s, bool h
 }
 
 // One sweep by those rules over rows and columns [M + 1, R - M - 1) from h into to.
-template <int M>
+template <class S, int M>
 __device__ void any_sweep(const float* h, float* to, float* g, int y0, int H, const ThermalArgs& a, bool& changed) {
+    constexpr int RW = S::RW, RH = S::RH, TX = S::TX, TY = S::TY, THREADS = S::THREADS;
     for (int i = threadIdx.x; i < RW * RH; i += THREADS) {
         const int row = i / RW, col = i % RW, y = y0 + row;
         if (row < M || row >= RH - M || col < M || col >= RW - M || y < 0 || y >= H) continue;
-        g[i] = give_rate(h, i, y + 1 < H, y > 0, a);
+        g[i] = give_rate<S>(h, i, y + 1 < H, y > 0, a);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < RW * RH; i += THREADS) {
         const int row = i / RW, col = i % RW, y = y0 + row;
         if (row <= M || row >= RH - M - 1 || col <= M || col >= RW - M - 1 || y < 0 || y >= H) continue;
-        to[i] = moved(h, g, i, y + 1 < H, y > 0, a);
+        to[i] = moved<S>(h, g, i, y + 1 < H, y > 0, a);
         if (__float_as_uint(to[i]) != __float_as_uint(h[i]) && row >= HALO && row < HALO + TY && col >= HALO &&
             col < HALO + TX)
             changed = true;
@@ -273,9 +295,11 @@ __device__ void any_sweep(const float* h, float* to, float* g, int y0, int H, co
 }
 
 // `k` sweeps (1 or 2) of the field `in` into `out`, a CTA a tile.
-__global__ void __launch_bounds__(THREADS, 5) thermal_sweeps_kernel(const float* __restrict__ in, float* __restrict__ out,
+template <class S>
+__global__ void __launch_bounds__(S::THREADS, S::MIN_CTAS) thermal_sweeps_kernel(const float* __restrict__ in, float* __restrict__ out,
                                                                     int W, int H, int k, ThermalArgs a, TileFlags fl,
                                                                     const __grid_constant__ RegionLoad rl) {
+    constexpr int RW = S::RW, RH = S::RH, TX = S::TX, TY = S::TY, THREADS = S::THREADS;
     __shared__ __align__(128) float sm_a[RW * RH];
     __shared__ __align__(16) float sm_b[RW * RH], sm_g[RW * RH];
     __shared__ __align__(8) unsigned long long bar;
@@ -337,19 +361,19 @@ __global__ void __launch_bounds__(THREADS, 5) thermal_sweeps_kernel(const float*
     const float* res = sm_b;
     if (a.plain) {
         // A region in which no cell gives has nothing to move in the second sweep either.
-        if (__syncthreads_or(give_pass<1>(sm_a, sm_b, sm_g, a, moved_any))) {
-            move_pass<2>(sm_a, sm_b, sm_g, a, moved_any);
+        if (__syncthreads_or(give_pass<S, 1>(sm_a, sm_b, sm_g, a, moved_any))) {
+            move_pass<S, 2>(sm_a, sm_b, sm_g, a, moved_any);
             __syncthreads();
             if (k == 2) {
-                if (__syncthreads_or(give_pass<3>(sm_b, sm_a, sm_g, a, moved_any)))
-                    move_pass<4>(sm_b, sm_a, sm_g, a, moved_any);
+                if (__syncthreads_or(give_pass<S, 3>(sm_b, sm_a, sm_g, a, moved_any)))
+                    move_pass<S, 4>(sm_b, sm_a, sm_g, a, moved_any);
                 res = sm_a;
             }
         }
     } else {
-        any_sweep<1>(sm_a, sm_b, sm_g, y0, H, a, moved_any);
+        any_sweep<S, 1>(sm_a, sm_b, sm_g, y0, H, a, moved_any);
         if (k == 2) {
-            any_sweep<3>(sm_b, sm_a, sm_g, y0, H, a, moved_any);
+            any_sweep<S, 3>(sm_b, sm_a, sm_g, y0, H, a, moved_any);
             res = sm_a;
         }
     }
@@ -373,9 +397,14 @@ __global__ void __launch_bounds__(THREADS, 5) thermal_sweeps_kernel(const float*
 
 cudaError_t launch(const float* in, float* out, int W, int H, int k, const ThermalArgs& a, cudaStream_t st,
                    TileFlags fl = TileFlags{nullptr, nullptr}, const RegionLoad* rl = nullptr) {
-    dim3 grid((W + TX - 1) / TX, (H + TY - 1) / TY);
     static const RegionLoad none{};
-    thermal_sweeps_kernel<<<grid, THREADS, 0, st>>>(in, out, W, H, k, a, fl, rl ? *rl : none);
+    auto run = [&](auto shape) {
+        using S = decltype(shape);
+        const dim3 grid((W + S::TX - 1) / S::TX, (H + S::TY - 1) / S::TY);
+        thermal_sweeps_kernel<S><<<grid, S::THREADS, 0, st>>>(in, out, W, H, k, a, fl, rl ? *rl : none);
+    };
+    if (small_tiles(W, H)) run(Small{});
+    else run(Wide{});
     return cudaGetLastError();
 }
 
@@ -404,10 +433,11 @@ RegionLoad region_load_of(const float* field, int W, int H, int* err) {
     RegionLoad rl{};
     rl.err = err;
     EncodeTiledFn enc = encode_tiled();
-    if (!enc || !err || W < 2 * RW || (((uintptr_t)field) & 15) != 0) return rl;
+    const int rw = small_tiles(W, H) ? Small::RW : Wide::RW, rh = small_tiles(W, H) ? Small::RH : Wide::RH;
+    if (!enc || !err || W < 2 * rw || (((uintptr_t)field) & 15) != 0) return rl;
     const cuuint64_t dims[2] = {(cuuint64_t)W, (cuuint64_t)H};
     const cuuint64_t strides[1] = {(cuuint64_t)W * sizeof(float)};
-    const cuuint32_t box[2] = {RW, RH};
+    const cuuint32_t box[2] = {(cuuint32_t)rw, (cuuint32_t)rh};
     const cuuint32_t estride[2] = {1, 1};
     if (enc(&rl.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)field, dims, strides, box, estride,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -464,7 +494,8 @@ cg_status thermal_sweeps_dev(cg_ctx* ctx, int W, int H, float* d_a, float* d_b, 
     // Per-tile change bits of the previous and the current launch. The first launch computes every
     // tile (the destination holds nothing yet); after it, both buffers hold a tile's bits whenever
     // that tile did not change, so the skip needs no copy.
-    const int tiles = ((W + TX - 1) / TX) * ((H + TY - 1) / TY);
+    const int tx = small_tiles(W, H) ? Small::TX : Wide::TX, ty = small_tiles(W, H) ? Small::TY : Wide::TY;
+    const int tiles = ((W + tx - 1) / tx) * ((H + ty - 1) / ty);
     CG_BUF(uint8_t, d_flags, ctx, S_THERMFLAG, 2 * (size_t)tiles);
     CG_BUF(int, d_err, ctx, S_THERMERR, 1);
     uint8_t* prev = d_flags;
