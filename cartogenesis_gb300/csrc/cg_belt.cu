@@ -748,6 +748,9 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
     const int bgrid = std::min(grid, (B + 255) / 256 + 1);
     CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_belt_sweeps, 512, 0));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "the belt's sweep kernel cannot be resident");
+    // One CTA an SM while a thread has two cells at most, for the shorter grid barriers; larger belts wait for
+    // their loads and take all that fit.
+    const int sweep_ctas = ctx->num_sms * std::min(per_sm, std::max(1, (B + F) / (ctx->num_sms * 1024)));
     CG_CUDA(ctx, cudaMemcpyAsync(d_next, d_h, N * 4, cudaMemcpyDeviceToDevice, sm));
     SweepArgs sa{};
     sa.swept = d_swept;
@@ -814,7 +817,7 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
         // The slopes.
         void* sargs[] = {&sa};
         ctx->launches++;
-        CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_belt_sweeps, ctx->num_sms, 512, sargs, 0, sm));
+        CG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_belt_sweeps, sweep_ctas, 512, sargs, 0, sm));
         CG_TRY_ST(seq_totals_f64_dev(ctx, totals, kSeqTotals));
         // The crust's answer to the rock taken so far (BeltErosion.kt:413-423).
         if (rebound && ((round + 1) % kReboundRounds == 0 || round == k.rounds - 1)) {

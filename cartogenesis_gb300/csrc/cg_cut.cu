@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256) k_bin_sums(const unsigned* __restrict__ c
 
 // SeaLevelStage.kt:614-622: the first bin that brings the weight below up to the target, the bins'
 // sequential sum told apart by predicted binades and chained (one thread adding 4096 doubles in turn took
-// 140 us, a CTA scan for every binade the sum grows through 70, this 17).
+// 140 us, a CTA scan for every binade the sum grows through 70, this 25).
 __global__ void __launch_bounds__(seqwalk::kSSThreads) k_bracket_bin(const double* __restrict__ hist, double target,
                                                                      CutState* s) {
     using namespace seqwalk;
