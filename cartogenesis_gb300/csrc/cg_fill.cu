@@ -218,7 +218,7 @@ __device__ __forceinline__ bool relax_tile(TileSmem& sm, int tile, float* __rest
         bool changed = false;
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            if (c[k] == before[k]) continue;
+            if (parent[k] == -2 || c[k] == before[k]) continue;   // a settled cell may hold NaN
             sf[r0 + k + 1][lx + 1] = c[k];
             changed = true;
             // A border cell, or the last column when the grid is narrower than a tile (its
