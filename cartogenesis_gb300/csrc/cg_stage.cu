@@ -192,46 +192,52 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
 
     // Phase boundaries of a round, for the per-phase device times of cg_round_stats (ev[8]: the end
     // of the uplift and the plate flexure). Two rounds' events in turn: a round's times are read after the
-    // next one's first synchronisation, so that the host does not wait for the end of a round.
-    cudaEvent_t events[2][9] = {};
+    // next one's first synchronisation, so that the host does not wait for the end of a round, or on the way
+    // out, whatever ends the rounds.
+    struct Times {
+        cg_round_stats* stats;
+        int first_round;
+        bool flexure;
+        int unread = -1;   // the round whose times are still to be read
+        cudaEvent_t events[2][9] = {};
+        void read() {      // once that round is over
+            if (unread < 0) return;
+            cudaEvent_t* ev = events[unread & 1];
+            float ms[8] = {0};
+            for (int i = 1; i < 8; ++i) cudaEventElapsedTime(&ms[i], ev[i - 1], ev[i]);
+            float total = 0.0f, ms_flexure = 0.0f;
+            if (flexure) {
+                cudaEventElapsedTime(&ms_flexure, ev[0], ev[8]);
+                cudaEventElapsedTime(&ms[1], ev[8], ev[1]);
+            }
+            cudaEventElapsedTime(&total, ev[0], ev[7]);
+            cg_round_stats& s = stats[unread - first_round];
+            s.ms_total = total;
+            s.ms_flexure = ms_flexure;
+            s.ms_cut = ms[1];
+            s.ms_fill = ms[2];
+            s.ms_route = ms[3];
+            s.ms_tree = ms[4];
+            s.ms_incise = ms[5];
+            s.ms_deposit = ms[6];
+            s.ms_relax = ms[7];
+            unread = -1;
+        }
+        ~Times() {
+            if (unread >= 0 && cudaEventSynchronize(events[unread & 1][7]) == cudaSuccess) read();
+            for (auto& set : events)
+                for (auto& e : set)
+                    if (e) cudaEventDestroy(e);
+        }
+    } times{stats, first_round, flexure};
     if (stats)
-        for (auto& set : events)
+        for (auto& set : times.events)
             for (auto& e : set) CG_CUDA(ctx, cudaEventCreate(&e));
-    struct Events {
-        cudaEvent_t (*ev)[9];
-        bool on;
-        ~Events() {
-            if (on)
-                for (int i = 0; i < 18; ++i) cudaEventDestroy(ev[i / 9][i % 9]);
-        }
-    } guard{events, stats != nullptr};
-    auto read_times = [&](int round) {   // of a round that is over
-        if (!stats || round < first_round) return;
-        cudaEvent_t* ev = events[round & 1];
-        float ms[8] = {0};
-        for (int i = 1; i < 8; ++i) cudaEventElapsedTime(&ms[i], ev[i - 1], ev[i]);
-        float total = 0.0f, ms_flexure = 0.0f;
-        if (flexure) {
-            cudaEventElapsedTime(&ms_flexure, ev[0], ev[8]);
-            cudaEventElapsedTime(&ms[1], ev[8], ev[1]);
-        }
-        cudaEventElapsedTime(&total, ev[0], ev[7]);
-        cg_round_stats& s = stats[round - first_round];
-        s.ms_total = total;
-        s.ms_flexure = ms_flexure;
-        s.ms_cut = ms[1];
-        s.ms_fill = ms[2];
-        s.ms_route = ms[3];
-        s.ms_tree = ms[4];
-        s.ms_incise = ms[5];
-        s.ms_deposit = ms[6];
-        s.ms_relax = ms[7];
-    };
 
     for (int round = first_round; round < end_round; ++round) {
         CG_TRY(cancelled(ctx));
         auto mark = [&](int i) {
-            if (stats) cudaEventRecord(events[round & 1][i], sm);
+            if (stats) cudaEventRecord(times.events[round & 1][i], sm);
         };
         float* cur = run.cur;
         const long long launches0 = ctx->launches;
@@ -245,7 +251,7 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
         int land_cells;
         CG_TRY(percentile_cut_dev(ctx, W, H, cur, p.sea_level, land_half, sea_half, stand_below_today(p, round),
                                   d_land, d_rel, &shoreline, &land_cells));
-        read_times(round - 1);
+        times.read();
         if (land_cells == 0) {   // HydraulicErosion.kt:856-858: the rounds stop where the land is gone
             run.done = true;
             run.next_round = round;
@@ -386,11 +392,12 @@ cg_status stage_rounds_dev(cg_ctx* ctx, StageRun& run, int end_round, cg_round_s
             s.ms_deposit_lakes = dc.ms_lakes;
             s.ms_deposit_seas = dc.ms_seas;
             s.ms_deposit_repairs = dc.ms_repairs;
+            times.unread = round;
         }
     }
-    if (stats && end_round > first_round) {
-        CG_CUDA(ctx, cudaEventSynchronize(events[(end_round - 1) & 1][7]));
-        read_times(end_round - 1);
+    if (times.unread >= 0) {
+        CG_CUDA(ctx, cudaEventSynchronize(times.events[times.unread & 1][7]));
+        times.read();
     }
     if (run.next_round >= p.hydraulic_rounds) run.done = true;
     return CG_OK;
