@@ -65,8 +65,10 @@ struct FillCounters {
 
 // (0) classes and initial levels.
 __global__ void k_fill_init(const uint8_t* __restrict__ land, const float* __restrict__ g, int W, int H,
-                            uint8_t* __restrict__ cls, float* __restrict__ f, int* __restrict__ ptr) {
+                            uint8_t* __restrict__ cls, float* __restrict__ f, int* __restrict__ ptr,
+                            int* __restrict__ left) {
     size_t N = (size_t)W * H;
+    if (blockIdx.x == 0 && threadIdx.x < 2) left[threadIdx.x] = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
         const int row = pdiv((int)i, W);
         if (!land[i]) {
@@ -106,22 +108,57 @@ __global__ void k_fill_init(const uint8_t* __restrict__ land, const float* __res
 // (1) every land cell's chain followed to its root, in place: a step replaces the cell's pointer by the one
 // it just read, p[i] <- p[p[i]], so cells above it on the chain skip what it has skipped. Whatever a
 // concurrent step lets a thread read is an ancestor of i on its chain, and the chain is finite. A cell whose
-// root is water or a polar outlet keeps its own height. One launch: jumping passes that each jumped every
-// cell once, with a host check every second pass, took 100 us at 1024 x 512 and 1.1 ms at 8192 x 4096.
-__global__ void k_drain_chains(int* p, const float* __restrict__ g, size_t N, uint8_t* cls, float* __restrict__ f) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
-        if (cls[i] != C_OPEN) continue;   // the roots' classes never change
-        int o = __ldcg(p + i);
-        for (int n = __ldcg(p + o); n != o; n = __ldcg(p + o)) {
-            __stcg(p + i, n);
-            o = n;
-        }
-        const uint8_t rc = cls[o];
-        if (rc == C_WATER || rc == C_SEED) {
-            cls[i] = C_DRAINED;
-            f[i] = g[i];
-        }
+// root is water or a polar outlet keeps its own height. True once the root is reached, `most` steps at most.
+__device__ __forceinline__ bool drain_chain(int* p, const float* __restrict__ g, size_t i, int most, uint8_t* cls,
+                                            float* __restrict__ f) {
+    int o = __ldcg(p + i);
+    for (int n = __ldcg(p + o); n != o; n = __ldcg(p + o)) {
+        if (most-- == 0) return false;
+        __stcg(p + i, n);
+        o = n;
     }
+    const uint8_t rc = cls[o];   // the roots' classes never change
+    if (rc == C_WATER || rc == C_SEED) {
+        cls[i] = C_DRAINED;
+        f[i] = g[i];
+    }
+    return true;
+}
+
+// A thread takes its cells in turn, and one whose chain runs through cells whose turn has not come takes them
+// a step each: with no limit a serpentine at 2048 x 1024 took 527 ms and a plane falling down an 8192 x 4096
+// map 69. So a cell takes kDrainSteps at most (`left` says that some needed more), and the rest is
+// k_relax_passes's to finish: 0.1 and 1.2 ms here, 0.06 and 1.8 there. (Passes that each jumped every cell
+// once, with a host check every second one: 0.2 and 1.5 ms.) Most chains of a world end here, in 8 us at
+// 1024 x 512 and 0.4 ms at 8192 x 4096; 16 to 64 steps are the same there, and fewer leave more to the passes.
+constexpr int kDrainSteps = 32;
+__global__ void k_drain_chains(int* p, const float* __restrict__ g, size_t N, uint8_t* cls, float* __restrict__ f,
+                               int* left) {
+    bool more = false;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x)
+        if (cls[i] == C_OPEN) more |= !drain_chain(p, g, i, kDrainSteps, cls, f);
+    if (more) *(volatile int*)left = 1;
+}
+
+// The chains that are left, every thread of a cooperative launch: passes of a few steps a cell, each from
+// pointers that much longer than the pass before, until none is short of its root. left[0] was set before
+// the launch; left[1] to left[3] take turns as the passes' answers, so that one is cleared while no CTA reads it.
+constexpr int kDrainAgain = 16;
+__device__ __noinline__ void drain_rest(int* p, const float* __restrict__ g, size_t N, uint8_t* cls, float* __restrict__ f,
+                                        int* left) {
+    cgr::grid_group grid = cgr::this_grid();
+    for (int now = 1;;) {
+        const int next = now == 3 ? 1 : now + 1;
+        bool more = false;
+        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x)
+            if (cls[i] == C_OPEN) more |= !drain_chain(p, g, i, kDrainAgain, cls, f);
+        if (blockIdx.x == 0 && threadIdx.x == 0) left[next] = 0;
+        if (more) *(volatile int*)(left + now) = 1;
+        grid.sync();
+        if (*(volatile int*)(left + now) == 0) break;
+        now = next;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) left[0] = 0;
 }
 
 // (2) tile relaxation. A CTA takes a 32x32 tile and relaxes its OPEN cells to local convergence. A warp
@@ -244,7 +281,7 @@ __device__ __forceinline__ bool relax_tile(TileSmem& sm, int tile, float* __rest
 struct RelaxArgs {
     float* f;
     const float* g;
-    const uint8_t* cls;
+    uint8_t* cls;
     const int* pin;
     int W, H, tiles_x, tiles_y;
     int* list[2];
@@ -252,11 +289,15 @@ struct RelaxArgs {
     int* count;   // [3]
     int* timed_out;
     int max_passes;
+    int* ptr;     // the cells' chains
+    int* left;    // [4]: whether chains are left (drain_rest)
 };
 
 __global__ void __launch_bounds__(256, 4) k_relax_passes(RelaxArgs a) {
     cgr::grid_group grid = cgr::this_grid();
     __shared__ TileSmem sm;
+    // Cells that drain were listed as open with their tiles; once settled they change nothing there.
+    if (*(volatile int*)a.left) drain_rest(a.ptr, a.g, (size_t)a.W * a.H, a.cls, a.f, a.left);
     int pass = 0, now = 0;   // count[now]: this pass's list
     for (; pass < a.max_passes; ++pass) {
         const int cur = pass & 1, nxt = cur ^ 1, then = now == 2 ? 0 : now + 1;
@@ -546,8 +587,9 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     CG_BUF(int, d_ptr, ctx, S_PTR, N);
     CG_BUF(int, d_pin, ctx, S_FILLQ, N);
     int tiles_x = (W + T - 1) / T, tiles_y = (H + T - 1) / T, tiles = tiles_x * tiles_y;
-    // Three list counts and the two tile lists' marks (zeroed before each relaxation), and the lists.
-    CG_BUF(int, d_marks, ctx, S_TILEFLAG, 2 * (size_t)tiles + 4);
+    // Three list counts and the two tile lists' marks (zeroed before each relaxation), the chains' words (not
+    // zeroed there), and the lists.
+    CG_BUF(int, d_marks, ctx, S_TILEFLAG, 2 * (size_t)tiles + 8);
     CG_BUF(int, d_lists, ctx, S_FILLLIST, 2 * (size_t)tiles);
     CG_BUF(FillCounters, d_cnt, ctx, S_FILLF, 1);
     RelaxArgs ra;
@@ -565,14 +607,16 @@ cg_status fill_depressions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land,
     ra.timed_out = &d_cnt->timed_out;
     ra.mark[0] = d_marks + 4;
     ra.mark[1] = ra.mark[0] + tiles;
+    ra.left = ra.mark[1] + tiles;
+    ra.ptr = d_ptr;
     ra.max_passes = 4 * (tiles_x + tiles_y) + 64;
     int per_sm = 0;
     CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_relax_passes, 256, 0));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "k_relax_passes cannot be resident");
     const int relax_grid = ctx->num_sms * std::min(per_sm, 8);
     int grid = ctx->num_sms * 8;
-    CG_LAUNCH(ctx) k_fill_init<<<grid, 256, 0, sm>>>(d_land, d_rel, W, H, d_cls, d_filled, d_ptr);
-    CG_LAUNCH(ctx) k_drain_chains<<<grid, 256, 0, sm>>>(d_ptr, d_rel, N, d_cls, d_filled);
+    CG_LAUNCH(ctx) k_fill_init<<<grid, 256, 0, sm>>>(d_land, d_rel, W, H, d_cls, d_filled, d_ptr, ra.left);
+    CG_LAUNCH(ctx) k_drain_chains<<<grid, 256, 0, sm>>>(d_ptr, d_rel, N, d_cls, d_filled, ra.left);
     CG_CHECK_LAUNCH(ctx);
 
     // Scratch of the level replays: a generation mark per cell, the level's cells and the heap, each
