@@ -759,6 +759,24 @@ __global__ void k_basin_finish(BasinDev b, int count, const uint8_t* __restrict_
 
 }  // namespace
 
+// The links, down then mask, and behind them the largest key and the number of sources. The mask is written a
+// word at a time, so it starts at one on grids of two cells too.
+struct Links {
+    uint8_t *down, *mask;
+    unsigned long long* max_key;
+    int* sources;
+};
+static size_t link_stride(size_t N) { return (N + 15) & ~(size_t)15; }
+static size_t link_bytes(size_t N) { return 2 * link_stride(N) + 32; }
+static Links links_at(uint8_t* d_links, size_t N) {
+    Links l;
+    l.down = d_links;
+    l.mask = d_links + link_stride(N);
+    l.max_key = reinterpret_cast<unsigned long long*>(l.mask + link_stride(N));
+    l.sources = reinterpret_cast<int*>(l.max_key + 1);
+    return l;
+}
+
 cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const int32_t* d_recv,
                         const float* d_weights, long long* d_key, int32_t* d_donors, float* d_area, int* h_levels,
                         const double* d_inflow, double* d_flow, ReadBack also) {
@@ -766,13 +784,12 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
     cudaStream_t sm = ctx->stream;
     int grid = ctx->num_sms * 8;
     CG_BUF(int32_t, d_pending, ctx, S_DEPTH, N);
-    // The links and, behind them, the largest key and the number of sources: zeroed together.
-    CG_BUF(uint8_t, d_links, ctx, S_LINKS, 2 * N + 32);
+    CG_BUF(uint8_t, d_links, ctx, S_LINKS, link_bytes(N));
     CG_BUF(int, d_sources, ctx, S_SOURCES, N);
-    uint8_t* d_down = d_links;
-    uint8_t* d_mask = d_links + N;
-    unsigned long long* d_max = reinterpret_cast<unsigned long long*>(d_links + ((2 * N + 15) & ~(size_t)15));
-    int* d_nsrc = reinterpret_cast<int*>(d_max + 1);
+    const Links links = links_at(d_links, N);
+    uint8_t *d_down = links.down, *d_mask = links.mask;
+    unsigned long long* d_max = links.max_key;
+    int* d_nsrc = links.sources;   // zeroed with the mask and the largest key
     CG_CUDA(ctx, cudaMemsetAsync(d_mask, 0, (uint8_t*)(d_nsrc + 1) - d_mask, sm));
     CG_LAUNCH(ctx) k_links<<<grid, 256, 0, sm>>>(d_land, d_recv, W, H, d_down, d_mask);
     CG_LAUNCH(ctx) k_sources<<<grid, 256, 0, sm>>>(d_land, d_mask, N, d_donors, d_pending, d_sources, d_nsrc);
@@ -803,10 +820,11 @@ cg_status tree_walk_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, const 
 cg_status flow_walk_dev(cg_ctx* ctx, int W, int H, long long* d_key, double* d_flow) {
     const size_t N = (size_t)W * H;
     CG_BUF(int32_t, d_pending, ctx, S_DEPTH, N);
-    CG_BUF(uint8_t, d_links, ctx, S_LINKS, 2 * N + 32);
+    CG_BUF(uint8_t, d_links, ctx, S_LINKS, link_bytes(N));
     CG_BUF(int, d_sources, ctx, S_SOURCES, N);
-    const int* d_nsrc = reinterpret_cast<const int*>(d_links + ((2 * N + 15) & ~(size_t)15)) + 2;
-    WalkArgs a{W, H, d_links, d_links + N, d_pending, d_key, nullptr, nullptr, nullptr, d_flow, d_sources, d_nsrc, nullptr};
+    const Links links = links_at(d_links, N);
+    WalkArgs a{W, H, links.down, links.mask, d_pending, d_key, nullptr, nullptr, nullptr, d_flow, d_sources, links.sources,
+               nullptr};
     const int ctas = ((int)std::min(N, (size_t)1 << 19) + 63) / 64;
     CG_LAUNCH(ctx) k_walk<WALK_FLOW><<<ctas, 64, 0, ctx->stream>>>(a);
     CG_CHECK_LAUNCH(ctx);
