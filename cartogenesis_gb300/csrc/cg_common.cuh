@@ -98,17 +98,17 @@ enum Slot {
     S_H0, S_H1, S_GIVE, S_UPLIFT, S_ROCK, S_RAIN, S_VEG, S_RUNOFF, S_ERODE, S_LAND, S_REL, S_FILLED,
     S_SURFACE, S_RECV, S_DONORS, S_KEY, S_ORDER, S_AREA, S_WATER, S_LABEL, S_PTR, S_SCRATCH0,
     S_SCRATCH1, S_SCRATCH2, S_SCRATCH3, S_ROWW, S_HIST, S_BRACKET, S_BRACKET2, S_SMALL, S_FLATS,
-    S_FLATIDX, S_FLATMEM, S_CG0, S_CG1, S_CG2, S_CG3, S_CG4, S_CG5, S_LEVELCNT, S_DEPTH, S_STATS,
+    S_FLATIDX, S_FLATMEM, S_CG0, S_CG1, S_CG2, S_CG3, S_CG4, S_CG5, S_LEVELCNT, S_DEPTH,
     S_BASIN, S_BASIN2, S_FILLQ, S_FILLF, S_FILLFLAG, S_TILEFLAG, S_SCRATCH4, S_SCRATCH5, S_THERMFLAG,
     S_LINKS, S_SOURCES, S_FILLLIST, S_CLAIM, S_FOOT, S_BREACH,
     // profile P2's deposition: the stage's state, a round's walk, and the mouths pass's own routing
-    S_SEDIMENT, S_STAMP, S_DEPWORDS, S_DEPMARK, S_SETTLED, S_LOAD, S_INCISED, S_DEPRANK, S_DEPLEVEL,
+    S_SEDIMENT, S_DEPWORDS, S_DEPMARK, S_SETTLED, S_LOAD, S_INCISED, S_DEPRANK, S_DEPLEVEL,
     S_HANDOFF, S_DEPUSED, S_DEPS0, S_DEPD0, S_DEPEVC, S_DEPEVK, S_DEPSEG, S_DEPEVENTS, S_DEPEVTOUCH,
     S_DEPSLOT0, S_DEPSLOT1, S_DEPSLOT2, S_DEPSLOT3, S_DEPSLOT4, S_DEPSLOT5, S_DEPSLOT6, S_DEPSLOT7,
     S_DEPHEAP, S_DEPTOUCH, S_DEPREPLAY, S_DEPSEGC,
     S_OM_LAND, S_OM_REL, S_OM_FILLED, S_OM_RECV, S_OM_KEY, S_OM_AREA, S_OM_RUNOFF, S_OM_DONORS,
-    S_FILLEB, S_THERMERR, S_SL_MASK, S_SL_LABEL, S_SL_SIZE, S_SL_WORDS, S_SL_LIST, S_SL_CHAIN, S_SL_STAMP, S_DEPSLOT8, S_DEPSLOT9, S_DEPSLOT10,
-    S_DEPCLAIM, S_DEPCANDOF, S_DEPCAND, S_DEPCANDN, S_DEPCANDOFF, S_DEPCANDW, S_DEPSLOTOFF, S_DEPACC, S_DEPOWN, S_DEPCELLCNT, S_DEPTIMERS, S_DEPRLIST, S_DEPWBITS, S_SS_EST, S_SS_SPEC, S_SS_WALK, S_SS_X, S_SS_MASK, S_SS_OUT, S_DEPFIRST, S_DEPTOUCHEV, S_RS_KEYS, S_RS_VALS, S_RS_HIST,
+    S_FILLEB, S_THERMERR, S_SL_MASK, S_SL_LABEL, S_SL_SIZE, S_SL_WORDS, S_SL_LIST, S_SL_CHAIN, S_SL_STAMP, S_DEPSLOT9, S_DEPSLOT10,
+    S_DEPCLAIM, S_DEPCANDOF, S_DEPCAND, S_DEPCANDN, S_DEPCANDOFF, S_DEPCANDW, S_DEPSLOTOFF, S_DEPCELLCNT, S_DEPTIMERS, S_DEPRLIST, S_DEPWBITS, S_SS_EST, S_SS_SPEC, S_SS_WALK, S_SS_X, S_SS_MASK, S_SS_OUT, S_DEPFIRST, S_DEPTOUCHEV, S_RS_KEYS, S_RS_VALS, S_RS_HIST,
     S_FX_TW, S_FX_A, S_FX_B, S_FX_MEAN, S_FX_REF, S_FX_DEFL, S_FX_UPL, S_FX_LOAD,
     // the belts' replay: its inputs, the belt and its frontier, the opening's routing, a round's state
     S_BT_H, S_BT_TECT, S_BT_WEAR, S_BT_ONSET, S_BT_UPLIFT, S_BT_RAIN, S_BT_COVER, S_BT_ROCK, S_BT_UNRES,

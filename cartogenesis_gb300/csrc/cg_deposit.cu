@@ -106,7 +106,6 @@ struct WalkDev {
     int* slot_n;            // per slot: admitted cells (a lake fan) or box tiles (a sea lobe)
     int* slot_box;          // per slot, a sea lobe's box in tiles: first column (may be < 0), first row, columns, rows
     int* slot_state;        // per slot: 1 while a lake fan waits to lay, 2 while a sea lobe waits, else 0
-    double* slot_laid;      // per slot: what its fan laid
     Touch* slot_touch;      // per slot: its fan's deposits, `cap` entries
     int* slot_touch_n;
     // A chunk's laying schedule: each (fan, admitted cell) pair, grouped by cell, knows the fan that
@@ -132,7 +131,6 @@ struct WalkDev {
     int* heap_admitted;
     unsigned long long* heap_sorted;   // per warp: a sea lobe's admitted cells by distance (`cap`)
     int lobe_words;         // words of a lobe's box in shared memory, even; 0: lobes take the heap
-    int* stamp;             // per cell: the stage's fan stamps
     // The level's fan deposits, for the repairs.
     Touch* touches;
     int touch_cap;
@@ -142,10 +140,8 @@ struct WalkDev {
     int* refit;             // cells to refit
     int* rlist;             // the log's entries on the cells to replay, grouped by cell (touch_cap)
     int* first;             // per cell: its earliest log entry being undone (kNoTouch at rest)
-    int* touch_ev;          // per level-log entry: its event's index
+    int* touch_ev;          // per level-log entry: its event's index, recorded as the log is assembled
     int* roff;              // per cell to replay + 1: its group's first entry
-    float* acc;             // per cell: a replayed settled height
-    uint8_t* own_done;      // per cell: the replay has taken the cell's own subtraction
     int* words;             // W_* control words
     unsigned long long* timers;   // T_*: nanoseconds of the walk's parts, kept by CTA 0's thread 0
 };
@@ -510,7 +506,6 @@ __device__ double lay_lake_warp(const WalkDev& w, int s, LakeFan& fan, double bu
         }
     }
     if (exact) laid = value(took);
-    if (lane == 1) w.slot_laid[s] = laid;
     if (lane == 0) w.slot_touch_n[s] = logged;
     return laid;
 }
@@ -840,9 +835,6 @@ __device__ void undo_from_grid(const WalkDev& w, int cut, int T) {
     }
 }
 
-// The level-log entry t's event (recorded as the log is assembled).
-__device__ __forceinline__ int event_of(const WalkDev& w, int t, int) { return w.touch_ev[t]; }
-
 // Whether the deposit into cell x by the fan of rank `rank` of level L makes a mouth conflict: x's
 // receiver lies on the level, is ranked after the fan, read its donors' settled heights and has a mouth of
 // its own (its step ends at the sea or in a lake), so its own walk, and with it its fan, are not the
@@ -883,7 +875,7 @@ __device__ void final_repairs_grid(const WalkDev& w, int L, int n, int touch_n, 
     for (int t = tid; t < T; t += stride) {
         const int x = w.touches[t].cell;
         if (!w.f.land[x]) continue;
-        const int rank = w.events[event_of(w, t, n)];
+        const int rank = w.events[w.touch_ev[t]];
         if (level_of_cell(w, x) == L && w.rank_of[x] > rank && atomicExch(&w.mark[x], gen) != gen) {
             const int i = atomicAdd(&w.words[W_NREPLAY], 1);
             w.replay[i] = x;
@@ -964,7 +956,7 @@ __device__ void final_repairs_grid(const WalkDev& w, int L, int n, int touch_n, 
         bool own = false;
         for (int a = 0; a < m; ++a) {
             const int t = g[a];
-            if (!own && w.events[event_of(w, t, n)] > rx) {
+            if (!own && w.events[w.touch_ev[t]] > rx) {
                 const double moved = w.f.incised_at[x];
                 if (moved > 0.0) acc -= (float)(moved * (double)w.p.to_relative);
                 own = true;
@@ -1422,7 +1414,6 @@ __global__ void k_rank_of(const int* __restrict__ order, int n, int* __restrict_
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) rank_of[order[k]] = k;
 }
 
-// Each level's first rank in the drainage order (level-major): level_start[levels] = n.
 // settle(): the stage's deposition laid on the rock at once; the sediment stays as the spoil the
 // mouths pass reads (HydraulicErosion.kt:1351-1364, 1451-1462).
 __global__ void k_settle(float* __restrict__ h, const float* __restrict__ sediment, size_t N) {
@@ -1498,16 +1489,14 @@ cg_status deposit_stage_reset_dev(cg_ctx* ctx, int W, int H) {
     const size_t N = (size_t)W * H;
     const size_t ids = schedule_ids(W, H);
     CG_BUF(float, d_sediment, ctx, S_SEDIMENT, N);
-    CG_BUF(int, d_stamp, ctx, S_STAMP, N);
     CG_BUF(int, d_mark, ctx, S_DEPMARK, N);
     CG_BUF(int, d_cellcnt, ctx, S_DEPCELLCNT, 2 * ids);
     CG_BUF(int, d_first, ctx, S_DEPFIRST, N);
     CG_BUF(int, d_words, ctx, S_DEPWORDS, W_WORDS);
     CG_LAUNCH(ctx) k_zero_float<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(d_sediment, N);
     CG_CHECK_LAUNCH(ctx);
-    // Fan ids and replay generations restart at 0, so every stamp and mark must too; the laying
-    // schedule's per-cell counts start at 0 (each chunk leaves them at 0).
-    CG_CUDA(ctx, cudaMemsetAsync(d_stamp, 0, N * sizeof(int), ctx->stream));
+    // The replays' generations restart at 0, so every mark must too; the laying schedule's per-cell counts
+    // start at 0 (each chunk leaves them at 0).
     CG_CUDA(ctx, cudaMemsetAsync(d_mark, 0, N * sizeof(int), ctx->stream));
     CG_CUDA(ctx, cudaMemsetAsync(d_cellcnt, 0, ids * sizeof(int), ctx->stream));
     CG_CUDA(ctx, cudaMemsetAsync(d_first, 0x7F, N * sizeof(int), ctx->stream));   // kNoTouch
@@ -1650,7 +1639,6 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     w.pool_base = d_pool_base;
     CG_BUF(long long, d_soff, ctx, S_DEPSLOTOFF, S);
     CG_BUF(int, d_sn, ctx, S_DEPSLOT7, 6 * S);
-    CG_BUF(double, d_slaid, ctx, S_DEPSLOT8, S);
     CG_BUF(Touch, d_stouch, ctx, S_DEPSLOT9, S * cap);
     CG_BUF(int, d_stn, ctx, S_DEPSLOT10, S);
     w.pair_cap = (int)std::min<size_t>(S * cap, (size_t)1 << 30);
@@ -1678,11 +1666,8 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     w.slot_n = d_sn;
     w.slot_state = d_sn + S;
     w.slot_box = d_sn + 2 * S;
-    w.slot_laid = d_slaid;
     w.slot_touch = d_stouch;
     w.slot_touch_n = d_stn;
-    CG_BUF(int, d_stamp, ctx, S_STAMP, N);
-    w.stamp = d_stamp;
     w.touch_cap = (int)std::min<size_t>(N, (size_t)1 << 26);
     CG_BUF(Touch, d_touch, ctx, S_DEPTOUCH, (size_t)w.touch_cap);
     w.touches = d_touch;
@@ -1698,14 +1683,10 @@ cg_status deposit_walk_dev(cg_ctx* ctx, const cg_erosion_params& cp, const Depos
     CG_BUF(int, d_tev, ctx, S_DEPTOUCHEV, (size_t)w.touch_cap);
     w.touch_ev = d_tev;
     w.roff = d_rlist + w.touch_cap;
-    CG_BUF(float, d_acc, ctx, S_DEPACC, N);
-    CG_BUF(uint8_t, d_own, ctx, S_DEPOWN, N);
-    w.acc = d_acc;
-    w.own_done = d_own;
     w.words = d_words;
     CG_BUF(unsigned long long, d_timers, ctx, S_DEPTIMERS, T_COUNT);
     w.timers = d_timers;
-    // The round's own counts (the fan ids, generations and wave numbers carry on through the stage).
+    // The round's own counts (the generations carry on through the stage).
     for (int word : {W_REPLAYED, W_WAVES, W_REFITTED, W_RELAID, W_ABORT})
         CG_CUDA(ctx, cudaMemsetAsync(d_words + word, 0, sizeof(int), sm));
     // A lobe's scratch in shared memory, for grids at least 4 wide whose lobes' boxes fit. The attribute is
