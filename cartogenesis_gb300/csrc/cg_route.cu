@@ -396,24 +396,26 @@ __device__ int steepest_neighbour(int W, int H, const double* __restrict__ rs, i
 }
 
 // Receivers of land cells (sea cells get -1). The facet rule's FP64 warp instructions cost the same
-// with one lane active as with 32, so each warp compacts the land cells of the chunks it scans (four cells
-// a lane, the fields' bytes a word at a time) into a small queue in shared memory and runs the rule 32 land
+// with one lane active as with 32, so each warp compacts the land cells of the chunks it scans (CELLS a lane;
+// four are the fields' bytes a word at a time) into a small queue in shared memory and runs the rule 32 land
 // cells at a time. `near` splits the work around the flats: 0 every land cell; 1 the cells with no raised
 // cell in their 3x3 block (their surface and their neighbours' are final before the flats are solved,
 // so this pass runs beside the flat solvers) and the sea; 2 the cells with a raised cell in their
 // 3x3 block, after the flats.
 constexpr int RECV_THREADS = 256;
 
+template <bool UNIT>
 __device__ __forceinline__ int receiver_of(int cell, const double* __restrict__ surface, int W, int H, Steps st,
-                                           long long seed, int by_facet, bool unit) {
+                                           long long seed, int by_facet) {
     const int row = pdiv(cell, W), col = pmod(cell, W);
     return !by_facet ? steepest_neighbour(W, H, surface, col, row, st)
-           : unit    ? facet_receiver_quick(W, H, surface, col, row, st, seed)
+           : UNIT    ? facet_receiver_quick(W, H, surface, col, row, st, seed)
                      : facet_receiver(W, H, surface, col, row, st, seed);
 }
 
-// For the four cells from `cell`, a byte each: nonzero where a raised cell is in the cell's 3x3 block.
-__device__ __forceinline__ unsigned near_raised4(const uint8_t* __restrict__ raised, int cell, int W, int H) {
+// For the CELLS cells from `cell`, a byte each: nonzero where a raised cell is in the cell's 3x3 block.
+template <int CELLS>
+__device__ __forceinline__ unsigned near_raised(const uint8_t* __restrict__ raised, int cell, int W, int H) {
     const int row = pdiv(cell, W), col = pmod(cell, W);
     unsigned long long any = 0;   // the columns from one before the cells to one after, a byte each
 #pragma unroll
@@ -422,46 +424,41 @@ __device__ __forceinline__ unsigned near_raised4(const uint8_t* __restrict__ rai
         if (nr < 0 || nr >= H) continue;
         const uint8_t* line = raised + (size_t)nr * W;
         any |= (unsigned long long)line[wrap_col(col - 1, W)] |
-               (unsigned long long)*reinterpret_cast<const unsigned*>(line + col) << 8 |
-               (unsigned long long)line[wrap_col(col + 4, W)] << 40;
+               (unsigned long long)line[wrap_col(col + CELLS, W)] << (8 * CELLS + 8);
+        if (CELLS == 4) any |= (unsigned long long)*reinterpret_cast<const unsigned*>(line + col) << 8;
+        else any |= (unsigned long long)line[col] << 8;
     }
     return (unsigned)(any | any >> 8 | any >> 16);
 }
 
-__global__ void __launch_bounds__(RECV_THREADS, 3) k_receivers(const uint8_t* __restrict__ land,
+template <int CELLS, bool UNIT>
+__global__ void __launch_bounds__(RECV_THREADS, CELLS == 4 && UNIT ? 3 : 1) k_receivers(const uint8_t* __restrict__ land,
                                                             const double* __restrict__ surface, int W, int H,
                                                             Steps st, long long seed, int by_facet,
                                                             const uint8_t* __restrict__ raised, int near,
                                                             int32_t* __restrict__ recv) {
+    static_assert(CELLS == 1 || CELLS == 4, "a byte or a word");
+    constexpr int CHUNK = 32 * CELLS;
     const unsigned FULL = 0xFFFFFFFFu;
-    __shared__ int queue[RECV_THREADS / 32][32 + 128];
+    __shared__ int queue[RECV_THREADS / 32][32 + CHUNK];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int* q = queue[warp];
-    const bool unit = st.ew == 1.0f && st.ns == 1.0f;
     const size_t N = (size_t)W * H;
     const size_t warps = (size_t)gridDim.x * (RECV_THREADS / 32);
     int n = 0;   // queued land cells (the same in every lane), under 32 between chunks
-    for (size_t base = ((size_t)blockIdx.x * (RECV_THREADS / 32) + warp) * 128;; base += warps * 128) {
+    for (size_t base = ((size_t)blockIdx.x * (RECV_THREADS / 32) + warp) * CHUNK;; base += warps * CHUNK) {
         const bool last = base >= N;
-        const size_t i = base + 4 * lane;
+        const size_t i = base + CELLS * lane;
+        const bool live = i < N;
         unsigned is_land = 0, is_near = 0;   // a byte a cell
-        if (i < N) {
-            if (W >= 4) {
-                is_land = *reinterpret_cast<const unsigned*>(land + i);
-                if (near && is_land) is_near = near_raised4(raised, (int)i, W, H);
-            } else {   // two columns at most: a row's neighbours are the row
-                for (int k = 0; k < 4 && i + k < N; ++k) {
-                    is_land |= (unsigned)land[i + k] << (8 * k);
-                    const int row = (int)(i + k) / W;
-                    for (int c = max(0, row - 1) * W; near && c < min(H, row + 2) * W; ++c)
-                        is_near |= (unsigned)raised[c] << (8 * k);
-                }
-            }
+        if (live) {
+            is_land = CELLS == 4 ? *reinterpret_cast<const unsigned*>(land + i) : land[i];
+            if (near && is_land) is_near = near_raised<CELLS>(raised, (int)i, W, H);
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < CELLS; ++k) {
             const bool on_land = (is_land >> (8 * k)) & 0xFFu;
-            if (!on_land && near != 2 && i + k < N) recv[i + k] = -1;
+            if (!on_land && near != 2 && live) recv[i + k] = -1;
             const bool l = on_land && (near == 0 || (((is_near >> (8 * k)) & 0xFFu) != 0) == (near == 2));
             const unsigned m = __ballot_sync(FULL, l);
             if (l) q[n + __popc(m & ((1u << lane) - 1u))] = (int)i + k;
@@ -472,7 +469,7 @@ __global__ void __launch_bounds__(RECV_THREADS, 3) k_receivers(const uint8_t* __
             const int some = min(n, 32);
             if (lane < some) {
                 const int cell = q[n - some + lane];
-                recv[cell] = receiver_of(cell, surface, W, H, st, seed, by_facet, unit);
+                recv[cell] = receiver_of<UNIT>(cell, surface, W, H, st, seed, by_facet);
             }
             n -= some;
             __syncwarp();
@@ -1700,6 +1697,24 @@ __global__ void k_flat_lists(const int* __restrict__ count, int flats, int* __re
 
 }  // namespace
 
+// Four cells a lane (the word loads need rows of four), but a cell a lane on small grids, where chunks of 128
+// cells leave most warps without one and a warp runs the rule four times in a row: a call without flats on
+// 128 x 64 cells twice as high as wide took 0.089 ms with chunks of 128 and takes 0.060, on 512 x 256 0.182 and
+// 0.146. At 1024 x 512 both take as long, and four a lane read less. The passes around the flats have fewer
+// idle warps beside the flat solvers: four a lane already at 256 x 256 (0.46 against 0.50 ms).
+// Square cells' rule is single precision and gains from a third CTA an SM (80 registers); the exact slopes of
+// other cells do not, and lose by the spills (2.98 against 2.74 ms for a call at 4096 x 2048).
+static void receivers_launch(cg_ctx* ctx, cudaStream_t stream, int W, int H, const uint8_t* d_land, const double* d_surface,
+                             Steps steps, int64_t seed, int by_facet, const uint8_t* d_raised, int near, int32_t* d_recv) {
+    const int ctas = ctx->num_sms * 8;
+    const bool words = W >= 4 && (size_t)W * H > (near == 0 ? (size_t)1 << 17 : (size_t)1 << 15);
+    const bool unit = steps.ew == 1.0f && steps.ns == 1.0f;   // square cells
+    auto kernel = unit ? (words ? k_receivers<4, true> : k_receivers<1, true>)
+                       : (words ? k_receivers<4, false> : k_receivers<1, false>);
+    CG_LAUNCH(ctx) kernel<<<ctas, RECV_THREADS, 0, stream>>>(d_land, d_surface, W, H, steps, (long long)seed, by_facet,
+                                                             d_raised, near, d_recv);
+}
+
 // FlowRouting.facetReceiver over a caller's routing surface (FlowRouting.kt:218-310, the rule
 // BeltErosion's rounds route the belts by): the facet receiver of every cell of d_mask, -1 elsewhere.
 cg_status facet_receivers_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, const double* d_surface,
@@ -1708,9 +1723,7 @@ cg_status facet_receivers_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_mask, 
     steps.ew = 1.0f;
     steps.ns = (float)r;
     steps.diag = (float)std::sqrt(1.0 + r * r);
-    CG_LAUNCH(ctx) k_receivers<<<ctx->num_sms * 8, RECV_THREADS, 0, ctx->stream>>>(d_mask, d_surface, W, H, steps,
-                                                                                  (long long)seed, 1, nullptr, 0,
-                                                                                  d_recv);
+    receivers_launch(ctx, ctx->stream, W, H, d_mask, d_surface, steps, seed, 1, nullptr, 0, d_recv);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }
@@ -1806,8 +1819,7 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
             CG_CUDA(ctx, cudaStreamWaitEvent(ctx->aux, ctx->fork, 0));
             CG_CUDA(ctx, cudaStreamWaitEvent(ctx->aux2, ctx->fork, 0));
             // The receivers away from the flats on the third stream, beside the flat solvers.
-            CG_LAUNCH(ctx) k_receivers<<<grid, RECV_THREADS, 0, ctx->aux2>>>(d_land, d_surface, W, H, steps,
-                                                                            (long long)seed, by, d_raised, 1, d_recv);
+            receivers_launch(ctx, ctx->aux2, W, H, d_land, d_surface, steps, seed, by, d_raised, 1, d_recv);
             CG_CHECK_LAUNCH(ctx);
             CG_CUDA(ctx, cudaEventRecord(ctx->join2, ctx->aux2));
             {
@@ -1857,8 +1869,7 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
             CG_CUDA(ctx, cudaStreamWaitEvent(sm, ctx->join, 0));
             CG_CUDA(ctx, cudaStreamWaitEvent(sm, ctx->join2, 0));
             // The receivers next to raised cells, now that the flats' surfaces are laid.
-            CG_LAUNCH(ctx) k_receivers<<<grid, RECV_THREADS, 0, sm>>>(d_land, d_surface, W, H, steps, (long long)seed,
-                                                                     by, d_raised, 2, d_recv);
+            receivers_launch(ctx, sm, W, H, d_land, d_surface, steps, seed, by, d_raised, 2, d_recv);
             CG_CHECK_LAUNCH(ctx);
             routed = true;
             if (kept_later) fc.d_kept = d_kept;
@@ -1868,8 +1879,7 @@ cg_status flow_directions_dev(cg_ctx* ctx, int W, int H, const uint8_t* d_land, 
         }
     }
     if (!routed) {
-        CG_LAUNCH(ctx) k_receivers<<<grid, RECV_THREADS, 0, sm>>>(d_land, d_surface, W, H, steps, (long long)seed, by,
-                                                                  nullptr, 0, d_recv);
+        receivers_launch(ctx, sm, W, H, d_land, d_surface, steps, seed, by, nullptr, 0, d_recv);
         CG_CHECK_LAUNCH(ctx);
     }
     if (counts) *counts = fc;
