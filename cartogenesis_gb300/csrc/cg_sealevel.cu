@@ -16,6 +16,7 @@
 // they would have one after another, and the next 32 start there: 11 to 17 basins a wave at 1024 x 512.
 // (One thread taking the basins in turn: 3.8 ms a pass there; one warp with the others loading ahead of
 // it 1.9; each walking twice instead of listing what it reads 0.85.)
+#include <algorithm>
 #include <cmath>
 
 #include "cg_common.cuh"
@@ -181,9 +182,12 @@ __device__ bool take_down(const NotchArgs& a, int cell, float cut_level, bool lo
     return false;
 }
 
-// A wave of the notch: `kNotchWarps` basins, `rank` this warp's among them. A stamp orders waves, then
-// the basins of a wave, the first the greatest.
-constexpr int kNotchWarps = 32;
+// A wave of the notch: up to `kNotchWarps` basins, `rank` this warp's among them. A stamp orders waves, then
+// the basins of a wave, the first the greatest. A basin's lists hold kNotchWords words for every cell that a
+// walk can reach, the whole map where the reach is wider than it: fewer basins a wave then, so that the lists
+// stay within kNotchScratch (4.8 GB at 2048 x 1024 with 32, and at 2^27 cells more than the GPU holds).
+constexpr int kNotchWarps = 32, kNotchWords = 18;
+constexpr size_t kNotchScratch = 512ull << 20;
 struct NotchTurn {
     int wave, rank;
     int* cut_cell;
@@ -329,11 +333,11 @@ __device__ int notch_basin(const NotchArgs& a, const Drowned& d, NotchTurn& t, i
     return n;
 }
 
-// The drowned basins in waves of up to 32, in order. The first basin of a wave never finds a clash, so
-// every wave cuts at least one.
+// The drowned basins in waves of up to a basin a warp, in order. The first basin of a wave never finds a clash,
+// so every wave cuts at least one.
 __global__ void __launch_bounds__(32 * kNotchWarps) k_notch_below_sea(NotchArgs a) {
     __shared__ int first_clash;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     NotchTurn t;
     t.wave = a.wave0;
     t.rank = warp;
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(32 * kNotchWarps) k_notch_below_sea(NotchArgs 
     for (int b0 = 0; b0 < a.count;) {
         ++t.wave;
         t.reads = 0;
-        if (threadIdx.x == 0) first_clash = kNotchWarps;
+        if (threadIdx.x == 0) first_clash = warps;
         const int b = b0 + warp;
         int n = 0, lowers = 0;
         Drowned d{};
@@ -468,7 +472,8 @@ extern "C" cg_status cg_sea_level_cut(cg_ctx* ctx, const cg_erosion_params* p, c
         // for the rounding of the sums.
         const float least = std::fmin(1.0f, rates.step_ns);
         const size_t cap = (size_t)std::fmin((double)N, 2.0 * std::ceil((double)rates.outlet_reach_cells / least) + 64.0) + 4;
-        CG_BUF(int, d_chain, ctx, S_SL_CHAIN, 18 * kNotchWarps * cap);
+        const size_t warps = std::max<size_t>(1, std::min<size_t>(kNotchWarps, kNotchScratch / (kNotchWords * sizeof(int) * cap)));
+        CG_BUF(int, d_chain, ctx, S_SL_CHAIN, kNotchWords * warps * cap);
         CG_BUF(int, d_stamp, ctx, S_SL_STAMP, N);
         if (pass == 0 || waves > (1 << 24)) {   // stamps stay within an int
             CG_CUDA(ctx, cudaMemsetAsync(d_stamp, 0, N * sizeof(int), sm));
@@ -492,9 +497,9 @@ extern "C" cg_status cg_sea_level_cut(cg_ctx* ctx, const cg_erosion_params* p, c
         a.count = drowned;
         a.list = d_list;
         a.chain = d_chain;
-        a.cut_cell = d_chain + kNotchWarps * cap;
-        a.cut_level = (float*)(d_chain + 4 * kNotchWarps * cap);
-        a.read_cell = d_chain + 7 * kNotchWarps * cap;
+        a.cut_cell = d_chain + warps * cap;
+        a.cut_level = (float*)(d_chain + 4 * warps * cap);
+        a.read_cell = d_chain + 7 * warps * cap;
         a.cap = (int)cap;
         a.stamp = d_stamp;
         a.wave0 = waves;
@@ -514,7 +519,7 @@ extern "C" cg_status cg_sea_level_cut(cg_ctx* ctx, const cg_erosion_params* p, c
         a.step_ns = rates.step_ns;
         a.step_diag = rates.step_diag;
         a.cells = d_words + 1;
-        CG_LAUNCH(ctx) k_notch_below_sea<<<1, 32 * kNotchWarps, 0, sm>>>(a);
+        CG_LAUNCH(ctx) k_notch_below_sea<<<1, 32 * (unsigned)warps, 0, sm>>>(a);
         CG_CHECK_LAUNCH(ctx);
         int cut = 0;
         CG_CUDA(ctx, cudaMemcpyAsync(&cut, d_words + 1, sizeof(int), cudaMemcpyDeviceToHost, sm));
