@@ -13,9 +13,9 @@ namespace {
 
 constexpr int kScanThreads = 256;
 constexpr int kScanTile = 4096;         // elements a CTA scans: 16 a thread
-constexpr int kScanDirect = 1 << 13;    // tiles whose sums every CTA adds up itself
+constexpr int kScanDirect = kScanTile;  // tiles whose sums every CTA adds up itself
 
-// The exclusive prefix of v over the CTA's threads, and the total; sh holds kScanThreads / 32 + 1 ints.
+// The exclusive prefix of v over the CTA's threads, and the total; sh holds kScanThreads / 32 ints.
 __device__ __forceinline__ int cta_prefix(int v, int* total, int* sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int x = v;
@@ -197,7 +197,8 @@ cg_status read_back(cg_ctx* ctx, std::initializer_list<ReadBack> parts) {
 
 // Two launches, the tiles' sums and the tiles, each CTA adding up the sums before its own: a level of
 // block scans and a pass adding their offsets took four to six. A read of up to kScanDirect sums a CTA
-// stays below the tile's own; longer inputs scan the sums first.
+// stays below the tile's own; longer inputs scan the sums first (at 8192 tiles the last pass takes 49 us
+// adding the sums up, and 42 after two launches of 3 and 4 that scan them).
 static cg_status scan_dev(cg_ctx* ctx, const int* d_in, int* d_out, int n, int** total) {
     if (n > 1 << 30) return fail(ctx, CG_BAD_ARG, "scan of %d elements is too long", n);
     const int tiles = (n + kScanTile - 1) / kScanTile;
