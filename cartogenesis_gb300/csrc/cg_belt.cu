@@ -748,7 +748,7 @@ cg_status belt_replay_dev(cg_ctx* ctx, const cg_erosion_params& p, float* d_h, c
     const int bgrid = std::min(grid, (B + 255) / 256 + 1);
     CG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_belt_sweeps, 512, 0));
     if (per_sm < 1) return fail(ctx, CG_CUDA, "the belt's sweep kernel cannot be resident");
-    // One CTA an SM while a thread has two cells at most, for the shorter grid barriers; larger belts wait for
+    // One CTA an SM while a thread has under four cells, for the shorter grid barriers; larger belts wait for
     // their loads and take all that fit.
     const int sweep_ctas = ctx->num_sms * std::min(per_sm, std::max(1, (B + F) / (ctx->num_sms * 1024)));
     CG_CUDA(ctx, cudaMemcpyAsync(d_next, d_h, N * 4, cudaMemcpyDeviceToDevice, sm));

@@ -24,13 +24,15 @@ import os
 BYTES_PER_CELL = {"ms_cut": 41.0, "ms_fill": 9.0, "ms_route": 28.0, "ms_tree": 20.0, "ms_incise": 32.0,
                   "ms_deposit": 81.0}
 PHASE_KERNELS = {
-    "ms_cut": "k_minmax, k_row_counts, k_bin_sums, k_bracket_*, k_land_and_water, k_uplift, k_unit_weights",
+    "ms_cut": "k_minmax, k_row_counts, k_bin_sums, k_bracket_*, k_sort_rank, k_land_and_water, k_uplift, k_unit_weights",
     "ms_fill": "k_fill_init, k_drain_chains, k_tiles_with_open, k_relax_passes, k_check_ties",
-    "ms_route": "k_surface, k_cc_*, k_flat_solve_warp/_sm/_cl, k_flat_solve, k_receivers",
+    "ms_route": "k_surface, k_cc_*, k_flat_solve_seg/_sm/_cl, k_flat_solve, k_receivers",
     "ms_tree": "k_links, k_sources, k_walk",
-    "ms_incise": "k_depth_*, k_incise_levels (P1, P2: the notch's k_footprint_*, k_breach_waves)",
-    "ms_deposit": "k_round_begin, k_rank_of, k_level_bounds, k_deposit_levels, k_settle, k_mouths_levels "
-                  "(last round: the closing breach's cut, fill, routing and notch)",
+    "ms_incise": "k_level_count_cta, k_level_scatter_cta, k_incise_levels (P1, P2: the notch's k_footprint_*, "
+                 "k_breach_waves)",
+    "ms_deposit": "k_round_begin, k_land_compact_ck, k_rs_*, k_rank_of, k_level_bounds, k_lake_candidates, "
+                  "k_admit_lakes, k_deposit_levels, k_settle, k_mouths_levels (last round: the closing breach's cut, "
+                  "fill, routing and notch)",
     "ms_relax": "thermal_sweeps_kernel",
     "ms_flexure": "k_uplift, k_flex_load, k_ss_*, k_fft_lines, k_transpose, k_flex_apply",
 }
