@@ -86,7 +86,7 @@ def roofline_entry(cfg, phase_ms_per_stage, root, traffic=None, fp64_gflops=None
     achieved = algo / (ms_launch / 1000.0) / 1e9 if ms_launch > 0 else 0.0
     phases = {}
     for k, v in phase_ms_per_stage.items():
-        if k == "ms_total" or v <= 0:
+        if k == "ms_total" or v <= 0 or (k == "ms_deposit" and p.profile == 0):   # P0: nothing between its events
             continue
         if k == "ms_flexure":
             gfs = flexure_flops_per_cell(p.width, p.height) * N / (v / rounds / 1000.0) / 1e9
