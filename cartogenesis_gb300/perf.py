@@ -15,8 +15,8 @@ mirrored grid take 5 flops per point per radix-2 stage, 20 (log2 W + log2 2H) fl
 and round, against the FP64 rate the bench measures on the GPU it runs on (cg_probe_fp64_rate). The
 kernels take the products, 2 of the 5, on the integer pipes and skip the mirrored half of the first
 pass, so the fraction is of the transform's arithmetic and not how busy the FP64 pipe is.
-The peak is the measured HBM copy bandwidth of the GB300s (MEASURED_PEAKS.json, written by
-the pool's driver), else the recipe's fallback of 6.8 TB/s.
+The peak is the measured HBM copy bandwidth of a GB300 (MEASURED_PEAKS.json), else 6.8 TB/s, an earlier
+measurement.
 """
 import json
 import os
